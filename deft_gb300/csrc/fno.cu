@@ -126,46 +126,57 @@ __global__ void __launch_bounds__(128) k_dft_z_fwd(const float *__restrict__ in,
 }
 
 // inv: out[l][z] (+)= sum_k Re[in[l][k] G[z][k]],  G = c_k s (cos, sin), z-major.
-// A block of 128 threads takes 64 lines: thread t keeps the table rows of
-// z = t mod 64 and z + 64 (per chunk of 128 z) in registers and walks every
-// second line (t / 64 picks the parity), so the line's Kz coefficients are
-// read by a whole warp at once (broadcast) and each feeds 4 multiply-adds.
-constexpr int kZiLines = 64;
+// N is a multiple of 4: a thread keeps the table rows of four consecutive z
+// in registers and walks lines of the block's tile, so each 16-byte read of
+// two of a line's coefficients (a broadcast) feeds 16 multiply-adds and the
+// result leaves as one 16-byte store.  The table's strided reads are paid
+// once per tile, so a tile is kZiLines lines where that still leaves every SM
+// two blocks, a quarter of them below.  91 us at
+// 96^3 with 16 channels and 12 modes when a thread held two z (8-byte reads,
+// 4 multiply-adds each), 73 us with four z and 64 lines, 44 us with 256.
+constexpr int kZiLines = 256;
 
 template <int KB>
 __global__ void __launch_bounds__(128) k_dft_z_inv(const float2 *__restrict__ in,
                                                    float *__restrict__ out,
                                                    const float2 *__restrict__ G, int L, int N,
-                                                   int Kz, int accumulate) {
-  __shared__ float2 cs[kZiLines * kMaxKz];
-  const int l0 = blockIdx.x * kZiLines;
-  const int nl = L - l0 < kZiLines ? L - l0 : kZiLines;
-  for (int i = threadIdx.x; i < kZiLines * Kz; i += blockDim.x)
-    cs[i] = i < nl * Kz ? in[(size_t)l0 * Kz + i] : make_float2(0.f, 0.f);
+                                                   int Kz, int accumulate, int lines) {
+  __shared__ __align__(16) float2 cs[kZiLines * KB];  // rows of KB, zero beyond Kz
+  const int l0 = blockIdx.x * lines;
+  const int nl = L - l0 < lines ? L - l0 : lines;
+  for (int i = threadIdx.x; i < nl * KB; i += blockDim.x) {
+    const int ll = i / KB, k = i - ll * KB;
+    cs[i] = k < Kz ? in[(size_t)(l0 + ll) * Kz + k] : make_float2(0.f, 0.f);
+  }
   __syncthreads();
-  const int zs = threadIdx.x & 63, par = threadIdx.x >> 6;
-  for (int zc = 0; zc < N; zc += 128) {
-    const int z0 = zc + zs, z1 = z0 + 64;
-    float2 g0[KB], g1[KB];
+  const int Q = N >> 2;  // quads of a line
+  const int per = Q < (int)blockDim.x ? Q : (int)blockDim.x;
+  const int sub = threadIdx.x / per, subs = blockDim.x / per;
+  if (sub >= subs) return;
+  for (int q = threadIdx.x - sub * per; q < Q; q += per) {
+    float2 g[KB][4];
 #pragma unroll
-    for (int k = 0; k < KB; k++) {
-      g0[k] = (k < Kz && z0 < N) ? G[(size_t)z0 * Kz + k] : make_float2(0.f, 0.f);
-      g1[k] = (k < Kz && z1 < N) ? G[(size_t)z1 * Kz + k] : make_float2(0.f, 0.f);
-    }
-    for (int ll = par; ll < nl; ll += 2) {
-      const float2 *c = cs + ll * Kz;
-      float v0 = 0.f, v1 = 0.f;
+    for (int j = 0; j < 4; j++)
 #pragma unroll
-      for (int k = 0; k < KB; k++) {
-        if (k < Kz) {
-          const float2 a = c[k];
-          v0 += a.x * g0[k].x - a.y * g0[k].y;
-          v1 += a.x * g1[k].x - a.y * g1[k].y;
+      for (int k = 0; k < KB; k++)
+        g[k][j] = k < Kz ? G[(size_t)(4 * q + j) * Kz + k] : make_float2(0.f, 0.f);
+    for (int ll = sub; ll < nl; ll += subs) {
+      float4 *o = reinterpret_cast<float4 *>(out + (size_t)(l0 + ll) * N) + q;
+      const float4 before = accumulate ? *o : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 *c = reinterpret_cast<const float4 *>(cs + ll * KB);
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int k2 = 0; k2 < KB / 2; k2++) {
+        const float4 a = c[k2];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          v[j] = fmaf(a.x, g[2 * k2][j].x, v[j]);
+          v[j] = fmaf(-a.y, g[2 * k2][j].y, v[j]);
+          v[j] = fmaf(a.z, g[2 * k2 + 1][j].x, v[j]);
+          v[j] = fmaf(-a.w, g[2 * k2 + 1][j].y, v[j]);
         }
       }
-      float *o = out + (size_t)(l0 + ll) * N;
-      if (z0 < N) o[z0] = accumulate ? o[z0] + v0 : v0;
-      if (z1 < N) o[z1] = accumulate ? o[z1] + v1 : v1;
+      *o = make_float4(before.x + v[0], before.y + v[1], before.z + v[2], before.w + v[3]);
     }
   }
 }
@@ -558,147 +569,233 @@ __global__ void k_project(const float *__restrict__ h, const __nv_bfloat16 *__re
   if (part) block_sum_store<2>(acc, part);
 }
 
-// Weight-gradient reductions over points: each block walks chunks of kChunk
-// points, stages the two factors in shared memory, and thread t accumulates
-// pair t of sum_p a[o][p] b[i][p] (t < C*C), or a row sum (C*C <= t < C*C+C).
-constexpr int kChunk = 64;
+// Weight-gradient reductions over points: a block walks chunks of kChunk
+// points, writes the two factors of a chunk to shared memory (point-major
+// rows of stride kCS: 16-byte rows, distinct banks for neighbouring rows) and
+// each warp adds its eighth of the chunk's points to its own copy of
+// sum_p a[o][p] b[i][p].  The outputs are tiled TO x TO over 16 lanes (TO =
+// C / 4; a lane's rows lie four apart), the warp's halves taking point quads
+// 16 points apart, so the words a load touches fall in distinct banks and
+// four points of 2 TO rows feed 4 TO^2 multiply-adds; the copies are added up
+// once per block.
+constexpr int kChunk = 256;
+constexpr int kCS = kChunk + 4;
+constexpr int kPwThreads = 128;  // two points a thread
+
+// acc[r][c] += sum over the warp's points of a[lane / 4 % 4 + 4 r] b[lane % 4 + 4 c],
+// row[r] += the same rows of a alone.
+template <int C>
+__device__ __forceinline__ void outer_accumulate(const float (*a)[kCS], const float (*b)[kCS],
+                                                 float (&acc)[C / 4][C / 4], float (&row)[C / 4]) {
+  constexpr int TO = C / 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
+  const int o0 = (lane >> 2) & 3, i0 = lane & 3;
+  constexpr int kPer = kChunk / (kPwThreads / 32);  // points of a warp
+#pragma unroll 2
+  for (int j = 0; j < kPer / 8; j++) {
+    const int p = warp * kPer + 32 * (j >> 2) + 4 * (j & 3) + 16 * half;
+    float4 av[TO], bv[TO];
+#pragma unroll
+    for (int r = 0; r < TO; r++) {
+      av[r] = *reinterpret_cast<const float4 *>(&a[o0 + 4 * r][p]);
+      bv[r] = *reinterpret_cast<const float4 *>(&b[i0 + 4 * r][p]);
+    }
+#pragma unroll
+    for (int r = 0; r < TO; r++) {
+      row[r] += (av[r].x + av[r].y) + (av[r].z + av[r].w);
+#pragma unroll
+      for (int c = 0; c < TO; c++) {
+        float t = acc[r][c];
+        t = fmaf(av[r].x, bv[c].x, t);
+        t = fmaf(av[r].y, bv[c].y, t);
+        t = fmaf(av[r].z, bv[c].z, t);
+        acc[r][c] = fmaf(av[r].w, bv[c].w, t);
+      }
+    }
+  }
+}
+
+// Adds the warps' copies (both halves) in a fixed order: out[o * C + i] and
+// out[C * C + o].  `red` holds kPwThreads / 32 * (C * C + C) floats and may
+// alias the chunk's rows (a barrier is taken first).
+template <int C>
+__device__ __forceinline__ void outer_store(float (&acc)[C / 4][C / 4], float (&row)[C / 4],
+                                            float *red, float *out) {
+  constexpr int TO = C / 4, NG = C * C + C, NW = kPwThreads / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int o0 = (lane >> 2) & 3, i0 = lane & 3;
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < TO; r++) {
+    const float rs = row[r] + __shfl_down_sync(0xffffffffu, row[r], 16);
+    if (lane < 16 && (lane & 3) == 0) red[warp * NG + C * C + o0 + 4 * r] = rs;
+#pragma unroll
+    for (int c = 0; c < TO; c++) {
+      const float x = acc[r][c] + __shfl_down_sync(0xffffffffu, acc[r][c], 16);
+      if (lane < 16) red[warp * NG + (o0 + 4 * r) * C + i0 + 4 * c] = x;
+    }
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < NG; t += kPwThreads) {
+    float x = 0.f;
+#pragma unroll
+    for (int w = 0; w < NW; w++) x += red[w * NG + t];
+    out[t] = x;
+  }
+}
+
+// hb[i] += sum_o W[o][i] zb (two points), W from shared memory.
+template <int C>
+__device__ __forceinline__ void add_row(const float *Wo, float2 zb, float2 (&hb)[C]) {
+#pragma unroll
+  for (int i4 = 0; i4 < C / 4; i4++) {
+    const float4 w = reinterpret_cast<const float4 *>(Wo)[i4];
+    hb[4 * i4].x = fmaf(w.x, zb.x, hb[4 * i4].x);
+    hb[4 * i4].y = fmaf(w.x, zb.y, hb[4 * i4].y);
+    hb[4 * i4 + 1].x = fmaf(w.y, zb.x, hb[4 * i4 + 1].x);
+    hb[4 * i4 + 1].y = fmaf(w.y, zb.y, hb[4 * i4 + 1].y);
+    hb[4 * i4 + 2].x = fmaf(w.z, zb.x, hb[4 * i4 + 2].x);
+    hb[4 * i4 + 2].y = fmaf(w.z, zb.y, hb[4 * i4 + 2].y);
+    hb[4 * i4 + 3].x = fmaf(w.w, zb.x, hb[4 * i4 + 3].x);
+    hb[4 * i4 + 3].y = fmaf(w.w, zb.y, hb[4 * i4 + 3].y);
+  }
+}
+
+template <int C> constexpr size_t pw_bwd_smem() {
+  return sizeof(float) * ((size_t)C * C + 2 * C * kCS);
+}
 
 // Backward of the projection and loss (loss = sum w (y - t)^2 / sum w).
 // hbar[j][r] = sum_c Q1[c][j] zbar_c with zbar_c = ybar Q2[c] gelu'(zq_c),
 // ybar = 2 w (y - t) / W.  Per-block partials [Q1 (C*C), q1 (C), Q2 (C), q2].
+// N^3 is a multiple of 64, so a thread's two points are both inside or both
+// outside.  Bound by its five C x N^3 passes (3 read, 1 written) and the
+// activation's arithmetic: 414 -> 81 us at 96^3, C = 16 (a quarter of the
+// threads formed the points and each weight product read two shared words).
 template <int C>
-__global__ void __launch_bounds__(256) k_project_bwd(
+__global__ void __launch_bounds__(kPwThreads) k_project_bwd(
     const float *__restrict__ h, const float *__restrict__ zq, const float *__restrict__ y,
-    const float *__restrict__ target, const float *__restrict__ w, float invW,
-    const __nv_bfloat16 *__restrict__ Q1, const __nv_bfloat16 *__restrict__ Q2,
-    float *__restrict__ hbar, float *__restrict__ part, long long NR) {
+    const float *__restrict__ target, const float *__restrict__ w,
+    const float *__restrict__ invWp, const __nv_bfloat16 *__restrict__ Q1,
+    const __nv_bfloat16 *__restrict__ Q2, float *__restrict__ hbar, float *__restrict__ part,
+    long long NR) {
   constexpr int NG = C * C + 2 * C + 1;
-  __shared__ float Q1s[C * C], Q2s[C];
-  __shared__ float zbs[C][kChunk], hs[C][kChunk], gs[C][kChunk], ybs[kChunk];
+  extern __shared__ __align__(16) float sm[];
+  float *Q1s = sm;
+  float(*zbs)[kCS] = reinterpret_cast<float(*)[kCS]>(sm + C * C);
+  float(*hs)[kCS] = zbs + C;
+  __shared__ float Q2s[C], red2[kPwThreads / 32][C + 1];
   for (int i = threadIdx.x; i < C * C; i += blockDim.x) Q1s[i] = bf(Q1, i);
   for (int i = threadIdx.x; i < C; i += blockDim.x) Q2s[i] = bf(Q2, i);
-  float accs[2] = {0.f, 0.f};  // gradient entries threadIdx.x and threadIdx.x + blockDim.x
+  const float invW = *invWp;
+  float acc[C / 4][C / 4] = {}, row[C / 4] = {}, ga[C] = {}, ya = 0.f;
   const long long nchunks = (NR + kChunk - 1) / kChunk;
   for (long long ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
     __syncthreads();
-    for (int p = threadIdx.x; p < kChunk; p += blockDim.x) {
-      const long long r = ch * kChunk + p;
-      if (r < NR) {
-        const float wr = w ? w[r] : 1.f;
-        const float yb = 2.f * wr * (y[r] - target[r]) * invW;
-        ybs[p] = yb;
-        float hb[C];
+    const int p = 2 * threadIdx.x;
+    const long long r = ch * kChunk + p;
+    const bool in = r < NR;
+    float2 yb = make_float2(0.f, 0.f), hb[C];
+    if (in) {
+      const float2 wr = w ? *reinterpret_cast<const float2 *>(w + r) : make_float2(1.f, 1.f);
+      const float2 yv = *reinterpret_cast<const float2 *>(y + r);
+      const float2 tv = *reinterpret_cast<const float2 *>(target + r);
+      yb = make_float2(2.f * wr.x * (yv.x - tv.x) * invW, 2.f * wr.y * (yv.y - tv.y) * invW);
+    }
+    ya += yb.x + yb.y;
 #pragma unroll
-        for (int i = 0; i < C; i++) {
-          hs[i][p] = h[(size_t)i * NR + r];
-          hb[i] = 0.f;
-        }
-#pragma unroll 1
-        for (int c = 0; c < C; c++) {
-          const float a = zq[(size_t)c * NR + r];
-          gs[c][p] = gelu(a);
-          const float zb = yb * Q2s[c] * gelu_d(a);
-          zbs[c][p] = zb;
+    for (int i = 0; i < C; i++) {
+      hb[i] = make_float2(0.f, 0.f);
+      *reinterpret_cast<float2 *>(&hs[i][p]) =
+          in ? *reinterpret_cast<const float2 *>(h + (size_t)i * NR + r) : hb[i];
+    }
 #pragma unroll
-          for (int i = 0; i < C; i++) hb[i] += Q1s[c * C + i] * zb;
-        }
+    for (int c = 0; c < C; c++) {
+      const float2 a = in ? *reinterpret_cast<const float2 *>(zq + (size_t)c * NR + r)
+                          : make_float2(0.f, 0.f);
+      ga[c] += yb.x * gelu(a.x) + yb.y * gelu(a.y);
+      const float2 zb =
+          make_float2(yb.x * Q2s[c] * gelu_d(a.x), yb.y * Q2s[c] * gelu_d(a.y));
+      *reinterpret_cast<float2 *>(&zbs[c][p]) = zb;
+      add_row<C>(Q1s + c * C, zb, hb);
+    }
+    if (in) {
 #pragma unroll
-        for (int i = 0; i < C; i++) hbar[(size_t)i * NR + r] = hb[i];
-      } else {
-        ybs[p] = 0.f;
-        for (int i = 0; i < C; i++) {
-          hs[i][p] = 0.f;
-          zbs[i][p] = 0.f;
-          gs[i][p] = 0.f;
-        }
-      }
+      for (int i = 0; i < C; i++) *reinterpret_cast<float2 *>(hbar + (size_t)i * NR + r) = hb[i];
     }
     __syncthreads();
-    for (int s2 = 0; s2 < 2; s2++) {
-      const int t = threadIdx.x + s2 * blockDim.x;
-      float acc = 0.f;
-      if (t < C * C) {
-        const int c = t / C, i = t % C;
-        for (int p = 0; p < kChunk; p++) acc += zbs[c][p] * hs[i][p];
-      } else if (t < C * C + C) {
-        const int c = t - C * C;
-        for (int p = 0; p < kChunk; p++) acc += zbs[c][p];
-      } else if (t < C * C + 2 * C) {
-        const int c = t - C * C - C;
-        for (int p = 0; p < kChunk; p++) acc += ybs[p] * gs[c][p];
-      } else if (t == C * C + 2 * C) {
-        for (int p = 0; p < kChunk; p++) acc += ybs[p];
-      }
-      accs[s2] += acc;
-    }
+    outer_accumulate<C>(zbs, hs, acc, row);
   }
-  for (int s2 = 0; s2 < 2; s2++) {
-    const int t = threadIdx.x + s2 * blockDim.x;
-    if (t < NG) part[(size_t)blockIdx.x * NG + t] = accs[s2];
+  float *out = part + (size_t)blockIdx.x * NG;
+  outer_store<C>(acc, row, &zbs[0][0], out);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int c = 0; c <= C; c++) {
+    float x = c < C ? ga[c < C ? c : 0] : ya;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) red2[warp][c] = x;
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c <= C; c += blockDim.x) {
+    float x = 0.f;
+    for (int k = 0; k < kPwThreads / 32; k++) x += red2[k][c];
+    out[C * C + C + c] = x;
   }
 }
 
 // Backward of a layer's pointwise part: zbar = hbar * act'(z) (written to
 // zbar), hprev_bar[i][r] = sum_o Wp[o][i] zbar[o][r] (written), per-block
-// partials [Wp (C*C), b (C)].
+// partials [Wp (C*C), b (C)].  Bound by its five C x N^3 passes (3 read, 2
+// written) and the activation's arithmetic: 464 -> 92 us at 96^3, C = 16.
 template <int C>
-__global__ void __launch_bounds__(256) k_layer_pw_bwd(
+__global__ void __launch_bounds__(kPwThreads) k_layer_pw_bwd(
     const float *__restrict__ hbar, const float *__restrict__ z, const float *__restrict__ hprev,
     const __nv_bfloat16 *__restrict__ Wp, float *__restrict__ zbar, float *__restrict__ hprev_bar,
     float *__restrict__ part, long long NR, int act) {
-  constexpr int NG = C * C + C;
-  __shared__ float Ws[C * C];
-  __shared__ float zbs[C][kChunk], hs[C][kChunk];
+  extern __shared__ __align__(16) float sm[];
+  float *Ws = sm;
+  float(*zbs)[kCS] = reinterpret_cast<float(*)[kCS]>(sm + C * C);
+  float(*hs)[kCS] = zbs + C;
   for (int i = threadIdx.x; i < C * C; i += blockDim.x) Ws[i] = bf(Wp, i);
-  float accs[2] = {0.f, 0.f};
+  float acc[C / 4][C / 4] = {}, row[C / 4] = {};
   const long long nchunks = (NR + kChunk - 1) / kChunk;
   for (long long ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
     __syncthreads();
-    for (int p = threadIdx.x; p < kChunk; p += blockDim.x) {
-      const long long r = ch * kChunk + p;
-      if (r < NR) {
-        float hb[C];
+    const int p = 2 * threadIdx.x;
+    const long long r = ch * kChunk + p;
+    const bool in = r < NR;
+    float2 hb[C];
 #pragma unroll
-        for (int i = 0; i < C; i++) {
-          hs[i][p] = hprev[(size_t)i * NR + r];
-          hb[i] = 0.f;
+    for (int i = 0; i < C; i++) {
+      hb[i] = make_float2(0.f, 0.f);
+      *reinterpret_cast<float2 *>(&hs[i][p]) =
+          in ? *reinterpret_cast<const float2 *>(hprev + (size_t)i * NR + r) : hb[i];
+    }
+#pragma unroll 4
+    for (int o = 0; o < C; o++) {
+      float2 zb = make_float2(0.f, 0.f);
+      if (in) {
+        zb = *reinterpret_cast<const float2 *>(hbar + (size_t)o * NR + r);
+        if (act) {
+          const float2 zv = *reinterpret_cast<const float2 *>(z + (size_t)o * NR + r);
+          zb.x *= gelu_d(zv.x);
+          zb.y *= gelu_d(zv.y);
         }
-#pragma unroll 1
-        for (int o = 0; o < C; o++) {
-          const float hbo = hbar[(size_t)o * NR + r];
-          const float zb = act ? hbo * gelu_d(z[(size_t)o * NR + r]) : hbo;
-          zbs[o][p] = zb;
-          zbar[(size_t)o * NR + r] = zb;
-#pragma unroll
-          for (int i = 0; i < C; i++) hb[i] += Ws[o * C + i] * zb;
-        }
-#pragma unroll
-        for (int i = 0; i < C; i++) hprev_bar[(size_t)i * NR + r] = hb[i];
-      } else {
-        for (int i = 0; i < C; i++) {
-          hs[i][p] = 0.f;
-          zbs[i][p] = 0.f;
-        }
+        *reinterpret_cast<float2 *>(zbar + (size_t)o * NR + r) = zb;
       }
+      *reinterpret_cast<float2 *>(&zbs[o][p]) = zb;
+      add_row<C>(Ws + o * C, zb, hb);
+    }
+    if (in) {
+#pragma unroll
+      for (int i = 0; i < C; i++)
+        *reinterpret_cast<float2 *>(hprev_bar + (size_t)i * NR + r) = hb[i];
     }
     __syncthreads();
-    for (int s2 = 0; s2 < 2; s2++) {
-      const int t = threadIdx.x + s2 * blockDim.x;
-      float acc = 0.f;
-      if (t < C * C) {
-        const int o = t / C, i = t % C;
-        for (int p = 0; p < kChunk; p++) acc += zbs[o][p] * hs[i][p];
-      } else if (t < NG) {
-        const int o = t - C * C;
-        for (int p = 0; p < kChunk; p++) acc += zbs[o][p];
-      }
-      accs[s2] += acc;
-    }
+    outer_accumulate<C>(zbs, hs, acc, row);
   }
-  for (int s2 = 0; s2 < 2; s2++) {
-    const int t = threadIdx.x + s2 * blockDim.x;
-    if (t < NG) part[(size_t)blockIdx.x * NG + t] = accs[s2];
-  }
+  outer_store<C>(acc, row, &zbs[0][0], part + (size_t)blockIdx.x * (C * C + C));
 }
 
 // Lift backward partials: [P (2C), p (C)].
@@ -723,14 +820,52 @@ __global__ void k_lift_bwd(const float *__restrict__ hbar, const float *__restri
   block_sum_store<NG>(g, part);
 }
 
-// Sums per-block partials [nblk][K] in a fixed order into grad (+=).
-__global__ void k_sum_partials(const float *__restrict__ part, int nblk, int K,
-                               float *__restrict__ grad) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= K) return;
+// Sums per-block partials [nblk][K] in a fixed order into grad (+=): a block
+// of 32 x 32 threads takes 32 columns, each thread every 32nd row, the 32 row
+// sums of a column added in order (one thread per column walking all rows
+// was latency-bound: 466 us at 3456 x 272 against 14 us at 608 x 272).
+__global__ void __launch_bounds__(1024) k_sum_partials(const float *__restrict__ part, int nblk,
+                                                       int K, float *__restrict__ grad) {
+  __shared__ double red[32][33];
+  const int k = blockIdx.x * 32 + threadIdx.x;
   double s = 0;
-  for (int b = 0; b < nblk; b++) s += part[(size_t)b * K + k];
-  grad[k] += (float)s;
+  if (k < K) {
+#pragma unroll 4
+    for (int b = threadIdx.y; b < nblk; b += 32) s += part[(size_t)b * K + k];
+  }
+  red[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0 && k < K) {
+    for (int w = 1; w < 32; w++) s += red[w][threadIdx.x];
+    grad[k] += (float)s;
+  }
+}
+
+// loss[0] = sum w (y - t)^2 / sum w and loss[1] = 1 / sum w from the
+// projection's per-block sums (FP64, fixed order; a weight sum of 0 counts
+// as 1), left on the device for the backward pass.
+__global__ void __launch_bounds__(256) k_loss(const float *__restrict__ part, int nblk,
+                                              float *__restrict__ loss) {
+  __shared__ double red[2][256];
+  double s = 0, w = 0;
+  for (int b = threadIdx.x; b < nblk; b += 256) {
+    s += part[2 * b];
+    w += part[2 * b + 1];
+  }
+  red[0][threadIdx.x] = s;
+  red[1][threadIdx.x] = w;
+  for (int o = 128; o > 0; o >>= 1) {
+    __syncthreads();
+    if (threadIdx.x < o) {
+      red[0][threadIdx.x] += red[0][threadIdx.x + o];
+      red[1][threadIdx.x] += red[1][threadIdx.x + o];
+    }
+  }
+  if (threadIdx.x == 0) {
+    const double W = red[1][0] > 0 ? red[1][0] : 1;
+    loss[0] = (float)(red[0][0] / W);
+    loss[1] = (float)(1.0 / W);
+  }
 }
 
 // Adam on the FP32 masters, then the BF16 copies.
@@ -841,10 +976,12 @@ struct deft_fno {
   float2 *A = nullptr, *B = nullptr, *S = nullptr, *S2 = nullptr;
   float *hb0 = nullptr, *hb1 = nullptr, *zb = nullptr;
   float *part = nullptr;
+  float *loss_d = nullptr;   // loss and 1 / sum of its weights (k_loss)
   double *bulk = nullptr;    // 2 N^3 doubles (bulk start, its gradient), allocated on first use
   double *part_d = nullptr;  // kNormBlocks FP64 partial sums
   long long launches = 0;    // kernel launches queued so far
   int nblk = 0;
+  int bwd_blk = 0;           // blocks of the pointwise backward kernels
   std::string err;
 };
 
@@ -882,12 +1019,13 @@ void launch_z_fwd(deft_fno *f, const float *in, float2 *out, const float2 *E) {
 }
 void launch_z_inv(deft_fno *f, const float2 *in, float *out, const float2 *G, int acc) {
   const int L = f->C * f->N * f->N;
-  const dim3 grid((L + kZiLines - 1) / kZiLines);
+  const int lines = L >= 2 * 152 * kZiLines ? kZiLines : kZiLines / 4;
+  const dim3 grid((L + lines - 1) / lines);
   switch (kz_block(f->Kz)) {
-    case 4: k_dft_z_inv<4><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc); break;
-    case 8: k_dft_z_inv<8><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc); break;
-    case 12: k_dft_z_inv<12><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc); break;
-    default: k_dft_z_inv<16><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc); break;
+    case 4: k_dft_z_inv<4><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc, lines); break;
+    case 8: k_dft_z_inv<8><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc, lines); break;
+    case 12: k_dft_z_inv<12><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc, lines); break;
+    default: k_dft_z_inv<16><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc, lines); break;
   }
 }
 void launch_axis(deft_fno *f, const float2 *in, float2 *out, const float2 *E, int outer, int Nin,
@@ -1148,6 +1286,15 @@ int deft_fno_create(int device, int N, int channels, int modes, int layers, unsi
   dev(&f->zb, act);
   f->nblk = grid_for(f->NR);
   dev(&f->part, sizeof(float) * (size_t)f->nblk * (C * C + 2 * C + 1 + 8));
+  {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const int nch = (int)((f->NR + kChunk - 1) / kChunk);
+    f->bwd_blk = 4 * (sms > 0 ? sms : 148);
+    if (f->bwd_blk > nch) f->bwd_blk = nch;
+    if (f->bwd_blk > f->nblk) f->bwd_blk = f->nblk;
+  }
+  dev(&f->loss_d, 2 * sizeof(float));
   dev(&f->part_d, sizeof(double) * kNormBlocks);
   if (!ok) {
     deft_fno_destroy(f);
@@ -1191,7 +1338,7 @@ int deft_fno_destroy(deft_fno *f) {
                   (void *)f->Eyi, (void *)f->Exf, (void *)f->Exi, (void *)f->zq, (void *)f->y,
                   (void *)f->mask, (void *)f->target, (void *)f->wt, (void *)f->A, (void *)f->B,
                   (void *)f->S, (void *)f->S2, (void *)f->hb0, (void *)f->hb1, (void *)f->zb,
-                  (void *)f->part, (void *)f->bulk, (void *)f->part_d})
+                  (void *)f->part, (void *)f->loss_d, (void *)f->bulk, (void *)f->part_d})
     cudaFree(q);
   for (float *q : f->h) cudaFree(q);
   for (float *q : f->z) cudaFree(q);
@@ -1232,6 +1379,24 @@ int deft_fno_set_params(deft_fno *f, const float *host) {
 
 namespace {
 
+void sum_partials(deft_fno *f, int nblk, int K, float *grad) {
+  k_sum_partials<<<(K + 31) / 32, dim3(32, 32), 0, f->stream>>>(f->part, nblk, K, grad);
+}
+
+template <int C> void project_bwd(deft_fno *f) {
+  k_project_bwd<C><<<f->bwd_blk, kPwThreads, pw_bwd_smem<C>(), f->stream>>>(
+      f->h[f->L], f->zq, f->y, f->target, f->wt, f->loss_d + 1, f->pb + f->oQ1, f->pb + f->oQ2,
+      f->hb0, f->part, f->NR);
+  sum_partials(f, f->bwd_blk, C * C + 2 * C + 1, f->g + f->oQ1);
+}
+
+template <int C> void layer_pw_bwd(deft_fno *f, int l, const float *hb, float *hb_next) {
+  k_layer_pw_bwd<C><<<f->bwd_blk, kPwThreads, pw_bwd_smem<C>(), f->stream>>>(
+      hb, f->z[l], f->h[l], f->pb + f->oWp[l], f->zb, hb_next, f->part, f->NR,
+      l < f->L - 1 ? 1 : 0);
+  sum_partials(f, f->bwd_blk, C * C + C, f->g + f->oWp[l]);
+}
+
 // Forward pass (and, with want_grad, the backward pass into f->g) on one
 // sample; mask / target / y_out are host or device arrays per `kind`.
 int eval_impl(deft_fno *f, const float *mask, float eta, const float *target, cudaMemcpyKind kin,
@@ -1245,69 +1410,41 @@ int eval_impl(deft_fno *f, const float *mask, float eta, const float *target, cu
   }
   if (int s = forward(f, eta, want_grad)) return s;
   project(f, f->zq, target ? f->target : nullptr, f->wt, target ? f->part : nullptr);
-  double W = 0, Ls = 0;
   if (target) {
-    std::vector<float> hpart(2 * (size_t)f->nblk);
-    cudaMemcpyAsync(hpart.data(), f->part, sizeof(float) * hpart.size(), cudaMemcpyDeviceToHost,
-                    f->stream);
-    if (cudaStreamSynchronize(f->stream) != cudaSuccess) return check(f, "fno loss");
-    for (int b = 0; b < f->nblk; b++) {
-      Ls += hpart[2 * b];
-      W += hpart[2 * b + 1];
-    }
-    if (loss) *loss = (float)(Ls / (W > 0 ? W : 1));
+    f->launches++;
+    k_loss<<<1, 256, 0, f->stream>>>(f->part, f->nblk, f->loss_d);
   }
   if (y_out) cudaMemcpyAsync(y_out, f->y, rb, kout, f->stream);
   if (want_grad && target) {
     f->launches += 4 + 9 * f->L;  // projection, lift and layer backward passes with their sums
     cudaMemsetAsync(f->g, 0, sizeof(float) * f->nparam, f->stream);
-    const float invW = (float)(1.0 / (W > 0 ? W : 1));
     // projection
-    if (C == 16)
-      k_project_bwd<16><<<f->nblk, kT, 0, f->stream>>>(f->h[f->L], f->zq, f->y, f->target, f->wt,
-                                                        invW, f->pb + f->oQ1, f->pb + f->oQ2,
-                                                        f->hb0, f->part, f->NR);
-    else if (C == 8)
-      k_project_bwd<8><<<f->nblk, kT, 0, f->stream>>>(f->h[f->L], f->zq, f->y, f->target, f->wt,
-                                                       invW, f->pb + f->oQ1, f->pb + f->oQ2,
-                                                       f->hb0, f->part, f->NR);
-    else
-      k_project_bwd<4><<<f->nblk, kT, 0, f->stream>>>(f->h[f->L], f->zq, f->y, f->target, f->wt,
-                                                       invW, f->pb + f->oQ1, f->pb + f->oQ2,
-                                                       f->hb0, f->part, f->NR);
-    const int NGp = C * C + 2 * C + 1;
-    k_sum_partials<<<(NGp + kT - 1) / kT, kT, 0, f->stream>>>(f->part, f->nblk, NGp,
-                                                              f->g + f->oQ1);
+    if (C == 16) project_bwd<16>(f);
+    else if (C == 8) project_bwd<8>(f);
+    else project_bwd<4>(f);
     float *hb = f->hb0, *hb_next = f->hb1;
     for (int l = f->L - 1; l >= 0; l--) {
-      const int actl = l < f->L - 1 ? 1 : 0;
-      if (C == 16)
-        k_layer_pw_bwd<16><<<f->nblk, kT, 0, f->stream>>>(hb, f->z[l], f->h[l], f->pb + f->oWp[l],
-                                                           f->zb, hb_next, f->part, f->NR, actl);
-      else if (C == 8)
-        k_layer_pw_bwd<8><<<f->nblk, kT, 0, f->stream>>>(hb, f->z[l], f->h[l], f->pb + f->oWp[l],
-                                                          f->zb, hb_next, f->part, f->NR, actl);
-      else
-        k_layer_pw_bwd<4><<<f->nblk, kT, 0, f->stream>>>(hb, f->z[l], f->h[l], f->pb + f->oWp[l],
-                                                          f->zb, hb_next, f->part, f->NR, actl);
-      const int NGl = C * C + C;
-      k_sum_partials<<<(NGl + kT - 1) / kT, kT, 0, f->stream>>>(f->part, f->nblk, NGl,
-                                                                f->g + f->oWp[l]);
+      if (C == 16) layer_pw_bwd<16>(f, l, hb, hb_next);
+      else if (C == 8) layer_pw_bwd<8>(f, l, hb, hb_next);
+      else layer_pw_bwd<4>(f, l, hb, hb_next);
       spectral_bwd(f, l, f->zb, hb_next);
       float *t = hb;
       hb = hb_next;
       hb_next = t;
     }
     if (C == 16)
-      k_lift_bwd<16><<<f->nblk, kT, 0, f->stream>>>(hb, f->mask, eta, f->part, f->NR);
+      k_lift_bwd<16><<<f->bwd_blk, kT, 0, f->stream>>>(hb, f->mask, eta, f->part, f->NR);
     else if (C == 8)
-      k_lift_bwd<8><<<f->nblk, kT, 0, f->stream>>>(hb, f->mask, eta, f->part, f->NR);
+      k_lift_bwd<8><<<f->bwd_blk, kT, 0, f->stream>>>(hb, f->mask, eta, f->part, f->NR);
     else
-      k_lift_bwd<4><<<f->nblk, kT, 0, f->stream>>>(hb, f->mask, eta, f->part, f->NR);
-    k_sum_partials<<<(3 * C + kT - 1) / kT, kT, 0, f->stream>>>(f->part, f->nblk, 3 * C,
-                                                                f->g + f->oP);
+      k_lift_bwd<4><<<f->bwd_blk, kT, 0, f->stream>>>(hb, f->mask, eta, f->part, f->NR);
+    sum_partials(f, f->bwd_blk, 3 * C, f->g + f->oP);
     if (int s = check(f, "fno backward")) return s;
   }
+  // the copy waits for the stream when its host side is pageable, so it
+  // comes after everything is queued
+  if (target && loss)
+    cudaMemcpyAsync(loss, f->loss_d, sizeof(float), cudaMemcpyDeviceToHost, f->stream);
   return check(f, "fno eval");
 }
 
