@@ -20,6 +20,7 @@
 // The k-space weights (src/ReciprocalOperators.h:94-235) are evaluated
 // analytically once per (grid, R) into a table, with the convolution
 // normalisation dV/V folded in.
+#include "df_phi.cuh"
 #include "fft_smem.cuh"
 #include "fmt_engine.h"
 #include "pencil_fft.cuh"
@@ -60,6 +61,10 @@ __device__ __forceinline__ T kcomp_t(const Geom &g, int c, int x, int y, int z) 
   if constexpr (sizeof(T) == 4)
     return g.Bmf[3 * c] * (float)wrapm(x, g.Nx) + g.Bmf[3 * c + 1] * (float)wrapm(y, g.Ny) +
            g.Bmf[3 * c + 2] * (float)z;
+  else if constexpr (is_df<T>)  // no FP64 arithmetic or conversions per element
+    return df_scale(dfl(g.Bmf[3 * c], g.Bml[3 * c]), (float)wrapm(x, g.Nx)) +
+           df_scale(dfl(g.Bmf[3 * c + 1], g.Bml[3 * c + 1]), (float)wrapm(y, g.Ny)) +
+           df_scale(dfl(g.Bmf[3 * c + 2], g.Bml[3 * c + 2]), (float)z);
   else
     return kcomp(g, c, x, y, z);
 }
@@ -131,6 +136,12 @@ __device__ __forceinline__ bool precond_active(float m, float nv) {
   const unsigned mb = __float_as_uint(m), nb = __float_as_uint(nv);
   return (mb << 1) != 0 && nb - 1u < 0x7F800000u;
 }
+
+// x != 0 (NaN included) without the FP64 pipe.
+__device__ __forceinline__ bool nonzero(double x) {
+  return ((unsigned long long)__double_as_longlong(x) << 1) != 0;
+}
+__device__ __forceinline__ bool nonzero(float x) { return x != 0.f; }
 
 // Deterministic block reduction of K doubles; thread 0 gets the sums.
 template <int K>
@@ -286,7 +297,7 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_r2c(const double *__restrict__ in,
     int ll, z;
     fdivmod(idx, g.fNz, ll, z);
     const int line = 2 * p0 + ll;
-    const T v = line < g.lines ? T(in[(size_t)line * g.Nz + z]) : T(0);
+    const T v = line < g.lines ? real_from<T>(in[(size_t)line * g.Nz + z]) : T(0);
     reinterpret_cast<T *>(&buf0[z * P + (ll >> 1)])[ll & 1] = v;
   }
   C *res = fft_tile<T, -1, RN>(buf0, buf1, fP, pz);
@@ -392,6 +403,7 @@ struct LocalArgs {
   //   H(k) = 1/nb + h33 w3^2 + 2 h32 w3 w2 + h22 w2^2 + hvv k^2 wv^2,
   // with h the Hessian of phi at the bulk weighted densities (0: off).
   float pc_inv_nb, pc_h33, pc_h32x2, pc_h22, pc_hvv, pc_inv_kTdV;
+  DfPhiConst dfk;  // the FP64 form's double-float Phi
 };
 
 // The bulk density nb in equilibrium with the chemical-potential term of f
@@ -497,6 +509,17 @@ template <int K>
 __device__ void finish_dots(double (&acc)[K], double *red, double *partials,
                             unsigned int *counter, double *out);
 
+// The double-float form's k = 0 entries, weighted in FP64: the table's
+// rounding of w(0) to a double-float would scale the mean of a field, and
+// with it every value of the gradient, which is a small difference of large
+// means.
+__device__ __forceinline__ double dc_w(int a, double R, const Geom &g) {
+  return (a == 0 ? (4 * M_PI / 3) * R * R * R : (4 * M_PI) * (R * R)) * g.scale;
+}
+__device__ __forceinline__ dfc dc_weight(dfc v, double w) {
+  return dfc{df_from(double(v.x) * w), df_from(double(v.y) * w)};
+}
+
 // x-FFT of n^, multiplication by the five weights, and the five inverse
 // x-FFTs one field at a time (three tiles of B lines: the forward result and
 // a ping-pong pair), which keeps B wide for coalesced column runs.
@@ -553,6 +576,8 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_x_conv_fwd(
         else w = slot == 0 ? w3[i] : slot == 1 ? w2[i] : wv[i];
         if (a < 2) {
           o = C{v.x * w, v.y * w};
+          if constexpr (is_df<T>)
+            if (i == 0) o = dc_weight(v, dc_w(a, lap->R, g));
         } else {
           int y, z;
           fdivmod(j, g.fNzH, y, z);
@@ -631,6 +656,11 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_x_conv_adj(
         o.x += q.y * w;  // times -i w
         o.y -= q.x * w;
       }
+      if constexpr (is_df<T>)
+        if (i == 0) {
+          const C d3 = dc_weight(r[0], dc_w(0, lap->R, g)), d2 = dc_weight(r[B], dc_w(1, lap->R, g));
+          o = C{d3.x + d2.x, d3.y + d2.y};
+        }
     }
     A[idx] = o;
   }
@@ -956,10 +986,9 @@ __device__ void z_r2c_store5(typename Cplx<T>::type *res, typename Cplx<T>::type
     const int b = a * P + (ll >> 1);
     const C zk = out[k * P5 + b];
     const C zm = out[(k == 0 ? 0 : Nz - k) * P5 + b];
-    const T h = T(0.5);
     C o;
-    if ((ll & 1) == 0) o = C{h * (zk.x + zm.x), h * (zk.y - zm.y)};
-    else o = C{h * (zk.y + zm.y), -h * (zk.x - zm.x)};
+    if ((ll & 1) == 0) o = C{half_of(zk.x + zm.x), half_of(zk.y - zm.y)};
+    else o = C{half_of(zk.y + zm.y), half_of(zm.x - zk.x)};
     S5[(size_t)a * g.NC + (size_t)line * NzH + k] = o;
   }
 }
@@ -972,22 +1001,17 @@ __device__ void z_r2c_store5(typename Cplx<T>::type *res, typename Cplx<T>::type
 #ifndef DEFT_Z_PHI_MIN_BLOCKS
 #define DEFT_Z_PHI_MIN_BLOCKS 5
 #endif
-// The FP64 form's Phi: FP64 (0) or double-float arithmetic (1).  Double-float
-// Phi needs 255 registers a thread (one block per SM) and measured 987 us
-// against 741 us at 128^3; capped at 128 registers it spills 1.7 KB.
-#ifndef DEFT_DF_PHI
-#define DEFT_DF_PHI 0
-#endif
-#ifndef DEFT_Z_PHI_DF_MIN_BLOCKS
-#define DEFT_Z_PHI_DF_MIN_BLOCKS 0
-#endif
-template <typename T> using PhiT = std::conditional_t<is_df<T> && !DEFT_DF_PHI, double, T>;
+// The pointwise logarithm of the FP64 forms: by table (logtab.cuh) beside the
+// double-float transforms.
+template <typename T> __device__ __forceinline__ Acc<T> local_log(Acc<T> x) {
+  if constexpr (is_df<T>) return log_tab(x);
+  else return wb_log<Acc<T>>(x);
+}
 template <typename T, bool GRAD, int RN = 0, typename R = double>
 __global__ void __launch_bounds__(kThreads,
                                   RN > 0 ? 2
                                          : (sizeof(T) == 4 ? DEFT_Z_PHI_MIN_BLOCKS
-                                                           : (is_df<T> ? DEFT_Z_PHI_DF_MIN_BLOCKS
-                                                                       : 0)))
+                                                           : (is_df<T> ? 2 : 0)))
     k_z_phi(typename Cplx<T>::type *S5,
                                                     const R *__restrict__ n,
                                                     const R *__restrict__ V, Geom g,
@@ -1004,39 +1028,44 @@ __global__ void __launch_bounds__(kThreads,
   const int Nz = g.Nz, P5 = 5 * P;
   const int p0 = blockIdx.x * P;
   C *res = z_load5_c2r<T, RN>(S5, A, Bf, g, pz, fP, f5P, p0);
-  // Phi and its partials in T (double-float in the FP64 form: FP64 only for
-  // its log), the energy sums and the local terms in U
+  // Phi and its partials in T (FP64 for double, double-float for dfl), the
+  // energy sums and the local terms in U
   using U = Acc<T>;
-  using Q = PhiT<T>;
   U tacc[kNumTerms] = {0, 0, 0, 0, 0, 0};
   const bool hs = la.terms & kTermHS;
   const U inv_nQ = U(la.inv_nQ);
-  const Q c = Q(la.dV * la.kT);
-  #pragma unroll 4
+  const U c = U(la.dV * la.kT);
+  #pragma unroll (is_df<T> ? 1 : 4)
   for (int idx = threadIdx.x; idx < 2 * P * Nz; idx += blockDim.x) {
     int ll, z;
     fdivmod(idx, g.fNz, ll, z);
     const int line = 2 * p0 + ll;
     T *cell = reinterpret_cast<T *>(res + z * P5 + (ll >> 1)) + (ll & 1);  // field 0
     const int fstride = 2 * P;  // T elements between fields
-    Q d[5] = {0, 0, 0, 0, 0};
+    T d[5] = {0, 0, 0, 0, 0};
     if (line < g.lines) {
       const size_t r = (size_t)line * Nz + z;
       if (hs) {
-        Q phi[3];
-        wb_phi<Q>(la.wr, Q(cell[0]), Q(cell[fstride]), Q(cell[2 * fstride]),
-                  Q(cell[3 * fstride]), Q(cell[4 * fstride]), phi, d);
-        tacc[0] += U(phi[0]);
-        tacc[1] += U(phi[1]);
-        tacc[2] += U(phi[2]);
+        T w[5];
+#pragma unroll
+        for (int a = 0; a < 5; a++) w[a] = cell[a * fstride];
+        if constexpr (is_df<T>) {
+          df_phi_point(la.wr, la.dfk, c, w, nonzero(nv), tacc, d);
+        } else {
+          T phi[3];
+          wb_phi<T>(la.wr, w[0], w[1], w[2], w[3], w[4], phi, d);
+          tacc[0] += phi[0];
+          tacc[1] += phi[1];
+          tacc[2] += phi[2];
+#pragma unroll
+          for (int a = 0; a < 5; a++) d[a] = c * d[a];
+        }
       }
-      const U nv = U(n[r]);
       if (la.terms & kTermIdeal) {
         // ln(n/nQ) once: the ideal-gas energy here, kept (lnq) for the
-        // gradient kernel of the same evaluation (FP64 forms: an FP64 log
-        // costs about 25 operations of GB300's narrow FP64 pipe)
-        const U lg = wb_log<U>(nv * inv_nQ);
-        tacc[3] += nv == U(0) ? U(0) : nv * (lg - U(1));
+        // gradient kernel of the same evaluation (FP64 forms)
+        const U lg = local_log<T>(nv * inv_nQ);
+        if (nonzero(nv)) tacc[3] += nv * (lg - U(1));
         if (lnq) lnq[r] = double(lg);
       }
       if (la.terms & kTermMu) tacc[4] += nv;
@@ -1044,7 +1073,7 @@ __global__ void __launch_bounds__(kThreads,
     }
     if (GRAD) {
 #pragma unroll
-      for (int a = 0; a < 5; a++) cell[a * fstride] = T(c * d[a]);
+      for (int a = 0; a < 5; a++) cell[a * fstride] = d[a];
     }
   }
   block_reduce_terms<U>(tacc, la, red, partials);
@@ -1060,6 +1089,11 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_grad(const typename Cplx<T>::type *__res
                                                      const double *__restrict__ V,
                                                      const double *__restrict__ mask,
                                                      double *__restrict__ grad, Geom g, FftPlan pz,
+// x / 2 (exact).
+__device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
+__device__ __forceinline__ double half_of(double x) { return 0.5 * x; }
+__device__ __forceinline__ dfl half_of(dfl x) { return df_ldexp(x, 0.5f); }
+
                                                      FastDiv fP, const LocalArgs *__restrict__ lap,
                                                      GradDots gd,
                                                      const double *__restrict__ lnq) {
@@ -1092,7 +1126,7 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_grad(const typename Cplx<T>::type *__res
     }
     U loc = 0;
     if (la.terms & kTermIdeal)
-      loc += U(la.kT) * (lnq ? U(lnq[r]) : wb_log<U>(U(n[r]) * U(la.inv_nQ)));
+      loc += U(la.kT) * (lnq ? U(lnq[r]) : local_log<T>(U(n[r]) * U(la.inv_nQ)));
     if (la.terms & kTermMu) loc += U(la.mu);
     if (la.terms & kTermVext) loc += U(V[r]);
     U gr = conv + U(la.dV) * loc;
@@ -1146,6 +1180,7 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_hess(const typename Cplx<T>::type *__res
     const size_t r = (size_t)line * Nz + z;
     const T *cell = reinterpret_cast<const T *>(res + z * P5 + (ll >> 1)) + (ll & 1);
     const int fs = 2 * P;
+      const U nv = U(n[r]);
     T h[kHessPacked];
     if (hs) {
       wb_hess<T>(la.wr, cell[0], cell[fs], cell[2 * fs], cell[3 * fs], cell[4 * fs], h);
@@ -1171,6 +1206,11 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_jac(typename Cplx<T>::type *S5, Geom g, 
   const int P = (int)fP.d;
   using C = typename Cplx<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  if constexpr (is_df<T>) {
+    tacc[0] *= la.dfk.s0;
+    tacc[1] *= la.dfk.s1;
+    tacc[2] *= la.dfk.s2;
+  }
   C *A = reinterpret_cast<C *>(smem_raw);
   C *Bf = A + g.Nz * 5 * P;
   const int Nz = g.Nz, P5 = 5 * P;
@@ -1715,7 +1755,7 @@ __global__ void k_c_df2d(const dfc *__restrict__ in, double2 *__restrict__ out, 
 __global__ void k_c_d2df(const double2 *__restrict__ in, dfc *__restrict__ out, int n) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double2 v = in[i];
-    out[i] = dfc{dfl(v.x), dfl(v.y)};
+    out[i] = dfc{df_from(v.x), df_from(v.y)};
   }
 }
 
@@ -3199,6 +3239,7 @@ class EngineImpl {
   void queue_energy(int nblk, int dk = 0, const double *dpart = nullptr, int gblk = 0) {
     pre(kK_reduce_terms);
     k_reduce_terms<<<1, kReduceThreads, 0, stream>>>(partials, nblk, g.dV, results, dpart, dk,
+    la.dfk = df_phi_const(la.wr, g.dV * f.kT);
                                                       gblk);
     post(kK_reduce_terms);
     if (!dev_only)

@@ -48,13 +48,17 @@ struct Geom {
   int NC;     // Nx*Ny*NzH complex points
   double Bm[9];  // k_c = sum_d Bm[3c+d] m_d  (2 pi R^-T)
   float Bmf[9];  // the same in FP32, for the mixed form
+  float Bml[9];  // Bm - Bmf in FP32 (Bmf + Bml: the double-float Bm)
   double dV, vol, dr, scale;  // scale = dV / vol (fft x dV then ifft x 1/V)
   FastDiv fNz, fNzH, fNy;     // division by Nz, Nz/2+1, Ny
 };
 
-// Fills the derived members (FP32 copy of Bm, fast dividers).
+// Fills the derived members (FP32 parts of Bm, fast dividers).
 inline void geom_finish(Geom &g) {
-  for (int i = 0; i < 9; i++) g.Bmf[i] = (float)g.Bm[i];
+  for (int i = 0; i < 9; i++) {
+    g.Bmf[i] = (float)g.Bm[i];
+    g.Bml[i] = (float)(g.Bm[i] - (double)g.Bmf[i]);
+  }
   g.fNz = make_fastdiv((unsigned)g.Nz);
   g.fNzH = make_fastdiv((unsigned)g.NzH);
   g.fNy = make_fastdiv((unsigned)g.Ny);

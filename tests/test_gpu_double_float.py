@@ -1,0 +1,62 @@
+"""The FP64 form's double-float kernels against the FP64 oracle where their
+branches meet: Phi in every density regime (dilute fluids, the series below
+n3 = 1/32 and 1/16, dense fluids, empty walls) for each hard-sphere kind.
+
+Tolerances.  A double-float operation rounds at 2^-47 or better and Phi's
+longest chains are some tens of them: 2^-42 of a partial's largest term.  The
+oracle's own ln(1 - n3) is FP64's, whose argument is rounded to 2^-53, i.e. to
+2^-53 / n3 of the logarithm; dilute cases allow four of those."""
+import math
+
+import numpy as np
+import pytest
+
+from deft_gb300 import _lib
+
+pytestmark = pytest.mark.gpu
+
+KINDS = [_lib.HS_WB_NOTENSOR, _lib.HS_RF, _lib.HS_WB_MARK2]
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from tests.capi import Ctx
+    c = Ctx(0)
+    yield c
+    c.close()
+
+
+def _check(ctx, O, lat, N, n, kind, n3, R=1.0, kT=1.0):
+    from tests.capi import Fmt, Grid
+    g = Grid(ctx, lat, N)
+    f = Fmt(g, R=R, kT=kT, terms=O.HS, functional=kind)
+    E, grad, terms = f.energy_grad(n)
+    P = O.Problem(lat, N, R=R, kT=kT, terms=O.HS, hs=kind)
+    Er, gr = P.energy_grad(n)
+    tol = 2.0 ** -42 + 4 * 2.0 ** -53 / n3
+    print(f"kind {kind} N {N} n3 {n3:.3g}: |dE/E| {abs(E / Er - 1):.2e} "
+          f"grad {np.abs(grad.reshape(-1) - gr.reshape(-1)).max() / np.abs(gr).max():.2e} "
+          f"(allowed {tol:.2e})")
+    assert abs(E / Er - 1) <= tol
+    assert np.abs(grad.reshape(-1) - gr.reshape(-1)).max() <= tol * np.abs(gr).max()
+    f.close()
+    g.close()
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("n3", [1e-12, 1e-7, 1e-3, 1 / 32, 1 / 16, 0.25, 0.48])
+def test_phi_regimes(ctx, oracle_mod, kind, n3):
+    N, lat = (12, 10, 14), np.diag([2.4, 2.0, 2.8])
+    rng = np.random.default_rng(int(1e6 * n3) + kind)
+    n = n3 / (4 * math.pi / 3) * (1 + 0.1 * rng.standard_normal(N))
+    _check(ctx, oracle_mod, lat, N, n.clip(0.5 * n3 / (4 * math.pi / 3)), kind, n3)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_phi_walls(ctx, oracle_mod, kind):
+    """Empty walls (n = 0) beside a dense fluid, non-unit R and kT."""
+    N, lat = (9, 8, 64), np.diag([1.8, 1.6, 12.8])
+    rng = np.random.default_rng(5)
+    n = 0.3 / (4 * math.pi / 3) / 0.8 ** 3 * (1 + 0.05 * rng.standard_normal(N))
+    n[:, :, 30:] = 0.0
+    _check(ctx, oracle_mod, lat, N, n, kind, 0.3, R=0.8, kT=1.7)
