@@ -966,6 +966,11 @@ __device__ typename Cplx<T>::type *z_load5_c2r(const typename Cplx<T>::type *__r
   return fft_tile<T, +1, RN>(A, Bf, f5P, pz);
 }
 
+// x / 2 (exact).
+__device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
+__device__ __forceinline__ double half_of(double x) { return 0.5 * x; }
+__device__ __forceinline__ dfl half_of(dfl x) { return df_ldexp(x, 0.5f); }
+
 // Forward z transform of the five real pairs held in `res` (same layout)
 // and the Hermitian split into the five half spectra of S5.
 template <typename T, int RN = 0>
@@ -1045,6 +1050,7 @@ __global__ void __launch_bounds__(kThreads,
     T d[5] = {0, 0, 0, 0, 0};
     if (line < g.lines) {
       const size_t r = (size_t)line * Nz + z;
+      const U nv = U(n[r]);
       if (hs) {
         T w[5];
 #pragma unroll
@@ -1076,6 +1082,11 @@ __global__ void __launch_bounds__(kThreads,
       for (int a = 0; a < 5; a++) cell[a * fstride] = d[a];
     }
   }
+  if constexpr (is_df<T>) {
+    tacc[0] *= la.dfk.s0;
+    tacc[1] *= la.dfk.s1;
+    tacc[2] *= la.dfk.s2;
+  }
   block_reduce_terms<U>(tacc, la, red, partials);
   if (!GRAD) return;
   __syncthreads();
@@ -1089,11 +1100,6 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_grad(const typename Cplx<T>::type *__res
                                                      const double *__restrict__ V,
                                                      const double *__restrict__ mask,
                                                      double *__restrict__ grad, Geom g, FftPlan pz,
-// x / 2 (exact).
-__device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
-__device__ __forceinline__ double half_of(double x) { return 0.5 * x; }
-__device__ __forceinline__ dfl half_of(dfl x) { return df_ldexp(x, 0.5f); }
-
                                                      FastDiv fP, const LocalArgs *__restrict__ lap,
                                                      GradDots gd,
                                                      const double *__restrict__ lnq) {
@@ -1180,7 +1186,6 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_hess(const typename Cplx<T>::type *__res
     const size_t r = (size_t)line * Nz + z;
     const T *cell = reinterpret_cast<const T *>(res + z * P5 + (ll >> 1)) + (ll & 1);
     const int fs = 2 * P;
-      const U nv = U(n[r]);
     T h[kHessPacked];
     if (hs) {
       wb_hess<T>(la.wr, cell[0], cell[fs], cell[2 * fs], cell[3 * fs], cell[4 * fs], h);
@@ -1206,11 +1211,6 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_jac(typename Cplx<T>::type *S5, Geom g, 
   const int P = (int)fP.d;
   using C = typename Cplx<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  if constexpr (is_df<T>) {
-    tacc[0] *= la.dfk.s0;
-    tacc[1] *= la.dfk.s1;
-    tacc[2] *= la.dfk.s2;
-  }
   C *A = reinterpret_cast<C *>(smem_raw);
   C *Bf = A + g.Nz * 5 * P;
   const int Nz = g.Nz, P5 = 5 * P;
@@ -3104,6 +3104,7 @@ class EngineImpl {
     la.wr.inv_4piR2 = 1.0 / (4 * M_PI * f.R * f.R);
     la.wr.kind = f.hs;
     la.terms = f.terms;
+    la.dfk = df_phi_const(la.wr, g.dV * f.kT);
     if (f.terms & kTermHS) {
       // the bulk solve runs once per (mu, kT, R, kind)
       if (!(pc_key_valid && pc_key.mu == f.mu && pc_key.kT == f.kT && pc_key.R == f.R &&
@@ -3239,7 +3240,6 @@ class EngineImpl {
   void queue_energy(int nblk, int dk = 0, const double *dpart = nullptr, int gblk = 0) {
     pre(kK_reduce_terms);
     k_reduce_terms<<<1, kReduceThreads, 0, stream>>>(partials, nblk, g.dV, results, dpart, dk,
-    la.dfk = df_phi_const(la.wr, g.dV * f.kT);
                                                       gblk);
     post(kK_reduce_terms);
     if (!dev_only)
