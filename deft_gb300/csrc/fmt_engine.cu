@@ -682,23 +682,28 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_x_conv_adj(
 // FFT along y of nf complex fields in place.  Columns c = x NzH + kz (all x
 // planes back to back); element y of column c at x Ny NzH + y NzH + kz.
 // grid = (column groups, fields).
-template <int SIGN, int W>
-__global__ void __launch_bounds__(pencil_threads<W>())
-    k_y_pencil(float2 *data, Geom g, const float2 *__restrict__ tw) {
-  constexpr int G = pencil_groups<W>(), P = 16 / W;
+// T = dfl: 128 registers, i.e. 16 warps per SM.  Mean of a one-field and a
+// five-field launch against the shared-memory passes: 128^3 53 -> 31 us, 256^3
+// 520 -> 300 us.
+template <int SIGN, int W, typename T = float>
+__global__ void __launch_bounds__(is_df<T> ? 32 * W : pencil_threads<W>(), is_df<T> ? 16 / W : 0)
+    k_y_pencil(typename Cplx<T>::type *data, Geom g,
+               const typename Cplx<T>::type *__restrict__ tw) {
+  using C = typename Cplx<T>::type;
+  constexpr int G = is_df<T> ? 1 : pencil_groups<W>(), P = 16 / W;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w = warp % W, grp = warp / W;
-  float2 *xs = reinterpret_cast<float2 *>(smem_raw) + grp * pencil_xs_elems<W>();
+  auto *xs = reinterpret_cast<typename PencilXs<T>::type *>(smem_raw) + grp * pencil_xs_elems<W>();
   const int c = (blockIdx.x * G + grp) * 32 + lane;
   const bool act = c < g.Nx * g.NzH;
   int x, kz;
   fdivmod(act ? c : 0, g.fNzH, x, kz);
-  float2 *base = data + (size_t)blockIdx.y * g.NC + (size_t)x * g.Ny * g.NzH + kz;
+  C *base = data + (size_t)blockIdx.y * g.NC + (size_t)x * g.Ny * g.NzH + kz;
   const int st = g.NzH;
-  float2 v[16];
+  C v[16];
 #pragma unroll
-  for (int m = 0; m < 16; m++) v[m] = act ? base[(w + W * m) * st] : make_float2(0.f, 0.f);
-  pencil_n2s<float, SIGN, W>(v, xs, w, lane, tw);
+  for (int m = 0; m < 16; m++) v[m] = act ? base[(w + W * m) * st] : C{0, 0};
+  pencil_n2s<T, SIGN, W>(v, xs, w, lane, tw);
   if (act) {
 #pragma unroll
     for (int i = 0; i < P; i++)
@@ -851,6 +856,163 @@ __global__ void __launch_bounds__(pencil_threads<W>(), W >= 16 ? 1 : 2)
   }
 }
 
+// The double-float forms of the two convolutions, one column group a block.
+// The weights come from the table (three reads a k-point).  Bound by the
+// double-float arithmetic, about 200 FP32 operations a complex point and
+// transform.  SPLIT false: a block takes all five fields one after another,
+// the spectrum waiting in thread-private shared slots (six transforms a
+// column; 128^3: 146 -> 109 us forward and 161 -> 100 us adjoint against the
+// shared-memory passes).  SPLIT true, for grids whose columns are too few to
+// fill the chip: a block per column group and field, each with its own
+// forward transform (64^3: 31 -> 20 us forward; adjoint, in two launches, 25
+// us either way).
+
+// The weight of field a at the frequencies a thread holds, applied to v:
+// sgn = 1 forward (times w3, w2, i k_c wv), -1 adjoint (odd weights negated).
+template <int W>
+__device__ __forceinline__ void pencil_weight_df(dfc (&v)[16], int a, int sgn,
+                                                 const dfl *__restrict__ tab, const Geom &g,
+                                                 int w, int y, int kz, int j, int J, double R) {
+  const bool act = j < J;
+  const int c = a < 2 ? 0 : a - 2;
+  const dfl kb = kcomp_t<dfl>(g, c, 0, y, kz), bx(g.Bmf[3 * c], g.Bml[3 * c]);
+#pragma unroll
+  for (int q = 0; q < 16; q++) {
+    const int f = pencil_freq<W>(w, q);
+    const dfl wt = act ? tab[(size_t)f * J + j] : dfl(0);
+    if (a < 2) {
+      if (q == 0 && w == 0 && j == 0) v[q] = dc_weight(v[q], dc_w(a, R, g));  // k = 0
+      else v[q] = dfc{v[q].x * wt, v[q].y * wt};
+    } else {
+      dfl wk = (df_scale(bx, (float)wrapm(f, g.Nx)) + kb) * wt;
+      if (sgn < 0) wk = -wk;
+      v[q] = dfc{-(v[q].y * wk), v[q].x * wk};  // times +-i wk
+    }
+  }
+}
+
+template <int W>
+__device__ __forceinline__ void pencil_load(dfc (&v)[16], const dfc *src, int w, int j, int J) {
+#pragma unroll
+  for (int m = 0; m < 16; m++) v[m] = j < J ? src[(size_t)(w + W * m) * J + j] : dfc{0, 0};
+}
+template <int W>
+__device__ __forceinline__ void pencil_store(const dfc (&v)[16], dfc *dst, int w, int j, int J) {
+  if (j < J) {
+#pragma unroll
+    for (int m = 0; m < 16; m++) dst[(size_t)(w + W * m) * J + j] = v[m];
+  }
+}
+
+template <int W, bool SPLIT>
+__global__ void __launch_bounds__(32 * W, 16 / W)
+    k_x_conv_fwd_pencil_df(const dfc *__restrict__ in, dfc *__restrict__ out5,
+                           const dfl *__restrict__ w3, const dfl *__restrict__ w2,
+                           const dfl *__restrict__ wv, Geom g, const dfc *__restrict__ tw,
+                           const LocalArgs *__restrict__ lap) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  dfl *xs = reinterpret_cast<dfl *>(smem_raw);
+  dfc *spec = reinterpret_cast<dfc *>(xs + pencil_xs_elems<W>());
+  const int J = g.Ny * g.NzH;
+  const int j = blockIdx.x * 32 + lane;
+  int y, kz;
+  fdivmod(j < J ? j : 0, g.fNzH, y, kz);
+  dfc v[16];
+  pencil_load<W>(v, in, w, j, J);
+  pencil_n2s<dfl, -1, W>(v, xs, w, lane, tw);
+  if constexpr (!SPLIT) {
+#pragma unroll
+    for (int q = 0; q < 16; q++) spec[q * blockDim.x + threadIdx.x] = v[q];
+  }
+#pragma unroll 1
+  for (int a = SPLIT ? blockIdx.y : 0; a < 5; a++) {
+    if constexpr (!SPLIT) {
+#pragma unroll
+      for (int q = 0; q < 16; q++) v[q] = spec[q * blockDim.x + threadIdx.x];
+    }
+    pencil_weight_df<W>(v, a, 1, a == 0 ? w3 : a == 1 ? w2 : wv, g, w, y, kz, j, J, lap->R);
+    pencil_s2n<dfl, +1, W>(v, xs, w, lane, tw);
+    pencil_store<W>(v, out5 + (size_t)a * g.NC, w, j, J);
+    if constexpr (SPLIT) break;
+  }
+}
+
+// All five fields of a column group; SPLIT: the weighted spectrum of one
+// field, written back in place for k_x_sum_pencil_df.
+template <int W, bool SPLIT>
+__global__ void __launch_bounds__(32 * W, 16 / W)
+    k_x_conv_adj_pencil_df(dfc *in5, dfc *__restrict__ out, const dfl *__restrict__ w3,
+                           const dfl *__restrict__ w2, const dfl *__restrict__ wv, Geom g,
+                           const dfc *__restrict__ tw, const LocalArgs *__restrict__ lap) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  dfl *xs = reinterpret_cast<dfl *>(smem_raw);
+  dfc *sum = reinterpret_cast<dfc *>(xs + pencil_xs_elems<W>());
+  const int J = g.Ny * g.NzH;
+  const int j = blockIdx.x * 32 + lane;
+  int y, kz;
+  fdivmod(j < J ? j : 0, g.fNzH, y, kz);
+  dfc v[16];
+#pragma unroll 1
+  for (int a = SPLIT ? blockIdx.y : 0; a < 5; a++) {
+    pencil_load<W>(v, in5 + (size_t)a * g.NC, w, j, J);
+    pencil_n2s<dfl, -1, W>(v, xs, w, lane, tw);
+    pencil_weight_df<W>(v, a, -1, a == 0 ? w3 : a == 1 ? w2 : wv, g, w, y, kz, j, J, lap->R);
+    if constexpr (SPLIT) {
+      // each thread's own slots, as rows of the spectral order
+      if (j < J) {
+        dfc *dst = in5 + (size_t)a * g.NC + j;
+#pragma unroll
+        for (int q = 0; q < 16; q++) dst[(size_t)(w * 16 + q) * J] = v[q];
+      }
+      break;
+    } else {
+#pragma unroll
+      for (int q = 0; q < 16; q++) {
+        dfc &o = sum[q * blockDim.x + threadIdx.x];
+        o = a == 0 ? v[q] : dfc{o.x + v[q].x, o.y + v[q].y};
+      }
+    }
+  }
+  if constexpr (!SPLIT) {
+#pragma unroll
+    for (int q = 0; q < 16; q++) v[q] = sum[q * blockDim.x + threadIdx.x];
+    pencil_s2n<dfl, +1, W>(v, xs, w, lane, tw);
+    pencil_store<W>(v, out, w, j, J);
+  }
+}
+
+// The split adjoint's second half: the five weighted spectra summed (in the
+// order of the fields) and transformed back.
+template <int W>
+__global__ void __launch_bounds__(32 * W, 16 / W)
+    k_x_sum_pencil_df(const dfc *__restrict__ in5, dfc *__restrict__ out, Geom g,
+                      const dfc *__restrict__ tw) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  dfl *xs = reinterpret_cast<dfl *>(smem_raw);
+  const int J = g.Ny * g.NzH;
+  const int j = blockIdx.x * 32 + lane;
+  dfc v[16];
+#pragma unroll
+  for (int q = 0; q < 16; q++) {
+    dfc o = dfc{0, 0};
+    if (j < J) {
+      const dfc *src = in5 + (size_t)(w * 16 + q) * J + j;
+      o = src[0];
+#pragma unroll
+      for (int a = 1; a < 5; a++) {
+        const dfc t = src[(size_t)a * g.NC];
+        o = dfc{o.x + t.x, o.y + t.y};
+      }
+    }
+    v[q] = o;
+  }
+  pencil_s2n<dfl, +1, W>(v, xs, w, lane, tw);
+  pencil_store<W>(v, out, w, j, J);
+}
+
 // The structure preconditioner along x, in place on one field: x-FFT, times
 // P(k) / N from the table P (layout x Ny NzH + y NzH + kz, k_pc_table),
 // inverse x-FFT (columns as in k_x_conv_fwd_pencil).
@@ -918,6 +1080,10 @@ __global__ void k_pc_table(float *__restrict__ P, Geom g, const LocalArgs *__res
 template <int W> constexpr size_t pencil_smem(bool conv) {
   return sizeof(float2) * pencil_groups<W>() * pencil_xs_elems<W>() +
          (conv ? (sizeof(float2) * 16 + sizeof(float) * 48) * pencil_threads<W>() : 0);
+}
+// Double-float: half-width exchange buffers, and the spectrum or sum slots.
+template <int W> constexpr size_t pencil_smem_df(bool conv) {
+  return sizeof(dfl) * pencil_xs_elems<W>() + (conv ? sizeof(dfc) * 16 * 32 * W : 0);
 }
 
 // Ideal-gas integrand kT n (ln(n/nQ) - 1) (src/IdealGas.cpp:68-72), 0 at
@@ -2390,6 +2556,7 @@ Tiles make_tiles(const Geom &g, size_t cs, size_t budget, const TileChoice *ov =
   t.Bxf = even_tiles(g.Ny * g.NzH, cap(budget / (3 * (size_t)g.Nx * cs), 16));
   t.Bxc = even_tiles(g.Ny * g.NzH, cap(budget / (10 * (size_t)g.Nx * cs), 16));
   t.Pz = even_tiles(pairs, cap(budget / (2 * (size_t)g.Nz * cs), 16));
+  if (t.Pz > 1 && t.Pz % 2 == 0) t.Pz -= 1;  // odd, as Pphi below
   int pm = cap(budget / (10 * (size_t)g.Nz * cs), 15);
   if (pm < 1) pm = 1;
   if (pm > 1 && pm % 2 == 0) pm -= 1;  // odd: conflict-free z-strided shared accesses
@@ -2783,6 +2950,13 @@ class EngineImpl {
       set_smem(k_x_conv_fwd_pencil<W>, pencil_smem<W>(true));
       set_smem(k_x_conv_adj_pencil<W>, pencil_smem<W>(true));
       set_smem(k_x_pc_pencil<W>, pencil_smem<W>(false));
+      set_smem(k_y_pencil<-1, W, dfl>, pencil_smem_df<W>(false));
+      set_smem(k_y_pencil<+1, W, dfl>, pencil_smem_df<W>(false));
+      set_smem(k_x_conv_fwd_pencil_df<W, false>, pencil_smem_df<W>(true));
+      set_smem(k_x_conv_adj_pencil_df<W, false>, pencil_smem_df<W>(true));
+      set_smem(k_x_conv_fwd_pencil_df<W, true>, pencil_smem_df<W>(false));
+      set_smem(k_x_conv_adj_pencil_df<W, true>, pencil_smem_df<W>(false));
+      set_smem(k_x_sum_pencil_df<W>, pencil_smem_df<W>(false));
     };
     smemp(std::integral_constant<int, 2>());
     smemp(std::integral_constant<int, 4>());
@@ -2833,10 +3007,11 @@ class EngineImpl {
     if (alloc(&results, sizeof(double) * 16) || alloc(&la_dev, sizeof(LocalArgs))) return -1;
     cudaError_t e = cudaMallocHost((void **)&results_host, sizeof(double) * 16);
     if (e != cudaSuccess) return fail("cudaMallocHost", e);
-    int dev = 0, sms = 0;
+    int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    dot_blocks = 4 * (sms > 0 ? sms : 148);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (nsm > 0) sms = nsm;
+    dot_blocks = 4 * sms;
     const int need = (g.NR + kThreads - 1) / kThreads;
     if (dot_blocks > need) dot_blocks = need;
     if (dot_blocks < 1) dot_blocks = 1;
@@ -2950,13 +3125,27 @@ class EngineImpl {
       for (int i = 0; i < 8; i++) c->radix[a][i] = i < pl[a]->npass ? pl[a]->radix[i] : 0;
   }
 
-  // Pencil kernels for the FP32 x and y transforms of lengths 32..256
-  // (DEFT_PENCIL=0 in the environment at grid creation selects the
-  // shared-memory Stockham kernels instead).
+  // Pencil kernels for the FP32 and double-float x and y transforms of
+  // lengths 32..256 (DEFT_PENCIL=0 in the environment at grid creation
+  // selects the shared-memory Stockham kernels instead, which are also what
+  // every other length takes).  Double-float ones also need a warp for every
+  // SM: their straight-line code (some 3000 instructions a transform) is
+  // fetched once per warp, and with fewer warps the fetches are what a launch
+  // takes (one field at 32^3, 34 warps: 6 us against 4 us).
   bool pencil_on = true;
   template <typename T> bool pencil(int axis) const {
-    return std::is_same<T, float>::value && pencil_on &&
-           pencil_w(axis == 0 ? g.Nx : axis == 1 ? g.Ny : g.Nz) > 0;
+    const int L = axis == 0 ? g.Nx : axis == 1 ? g.Ny : g.Nz;
+    if (std::is_same<T, double>::value || !pencil_on || pencil_w(L) == 0) return false;
+    const int cols = axis == 0 ? g.Ny * g.NzH : g.Nx * g.NzH;
+    return !is_df<T> || (cols + 31) / 32 * (L / 16) >= sms;
+  }
+  // The double-float x convolutions run a block per column group and field
+  // where the column groups alone leave the SMs fewer than eight warps each
+  // (two a scheduler: below that the extra forward transforms cost less than
+  // the idle issue slots).
+  int sms = 148;
+  template <int W> bool split_x_df() const {
+    return (g.Ny * g.NzH + 31) / 32 * W < 8 * sms;
   }
   // Calls f(std::integral_constant<int, W>()) for the pencil width of length L.
   template <typename F> static void with_w(int L, F &&f) {
@@ -2993,19 +3182,20 @@ class EngineImpl {
     dim3 grid((g.NzH + t.By - 1) / t.By, g.Nx, nf);
     const int kid = kslot<T>(nf == 1 ? kK_y_fft1 : kK_y_fft5);
     pre(kid);
-    if constexpr (std::is_same<T, float>::value) {
+    if constexpr (!std::is_same<T, double>::value) {
       if (pencil<T>(1)) {
         with_w(g.Ny, [&](auto wc) {
           constexpr int W = decltype(wc)::value;
-          const int cols = 32 * pencil_groups<W>();
+          const int cols = 32 * (is_df<T> ? 1 : pencil_groups<W>());
+          const int threads = is_df<T> ? 32 * W : pencil_threads<W>();
           const dim3 pg((g.Nx * g.NzH + cols - 1) / cols, nf);
-          const float2 *tw = reinterpret_cast<const float2 *>(plan<T>(1).tw);
+          using C = typename Cplx<T>::type;
+          const C *tw = reinterpret_cast<const C *>(plan<T>(1).tw);
+          const size_t sm = is_df<T> ? pencil_smem_df<W>(false) : pencil_smem<W>(false);
           if (sign < 0)
-            k_y_pencil<-1, W><<<pg, pencil_threads<W>(), pencil_smem<W>(false), stream>>>(
-                reinterpret_cast<float2 *>(data), g, tw);
+            k_y_pencil<-1, W, T><<<pg, threads, sm, stream>>>(data, g, tw);
           else
-            k_y_pencil<+1, W><<<pg, pencil_threads<W>(), pencil_smem<W>(false), stream>>>(
-                reinterpret_cast<float2 *>(data), g, tw);
+            k_y_pencil<+1, W, T><<<pg, threads, sm, stream>>>(data, g, tw);
         });
         post(kid);
         return;
@@ -3028,11 +3218,24 @@ class EngineImpl {
     if (pencil<T>(0)) {
       with_w(g.Nx, [&](auto wc) {
         constexpr int W = decltype(wc)::value;
-        const int cols = 32 * pencil_groups<W>();
-        k_x_conv_adj_pencil<W><<<(g.Ny * g.NzH + cols - 1) / cols, pencil_threads<W>(),
-                                 pencil_smem<W>(true), stream>>>(
-            reinterpret_cast<const float2 *>(spec5<T>()), reinterpret_cast<float2 *>(spec0<T>()),
-            g, reinterpret_cast<const float2 *>(plan<T>(0).tw), la_dev);
+        const int blocks = (g.Ny * g.NzH + 32 * pencil_groups<W>() - 1) / (32 * pencil_groups<W>());
+        if constexpr (is_df<T>) {
+          const int groups = (g.Ny * g.NzH + 31) / 32;
+          if (split_x_df<W>()) {
+            k_x_conv_adj_pencil_df<W, true><<<dim3(groups, 5), 32 * W, pencil_smem_df<W>(false),
+                                              stream>>>(spec5<T>(), spec0<T>(), w3d, w2d, wvd, g,
+                                                        tw_xd, la_dev);
+            post(kK_x_conv_adj);
+            pre(kK_x_conv_adj);
+            k_x_sum_pencil_df<W><<<groups, 32 * W, pencil_smem_df<W>(false), stream>>>(
+                spec5<T>(), spec0<T>(), g, tw_xd);
+          } else {
+            k_x_conv_adj_pencil_df<W, false><<<groups, 32 * W, pencil_smem_df<W>(true), stream>>>(
+                spec5<T>(), spec0<T>(), w3d, w2d, wvd, g, tw_xd, la_dev);
+          }
+        } else if constexpr (std::is_same<T, float>::value)
+          k_x_conv_adj_pencil<W><<<blocks, pencil_threads<W>(), pencil_smem<W>(true), stream>>>(
+              spec5<T>(), spec0<T>(), g, reinterpret_cast<const float2 *>(plan<T>(0).tw), la_dev);
       });
       return;
     }
@@ -3073,11 +3276,19 @@ class EngineImpl {
     if (pencil<T>(0)) {
       with_w(g.Nx, [&](auto wc) {
         constexpr int W = decltype(wc)::value;
-        const int cols = 32 * pencil_groups<W>();
-        k_x_conv_fwd_pencil<W><<<(g.Ny * g.NzH + cols - 1) / cols, pencil_threads<W>(),
-                                 pencil_smem<W>(true), stream>>>(
-            reinterpret_cast<const float2 *>(spec0<T>()), reinterpret_cast<float2 *>(spec5<T>()),
-            g, reinterpret_cast<const float2 *>(plan<T>(0).tw), la_dev);
+        const int blocks = (g.Ny * g.NzH + 32 * pencil_groups<W>() - 1) / (32 * pencil_groups<W>());
+        if constexpr (is_df<T>) {
+          const int groups = (g.Ny * g.NzH + 31) / 32;
+          if (split_x_df<W>())
+            k_x_conv_fwd_pencil_df<W, true><<<dim3(groups, 5), 32 * W, pencil_smem_df<W>(false),
+                                              stream>>>(spec0<T>(), spec5<T>(), w3d, w2d, wvd, g,
+                                                        tw_xd, la_dev);
+          else
+            k_x_conv_fwd_pencil_df<W, false><<<groups, 32 * W, pencil_smem_df<W>(true), stream>>>(
+                spec0<T>(), spec5<T>(), w3d, w2d, wvd, g, tw_xd, la_dev);
+        } else if constexpr (std::is_same<T, float>::value)
+          k_x_conv_fwd_pencil<W><<<blocks, pencil_threads<W>(), pencil_smem<W>(true), stream>>>(
+              spec0<T>(), spec5<T>(), g, reinterpret_cast<const float2 *>(plan<T>(0).tw), la_dev);
       });
     } else {
       with_rn<T>(plan<T>(0), [&](auto rn) {

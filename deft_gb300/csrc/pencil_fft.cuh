@@ -3,7 +3,8 @@
 //
 // A column is a line of L complex elements with a constant stride in global
 // memory; the 32 columns of a group are adjacent in memory, so a warp's load
-// or store of one row is one contiguous 256-byte (FP32) run.  The transform
+// or store of one row is one contiguous 256-byte (FP32) or 512-byte
+// (double-float) run.  The transform
 // is the two-stage Cooley-Tukey split L = 16 x W:
 //
 //   natural distribution:  element n = w + W m sits in warp w, slot m (m < 16)
@@ -18,8 +19,10 @@
 // twiddle index is uniform across a warp, so the table reads are broadcasts.
 //
 // Exchange buffer layout: xs[(w * 16 + k1) * 32 + lane], conflict-free for
-// both the writes and the reads.  Every thread of the block must call the
-// transforms (they synchronise the block).
+// both the writes and the reads.  Double-float elements (16 bytes) cross in two
+// rounds, real parts and then imaginary parts, through a buffer of half the
+// size.  Every thread of the block must call the transforms (they synchronise
+// the block).
 #pragma once
 
 #include "fft_smem.cuh"
@@ -32,6 +35,38 @@ template <int W> constexpr int pencil_threads() { return 32 * W * pencil_groups<
 // Exchange-buffer elements of one column group.
 template <int W> constexpr int pencil_xs_elems() { return 16 * W * 32; }
 
+// Element of the exchange buffer.
+template <typename T> struct PencilXs { using type = typename Cplx<T>::type; };
+template <> struct PencilXs<dfl> { using type = dfl; };
+
+// v[r] of the writers' slots (row wr(r)) to v[s] of the readers' (row rd(s)).
+template <typename T, typename WR, typename RD>
+__device__ __forceinline__ void pencil_exchange(typename Cplx<T>::type (&v)[16],
+                                                typename PencilXs<T>::type *xs, int lane, WR wr,
+                                                RD rd) {
+  if constexpr (sizeof(typename PencilXs<T>::type) == sizeof(typename Cplx<T>::type)) {
+    __syncthreads();  // the buffer's previous contents have been read
+#pragma unroll
+    for (int q = 0; q < 16; q++) xs[wr(q) * 32 + lane] = v[q];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 16; q++) v[q] = xs[rd(q) * 32 + lane];
+  } else {
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 16; q++) xs[wr(q) * 32 + lane] = v[q].x;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 16; q++) v[q].x = xs[rd(q) * 32 + lane];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 16; q++) xs[wr(q) * 32 + lane] = v[q].y;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 16; q++) v[q].y = xs[rd(q) * 32 + lane];
+  }
+}
+
 // The pencil length for W (L = 16 W) and the W of a length (0: no pencil).
 inline int pencil_w(int L) {
   return (L == 32 || L == 64 || L == 128 || L == 256) ? L / 16 : 0;
@@ -41,7 +76,7 @@ inline int pencil_w(int L) {
 // v[i W + k2] = X[k1 + 16 k2] (k1 = w 16/W + i) out.
 template <typename T, int S, int W>
 __device__ __forceinline__ void pencil_n2s(typename Cplx<T>::type (&v)[16],
-                                           typename Cplx<T>::type *xs, int w, int lane,
+                                           typename PencilXs<T>::type *xs, int w, int lane,
                                            const typename Cplx<T>::type *__restrict__ tw) {
   using C = typename Cplx<T>::type;
   constexpr int P = 16 / W;
@@ -50,16 +85,9 @@ __device__ __forceinline__ void pencil_n2s(typename Cplx<T>::type (&v)[16],
 #pragma unroll
     for (int k1 = 1; k1 < 16; k1++) v[k1] = c_mul(v[k1], tw_load<S>(tw, w * k1));
   }
-  __syncthreads();  // the buffer's previous contents have been read
-#pragma unroll
-  for (int k1 = 0; k1 < 16; k1++) xs[(w * 16 + k1) * 32 + lane] = v[k1];
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < P; i++) {
-    const int k1 = w * P + i;
-#pragma unroll
-    for (int ww = 0; ww < W; ww++) v[i * W + ww] = xs[(ww * 16 + k1) * 32 + lane];
-  }
+  pencil_exchange<T>(
+      v, xs, lane, [w](int k1) { return w * 16 + k1; },
+      [w](int q) { return (q % W) * 16 + w * P + q / W; });
 #pragma unroll
   for (int i = 0; i < P; i++) dft_m<S, T, C, W>(&v[i * W]);  // over w
 }
@@ -68,7 +96,7 @@ __device__ __forceinline__ void pencil_n2s(typename Cplx<T>::type (&v)[16],
 // pencil_n2s.  v[i W + k2] = Y[k1 + 16 k2] in, v[m] = y[w + W m] out.
 template <typename T, int S, int W>
 __device__ __forceinline__ void pencil_s2n(typename Cplx<T>::type (&v)[16],
-                                           typename Cplx<T>::type *xs, int w, int lane,
+                                           typename PencilXs<T>::type *xs, int w, int lane,
                                            const typename Cplx<T>::type *__restrict__ tw) {
   using C = typename Cplx<T>::type;
   constexpr int P = 16 / W;
@@ -80,16 +108,9 @@ __device__ __forceinline__ void pencil_s2n(typename Cplx<T>::type (&v)[16],
 #pragma unroll
     for (int ww = 1; ww < W; ww++) v[i * W + ww] = c_mul(v[i * W + ww], tw_load<S>(tw, ww * k1));
   }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < P; i++) {
-    const int k1 = w * P + i;
-#pragma unroll
-    for (int ww = 0; ww < W; ww++) xs[(ww * 16 + k1) * 32 + lane] = v[i * W + ww];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k1 = 0; k1 < 16; k1++) v[k1] = xs[(w * 16 + k1) * 32 + lane];
+  pencil_exchange<T>(
+      v, xs, lane, [w](int q) { return (q % W) * 16 + w * P + q / W; },
+      [w](int k1) { return w * 16 + k1; });
   dft16<S, T>(v);  // over k1: y[w + W m] at v[m]
 }
 
