@@ -7,14 +7,16 @@
 // applies the inter-pass twiddles from a global table of L roots
 // exp(-2 pi i t / L), runs a register DFT of length r and writes the
 // self-sorted result into the other buffer (ping-pong), so no bit-reversal
-// pass is needed.  Radices 2, 3, 4, 5 and 8 are hand-written; any other
-// prime factor up to 13 goes through a direct DFT from the same table.
+// pass is needed.  Radices 2, 3, 4, 5 and 8 are hand-written; 7, 11 and 13 are
+// folded DFTs with compile-time roots (dft_prime).
 //
 // Sign convention (FFTW's, which the reference links): SIGN = -1 forward,
 // +1 backward, both unnormalised.
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "dfloat.cuh"
 #include "fastdiv.cuh"
@@ -44,6 +46,13 @@ struct FftPlan {
   const void *tw;          // device table, n entries of Cplx<T>
   int reg;                 // 1: register-resident two-stage transform (radix order 16, n/16)
 };
+
+// Whether a plan has a pass of radix 7, 11 or 13.
+inline bool plan_has_prime(const FftPlan &p) {
+  for (int i = 0; i < p.npass; i++)
+    if (p.radix[i] == 7 || p.radix[i] > 8) return !p.reg;
+  return false;
+}
 
 // Fills ns[] once radix[] and npass are set.
 inline void plan_fill_ns(FftPlan &p) {
@@ -126,6 +135,94 @@ template <int SIGN, typename T, typename C> __device__ __forceinline__ void dft5
   v[3] = C{m2.x + n2.y, m2.y - n2.x};
 }
 
+// Cosines and sines of 2 pi m / R, 1 <= m <= R / 2 (folded at compile time).
+template <int R> __host__ __device__ constexpr double root_cos(int m) {
+  if (R == 7) {
+    if (m == 1) return 0.623489801858733530525;
+    if (m == 2) return -0.222520933956314404289;
+    if (m == 3) return -0.900968867902419126236;
+  }
+  if (R == 11) {
+    if (m == 1) return 0.841253532831181168862;
+    if (m == 2) return 0.415415013001886425529;
+    if (m == 3) return -0.142314838273285140444;
+    if (m == 4) return -0.654860733945285064057;
+    if (m == 5) return -0.95949297361449738989;
+  }
+  if (R == 13) {
+    if (m == 1) return 0.8854560256532098959;
+    if (m == 2) return 0.568064746731155802512;
+    if (m == 3) return 0.120536680255323053349;
+    if (m == 4) return -0.35460488704253562597;
+    if (m == 5) return -0.748510748171101098635;
+    if (m == 6) return -0.970941817426052027157;
+  }
+  return 0.0;
+}
+template <int R> __host__ __device__ constexpr double root_sin(int m) {
+  if (R == 7) {
+    if (m == 1) return 0.781831482468029808708;
+    if (m == 2) return 0.974927912181823607018;
+    if (m == 3) return 0.433883739117558120476;
+  }
+  if (R == 11) {
+    if (m == 1) return 0.540640817455597582108;
+    if (m == 2) return 0.909631995354518371412;
+    if (m == 3) return 0.989821441880932732376;
+    if (m == 4) return 0.755749574354258283774;
+    if (m == 5) return 0.281732556841429697711;
+  }
+  if (R == 13) {
+    if (m == 1) return 0.464723172043768545656;
+    if (m == 2) return 0.82298386589365639458;
+    if (m == 3) return 0.992708874098053992801;
+    if (m == 4) return 0.93501624268541482344;
+    if (m == 5) return 0.663122658240795202377;
+    if (m == 6) return 0.239315664287557767149;
+  }
+  return 0.0;
+}
+template <int R> __host__ __device__ constexpr double prime_cos(int m) {
+  return root_cos<R>(m % R <= R / 2 ? m % R : R - m % R);
+}
+template <int R> __host__ __device__ constexpr double prime_sin(int m) {
+  return m % R <= R / 2 ? root_sin<R>(m % R) : -root_sin<R>(R - m % R);
+}
+
+// DFT of odd prime length R in registers, folded over the pairs (s, R - s):
+// with t_s = v_s + v_{R-s}, u_s = v_s - v_{R-s},
+//   X_o, X_{R-o} = v_0 + sum_s cos(2 pi s o / R) t_s  +- SIGN i sum_s sin(2 pi s o / R) u_s,
+// (R-1)^2 real products instead of the direct form's 4 (R-1)^2.  Each output
+// goes to store(o, X_o) as it is formed, so that only t and u stay live.
+template <int SIGN, typename T, typename C, int R, typename F>
+__device__ __forceinline__ void dft_prime(const C *v, F store) {
+  constexpr int H = R / 2;
+  C t[H], u[H];
+  const C v0 = v[0];
+  C sum = v0;
+#pragma unroll
+  for (int s = 0; s < H; s++) {
+    t[s] = c_add(v[s + 1], v[R - 1 - s]);
+    u[s] = c_sub(v[s + 1], v[R - 1 - s]);
+    sum = c_add(sum, t[s]);
+  }
+#pragma unroll
+  for (int o = 1; o <= H; o++) {
+    C a = v0, b;
+#pragma unroll
+    for (int s = 1; s <= H; s++) {
+      const T ck = T(prime_cos<R>(s * o)), sk = T(SIGN * prime_sin<R>(s * o));
+      a = C{a.x + ck * t[s - 1].x, a.y + ck * t[s - 1].y};
+      if (s == 1) b = C{sk * u[0].x, sk * u[0].y};
+      else b = C{b.x + sk * u[s - 1].x, b.y + sk * u[s - 1].y};
+    }
+    store(o, C{a.x - b.y, a.y + b.x});
+    store(R - o, C{a.x + b.y, a.y - b.x});
+  }
+  store(0, sum);
+}
+
+
 template <int SIGN, typename C> __device__ __forceinline__ C tw_load(const C *tw, int t) {
   C w = ldg_c(&tw[t]);
   if (SIGN > 0) w.y = -w.y;
@@ -154,48 +251,17 @@ __device__ __forceinline__ void fft_pass(const typename Cplx<T>::type *__restric
 #pragma unroll
       for (int s = 1; s < R; ++s) v[s] = c_mul(v[s], tw_load<SIGN>(tw, s * k * twstep));
     }
-    if constexpr (R == 2) dft2<SIGN>(v[0], v[1]);
-    else if constexpr (R == 4) dft4<SIGN>(v[0], v[1], v[2], v[3]);
-    else if constexpr (R == 8) dft8<SIGN, T>(v);
-    else if constexpr (R == 3) dft3<SIGN, T>(v);
-    else if constexpr (R == 5) dft5<SIGN, T>(v);
     const int base = q * Ns * R + k;
+    if constexpr (R > 5 && R != 8) {
+      dft_prime<SIGN, T, C, R>(v, [&](int o, C x) { dst[(base + o * Ns) * B + bl] = x; });
+    } else {
+      if constexpr (R == 2) dft2<SIGN>(v[0], v[1]);
+      else if constexpr (R == 4) dft4<SIGN>(v[0], v[1], v[2], v[3]);
+      else if constexpr (R == 8) dft8<SIGN, T>(v);
+      else if constexpr (R == 3) dft3<SIGN, T>(v);
+      else dft5<SIGN, T>(v);
 #pragma unroll
-    for (int s = 0; s < R; ++s) dst[(base + s * Ns) * B + bl] = v[s];
-  }
-}
-
-// Direct-DFT pass for any prime radix r <= kMaxRadix.
-template <typename T, int SIGN>
-__device__ void fft_pass_generic(const typename Cplx<T>::type *__restrict__ src,
-                                 typename Cplx<T>::type *__restrict__ dst, const FastDiv &bd,
-                                 int L, const FastDiv &nsd, int r,
-                                 const typename Cplx<T>::type *__restrict__ tw) {
-  using C = typename Cplx<T>::type;
-  const int B = (int)bd.d, Ns = (int)nsd.d;
-  const int m = L / r;
-  const int twstep = L / (Ns * r);
-  const int total = m * B;
-  for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-    int j, bl, q, k;
-    fdivmod(idx, bd, j, bl);
-    fdivmod(j, nsd, q, k);
-    C v[kMaxRadix];
-    for (int s = 0; s < r; ++s) {
-      C a = src[(j + s * m) * B + bl];
-      if (k && s) a = c_mul(a, tw_load<SIGN>(tw, s * k * twstep));
-      v[s] = a;
-    }
-    const int base = q * Ns * r + k;
-    for (int o = 0; o < r; ++o) {
-      C acc = v[0];
-      int t = 0;  // (s * o) mod r, stepped without a divide
-      for (int s = 1; s < r; ++s) {
-        t += o;
-        if (t >= r) t -= r;
-        acc = c_add(acc, c_mul(v[s], tw_load<SIGN>(tw, t * m)));
-      }
-      dst[(base + o * Ns) * B + bl] = acc;
+      for (int s = 0; s < R; ++s) dst[(base + s * Ns) * B + bl] = v[s];
     }
   }
 }
@@ -338,7 +404,10 @@ inline bool reg_fft_length(int n) { return n == 32 || n == 64 || n == 128 || n =
 // Returns the buffer that holds the result.  Ends with __syncthreads().  RN > 0
 // selects the register-resident transform of length RN (in place in `a`);
 // kernels are instantiated per RN so that the register cost of that path
-// never lands on the shared-memory one.
+// never lands on the shared-memory one.  For the same reason the double-float
+// passes of radix 7, 11 and 13 are in the instantiation RN = -1 only (plans
+// with such a factor; with them in every kernel a 96^3 grid's x and y kernels
+// took 10 to 20 % longer).
 template <typename T, int SIGN, int RN = 0>
 __device__ typename Cplx<T>::type *fft_tile(typename Cplx<T>::type *a, typename Cplx<T>::type *b,
                                             const FastDiv &bd, const FftPlan &p) {
@@ -359,7 +428,13 @@ __device__ typename Cplx<T>::type *fft_tile(typename Cplx<T>::type *a, typename 
       case 4: fft_pass<T, SIGN, 4>(src, dst, bd, p.n, nsd, tw); break;
       case 5: fft_pass<T, SIGN, 5>(src, dst, bd, p.n, nsd, tw); break;
       case 8: fft_pass<T, SIGN, 8>(src, dst, bd, p.n, nsd, tw); break;
-      default: fft_pass_generic<T, SIGN>(src, dst, bd, p.n, nsd, r, tw); break;
+      default:
+        if constexpr (RN < 0 || !std::is_same<T, dfl>::value) {
+          if (r == 7) fft_pass<T, SIGN, 7>(src, dst, bd, p.n, nsd, tw);
+          else if (r == 11) fft_pass<T, SIGN, 11>(src, dst, bd, p.n, nsd, tw);
+          else fft_pass<T, SIGN, 13>(src, dst, bd, p.n, nsd, tw);
+        }
+        break;
     }
     __syncthreads();
     C *t = src;

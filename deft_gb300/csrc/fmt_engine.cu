@@ -277,7 +277,10 @@ __device__ __forceinline__ void unpack_r2c_store(const typename Cplx<T>::type *r
 // registers a thread.  The shared-memory ones set no minimum, which leaves
 // ptxas its own occupancy heuristic (40-64 registers); a minimum of one block
 // let it double their registers and cost a third of their speed.
-#define DEFT_FFT_BOUNDS(RN) __launch_bounds__(kThreads, (RN) > 0 ? 2 : 0)
+// The instantiations with the prime radices 7, 11 and 13 in FP64 or
+// double-float are held to 80 registers (three blocks).
+#define DEFT_FFT_BOUNDS(RN) \
+  __launch_bounds__(kThreads, (RN) > 0 ? 2 : (sizeof(T) == 4 || (is_df<T> && (RN) == 0) ? 0 : 3))
 
 // Real fields -> half-complex along z.  grid.x = pair tiles, grid.y = field.
 template <typename T, int RN = 0>
@@ -305,8 +308,8 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_r2c(const double *__restrict__ in,
 }
 
 // Half-complex along z -> real fields.  grid.x = pair tiles, grid.y = field.
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_z_c2r(const typename Cplx<T>::type *__restrict__ in,
+template <typename T, int RN = 0>
+__global__ void DEFT_FFT_BOUNDS(RN) k_z_c2r(const typename Cplx<T>::type *__restrict__ in,
                                                     double *__restrict__ out, Geom g, FftPlan pz,
                                                     FastDiv fP, double s) {
   const int P = (int)fP.d;
@@ -318,7 +321,7 @@ __global__ void __launch_bounds__(kThreads) k_z_c2r(const typename Cplx<T>::type
   in += (size_t)blockIdx.y * g.NC;
   out += (size_t)blockIdx.y * g.NR;
   pack_c2r<T>(in, buf0, g, p0, P);
-  C *res = fft_tile<T, +1>(buf0, buf1, fP, pz);
+  C *res = fft_tile<T, +1, RN>(buf0, buf1, fP, pz);
   #pragma unroll 4
   for (int idx = threadIdx.x; idx < 2 * P * g.Nz; idx += blockDim.x) {
     int ll, z;
@@ -364,8 +367,8 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_y_fft(typename Cplx<T>::type *data, Geom g
 }
 
 // Plain FFT along x (stride Ny*NzH), optional scale.  grid.x = line tiles.
-template <typename T, int SIGN>
-__global__ void __launch_bounds__(kThreads) k_x_fft(typename Cplx<T>::type *data, Geom g,
+template <typename T, int SIGN, int RN = 0>
+__global__ void DEFT_FFT_BOUNDS(RN) k_x_fft(typename Cplx<T>::type *data, Geom g,
                                                     FftPlan px, FastDiv fB, T s) {
   const int B = (int)fB.d;
   using C = typename Cplx<T>::type;
@@ -381,7 +384,7 @@ __global__ void __launch_bounds__(kThreads) k_x_fft(typename Cplx<T>::type *data
     j += j0;
     buf0[idx] = j < J ? data[(size_t)e * J + j] : C{0, 0};
   }
-  C *res = fft_tile<T, SIGN>(buf0, buf1, fB, px);
+  C *res = fft_tile<T, SIGN, RN>(buf0, buf1, fB, px);
   #pragma unroll 4
   for (int idx = threadIdx.x; idx < g.Nx * B; idx += blockDim.x) {
     int e, j;
@@ -1182,7 +1185,7 @@ template <typename T, bool GRAD, int RN = 0, typename R = double>
 __global__ void __launch_bounds__(kThreads,
                                   RN > 0 ? 2
                                          : (sizeof(T) == 4 ? DEFT_Z_PHI_MIN_BLOCKS
-                                                           : (is_df<T> ? 2 : 0)))
+                                                           : (is_df<T> ? 3 : 0)))
     k_z_phi(typename Cplx<T>::type *S5,
                                                     const R *__restrict__ n,
                                                     const R *__restrict__ V, Geom g,
@@ -2463,9 +2466,15 @@ bool factorize(int n, FftPlan &p) {
   int k = 0;
   p.n = n;
   p.reg = 0;
-  while (n % 8 == 0 && k < kMaxPasses) { p.radix[k++] = 8; n /= 8; }
-  while (n % 4 == 0 && k < kMaxPasses) { p.radix[k++] = 4; n /= 4; }
-  while (n % 2 == 0 && k < kMaxPasses) { p.radix[k++] = 2; n /= 2; }
+  int e = 0;
+  while (n % 2 == 0) { e++; n /= 2; }
+  // eights, then fours; a lone radix-2 pass moves every element for one
+  // addition, so 8 x 2 becomes 4 x 4 (x convolutions of an 80^3 grid 60 -> 54
+  // us, Phi at 128^3 297 -> 287)
+  const int eights = e / 3 - (e % 3 == 1 && e > 1 ? 1 : 0);
+  for (int i = 0; i < eights; i++, e -= 3) p.radix[k++] = 8;
+  for (; e >= 2; e -= 2) p.radix[k++] = 4;
+  if (e) p.radix[k++] = 2;
   const int primes[] = {3, 5, 7, 11, 13};
   for (int q : primes)
     while (n % q == 0 && k < kMaxPasses) { p.radix[k++] = q; n /= q; }
@@ -2547,6 +2556,17 @@ void finish_tiles(Tiles &t, const Geom &g, size_t cs) {
 
 // Built-in rule: the widest tiles within `budget` bytes of shared memory (at
 // most 16 columns / pairs), evened out over the lines; overrides from `ov`.
+// The FP64 and double-float kernels (16-byte elements) are issue-bound, so
+// their z and x-convolution tiles are as wide as one round of the block's 256
+// threads takes in a pass, and no wider than leaves every SM a block:
+//   Phi: 5 P lines of Nz / 8 butterflies (128^3: 3 pairs, 256^3: 2 pairs 2480
+//     us against 2690 with 1; 96^3: 4 pairs 151 us against 174 with 5; 32^3:
+//     3 pairs 23.5 us against 34.8 with 15)
+//   one-field z kernels: an odd count near 1100 / Nz (96^3: 11, r2c 23.8 us
+//     against 26.2 with 15; 128^3: 9, 46 against 55; 64^3: 7, 13.6 against 16)
+//   x convolutions: forward 256 / (Nx / smallest radix) columns (96^3: 8, 59 us
+//     against 65 with 16), adjoint four (96^3 63 us against 76 with 6, 77^3 61
+//     against 71 with 7).
 Tiles make_tiles(const Geom &g, size_t cs, size_t budget, const TileChoice *ov = nullptr) {
   Tiles t;
   const int pairs = (g.lines + 1) / 2;
@@ -2560,6 +2580,21 @@ Tiles make_tiles(const Geom &g, size_t cs, size_t budget, const TileChoice *ov =
   int pm = cap(budget / (10 * (size_t)g.Nz * cs), 15);
   if (pm < 1) pm = 1;
   if (pm > 1 && pm % 2 == 0) pm -= 1;  // odd: conflict-free z-strided shared accesses
+  if (cs == 16) {
+    constexpr int kSms = 152;
+    auto least = [](int a, int b) { return a < b ? a : b; };
+    auto most = [](int a, int b) { return a > b ? a : b; };
+    const int fit = cap(budget / (10 * (size_t)g.Nz * cs), 15);
+    pm = most(1, least(most(fit, g.Nz > 192 ? 2 : 1), least((2 * 409 / g.Nz + 1) / 2, most(1, pairs / kSms))));
+    if (10 * (size_t)g.Nz * pm * cs > 200 * 1024) pm = 1;
+    t.Pz = most(1, least(t.Pz, least(1100 / g.Nz, most(2, pairs / (2 * kSms))) | 1));
+    int rmin = 8;
+    FftPlan px;
+    if (factorize(g.Nx, px))
+      for (int i = 0; i < px.npass; i++) rmin = least(rmin, px.radix[i]);
+    t.Bxf = least(t.Bxf, most(4, 256 * rmin / g.Nx));
+    t.Bxc = least(t.Bxc, 4);
+  }
   t.Pphi = pm < pairs ? pm : pairs;
   if (ov) {
     if (ov->By > 0) t.By = ov->By < g.NzH ? ov->By : g.NzH;
@@ -2623,8 +2658,9 @@ const char *const kKernelNames[kNumKernels] = {
     "diag_precond", "precond_dots", "newton_update", "device_control", "struct_pc"};
 
 // Calls f(std::integral_constant<int, RN>()) with RN = the plan's length
-// when it is an FP32 plan marked for the register-resident transform, else
-// RN = 0 (shared-memory passes): picks the kernel instantiation to launch.
+// when it is an FP32 plan marked for the register-resident transform, RN = -1
+// for a double-float plan with a radix of 7, 11 or 13, else RN = 0
+// (shared-memory passes): picks the kernel instantiation to launch.
 template <typename T, typename F> void with_rn(const FftPlan &p, F &&f) {
   if constexpr (sizeof(T) == 4) {
     if (p.reg) {
@@ -2635,6 +2671,12 @@ template <typename T, typename F> void with_rn(const FftPlan &p, F &&f) {
         case 256: f(std::integral_constant<int, 256>()); return;
         default: break;
       }
+    }
+  }
+  if constexpr (is_df<T>) {
+    if (plan_has_prime(p)) {
+      f(std::integral_constant<int, -1>());
+      return;
     }
   }
   f(std::integral_constant<int, 0>());
@@ -2908,20 +2950,25 @@ class EngineImpl {
     set_smem(k_z_phi<double, false>, t64.smem_phi);
     set_smem(k_z_phi<double, true>, t64.smem_phi);
     set_smem(k_z_grad<double>, t64.smem_z);
-    set_smem(k_z_r2c<dfl>, t64.smem_z);
-    set_smem(k_x_fft<dfl, -1>, t64.smem_x2);
-    set_smem(k_x_fft<dfl, +1>, t64.smem_x2);
-    set_smem(k_z_c2r<dfl>, t64.smem_z);
     set_smem(k_x_fft<float, -1>, t32.smem_x2);
     set_smem(k_x_fft<float, +1>, t32.smem_x2);
     set_smem(k_z_c2r<float>, t32.smem_z);
-    set_smem(k_y_fft<dfl, -1>, t64.smem_y);
-    set_smem(k_y_fft<dfl, +1>, t64.smem_y);
-    set_smem(k_x_conv_fwd<dfl>, t64.smem_xf);
-    set_smem(k_x_conv_adj<dfl>, t64.smem_xc);
-    set_smem(k_z_phi<dfl, false>, t64.smem_phi);
-    set_smem(k_z_phi<dfl, true>, t64.smem_phi);
-    set_smem(k_z_grad<dfl>, t64.smem_z);
+    auto smemd = [&](auto rn) {
+      constexpr int RN = decltype(rn)::value;
+      set_smem(k_z_r2c<dfl, RN>, t64.smem_z);
+      set_smem(k_z_c2r<dfl, RN>, t64.smem_z);
+      set_smem(k_x_fft<dfl, -1, RN>, t64.smem_x2);
+      set_smem(k_x_fft<dfl, +1, RN>, t64.smem_x2);
+      set_smem(k_y_fft<dfl, -1, RN>, t64.smem_y);
+      set_smem(k_y_fft<dfl, +1, RN>, t64.smem_y);
+      set_smem(k_x_conv_fwd<dfl, RN>, t64.smem_xf);
+      set_smem(k_x_conv_adj<dfl, RN>, t64.smem_xc);
+      set_smem(k_z_phi<dfl, false, RN>, t64.smem_phi);
+      set_smem(k_z_phi<dfl, true, RN>, t64.smem_phi);
+      set_smem(k_z_grad<dfl, RN>, t64.smem_z);
+    };
+    smemd(std::integral_constant<int, 0>());
+    smemd(std::integral_constant<int, -1>());
     {
       const char *ev = getenv("DEFT_FP64_TRANSFORMS");
       df_on = !(ev && !strcmp(ev, "fp64"));
@@ -3894,8 +3941,10 @@ int Engine::fft(const double *in, double2 *out, Arith a) {
     e.z_r2c_spec0<dfl>(in);
     e.y_fft<dfl>(w, 1, -1);
     e.pre(kK_x_fft);
-    k_x_fft<dfl, -1><<<e.x_tiles(e.t64.Bx), kThreads, e.t64.smem_x2, e.stream>>>(
-        w, e.g, e.pxd, e.t64.fBx, dfl(e.g.dV));
+    with_rn<dfl>(e.pxd, [&](auto rn) {
+      k_x_fft<dfl, -1, decltype(rn)::value><<<e.x_tiles(e.t64.Bx), kThreads, e.t64.smem_x2,
+                                              e.stream>>>(w, e.g, e.pxd, e.t64.fBx, dfl(e.g.dV));
+    });
     e.post(kK_x_fft);
     k_c_df2d<<<e.dot_blocks, kThreads, 0, e.stream>>>(w, out, e.g.NC);
     return e.check("fft");
@@ -3932,13 +3981,18 @@ int Engine::ifft(const double2 *in, double *out, Arith a) {
     dfc *w = reinterpret_cast<dfc *>(e.S0);
     k_c_d2df<<<e.dot_blocks, kThreads, 0, e.stream>>>(in, w, e.g.NC);
     e.pre(kK_x_fft);
-    k_x_fft<dfl, +1><<<e.x_tiles(e.t64.Bx), kThreads, e.t64.smem_x2, e.stream>>>(
-        w, e.g, e.pxd, e.t64.fBx, dfl(1));
+    with_rn<dfl>(e.pxd, [&](auto rn) {
+      k_x_fft<dfl, +1, decltype(rn)::value><<<e.x_tiles(e.t64.Bx), kThreads, e.t64.smem_x2,
+                                              e.stream>>>(w, e.g, e.pxd, e.t64.fBx, dfl(1));
+    });
     e.post(kK_x_fft);
     e.y_fft<dfl>(w, 1, +1);
     e.pre(kK_z_c2r);
-    k_z_c2r<dfl><<<dim3(e.pairs_tiles(e.t64.Pz), 1), kThreads, e.t64.smem_z, e.stream>>>(
-        w, out, e.g, e.pzd, e.t64.fPz, 1.0 / e.g.vol);
+    with_rn<dfl>(e.pzd, [&](auto rn) {
+      k_z_c2r<dfl, decltype(rn)::value><<<dim3(e.pairs_tiles(e.t64.Pz), 1), kThreads,
+                                          e.t64.smem_z, e.stream>>>(w, out, e.g, e.pzd,
+                                                                    e.t64.fPz, 1.0 / e.g.vol);
+    });
     e.post(kK_z_c2r);
     return e.check("ifft");
   }
@@ -3969,8 +4023,11 @@ int Engine::weighted(const FmtSpec &f, const double *n, double *out5, Arith a) {
   if (a == kArithDF && e.df_on) {
     if (e.upload_args(f) || e.ensure_table<dfl>(f.R) || e.forward_weighted<dfl>(f, n)) return -1;
     e.pre(kK_z_c2r);
-    k_z_c2r<dfl><<<dim3(e.pairs_tiles(e.t64.Pz), 5), kThreads, e.t64.smem_z, e.stream>>>(
-        e.spec5<dfl>(), out5, e.g, e.pzd, e.t64.fPz, 1.0);
+    with_rn<dfl>(e.pzd, [&](auto rn) {
+      k_z_c2r<dfl, decltype(rn)::value><<<dim3(e.pairs_tiles(e.t64.Pz), 5), kThreads,
+                                          e.t64.smem_z, e.stream>>>(e.spec5<dfl>(), out5, e.g,
+                                                                    e.pzd, e.t64.fPz, 1.0);
+    });
     e.post(kK_z_c2r);
     return e.check("weighted");
   }

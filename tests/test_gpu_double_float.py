@@ -1,8 +1,8 @@
 """The FP64 form's double-float kernels against the FP64 oracle where their
 branches meet: Phi in every density regime (dilute fluids, the series below
 n3 = 1/32 and 1/16, dense fluids, empty walls) for each hard-sphere kind, and
-the register-resident x and y transforms at the lengths they take, with odd
-and mixed companions.
+the x and y transforms at the lengths their register form takes and at odd
+and prime-factor lengths.
 
 Tolerances.  A double-float operation rounds at 2^-47 or better and Phi's
 longest chains are some tens of them: 2^-42 of a partial's largest term.  The
@@ -65,10 +65,11 @@ def test_phi_walls(ctx, oracle_mod, kind):
 
 
 @pytest.mark.parametrize("N", [(32, 32, 32), (64, 32, 15), (32, 64, 9), (128, 32, 6), (32, 128, 7),
-                               (256, 32, 4), (32, 256, 4), (33, 64, 10), (64, 30, 11)])
-def test_register_transforms(ctx, oracle_mod, N):
+                               (256, 32, 4), (32, 256, 4), (33, 64, 10), (64, 30, 11),
+                               (26, 49, 22), (143, 16, 7), (16, 77, 169)])
+def test_transform_lengths(ctx, oracle_mod, N):
     """Lengths 32 to 256 along x and y (and neighbours that are not), columns
-    that do not fill a group."""
+    that do not fill a group, prime factors 7, 11 and 13 on each axis."""
     lat = np.array([[0.2 * N[0], 0.1, 0.0], [0.0, 0.2 * N[1], 0.2], [0.3, 0.0, 0.25 * N[2]]])
     rng = np.random.default_rng(sum(N))
     n = 0.2 / (4 * math.pi / 3) * (1 + 0.2 * rng.standard_normal(N)).clip(0.1)
