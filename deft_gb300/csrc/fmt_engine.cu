@@ -143,27 +143,71 @@ __device__ __forceinline__ bool nonzero(double x) {
 }
 __device__ __forceinline__ bool nonzero(float x) { return x != 0.f; }
 
-// Deterministic block reduction of K doubles; thread 0 gets the sums.
+// Sums K doubles over a warp: at each of the first steps a lane keeps half of
+// the values it still holds and sends the other half away, so six values
+// take eight FP64 additions a lane instead of thirty (a warp-wide addition
+// occupies a scheduler's FP64 pipe for 64 cycles).  On return v[0] holds the
+// sum of value warp_sum_slot<K>(lane) (-1: padding).
+template <int K, int O, typename A>
+__device__ __forceinline__ void warp_sum_step(A &v, int lane) {
+  if constexpr (O > 0) {
+    if constexpr (K == 1) {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+      warp_sum_step<1, O / 2>(v, lane);
+    } else {
+      constexpr int H = (K + 1) / 2;
+      const bool up = lane & O;
+#pragma unroll
+      for (int i = 0; i < H; i++) {
+        const double hi = H + i < K ? v[H + i < K ? H + i : 0] : 0.0;
+        const double send = up ? v[i] : hi;
+        v[i] = (up ? hi : v[i]) + __shfl_xor_sync(0xffffffffu, send, O);
+      }
+      warp_sum_step<H, O / 2>(v, lane);
+    }
+  }
+}
+template <int K, int O = 16> __device__ __forceinline__ int warp_sum_slot(int lane) {
+  if constexpr (K == 1 || O == 0) {
+    return 0;
+  } else {
+    constexpr int H = (K + 1) / 2;
+    const int s = warp_sum_slot<H, O / 2>(lane);
+    const int t = s + ((lane & O) ? H : 0);
+    return s >= 0 && t < K ? t : -1;
+  }
+}
+// Lanes that share a slot's sum differ in the low bits only: one writes it.
+template <int K> __host__ __device__ constexpr int warp_sum_same() {
+  int k = K, o = 32;
+  while (k > 1) {
+    k = (k + 1) / 2;
+    o /= 2;
+  }
+  return o;  // lanes per slot
+}
+template <int K>
+__device__ __forceinline__ void warp_sum_store(double (&v)[K], double *dst /* K */) {
+  const int lane = threadIdx.x & 31;
+  warp_sum_step<K, 16>(v, lane);
+  const int slot = warp_sum_slot<K>(lane);
+  if (slot >= 0 && lane % warp_sum_same<K>() == 0) dst[slot] = v[0];
+}
+
+// Deterministic block reduction of K doubles; thread 0 gets the sums (lane k
+// of the first warp adds the warps' sums of value k, in order).
 template <int K>
 __device__ void block_reduce(double (&v)[K], double *smem /* 32*K */) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    double x = v[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    v[k] = x;
-  }
-  if (lane == 0)
-    for (int k = 0; k < K; k++) smem[warp * K + k] = v[k];
+  warp_sum_store<K>(v, smem + warp * K);
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (warp == 0) {
     const int nw = (blockDim.x + 31) >> 5;
-    for (int k = 0; k < K; k++) {
-      double s = 0;
-      for (int w = 0; w < nw; w++) s += smem[w * K + k];
-      v[k] = s;
-    }
+    double s = 0;
+    if (lane < K)
+      for (int w = 0; w < nw; w++) s += smem[w * K + lane];
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = __shfl_sync(0xffffffffu, s, k);
   }
 }
 
@@ -174,22 +218,25 @@ template <typename T, typename LA>
 __device__ void block_reduce_terms(T (&t)[6], const LA &la, double *red /* 32*6 */,
                                    double *partials) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if constexpr (sizeof(T) == 8) {
+    warp_sum_store<6>(t, red + warp * 6);
+  } else {
 #pragma unroll
-  for (int k = 0; k < 6; k++) {
-    T x = t[k];
+    for (int k = 0; k < 6; k++) {
+      T x = t[k];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) red[warp * 6 + k] = double(x);
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (lane == 0) red[warp * 6 + k] = double(x);
+    }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const double scale[6] = {la.kT, la.kT, la.kT, la.kT, la.mu, 1.0};
+  if (threadIdx.x < 6) {
+    const int k = threadIdx.x;
+    const double scale = k < 4 ? la.kT : k == 4 ? la.mu : 1.0;
     const int nw = (blockDim.x + 31) >> 5;
-    for (int k = 0; k < 6; k++) {
-      double sum = 0;
-      for (int w = 0; w < nw; w++) sum += red[w * 6 + k];
-      partials[(size_t)blockIdx.x * 6 + k] = scale[k] * sum;
-    }
+    double sum = 0;
+    for (int w = 0; w < nw; w++) sum += red[w * 6 + k];
+    partials[(size_t)blockIdx.x * 6 + k] = scale * sum;
   }
 }
 
@@ -1948,61 +1995,49 @@ __global__ void __launch_bounds__(kThreads) k_local_energy(const double *__restr
     for (int t = 0; t < kNumTerms; t++) partials[(size_t)blockIdx.x * kNumTerms + t] = acc[t];
 }
 
-// Sums per-block energy partials in a fixed order: out[t] = dV sum, out[6] = E.
-// One block (a 1024-thread block measured slower: 27 vs 18 us at 128^3).
+// Energy terms (out[t] = dV times the sum of the blocks' partials, t < 6, and
+// out[6] = their total) and, with dk > 0, the gradient dot products of k_z_grad
+// (out[8..8+dk)), each summed in a fixed order.  A block per sum (the FP64
+// pipe of one SM, two lanes wide, took 91 us for the 16384 x 6 partials of a
+// 256^3 evaluation and 13 us at 128^3); the last to finish forms the total.
+// A single block (counter may be null) takes the sums one after another.
 constexpr int kReduceThreads = kThreads;
-// Energy terms (out[0..6), total in out[6]) and, with dk > 0, the gradient
-// dot products of k_z_grad (out[8..8+dk)), both summed in block order.
-__global__ void k_reduce_terms(const double *partials, int nblk, double dV, double *out,
-                               const double *dpart = nullptr, int dk = 0, int dblk = 0) {
-  __shared__ double red[32 * kNumTerms];
-  double acc[kNumTerms] = {0, 0, 0, 0, 0, 0};
-  // four blocks' partials in flight per thread and step (one block is
-  // latency-bound on these loads), then the remainder; a fixed order
-  int b = threadIdx.x;
-  for (; b + 3 * (int)blockDim.x < nblk; b += 4 * blockDim.x) {
-    double v[4][kNumTerms];
+constexpr int kReduceBlocks = kNumTerms;
+__global__ void __launch_bounds__(kReduceThreads)
+    k_reduce_terms(const double *partials, int nblk, double dV, double *out,
+                   unsigned int *counter = nullptr, const double *dpart = nullptr, int dk = 0,
+                   int dblk = 0) {
+  __shared__ double red[32];
+  for (int t = blockIdx.x; t < kNumTerms + dk; t += gridDim.x) {
+    const bool term = t < kNumTerms;
+    const double *p = term ? partials + t : dpart + (t - kNumTerms);
+    const int n = term ? nblk : dblk, ld = term ? kNumTerms : 3;
+    double acc[1] = {0};
+    int b = threadIdx.x;
+    // four blocks' partials in flight per thread and step
+    for (; b + 3 * kReduceThreads < n; b += 4 * kReduceThreads) {
+      double v[4];
 #pragma unroll
-    for (int u = 0; u < 4; u++)
+      for (int u = 0; u < 4; u++) v[u] = p[(size_t)(b + u * kReduceThreads) * ld];
 #pragma unroll
-      for (int t = 0; t < kNumTerms; t++)
-        v[u][t] = partials[(size_t)(b + u * blockDim.x) * kNumTerms + t];
-#pragma unroll
-    for (int u = 0; u < 4; u++)
-#pragma unroll
-      for (int t = 0; t < kNumTerms; t++) acc[t] += v[u][t];
+      for (int u = 0; u < 4; u++) acc[0] += v[u];
+    }
+    for (; b < n; b += kReduceThreads) acc[0] += p[(size_t)b * ld];
+    __syncthreads();  // the previous sum's readers of red are done
+    block_reduce<1>(acc, red);
+    if (threadIdx.x == 0) {
+      if (term) out[t] = acc[0] * dV;
+      else out[8 + t - kNumTerms] = acc[0];
+    }
   }
-  for (; b < nblk; b += blockDim.x)
-    for (int t = 0; t < kNumTerms; t++) acc[t] += partials[(size_t)b * kNumTerms + t];
-  block_reduce<kNumTerms>(acc, red);
   if (threadIdx.x == 0) {
-    double E = 0;
-    for (int t = 0; t < kNumTerms; t++) {
-      out[t] = acc[t] * dV;
-      E += out[t];
+    __threadfence();
+    if (gridDim.x == 1 || atomicAdd(counter, 1u) == gridDim.x - 1) {
+      __threadfence();
+      const volatile double *o = out;  // pairwise: three dependent additions
+      out[kNumTerms] = (o[3] + o[4]) + ((o[1] + o[2]) + (o[0] + o[5]));
+      if (gridDim.x > 1) *counter = 0;
     }
-    out[kNumTerms] = E;
-  }
-  if (dk > 0) {
-    __syncthreads();
-    double d[3] = {0, 0, 0};
-    int b2 = threadIdx.x;
-    for (; b2 + 3 * (int)blockDim.x < dblk; b2 += 4 * blockDim.x) {
-      double v[4][3];
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-#pragma unroll
-        for (int t = 0; t < 3; t++) v[u][t] = dpart[(size_t)(b2 + u * blockDim.x) * 3 + t];
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-#pragma unroll
-        for (int t = 0; t < 3; t++) d[t] += v[u][t];
-    }
-    for (; b2 < dblk; b2 += blockDim.x)
-      for (int t = 0; t < 3; t++) d[t] += dpart[(size_t)b2 * 3 + t];
-    block_reduce<3>(d, red);
-    if (threadIdx.x == 0)
-      for (int t = 0; t < dk; t++) out[8 + t] = d[t];
   }
 }
 
@@ -3497,8 +3532,8 @@ class EngineImpl {
   // With gd, also the gradient dot products k_z_grad took (results[8..11)).
   void queue_energy(int nblk, int dk = 0, const double *dpart = nullptr, int gblk = 0) {
     pre(kK_reduce_terms);
-    k_reduce_terms<<<1, kReduceThreads, 0, stream>>>(partials, nblk, g.dV, results, dpart, dk,
-                                                      gblk);
+    k_reduce_terms<<<kReduceBlocks + dk, kReduceThreads, 0, stream>>>(
+        partials, nblk, g.dV, results, dot_counter, dpart, dk, gblk);
     post(kK_reduce_terms);
     if (!dev_only)
       cudaMemcpyAsync(results_host, results, sizeof(double) * (dk ? 11 : 8),
