@@ -111,8 +111,54 @@ __device__ __forceinline__ void df_m2(dfl e, dfl om, dfl l, dfl &P2, dfl &dP2, d
   }
 }
 
+// Whether the double-float formulas cover a point: 1 - n3 well inside (0, inf)
+// and the powers of n2, v inside FP32's range.
+__device__ __forceinline__ bool df_point_ok(dfl om, dfl n2, dfl v2, bool fluid) {
+  const float a = fabsf(n2.hi);
+  return om.hi > 0x1p-20f && om.hi < 0x1p20f && a < 1e9f && v2.hi < 1e18f &&
+         (a > 1e-9f || !fluid);
+}
+__device__ __forceinline__ dfl df_one_minus(dfl x) {
+  const dfl t = df_two_sum(1.0f, -x.hi);
+  return df_fast_two_sum(t.hi, t.lo - x.lo);
+}
+
+// S'' (wb_phi.cuh) with S and S' as df_S gives them.
+__device__ __forceinline__ dfl df_d2S(dfl n3, dfl om, dfl l) {
+  if (fabsf(n3.hi) < 0.03125f) {
+    auto c = [](int j) { return 2.0 * (j - 1) / (double(j + 1) * (j + 2)); };  // j (j-1) c_j
+    const float ef = n3.hi;
+    float d = 0.f;
+#pragma unroll
+    for (int j = 11; j > 6; j--) d = fmaf(d, ef, (float)c(j));
+    dfl s = df_scale(n3, d);
+#pragma unroll
+    for (int j = 6; j >= 2; j--) {
+      s = dfl(c(j)) + s;
+      if (j > 2) s = s * n3;
+    }
+    return -s;
+  }
+  const dfl ol = om * l, g = n3 + om * ol, dg = n3 - df_ldexp(ol, 2.0f);
+  const dfl ie = df_rcp(n3), ie2 = ie * ie, d2g = dfl(3) + df_ldexp(l, 2.0f);
+  return (d2g - df_ldexp(dg * ie, 4.0f) + df_scale(g * ie2, 6.0f)) * ie2;
+}
+
+// The third term's f3 without its constant (White Bear: S u^2, Rosenfeld: u^2)
+// and its derivative.
+__device__ __forceinline__ void df_S(dfl n3, dfl om, dfl l, dfl &S, dfl &dS) {
+  if (fabsf(n3.hi) < 0.03125f) {
+    df_S_series(n3, S, dS);
+  } else {
+    const dfl ol = om * l, g = n3 + om * ol, dg = n3 - df_ldexp(ol, 2.0f);
+    const dfl ie = df_rcp(n3), gi = g * ie, ie2 = ie * ie;
+    S = gi * ie;
+    dS = (dg - df_ldexp(gi, 2.0f)) * ie2;
+  }
+}
+
 // The FP64 formulas: p[3] = the sums' terms, d = c times the partials.
-__device__ __noinline__ void df_phi_fp64(const WbRadius &r, const DfPhiConst &k, double c,
+static __device__ __noinline__ void df_phi_fp64(const WbRadius &r, const DfPhiConst &k, double c,
                                          const dfl *w, double *p, dfl *d) {
   double phi[3], g[5];
   wb_phi<double>(r, to_double(w[0]), to_double(w[1]), to_double(w[2]), to_double(w[3]),
@@ -132,11 +178,8 @@ __device__ __forceinline__ void df_phi_point(const WbRadius &r, const DfPhiConst
                                              dfl (&d)[5]) {
   const dfl n3 = w[0], n2 = w[1];
   const dfl v2 = w[2] * w[2] + w[3] * w[3] + w[4] * w[4];
-  const dfl t = df_two_sum(1.0f, -n3.hi);
-  const dfl om = df_fast_two_sum(t.hi, t.lo - n3.lo);
-  const float an2 = fabsf(n2.hi);
-  if (!(om.hi > 0x1p-20f && om.hi < 0x1p20f && an2 < 1e9f && v2.hi < 1e18f &&
-        (an2 > 1e-9f || !fluid))) {
+  const dfl om = df_one_minus(n3);
+  if (!df_point_ok(om, n2, v2, fluid)) {
     dfl wl[5] = {w[0], w[1], w[2], w[3], w[4]}, dl[5];
     double p[3];
     df_phi_fp64(r, k, c, wl, p, dl);
@@ -154,14 +197,7 @@ __device__ __forceinline__ void df_phi_point(const WbRadius &r, const DfPhiConst
     df3 = df_ldexp(u2 * u, 2.0f);
   } else if (r.kind == kHsWhiteBear) {
     dfl S, dS;
-    if (fabsf(n3.hi) < 0.03125f) {
-      df_S_series(n3, S, dS);
-    } else {
-      const dfl ol = om * l, g = n3 + om * ol, dg = n3 - df_ldexp(ol, 2.0f);
-      const dfl ie = df_rcp(n3), gi = g * ie, ie2 = ie * ie;
-      S = gi * ie;
-      dS = (dg - df_ldexp(gi, 2.0f)) * ie2;
-    }
+    df_S(n3, om, l, S, dS);
     f3 = S * u2;
     df3 = (dS + df_ldexp(S * u, 2.0f)) * u2;
   } else {

@@ -84,6 +84,7 @@ __device__ __forceinline__ float d2f_small(double d) {
 // A real of the transforms' type from FP64 data.
 template <typename T> __device__ __forceinline__ T real_from(double d) { return T(d); }
 template <> __device__ __forceinline__ dfl real_from<dfl>(double d) { return df_from(d); }
+template <typename T> __device__ __forceinline__ T real_from(dfl d) { return T(d); }
 
 // Knuth's TwoSum: s + e == a + b exactly.
 __device__ __forceinline__ dfl df_two_sum(float a, float b) {
@@ -118,7 +119,6 @@ __device__ __forceinline__ bool operator==(dfl a, dfl b) { return a.hi == b.hi &
 __device__ __forceinline__ bool operator<(dfl a, dfl b) {
   return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo);
 }
-__device__ __forceinline__ dfl fabs(dfl a) { return a.hi < 0.f ? -a : a; }
 // Quotient by one correction step (the long division of Dekker 1971):
 // q1 = a.hi / b.hi in FP32, the remainder r = a - q1 b in double-float,
 // q = q1 + r.hi / b.hi; relative error about 2^-44.
@@ -145,7 +145,7 @@ struct tfl {
   float a, b, c;
   tfl() = default;
   __host__ __device__ constexpr tfl(float x, float y, float z) : a(x), b(y), c(z) {}
-  __host__ __device__ constexpr tfl(double d)
+  __host__ __device__ explicit constexpr tfl(double d)
       : a((float)d), b((float)(d - (double)(float)d)),
         c((float)((d - (double)(float)d) - (double)(float)(d - (double)(float)d))) {}
 };

@@ -20,6 +20,7 @@
 // The k-space weights (src/ReciprocalOperators.h:94-235) are evaluated
 // analytically once per (grid, R) into a table, with the convolution
 // normalisation dV/V folded in.
+#include "block_sum.cuh"
 #include "df_phi.cuh"
 #include "fft_smem.cuh"
 #include "fmt_engine.h"
@@ -143,74 +144,6 @@ __device__ __forceinline__ bool nonzero(double x) {
 }
 __device__ __forceinline__ bool nonzero(float x) { return x != 0.f; }
 
-// Sums K doubles over a warp: at each of the first steps a lane keeps half of
-// the values it still holds and sends the other half away, so six values
-// take eight FP64 additions a lane instead of thirty (a warp-wide addition
-// occupies a scheduler's FP64 pipe for 64 cycles).  On return v[0] holds the
-// sum of value warp_sum_slot<K>(lane) (-1: padding).
-template <int K, int O, typename A>
-__device__ __forceinline__ void warp_sum_step(A &v, int lane) {
-  if constexpr (O > 0) {
-    if constexpr (K == 1) {
-      v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
-      warp_sum_step<1, O / 2>(v, lane);
-    } else {
-      constexpr int H = (K + 1) / 2;
-      const bool up = lane & O;
-#pragma unroll
-      for (int i = 0; i < H; i++) {
-        const double hi = H + i < K ? v[H + i < K ? H + i : 0] : 0.0;
-        const double send = up ? v[i] : hi;
-        v[i] = (up ? hi : v[i]) + __shfl_xor_sync(0xffffffffu, send, O);
-      }
-      warp_sum_step<H, O / 2>(v, lane);
-    }
-  }
-}
-template <int K, int O = 16> __device__ __forceinline__ int warp_sum_slot(int lane) {
-  if constexpr (K == 1 || O == 0) {
-    return 0;
-  } else {
-    constexpr int H = (K + 1) / 2;
-    const int s = warp_sum_slot<H, O / 2>(lane);
-    const int t = s + ((lane & O) ? H : 0);
-    return s >= 0 && t < K ? t : -1;
-  }
-}
-// Lanes that share a slot's sum differ in the low bits only: one writes it.
-template <int K> __host__ __device__ constexpr int warp_sum_same() {
-  int k = K, o = 32;
-  while (k > 1) {
-    k = (k + 1) / 2;
-    o /= 2;
-  }
-  return o;  // lanes per slot
-}
-template <int K>
-__device__ __forceinline__ void warp_sum_store(double (&v)[K], double *dst /* K */) {
-  const int lane = threadIdx.x & 31;
-  warp_sum_step<K, 16>(v, lane);
-  const int slot = warp_sum_slot<K>(lane);
-  if (slot >= 0 && lane % warp_sum_same<K>() == 0) dst[slot] = v[0];
-}
-
-// Deterministic block reduction of K doubles; thread 0 gets the sums (lane k
-// of the first warp adds the warps' sums of value k, in order).
-template <int K>
-__device__ void block_reduce(double (&v)[K], double *smem /* 32*K */) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  warp_sum_store<K>(v, smem + warp * K);
-  __syncthreads();
-  if (warp == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    double s = 0;
-    if (lane < K)
-      for (int w = 0; w < nw; w++) s += smem[w * K + lane];
-#pragma unroll
-    for (int k = 0; k < K; k++) v[k] = __shfl_sync(0xffffffffu, s, k);
-  }
-}
-
 // Per-block energy partials of the six terms: warp sums in the kernel's
 // arithmetic type T (no FP64 work per thread in the FP32 kernels), then the
 // warps' sums in FP64 in a fixed order, scaled by kT (phi, ideal gas), mu, 1.
@@ -330,8 +263,8 @@ __device__ __forceinline__ void unpack_r2c_store(const typename Cplx<T>::type *r
   __launch_bounds__(kThreads, (RN) > 0 ? 2 : (sizeof(T) == 4 || (is_df<T> && (RN) == 0) ? 0 : 3))
 
 // Real fields -> half-complex along z.  grid.x = pair tiles, grid.y = field.
-template <typename T, int RN = 0>
-__global__ void DEFT_FFT_BOUNDS(RN) k_z_r2c(const double *__restrict__ in,
+template <typename T, int RN = 0, typename R = double>
+__global__ void DEFT_FFT_BOUNDS(RN) k_z_r2c(const R *__restrict__ in,
                                                     typename Cplx<T>::type *__restrict__ out,
                                                     Geom g, FftPlan pz, FastDiv fP, T s) {
   const int P = (int)fP.d;
@@ -354,10 +287,11 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_r2c(const double *__restrict__ in,
   unpack_r2c_store<T>(res, out, g, p0, P, s);
 }
 
-// Half-complex along z -> real fields.  grid.x = pair tiles, grid.y = field.
-template <typename T, int RN = 0>
+// Half-complex along z -> real fields (times s for FP64 ones).  grid.x = pair
+// tiles, grid.y = field.
+template <typename T, int RN = 0, typename R = double>
 __global__ void DEFT_FFT_BOUNDS(RN) k_z_c2r(const typename Cplx<T>::type *__restrict__ in,
-                                                    double *__restrict__ out, Geom g, FftPlan pz,
+                                                    R *__restrict__ out, Geom g, FftPlan pz,
                                                     FastDiv fP, double s) {
   const int P = (int)fP.d;
   using C = typename Cplx<T>::type;
@@ -376,7 +310,8 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_c2r(const typename Cplx<T>::type *__rest
     const int line = 2 * p0 + ll;
     if (line >= g.lines) continue;
     const C v = res[z * P + (ll >> 1)];
-    out[(size_t)line * g.Nz + z] = double((ll & 1) ? v.y : v.x) * s;
+    if constexpr (std::is_same<R, dfl>::value) out[(size_t)line * g.Nz + z] = (ll & 1) ? v.y : v.x;
+    else out[(size_t)line * g.Nz + z] = double((ll & 1) ? v.y : v.x) * s;
   }
 }
 
@@ -721,6 +656,157 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_x_conv_adj(
     fdivmod(idx, fB, e, j);
     j += j0;
     if (j < J) out[(size_t)e * J + j] = res[idx];
+  }
+}
+
+// Weight `a` of the set at k, applied to v (sgn = -1: its adjoint).  kx .. kz
+// are only formed for the patterns that read them.
+template <typename K>
+__device__ __forceinline__ dfc apply_weight(dfc v, const FieldWeights &fw, int a, int sgn,
+                                            size_t i, K k) {
+  const int p = fw.pat[a];
+  if (p == kWtScalar) {
+    if (i == 0) return dc_weight(v, fw.dc[a]);
+    const dfl w = fw.r0[a][i];
+    return dfc{v.x * w, v.y * w};
+  }
+  if (p < kWtDiag) {
+    dfl w = k(p - kWtVector) * fw.r0[a][i];
+    if (sgn < 0) w = -w;
+    return dfc{-(v.y * w), v.x * w};  // times +-i w
+  }
+  dfl w;
+  if (p < kWtXY) {
+    const dfl kc = k(p - kWtDiag);
+    w = fw.r0[a][i] + kc * kc * fw.r1[a][i];
+  } else {
+    w = k(p - kWtXY) * k((p - kWtXY + 1) % 3) * fw.r1[a][i];
+  }
+  return dfc{v.x * w, v.y * w};
+}
+
+// The set's weighted copies of one spectrum along x: x-FFT, then per field its
+// weight and an inverse x-FFT (three tiles of B lines, as k_x_conv_fwd).
+template <int RN = 0, typename T = dfl>
+__global__ void DEFT_FFT_BOUNDS(RN) k_x_fan_out(const dfc *__restrict__ in,
+                                                dfc *__restrict__ out, FieldWeights fw, int sgn,
+                                                Geom g, FftPlan px, FastDiv fB) {
+  const int B = (int)fB.d;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  dfc *bufA = reinterpret_cast<dfc *>(smem_raw);
+  dfc *bufB = bufA + g.Nx * B, *bufC = bufB + g.Nx * B;
+  const int J = g.Ny * g.NzH, j0 = blockIdx.x * B;
+#pragma unroll 4
+  for (int idx = threadIdx.x; idx < g.Nx * B; idx += blockDim.x) {
+    int e, j;
+    fdivmod(idx, fB, e, j);
+    j += j0;
+    bufA[idx] = j < J ? in[(size_t)e * J + j] : dfc{0, 0};
+  }
+  const dfc *R0 = fft_tile<dfl, -1, RN>(bufA, bufB, fB, px);
+  dfc *F1 = (R0 == bufA) ? bufB : bufA, *F2 = bufC;
+  for (int a = 0; a < fw.n; a++) {
+    for (int idx = threadIdx.x; idx < g.Nx * B; idx += blockDim.x) {
+      int e, j, y, z;
+      fdivmod(idx, fB, e, j);
+      j += j0;
+      fdivmod(j < J ? j : 0, g.fNzH, y, z);
+      F1[idx] = j < J ? apply_weight(R0[idx], fw, a, sgn, (size_t)e * J + j,
+                                     [&](int c) { return kcomp_t<dfl>(g, c, e, y, z); })
+                      : dfc{0, 0};
+    }
+    const dfc *res = fft_tile<dfl, +1, RN>(F1, F2, fB, px);
+    dfc *dst = out + (size_t)a * g.NC;
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < g.Nx * B; idx += blockDim.x) {
+      int e, j;
+      fdivmod(idx, fB, e, j);
+      j += j0;
+      if (j < J) dst[(size_t)e * J + j] = res[idx];
+    }
+    __syncthreads();
+  }
+}
+
+// The other direction: x-FFT of each field, its weight, the sum over the
+// fields (a third tile), inverse x-FFT of the sum.
+template <int RN = 0, typename T = dfl>
+__global__ void DEFT_FFT_BOUNDS(RN) k_x_fan_in(const dfc *__restrict__ in, dfc *__restrict__ out,
+                                               FieldWeights fw, int sgn, Geom g, FftPlan px,
+                                               FastDiv fB) {
+  const int B = (int)fB.d;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  dfc *bufA = reinterpret_cast<dfc *>(smem_raw);
+  dfc *bufB = bufA + g.Nx * B, *sum = bufB + g.Nx * B;
+  const int J = g.Ny * g.NzH, j0 = blockIdx.x * B;
+  for (int a = 0; a < fw.n; a++) {
+    const dfc *src = in + (size_t)a * g.NC;
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < g.Nx * B; idx += blockDim.x) {
+      int e, j;
+      fdivmod(idx, fB, e, j);
+      j += j0;
+      bufA[idx] = j < J ? src[(size_t)e * J + j] : dfc{0, 0};
+    }
+    const dfc *res = fft_tile<dfl, -1, RN>(bufA, bufB, fB, px);
+    for (int idx = threadIdx.x; idx < g.Nx * B; idx += blockDim.x) {
+      int e, j, y, z;
+      fdivmod(idx, fB, e, j);
+      j += j0;
+      fdivmod(j < J ? j : 0, g.fNzH, y, z);
+      dfc t = dfc{0, 0};
+      if (j < J)
+        t = apply_weight(res[idx], fw, a, sgn, (size_t)e * J + j,
+                         [&](int c) { return kcomp_t<dfl>(g, c, e, y, z); });
+      sum[idx] = a == 0 ? t : c_add(sum[idx], t);
+    }
+    __syncthreads();
+  }
+  const dfc *res = fft_tile<dfl, +1, RN>(sum, bufA, fB, px);
+#pragma unroll 4
+  for (int idx = threadIdx.x; idx < g.Nx * B; idx += blockDim.x) {
+    int e, j;
+    fdivmod(idx, fB, e, j);
+    j += j0;
+    if (j < J) out[(size_t)e * J + j] = res[idx];
+  }
+}
+
+// Radial part `kind` of a weight at every k of the half spectrum, times the
+// convolution's scale (formulas and thresholds of contact_math.cuh and
+// tensor.cu; the vector shell primes take their closed form above kR = 1e-5
+// on every axis).
+__global__ void k_radial_table(int kind, Geom g, double R, dfl *__restrict__ out) {
+  const double fp = 4 * M_PI;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.NC; i += gridDim.x * blockDim.x) {
+    int t, z, x, y;
+    fdivmod(i, g.fNzH, t, z);
+    fdivmod(t, g.fNy, x, y);
+    const double kx = kcomp(g, 0, x, y, z), ky = kcomp(g, 1, x, y, z), kz = kcomp(g, 2, x, y, z);
+    const double k2 = kx * kx + ky * ky + kz * kz, k = sqrt(k2);
+    const double smear = exp(-6.0 * k2 * g.dr * g.dr);
+    double w = 0;
+    if (kind == kRadStep || kind == kRadShell || kind == kRadVShell) {
+      double a, b, c;
+      weights_at(k2, R, g.dr, a, b, c);
+      w = kind == kRadStep ? a : kind == kRadShell ? b : c;
+    } else if (kind == kRadShell2R) {
+      double a, c;
+      weights_at(k2, 2 * R, g.dr, a, w, c);
+    } else if (kind == kRadGauss) {
+      w = exp(-0.5 * k2 * R * R);
+    } else {
+      const double q = k * R;
+      double s, c;
+      sincos(q, &s, &c);
+      if (kind == kRadShellPrime) w = q > 1e-5 ? smear * fp * (s / k + R * c) : 2 * fp * R;
+      else if (kind == kRadVShellPrime) w = q > 1e-5 ? smear * fp * R * s / k : fp * R * R;
+      else if (q > 0 && kind == kRadTensorA)
+        w = smear * fp * R * R * (s / q * (1 / (q * q) - 1.0 / 3) - c / (q * q));
+      else if (q > 0)
+        w = smear * fp * R * R / k2 * (s / q * (1 - 3 / (q * q)) + 3 * c / (q * q));
+    }
+    out[i] = df_from(w * g.scale);
   }
 }
 
@@ -1980,13 +2066,23 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) k_local_energy(const double *__restrict__ n,
                                                            const double *__restrict__ V, Geom g,
                                                            const LocalArgs *__restrict__ lap,
-                                                           double *partials) {
+                                                           double *partials,
+                                                           double *__restrict__ lnq) {
   const LocalArgs la = *lap;
   __shared__ double red[32 * kNumTerms];
   double acc[kNumTerms] = {0, 0, 0, 0, 0, 0};
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < g.NR; r += gridDim.x * blockDim.x) {
     const double nv = n[r];
-    if (la.terms & kTermIdeal) acc[3] += ideal_energy<T>(nv, la);
+    if (la.terms & kTermIdeal) {
+      if constexpr (is_df<T>) {
+        // by table, and kept for the gradient kernel of the same evaluation
+        const double lg = log_tab(nv * la.inv_nQ);
+        if (nonzero(nv)) acc[3] += la.kT * nv * (lg - 1.0);
+        if (lnq) lnq[r] = lg;
+      } else {
+        acc[3] += ideal_energy<T>(nv, la);
+      }
+    }
     if (la.terms & kTermMu) acc[4] += la.mu * nv;
     if (la.terms & kTermVext) acc[5] += V[r] * nv;
   }
@@ -2827,6 +2923,7 @@ class EngineImpl {
     cudaFree(hess);
     cudaFree(pc_table);
     cudaFree(lnq);
+    for (Radial &r : radials) cudaFree(r.tab);
     clear_graphs();
     cudaFree(la_dev);
     cudaFree(hloc);
@@ -3001,6 +3098,10 @@ class EngineImpl {
       set_smem(k_z_phi<dfl, false, RN>, t64.smem_phi);
       set_smem(k_z_phi<dfl, true, RN>, t64.smem_phi);
       set_smem(k_z_grad<dfl, RN>, t64.smem_z);
+      set_smem(k_z_r2c<dfl, RN, dfl>, t64.smem_z);
+      set_smem(k_z_c2r<dfl, RN, dfl>, t64.smem_z);
+      set_smem(k_x_fan_out<RN>, t64.smem_xf);
+      set_smem(k_x_fan_in<RN>, t64.smem_xf);
     };
     smemd(std::integral_constant<int, 0>());
     smemd(std::integral_constant<int, -1>());
@@ -3350,6 +3451,73 @@ class EngineImpl {
     post(kslot<T>(kK_z_r2c));
   }
 
+  // Sets of convolutions (Engine::fan_out, fan_in).
+  struct Radial {
+    dfl *tab = nullptr;
+    double R = -1;
+  };
+  Radial radials[kNumRadial];
+  const dfl *radial(int kind, double R) {
+    Radial &r = radials[kind];
+    if (!r.tab && alloc(&r.tab, sizeof(dfl) * (size_t)g.NC)) return nullptr;
+    if (r.R != R) {
+      const int blocks = (g.NC + kThreads - 1) / kThreads;
+      pre(kK_weight_table);
+      k_radial_table<<<blocks < 4096 ? blocks : 4096, kThreads, 0, stream>>>(kind, g, R, r.tab);
+      post(kK_weight_table);
+      if (check("weight table")) return nullptr;
+      r.R = R;
+    }
+    return r.tab;
+  }
+  // The z transform of nf real fields (FP64 or double-float) into spec.
+  template <typename R> void z_r2c_df(const R *in, dfc *spec, int nf) {
+    pre(kK_z_r2c);
+    with_rn<dfl>(pzd, [&](auto rn) {
+      k_z_r2c<dfl, decltype(rn)::value, R><<<dim3(pairs_tiles(t64.Pz), nf), kThreads, t64.smem_z,
+                                             stream>>>(in, spec, g, pzd, t64.fPz, dfl(1));
+    });
+    post(kK_z_r2c);
+  }
+  template <typename R> void z_c2r_df(const dfc *spec, R *out, int nf) {
+    pre(kK_z_c2r);
+    with_rn<dfl>(pzd, [&](auto rn) {
+      k_z_c2r<dfl, decltype(rn)::value, R><<<dim3(pairs_tiles(t64.Pz), nf), kThreads, t64.smem_z,
+                                             stream>>>(spec, out, g, pzd, t64.fPz, 1.0);
+    });
+    post(kK_z_c2r);
+  }
+  template <typename R> int spectrum(const R *in) {
+    z_r2c_df(in, spec0<dfl>(), 1);
+    y_fft<dfl>(spec0<dfl>(), 1, -1);
+    return check("spectrum");
+  }
+  int fan_out(const FieldWeights &w, int sgn, dfc *spec, dfl *out) {
+    pre(kK_x_conv_fwd);
+    with_rn<dfl>(pxd, [&](auto rn) {
+      k_x_fan_out<decltype(rn)::value><<<x_tiles(t64.Bxf), kThreads, t64.smem_xf, stream>>>(
+          spec0<dfl>(), spec, w, sgn, g, pxd, t64.fBxf);
+    });
+    post(kK_x_conv_fwd);
+    y_fft<dfl>(spec, w.n, +1);
+    z_c2r_df(spec, out, w.n);
+    return check("fan out");
+  }
+  template <typename R>
+  int fan_in(const FieldWeights &w, int sgn, const dfl *in, dfc *spec, R *out) {
+    z_r2c_df(in, spec, w.n);
+    y_fft<dfl>(spec, w.n, -1);
+    pre(kK_x_conv_adj);
+    with_rn<dfl>(pxd, [&](auto rn) {
+      k_x_fan_in<decltype(rn)::value><<<x_tiles(t64.Bxf), kThreads, t64.smem_xf, stream>>>(
+          spec, spec0<dfl>(), w, sgn, g, pxd, t64.fBxf);
+    });
+    post(kK_x_conv_adj);
+    y_fft<dfl>(spec0<dfl>(), 1, +1);
+    z_c2r_df(spec0<dfl>(), out, 1);
+    return check("fan in");
+  }
+
   template <typename T, typename R = double> int forward_weighted(const FmtSpec &f, const R *n) {
     const Tiles &t = tl<T>();
     z_r2c_spec0<T, R>(n);
@@ -3569,7 +3737,7 @@ class EngineImpl {
            double *E_host, double *terms_host, int kd = 0, const double *const *da = nullptr,
            const double *const *db = nullptr, double *dots_host = nullptr) {
     if ((f.terms & kTermHS) && ensure_table<T>(f.R)) return -1;
-    if (sizeof(T) != 4 && grad && (f.terms & kTermHS) && ensure_lnq()) return -1;
+    if (sizeof(T) != 4 && grad && (is_df<T> || (f.terms & kTermHS)) && ensure_lnq()) return -1;
     if (upload_args(f)) return -1;
     const GraphKey key =
         graph_key(grad ? 1 : 0, is_df<T> ? 9 : (int)sizeof(T), f, n, V, mask, grad, kd, da, db);
@@ -3687,7 +3855,8 @@ class EngineImpl {
       nblk = 4 * 152;
       if constexpr (r64) {
         pre(kslot<T>(kK_local_energy));
-        k_local_energy<Acc<T>><<<nblk, kThreads, 0, stream>>>(n, V, g, la_dev, partials);
+        k_local_energy<T><<<nblk, kThreads, 0, stream>>>(n, V, g, la_dev, partials,
+                                                         grad ? lnq_for<T>(f) : nullptr);
         post(kslot<T>(kK_local_energy));
       } else {
         err = "FP32 vectors need the hard-sphere term";
@@ -3709,7 +3878,7 @@ class EngineImpl {
         with_rn<T>(plan<T>(2), [&](auto rn) {
           k_z_grad<T, decltype(rn)::value><<<pairs_tiles(t.Pz), kThreads, t.smem_z, stream>>>(
               spec0<T>(), n, V, mask, grad, g, plan<T>(2), t.fPz, la_dev, gd ? *gd : GradDots{},
-              (f.terms & kTermHS) ? lnq_for<T>(f) : nullptr);
+              lnq_for<T>(f));
         });
       } else {
         err = "FP32 vectors need the warp z transforms";
@@ -3826,7 +3995,9 @@ class EngineImpl {
   double *lnq = nullptr;
   int ensure_lnq() { return lnq ? 0 : alloc(&lnq, sizeof(double) * (size_t)g.NR); }
   template <typename T> double *lnq_for(const FmtSpec &f) const {
-    return (sizeof(T) != 4 && (f.terms & kTermIdeal)) ? lnq : nullptr;
+    return (sizeof(T) != 4 && (f.terms & kTermIdeal) && (is_df<T> || (f.terms & kTermHS)))
+               ? lnq
+               : nullptr;
   }
   float *pc_table = nullptr;  // P(k) / N of the structure preconditioner
   LocalArgs pc_table_la{};    // the parameters it was made for
@@ -4042,6 +4213,20 @@ int Engine::ifft(const double2 *in, double *out, Arith a) {
       e.S0, out, e.g, e.pz, e.t64.fPz, 1.0 / e.g.vol);
     e.post(kK_z_c2r);
   return e.check("ifft");
+}
+
+bool Engine::df_on() const { return impl_->df_on; }
+const dfl *Engine::radial(int kind, double R) { return impl_->radial(kind, R); }
+int Engine::spectrum(const double *in) { return impl_->spectrum(in); }
+int Engine::spectrum(const dfl *in) { return impl_->spectrum(in); }
+int Engine::fan_out(const FieldWeights &w, int sgn, dfc *spec, dfl *out) {
+  return impl_->fan_out(w, sgn, spec, out);
+}
+int Engine::fan_in(const FieldWeights &w, int sgn, const dfl *in, dfc *spec, double *out) {
+  return impl_->fan_in(w, sgn, in, spec, out);
+}
+int Engine::fan_in(const FieldWeights &w, int sgn, const dfl *in, dfc *spec, dfl *out) {
+  return impl_->fan_in(w, sgn, in, spec, out);
 }
 
 int Engine::weighted(const FmtSpec &f, const double *n, double *out5, Arith a) {
@@ -4667,7 +4852,7 @@ int noalloc_energy_grad(const GridSpec &s, const FmtSpec &f, const double *n, co
                                                               t.f5Bxc, la_dev);
     k_y_fft<double, +1><<<ygrid1, kThreads, t.smem_y, stream>>>(S0, g, py, t.fBy);
   } else {
-    k_local_energy<double><<<nblk, kThreads, 0, stream>>>(n, V, g, la_dev, partials);
+    k_local_energy<double><<<nblk, kThreads, 0, stream>>>(n, V, g, la_dev, partials, nullptr);
   }
   k_z_grad<double><<<ptiles_z, kThreads, t.smem_z, stream>>>(S0, n, V, mask, grad, g, pz, t.fPz,
                                                              la_dev, GradDots{}, nullptr);

@@ -7,6 +7,7 @@
 
 #include <cuda_runtime.h>
 
+#include "dfloat.cuh"
 #include "fastdiv.cuh"
 
 #include <string>
@@ -77,6 +78,40 @@ struct TileChoice {
   int radix[3][8] = {};  // axes x, y, z
 };
 
+// Radial parts of the convolution weights at |k|, as functions of a length R
+// (dV / V, the scale of a convolution, folded in by Engine::radial).
+enum RadialKind {
+  kRadStep,         // step theta(R - r)
+  kRadShell,        // shell delta(R - r)
+  kRadVShell,       // vector shells: weight i k_c times this
+  kRadShellPrime,   // -shell'
+  kRadVShellPrime,  // vector shell primes: i k_c times this
+  kRadShell2R,      // shell of radius 2 R
+  kRadGauss,        // exp(-k^2 R^2 / 2), without the smearing
+  kRadTensorA,      // tensor shells: xx = this + k_x^2 (kRadTensorB), xy = k_x k_y (kRadTensorB)
+  kRadTensorB,
+  kNumRadial
+};
+
+// A set of up to eleven k-space weights built from radial tables: field a's
+// weight is r0 (real, DC value dc at k = 0), i k_c r0 (vector), r0 + k_c^2 r1 or
+// k_p k_q r1 (tensor; 0 at k = 0).
+constexpr int kMaxWeights = 11;
+enum WeightPattern { kWtScalar = 0, kWtVector = 1, kWtDiag = 4, kWtXY = 7, kWtYZ = 8, kWtZX = 9 };
+struct FieldWeights {
+  int n = 0;
+  int pat[kMaxWeights];
+  const dfl *r0[kMaxWeights];
+  const dfl *r1[kMaxWeights];
+  double dc[kMaxWeights];
+  void add(int p, const dfl *a, const dfl *b = nullptr, double d = 0) {
+    pat[n] = p;
+    r0[n] = a;
+    r1[n] = b;
+    dc[n++] = d;
+  }
+};
+
 // The bulk density in equilibrium with the chemical-potential term mu
 // (integrand mu n) for hard-sphere kind hs (White Bear, Rosenfeld, mark II)
 // plus the ideal gas; 0 when there is none.  Host code.
@@ -117,6 +152,22 @@ class Engine {
   // n3, n2, n2x, n2y, n2z (5*NR reals): FP32 transforms when f is mixed,
   // else those of `a`.
   int weighted(const FmtSpec &f, const double *n, double *out5, Arith a = kArithFP64);
+
+  // Sets of convolutions in double-float arithmetic (df_on: the engine's
+  // double-float transforms are in use).  Fields are double-floats, NR each,
+  // one after another.  radial: a weight table, kept per (kind, R); nullptr on
+  // failure.  spectrum: the z and y transforms of a real field (the x axis is
+  // left to the convolutions).  fan_out: w.n weighted copies of that field,
+  // sgn = -1 for the adjoint weights (odd ones negated).  fan_in: the sum over
+  // w.n fields of their weighted transforms, transformed back (FP64 or
+  // double-float out).  spec: w.n NC complex scratch.
+  bool df_on() const;
+  const dfl *radial(int kind, double R);
+  int spectrum(const double *in);
+  int spectrum(const dfl *in);
+  int fan_out(const FieldWeights &w, int sgn, dfc *spec, dfl *out);
+  int fan_in(const FieldWeights &w, int sgn, const dfl *in, dfc *spec, double *out);
+  int fan_in(const FieldWeights &w, int sgn, const dfl *in, dfc *spec, dfl *out);
 
   // Energy (terms_host gets the 6 per-term energies, may be null).
   // V, mask may be null when the corresponding term flag is off.

@@ -74,3 +74,48 @@ def test_transform_lengths(ctx, oracle_mod, N):
     rng = np.random.default_rng(sum(N))
     n = 0.2 / (4 * math.pi / 3) * (1 + 0.2 * rng.standard_normal(N)).clip(0.1)
     _check(ctx, oracle_mod, lat, N, n, _lib.HS_WB_NOTENSOR, 0.2)
+
+
+@pytest.mark.parametrize("kind", [_lib.HS_WB_TENSOR, _lib.HS_TARAZONA])
+@pytest.mark.parametrize("N,n3", [((7, 11, 13), 0.3), ((16, 9, 25), 1 / 32), ((33, 8, 12), 1e-8),
+                                  ((1, 1, 64), 0.4)])
+def test_tensor_sets(ctx, oracle_mod, kind, N, n3):
+    """The eleven convolutions and their adjoints on odd, prime and
+    one-dimensional grids, each branch of the third term, with empty walls
+    where the fluid is dense."""
+    lat = np.array([[0.2 * N[0], 0.1, 0.0], [0.0, 0.2 * N[1], 0.1], [0.1, 0.0, 0.2 * N[2]]])
+    rng = np.random.default_rng(N[0] + kind)
+    n = n3 / (4 * math.pi / 3) * (1 + 0.1 * rng.standard_normal(N)).clip(0.5)
+    if n3 > 0.1:
+        n[:, :, N[2] // 2:] = 0.0
+    _check(ctx, oracle_mod, lat, N, n, kind, n3)
+
+
+@pytest.mark.parametrize("N", [(7, 11, 13), (16, 9, 25), (12, 20, 14)])
+def test_water_sets(ctx, oracle_mod, N):
+    """The water terms around a nearly empty cavity (1e-5 of the liquid): their
+    energy and gradient against the oracle's.  The pass has some hundred
+    double-float operations in a row and divides by the shell density, which
+    falls to 1e-3 of the liquid's in the cavity: 2^-42 / 1e-3 of the largest
+    entry."""
+    from tests.capi import Fmt, Grid
+    from tests.golden.cases import WATER_KT, WATER_N, WATER_R, WATER_SAFT
+    O = oracle_mod
+    lat = np.diag([0.6 * v for v in N])
+    rng = np.random.default_rng(sum(N))
+    n = WATER_N * (1 + 0.1 * rng.standard_normal(N)).clip(0.3)
+    n[: N[0] // 3, : N[1] // 3] = 1e-5 * WATER_N
+    P = O.Problem(lat, N, R=WATER_R, kT=WATER_KT, mu=0.01, terms=O.HS | O.IDEAL | O.MU,
+                  saft=WATER_SAFT)
+    Er, gr = P.energy_grad(n)
+    g = Grid(ctx, lat, N)
+    f = Fmt(g, R=WATER_R, kT=WATER_KT, mu=0.01,
+            terms=_lib.TERM_HS | _lib.TERM_IDEAL | _lib.TERM_MU | _lib.TERM_SAFT)
+    sp = np.array(WATER_SAFT)
+    _lib.check(f.L.deft_fmt_set_saft(f.h, sp.ctypes.data))
+    E, grad, _ = f.energy_grad(n)
+    err = np.abs(grad.reshape(-1) - gr.reshape(-1)).max() / np.abs(gr).max()
+    print(f"N {N}: |dE/E| {abs(E / Er - 1):.2e} grad {err:.2e}")
+    assert abs(E / Er - 1) <= 2.0 ** -42 and err <= 2.0 ** -42 * 1e3
+    f.close()
+    g.close()
