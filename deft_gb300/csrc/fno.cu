@@ -303,6 +303,338 @@ __global__ void __launch_bounds__(256) k_dft_tile(const float2 *__restrict__ in,
   }
 }
 
+// ---------------------------------------------------------------------------
+// z and y transforms of a whole (channel, x) slab in one block, for grids whose
+// slab of N x N reals fits in shared memory beside another block's (slab_ok).
+// Both axes are folded: with e_n = a_n + a_{N-n}, o_n = a_n - a_{N-n} a
+// transform's cosine sums read e and its sine sums o, half the products, and
+// along y the sums for +k and -k are the same two.  Yc[n][k] = (cos, sin) of 2
+// pi k n / N, k <= m (the last for ky = -m).
+
+// Row stride of the slab tile: 16-byte rows, and the eight rows one load
+// instruction touches in distinct banks.
+__host__ __device__ inline int slab_stride(int N) { return N + (N % 8 == 0 ? 4 : 8); }
+__host__ __device__ inline int slab_chunks(int N) { return (N + 31) / 32; }
+__host__ __device__ constexpr int slab_jp(int KB) { return KB / 4 == 3 ? 4 : KB / 4; }
+size_t slab_fwd_smem(int N, int m, int KB) {
+  return sizeof(float) * 32 * slab_chunks(N) * slab_stride(N) +
+         sizeof(float2) * ((size_t)(N / 2 + 1) * (4 * slab_jp(KB) + m + 1));
+}
+size_t slab_inv_smem(int N, int m, int KB) {
+  return sizeof(float2) *
+         ((size_t)N * KB + (size_t)KB * N + 2 * (size_t)(m + 1) * KB + (size_t)(N / 2 + 1) * (m + 1));
+}
+// Two slab blocks per SM (up to N = 148).
+bool slab_ok(int N, int m) { return slab_fwd_smem(N, m, (m + 3) / 4 * 4) <= 110 * 1024; }
+
+// 16-byte asynchronous copies to shared memory.
+__device__ __forceinline__ void copy_async16(float *dst, const float *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src));
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;"); }
+template <int N> __device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+// Analysis: out[slab][ky][kz] = sum_y e^{-i ky y} sum_z E[z][kz] in[slab][y][z].
+// Along z two warps share 32 lines, each taking every second quad of z; lane
+// (lg = lane / 4, mg = lane % 4) holds lines lg + 8 r (r < 4) and modes mg + 4 j, so
+// a quad's three row reads a line and two table words a z feed 96 multiply-adds
+// and 32 additions.  The slab's second half
+// arrives while the first is transformed.  128^3, 16 channels, 12 modes: 66 us
+// against 101 for the z axis and 26 to 55 for the y axis before.
+template <int KB>
+__global__ void __launch_bounds__(384) k_slab_fwd(const float *__restrict__ in,
+                                                  float2 *__restrict__ out,
+                                                  const float2 *__restrict__ E,
+                                                  const float2 *__restrict__ Yc, int N, int Kz,
+                                                  int m) {
+  constexpr int J = KB / 4, JP = slab_jp(KB);
+  extern __shared__ __align__(16) float sm[];
+  const int S = slab_stride(N), rows = 32 * slab_chunks(N), H = N / 2;
+  float *tile = sm;                                              // [rows][S]
+  float2 *T = reinterpret_cast<float2 *>(tile + rows * S);       // [H + 1][4][JP]
+  float2 *Ys = T + (size_t)(H + 1) * 4 * JP;                     // [H + 1][m + 1]
+  const float *src = in + (size_t)blockIdx.x * N * N;
+  const int N4 = N >> 2, nq = N / 8;  // whole quads below N / 2
+  // the quads of z below nq / 2 and their mirrors, then the rest: the first
+  // half is transformed while the second is on its way
+  const int q1 = nq / 2;
+  auto stage = [&](int lo, int count) {  // `count` quads from lo, and nothing else
+    const int per = blockDim.x / count, q = threadIdx.x % count, l0 = threadIdx.x / count;
+    if (l0 < per) {
+      for (int ll = l0; ll < N; ll += per)
+        copy_async16(tile + ll * S + 4 * (lo + q), src + (size_t)ll * N + 4 * (lo + q));
+    }
+  };
+  if (q1 > 0) {
+    stage(0, q1);
+    stage(N4 - q1, q1);
+  }
+  copy_commit();
+  stage(q1, N4 - 2 * q1);
+  copy_commit();
+  for (int i = threadIdx.x; i < (rows - N) * S; i += blockDim.x) tile[N * S + i] = 0.f;
+  for (int i = threadIdx.x; i < (H + 1) * 4 * JP; i += blockDim.x) {
+    const int z = i / (4 * JP), r = i - z * 4 * JP, kk = r / JP + 4 * (r % JP);
+    T[i] = kk < Kz && r % JP < J ? E[z * Kz + kk] : make_float2(0.f, 0.f);
+  }
+  for (int i = threadIdx.x; i < (H + 1) * (m + 1); i += blockDim.x) Ys[i] = Yc[i];
+  copy_wait<1>();
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, chunk = w >> 1, par = w & 1;
+  const int lg = lane >> 2, mg = lane & 3;
+  const float *row0 = tile + (32 * chunk + lg) * S;
+  float2 acc[4][J];
+#pragma unroll
+  for (int r = 0; r < 4; r++)
+#pragma unroll
+    for (int j = 0; j < J; j++) acc[r][j] = make_float2(0.f, 0.f);
+  auto load_t = [&](int z, float2(&t)[J]) {
+    const float2 *p = T + (z * 4 + mg) * JP;
+    if constexpr (J == 1) {
+      t[0] = p[0];
+    } else {
+#pragma unroll
+      for (int j = 0; j + 1 < J + 1; j += 2) {
+        const float4 v = reinterpret_cast<const float4 *>(p)[j / 2];
+        t[j] = make_float2(v.x, v.y);
+        if (j + 1 < J) t[j + 1] = make_float2(v.z, v.w);
+      }
+    }
+  };
+  auto add = [&](int r, float a, float b, const float2(&t)[J]) {
+    const float e = a + b, o = a - b;
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+      acc[r][j].x = fmaf(e, t[j].x, acc[r][j].x);
+      acc[r][j].y = fmaf(o, t[j].y, acc[r][j].y);
+    }
+  };
+#pragma unroll 1
+  for (int q = par, half = 0; half < 2; q += 2) {
+    if (q >= (half ? nq : q1)) {
+      if (half++) break;
+      copy_wait<0>();
+      __syncthreads();
+      if (q >= nq) break;
+    }
+    float4 a[4], b[4];
+    float b0[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      const float *row = row0 + 8 * r * S;
+      a[r] = *reinterpret_cast<const float4 *>(row + 4 * q);
+      b[r] = *reinterpret_cast<const float4 *>(row + N - 4 * q - 4);
+      b0[r] = q ? row[N - 4 * q] : 0.f;  // z = 0 has no partner
+    }
+    float2 t[J];
+    load_t(4 * q, t);
+#pragma unroll
+    for (int r = 0; r < 4; r++) add(r, a[r].x, b0[r], t);
+    load_t(4 * q + 1, t);
+#pragma unroll
+    for (int r = 0; r < 4; r++) add(r, a[r].y, b[r].w, t);
+    load_t(4 * q + 2, t);
+#pragma unroll
+    for (int r = 0; r < 4; r++) add(r, a[r].z, b[r].z, t);
+    load_t(4 * q + 3, t);
+#pragma unroll
+    for (int r = 0; r < 4; r++) add(r, a[r].w, b[r].y, t);
+  }
+  if (par == 0) {
+    // what is left below N / 2 (N = 4 mod 8), and z = N / 2 itself
+#pragma unroll 1
+    for (int z = 4 * nq; z <= H; z++) {
+      float2 t[J];
+      load_t(z, t);
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const float *row = row0 + 8 * r * S;
+        add(r, row[z], z > 0 && z < H ? row[N - z] : 0.f, t);
+      }
+    }
+  }
+  // the two warps' halves added, as R[y][kz] in the tile's place
+  __syncthreads();
+  float2 *R = reinterpret_cast<float2 *>(sm);  // [N][KB]
+#pragma unroll
+  for (int half = 1; half >= 0; half--) {
+    if (par == half) {
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const int l = 32 * chunk + lg + 8 * r;
+        if (l < N) {
+#pragma unroll
+          for (int j = 0; j < J; j++) {
+            float2 &d = R[l * KB + mg + 4 * j];
+            const float2 v = acc[r][j];
+            d = half ? v : make_float2(d.x + v.x, d.y + v.y);
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  // y: a thread takes two k of one kz over a share of n, the shares added up
+  // through shared memory (behind R)
+  float2 *o = out + (size_t)blockIdx.x * 2 * m * Kz;
+  const int kp = (m + 2) / 2, items = kp * Kz;
+  int shares = blockDim.x / items;
+  const int room = (int)(((size_t)rows * S - (size_t)N * KB * 2) / (8 * (size_t)items));
+  shares = shares < 1 || room < 1 ? 1 : (shares < room ? shares : room);
+  float4 *part = reinterpret_cast<float4 *>(R + (size_t)N * KB);  // [share][k][item]: (c, s)
+  for (int it0 = 0; it0 < items; it0 += blockDim.x) {
+    const int sh = threadIdx.x / items;
+    const int it = shares > 1 ? (int)threadIdx.x - sh * items : it0 + (int)threadIdx.x;
+    const bool on = shares > 1 ? sh < shares : it < items;
+    const int k0 = 2 * (it / Kz), kz = it % Kz, k1 = k0 < m ? k0 + 1 : k0;
+    float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0;
+    if (on) {
+      const float2 *rp = R + kz;
+      const int s0 = shares > 1 ? sh : 0;
+      auto add2 = [&](float2 e, float2 od, int n) {
+        const float2 ya = Ys[n * (m + 1) + k0], yb = Ys[n * (m + 1) + k1];
+        v0.x = fmaf(e.x, ya.x, v0.x);
+        v0.y = fmaf(e.y, ya.x, v0.y);
+        v0.z = fmaf(od.x, ya.y, v0.z);
+        v0.w = fmaf(od.y, ya.y, v0.w);
+        v1.x = fmaf(e.x, yb.x, v1.x);
+        v1.y = fmaf(e.y, yb.x, v1.y);
+        v1.z = fmaf(od.x, yb.y, v1.z);
+        v1.w = fmaf(od.y, yb.y, v1.w);
+      };
+      if (s0 == 0) {
+        add2(rp[0], make_float2(0.f, 0.f), 0);
+        add2(rp[H * KB], make_float2(0.f, 0.f), H);
+      }
+#pragma unroll 4
+      for (int n = 1 + s0; n < H; n += shares) {
+        const float2 p = rp[n * KB], q = rp[(N - n) * KB];
+        add2(make_float2(p.x + q.x, p.y + q.y), make_float2(p.x - q.x, p.y - q.y), n);
+      }
+    }
+    if (shares > 1) {
+      if (on) {
+        part[(sh * 2) * items + it] = v0;
+        part[(sh * 2 + 1) * items + it] = v1;
+      }
+      __syncthreads();
+      if (sh == 0) {
+        for (int u = 1; u < shares; u++) {
+          const float4 a = part[(u * 2) * items + it], c = part[(u * 2 + 1) * items + it];
+          v0 = make_float4(v0.x + a.x, v0.y + a.y, v0.z + a.z, v0.w + a.w);
+          v1 = make_float4(v1.x + c.x, v1.y + c.y, v1.z + c.z, v1.w + c.w);
+        }
+      }
+    }
+    if (on && (shares == 1 || sh == 0)) {
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const int kk = k0 + u;
+        const float4 v = u ? v1 : v0;
+        if (kk > m) continue;
+        if (kk < m) o[kk * Kz + kz] = make_float2(v.x + v.w, v.y - v.z);
+        if (kk > 0) o[(2 * m - kk) * Kz + kz] = make_float2(v.x - v.w, v.y + v.z);
+      }
+    }
+    if (shares > 1) break;
+  }
+}
+
+// The slab's coefficients B[ky][kz] as the folded pairs P_k = B_k + B_{-k}, Q_k =
+// B_k - B_{-k} (k = 0: B_0, 0; k = m: B_{-m}, -B_{-m}), rows of ld.
+__device__ __forceinline__ void slab_pairs(const float2 *__restrict__ B, int m, int Kz, float2 &P,
+                                           float2 &Q, int k, int kz) {
+  const float2 a = k < m ? B[k * Kz + kz] : make_float2(0.f, 0.f);
+  const float2 b = k > 0 ? B[(2 * m - k) * Kz + kz] : make_float2(0.f, 0.f);
+  P = make_float2(a.x + b.x, a.y + b.y);
+  Q = k ? make_float2(a.x - b.x, a.y - b.y) : make_float2(0.f, 0.f);
+}
+
+// Synthesis: out[slab][y][z] (+)= sum_kz Re[G[z][kz] sum_ky e^{+i ky y} B[slab][ky][kz]].
+// The y sums go to shared memory (y and N - y together), then the z synthesis of
+// k_dft_z_inv.  96^3, 16 channels, 12 modes: 47 us against 44 and 25 for the
+// two launches.
+template <int KB>
+__global__ void __launch_bounds__(128) k_slab_inv(const float2 *__restrict__ in,
+                                                  float *__restrict__ out,
+                                                  const float2 *__restrict__ G,
+                                                  const float2 *__restrict__ Yc, int N, int Kz,
+                                                  int m, int accumulate) {
+  extern __shared__ __align__(16) float sm[];
+  const int H = N / 2;
+  float2 *A = reinterpret_cast<float2 *>(sm);  // [N][KB]
+  float2 *Gs = A + (size_t)N * KB;             // [KB][N]
+  float2 *P = Gs + (size_t)KB * N, *Q = P + (m + 1) * KB;
+  float2 *Ys = Q + (m + 1) * KB;               // [H + 1][m + 1]
+  const float2 *B = in + (size_t)blockIdx.x * 2 * m * Kz;
+  for (int i = threadIdx.x; i < N * KB; i += blockDim.x) {
+    const int z = i / KB, k = i - z * KB;
+    Gs[k * N + z] = k < Kz ? G[z * Kz + k] : make_float2(0.f, 0.f);
+  }
+  for (int i = threadIdx.x; i < (m + 1) * KB; i += blockDim.x) {
+    const int k = i / KB, kz = i - k * KB;
+    float2 p = make_float2(0.f, 0.f), q = p;
+    if (kz < Kz) slab_pairs(B, m, Kz, p, q, k, kz);
+    P[i] = p;
+    Q[i] = q;
+  }
+  for (int i = threadIdx.x; i < (H + 1) * (m + 1); i += blockDim.x) Ys[i] = Yc[i];
+  __syncthreads();
+  for (int it = threadIdx.x; it < (H + 1) * KB; it += blockDim.x) {
+    const int n = it / KB, kz = it - n * KB;
+    float2 u = P[kz], v = make_float2(0.f, 0.f);
+#pragma unroll 4
+    for (int k = 1; k <= m; k++) {
+      const float2 p = P[k * KB + kz], q = Q[k * KB + kz], y = Ys[n * (m + 1) + k];
+      u.x = fmaf(p.x, y.x, u.x);
+      u.y = fmaf(p.y, y.x, u.y);
+      v.x = fmaf(-q.y, y.y, v.x);
+      v.y = fmaf(q.x, y.y, v.y);
+    }
+    A[n * KB + kz] = make_float2(u.x + v.x, u.y + v.y);
+    if (n > 0 && n < H) A[(N - n) * KB + kz] = make_float2(u.x - v.x, u.y - v.y);
+  }
+  __syncthreads();
+  const int Qd = N >> 2;  // quads of a line
+  const int per = Qd < (int)blockDim.x ? Qd : (int)blockDim.x;
+  const int sub = threadIdx.x / per, subs = blockDim.x / per;
+  if (sub >= subs) return;
+  float *base = out + (size_t)blockIdx.x * N * N;
+  for (int q = threadIdx.x - sub * per; q < Qd; q += per) {
+    float2 g[KB][4];
+#pragma unroll
+    for (int k = 0; k < KB; k++) {
+      const float4 *gp = reinterpret_cast<const float4 *>(Gs + (size_t)k * N + 4 * q);
+      const float4 g0 = gp[0], g1 = gp[1];
+      g[k][0] = make_float2(g0.x, g0.y);
+      g[k][1] = make_float2(g0.z, g0.w);
+      g[k][2] = make_float2(g1.x, g1.y);
+      g[k][3] = make_float2(g1.z, g1.w);
+    }
+    for (int ll = sub; ll < N; ll += subs) {
+      float4 *o = reinterpret_cast<float4 *>(base + (size_t)ll * N) + q;
+      const float4 before = accumulate ? *o : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 *c = reinterpret_cast<const float4 *>(A + ll * KB);
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int k2 = 0; k2 < KB / 2; k2++) {
+        const float4 a = c[k2];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          v[j] = fmaf(a.x, g[2 * k2][j].x, v[j]);
+          v[j] = fmaf(-a.y, g[2 * k2][j].y, v[j]);
+          v[j] = fmaf(a.z, g[2 * k2 + 1][j].x, v[j]);
+          v[j] = fmaf(-a.w, g[2 * k2 + 1][j].y, v[j]);
+        }
+      }
+      *o = make_float4(before.x + v[0], before.y + v[1], before.z + v[2], before.w + v[3]);
+    }
+  }
+}
+
 // Spectral mixing U[o][k] = sum_i W[i][o][k] V[i][k]  (W bf16 complex).
 __global__ void k_spec_mix(const float2 *__restrict__ V, const __nv_bfloat16 *__restrict__ W,
                            float2 *__restrict__ U, int C, int K) {
@@ -490,6 +822,142 @@ __global__ void __launch_bounds__(256) k_layer_synth_pw(const float2 *__restrict
       if (act) acc = make_float2(gelu(acc.x), gelu(acc.y));
       *reinterpret_cast<float2 *>(hn + (size_t)o * NR + r) = acc;
     }
+  }
+}
+
+// The inference layer from the x-synthesised coefficients B[c][x][ky][kz]: a
+// block holds one x's coefficients of every channel (folded pairs, slab_pairs)
+// and walks lines y of a share of that x: per pass the y sums of its lines go
+// to shared memory, then a thread synthesises z and N - z together (their
+// cosine and sine sums; thread 0 of a line takes z = 0 and N / 2, whose sine
+// table is the half difference of the two cosines and multiplies the real part
+// again, so its coefficients stand in a second array as (re, re)), adds the
+// pointwise layer and activates.  The previous layer's values are loaded before
+// the sums, the next pass's y sums are formed while this pass's lines are in
+// flight (two buffers).  Bound by issue and
+// latency at two blocks per SM (128 registers): 142 us at 128^3, 16 channels, 12
+// modes, against 131 without the y sums and 44 for those (packed f32x2
+// multiply-adds: 148).
+template <int C>
+size_t synth_smem(int N, int m, int Kz) {
+  const int lpb = 256 / (N / 2);
+  return sizeof(float) * (C * C + C) +
+         sizeof(float2) * ((size_t)Kz * (N / 2) + (size_t)N * (m + 1) +
+                           2 * (size_t)C * (m + 1) * Kz + 4 * (size_t)lpb * C * Kz);
+}
+template <int C>
+__global__ void __launch_bounds__(256, 2) k_layer_synth(const float2 *__restrict__ B,
+                                                        const float2 *__restrict__ G,
+                                                        const float2 *__restrict__ Yc,
+                                                        const float *__restrict__ h,
+                                                        float *__restrict__ hn,
+                                                        const __nv_bfloat16 *__restrict__ Wp,
+                                                        const __nv_bfloat16 *__restrict__ b, int N,
+                                                        int Kz, int m, int act) {
+  extern __shared__ __align__(16) float sm[];
+  const int H = N >> 1, lpb = 256 / H;
+  float *Ws = sm;                                       // [C][C]
+  float *bs = Ws + C * C;                               // [C]
+  float2 *As = reinterpret_cast<float2 *>(bs + C);      // [2][lpb][Kz][C]: (re, im)
+  float2 *Ax = As + 2 * (size_t)lpb * Kz * C;           // the same as (re, re)
+  float2 *Gs = Ax + 2 * (size_t)lpb * Kz * C;           // [Kz][H]
+  float2 *Ys = Gs + (size_t)Kz * H;                     // [N][m + 1]
+  float2 *P = Ys + (size_t)N * (m + 1);                 // [m + 1][Kz][C]
+  float2 *Q = P + (size_t)(m + 1) * Kz * C;
+  const int x = blockIdx.x;
+  for (int i = threadIdx.x; i < C * C; i += blockDim.x) Ws[i] = bf(Wp, i);
+  for (int i = threadIdx.x; i < C; i += blockDim.x) bs[i] = bf(b, i);
+  for (int i = threadIdx.x; i < Kz * H; i += blockDim.x) {
+    const int k = i / H, z = i - k * H;
+    const float2 g = G[(size_t)z * Kz + k];
+    if (z == 0) {
+      const float gh = G[(size_t)H * Kz + k].x;
+      Gs[i] = make_float2(0.5f * (g.x + gh), 0.5f * (gh - g.x));
+    } else {
+      Gs[i] = g;
+    }
+  }
+  for (int i = threadIdx.x; i < N * (m + 1); i += blockDim.x) Ys[i] = Yc[i];
+  for (int i = threadIdx.x; i < (m + 1) * Kz * C; i += blockDim.x) {
+    const int c = i / ((m + 1) * Kz), r = i - c * (m + 1) * Kz, k = r / Kz, kz = r - k * Kz;
+    slab_pairs(B + ((size_t)c * N + x) * 2 * m * Kz, m, Kz, P[r * C + c], Q[r * C + c], k, kz);
+  }
+  const long long NR = (long long)N * N * N;
+  const int y0 = (int)((long long)N * blockIdx.y / gridDim.y);
+  const int y1 = (int)((long long)N * (blockIdx.y + 1) / gridDim.y);
+  // y sums of lines ya .. ya + lpb into buffer `buf`
+  auto lines_to = [&](int ya, int buf) {
+    for (int i = threadIdx.x; i < lpb * Kz * C; i += blockDim.x) {
+      const int ll = i / (Kz * C), r = i - ll * Kz * C, y = ya + ll;
+      if (y >= y1) continue;
+      const float2 *yp = Ys + (size_t)y * (m + 1);
+      float2 u = P[r], v = make_float2(0.f, 0.f);
+#pragma unroll 4
+      for (int k = 1; k <= m; k++) {
+        const float2 p = P[(size_t)k * Kz * C + r], q = Q[(size_t)k * Kz * C + r], cs = yp[k];
+        u.x = fmaf(p.x, cs.x, u.x);
+        u.y = fmaf(p.y, cs.x, u.y);
+        v.x = fmaf(-q.y, cs.y, v.x);
+        v.y = fmaf(q.x, cs.y, v.y);
+      }
+      const float2 a = make_float2(u.x + v.x, u.y + v.y);
+      As[(size_t)buf * lpb * Kz * C + i] = a;
+      Ax[(size_t)buf * lpb * Kz * C + i] = make_float2(a.x, a.x);
+    }
+  };
+  __syncthreads();
+  lines_to(y0, 0);
+  __syncthreads();
+  const int tl = threadIdx.x / H, zp = threadIdx.x - tl * H, zm = zp ? N - zp : H;
+  int buf = 0;
+  for (int ya = y0; ya < y1; ya += lpb, buf ^= 1) {
+    const int y = ya + tl;
+    const bool on = tl < lpb && y < y1;
+    const size_t r0 = ((size_t)x * N + (on ? y : y0)) * N;
+    float2 hv[C];
+#pragma unroll
+    for (int i = 0; i < C; i++)
+      hv[i] = make_float2(h[(size_t)i * NR + r0 + zp], h[(size_t)i * NR + r0 + zm]);
+    if (ya + lpb < y1) lines_to(ya + lpb, buf ^ 1);
+    if (on) {
+      const float2 *a = (zp ? As : Ax) + ((size_t)buf * lpb + tl) * Kz * C;
+      float2 spec[C];  // (cosine, sine) sums
+#pragma unroll
+      for (int c = 0; c < C; c++) spec[c] = make_float2(0.f, 0.f);
+      for (int k = 0; k < Kz; k++) {
+        const float2 g = Gs[(size_t)k * H + zp];
+        const float4 *ak = reinterpret_cast<const float4 *>(a + k * C);
+#pragma unroll
+        for (int c2 = 0; c2 < C / 2; c2++) {
+          const float4 ac = ak[c2];  // channels 2 c2, 2 c2 + 1
+          spec[2 * c2].x = fmaf(ac.x, g.x, spec[2 * c2].x);
+          spec[2 * c2].y = fmaf(ac.y, g.y, spec[2 * c2].y);
+          spec[2 * c2 + 1].x = fmaf(ac.z, g.x, spec[2 * c2 + 1].x);
+          spec[2 * c2 + 1].y = fmaf(ac.w, g.y, spec[2 * c2 + 1].y);
+        }
+      }
+#pragma unroll
+      for (int o = 0; o < C; o++) {
+        float2 acc = make_float2(spec[o].x - spec[o].y + bs[o], spec[o].x + spec[o].y + bs[o]);
+        const float4 *wr = reinterpret_cast<const float4 *>(Ws + o * C);
+#pragma unroll
+        for (int i4 = 0; i4 < C / 4; i4++) {
+          const float4 w = wr[i4];
+          acc.x = fmaf(w.x, hv[4 * i4].x, acc.x);
+          acc.y = fmaf(w.x, hv[4 * i4].y, acc.y);
+          acc.x = fmaf(w.y, hv[4 * i4 + 1].x, acc.x);
+          acc.y = fmaf(w.y, hv[4 * i4 + 1].y, acc.y);
+          acc.x = fmaf(w.z, hv[4 * i4 + 2].x, acc.x);
+          acc.y = fmaf(w.z, hv[4 * i4 + 2].y, acc.y);
+          acc.x = fmaf(w.w, hv[4 * i4 + 3].x, acc.x);
+          acc.y = fmaf(w.w, hv[4 * i4 + 3].y, acc.y);
+        }
+        if (act) acc = make_float2(gelu(acc.x), gelu(acc.y));
+        hn[(size_t)o * NR + r0 + zp] = acc.x;
+        hn[(size_t)o * NR + r0 + zm] = acc.y;
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -969,6 +1437,8 @@ struct deft_fno {
   float2 *Gzi = nullptr;  // [N][Kz] synthesis c_k / N^3
   float2 *Gza = nullptr;  // [N][Kz] adjoint of the forward z transform (c = 1, s = 1)
   float2 *Eyf = nullptr, *Eyi = nullptr, *Exf = nullptr, *Exi = nullptr;
+  float2 *Yc = nullptr;  // [N][m + 1] (cos, sin) of the slab kernels
+  bool slab = false;      // slab kernels for the z and y axes
   // activations
   std::vector<float *> h, z;  // h[0..L], z[0..L-1]
   std::vector<float2 *> V;    // V[l] spectral inputs per layer
@@ -1068,53 +1538,123 @@ void launch_axis(deft_fno *f, const float2 *in, float2 *out, const float2 *E, in
                                                                               Nin, Mout, inner);
 }
 
-// Forward through the spectral part of layer l: S (in zbuf) = Finv(W F h);
-// without zout, stops before the z synthesis (its coefficients in f->A).
-void spectral_fwd(deft_fno *f, int l, const float *hin, float *zout) {
+// The shared-memory cap of a kernel, for the current device.
+template <typename K> void allow_smem(K kernel, size_t bytes) {
+  if (bytes > 48 * 1024)
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+// Calls g(std::integral_constant<int, KB>()) with Kz rounded up to the register tile.
+template <typename F> void with_kb(int Kz, F &&g) {
+  switch (kz_block(Kz)) {
+    case 4: g(std::integral_constant<int, 4>()); break;
+    case 8: g(std::integral_constant<int, 8>()); break;
+    case 12: g(std::integral_constant<int, 12>()); break;
+    default: g(std::integral_constant<int, 16>()); break;
+  }
+}
+
+// z (table E) and y analysis of C fields: f->B [C N Ky Kz].
+void analyse_zy(deft_fno *f, const float *in, const float2 *E) {
   const int C = f->C, N = f->N;
-  launch_z_fwd(f, hin, f->A, f->Ezf);                               // [C N N Kz]
-  launch_axis(f, f->A, f->B, f->Eyf, C * N, N, f->Ky, f->Kz);       // [C N Ky Kz]
+  f->launches++;
+  if (!f->slab) {
+    f->launches++;
+    launch_z_fwd(f, in, f->A, E);                                // [C N N Kz]
+    launch_axis(f, f->A, f->B, f->Eyf, C * N, N, f->Ky, f->Kz);  // [C N Ky Kz]
+    return;
+  }
+  with_kb(f->Kz, [&](auto kb) {
+    constexpr int KB = decltype(kb)::value;
+    const size_t sm = slab_fwd_smem(N, f->m, KB);
+    allow_smem(k_slab_fwd<KB>, sm);
+    k_slab_fwd<KB><<<C * N, 64 * slab_chunks(N), sm, f->stream>>>(in, f->B, E, f->Yc, N, f->Kz,
+                                                                  f->m);
+  });
+}
+// y and z (table G) synthesis of f->B into C fields.
+void synthesise_yz(deft_fno *f, float *out, const float2 *G, int accumulate) {
+  const int C = f->C, N = f->N;
+  f->launches++;
+  if (!f->slab) {
+    f->launches++;
+    launch_axis(f, f->B, f->A, f->Eyi, C * N, f->Ky, N, f->Kz);  // [C N N Kz]
+    launch_z_inv(f, f->A, out, G, accumulate);
+    return;
+  }
+  with_kb(f->Kz, [&](auto kb) {
+    constexpr int KB = decltype(kb)::value;
+    const size_t sm = slab_inv_smem(N, f->m, KB);
+    allow_smem(k_slab_inv<KB>, sm);
+    k_slab_inv<KB><<<C * N, 128, sm, f->stream>>>(f->B, out, G, f->Yc, N, f->Kz, f->m, accumulate);
+  });
+}
+
+// Forward through the spectral part of layer l up to the x synthesis: its
+// coefficients in f->B.
+void spectral_fwd(deft_fno *f, int l, const float *hin) {
+  const int C = f->C, N = f->N;
+  analyse_zy(f, hin, f->Ezf);
   launch_axis(f, f->B, f->V[l], f->Exf, C, N, f->Kx, f->Ky * f->Kz);  // [C Kx Ky Kz]
   k_spec_mix<<<(C * f->K + kT - 1) / kT, kT, 0, f->stream>>>(f->V[l], f->pb + f->oW[l], f->S, C,
                                                               f->K);
-  launch_axis(f, f->S, f->B, f->Exi, C, f->Kx, N, f->Ky * f->Kz);   // [C N Ky Kz]
-  launch_axis(f, f->B, f->A, f->Eyi, C * N, f->Ky, N, f->Kz);       // [C N N Kz]
-  if (zout) launch_z_inv(f, f->A, zout, f->Gzi, 0);
+  launch_axis(f, f->S, f->B, f->Exi, C, f->Kx, N, f->Ky * f->Kz);  // [C N Ky Kz]
+  f->launches += 3;
 }
 
-// The inference layer: synthesis of f->A fused into the pointwise layer.
+// The inference layer: y and z synthesis fused with the pointwise layer (slab
+// grids), else the z synthesis fused with it.
 template <int C>
-void launch_layer_synth_pw(deft_fno *f, int l) {
-  const int N = f->N, half = N / 2, lpb = 256 / half;
-  const size_t sm = sizeof(float) * (C * C + ((C + 3) & ~3)) +
-                    sizeof(float2) * ((size_t)f->Kz * N + (size_t)lpb * C * f->Kz);
-  if (sm > 48 * 1024)
-    cudaFuncSetAttribute(k_layer_synth_pw<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sm);
+void launch_layer_synth(deft_fno *f, int l) {
+  const int N = f->N, half = N / 2, lpb = 256 / half, act = l < f->L - 1 ? 1 : 0;
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (sms <= 0) sms = 148;
+  f->launches++;
+  if (f->slab) {
+    const size_t sm = synth_smem<C>(N, f->m, f->Kz);
+    allow_smem(k_layer_synth<C>, sm);
+    // blocks per x: the fewest rounds of two blocks per SM, a round costing
+    // its passes and about two more for the block's tables
+    const int most = (N + lpb - 1) / lpb;
+    int share = 1, best = 0;
+    for (int k = 1; k <= most && k <= 16; k++) {
+      const int cost = (N * k + 2 * sms - 1) / (2 * sms) * (((N + k - 1) / k + lpb - 1) / lpb + 2);
+      if (k == 1 || cost < best) {
+        best = cost;
+        share = k;
+      }
+    }
+    k_layer_synth<C><<<dim3(N, share), 256, sm, f->stream>>>(
+        f->B, f->Gzi, f->Yc, f->h[l], f->h[l + 1], f->pb + f->oWp[l], f->pb + f->ob[l], N, f->Kz,
+        f->m, act);
+    return;
+  }
+  f->launches++;
+  launch_axis(f, f->B, f->A, f->Eyi, C * N, f->Ky, N, f->Kz);  // [C N N Kz]
+  const size_t sm = sizeof(float) * (C * C + ((C + 3) & ~3)) +
+                    sizeof(float2) * ((size_t)f->Kz * N + (size_t)lpb * C * f->Kz);
+  allow_smem(k_layer_synth_pw<C>, sm);
   const int lines = N * N;
-  int grid = 4 * (sms > 0 ? sms : 148);
+  int grid = 4 * sms;
   const int need = (lines + lpb - 1) / lpb;
   if (grid > need) grid = need;
   k_layer_synth_pw<C><<<grid, 256, sm, f->stream>>>(f->A, f->Gzi, f->h[l], f->h[l + 1],
                                                     f->pb + f->oWp[l], f->pb + f->ob[l], N, f->Kz,
-                                                    l < f->L - 1 ? 1 : 0);
+                                                    act);
 }
 
-// Adjoint of spectral_fwd for upstream zbar: adds K^T zbar to hin_bar and
+// Adjoint of the spectral part for upstream zbar: adds K^T zbar to hin_bar and
 // accumulates W grads.
 void spectral_bwd(deft_fno *f, int l, const float *zbar, float *hin_bar) {
   const int C = f->C, N = f->N;
-  launch_z_fwd(f, zbar, f->A, f->Ezb);                              // A'bar
-  launch_axis(f, f->A, f->B, f->Eyf, C * N, N, f->Ky, f->Kz);       // B'bar
+  analyse_zy(f, zbar, f->Ezb);                                      // B'bar
   launch_axis(f, f->B, f->S, f->Exf, C, N, f->Kx, f->Ky * f->Kz);   // Ubar
   k_spec_mix_bwd<<<(C * f->K + kT - 1) / kT, kT, 0, f->stream>>>(
       f->V[l], f->pb + f->oW[l], f->S, f->S2, f->g + f->oW[l], C, f->K);  // Vbar
   launch_axis(f, f->S2, f->B, f->Exi, C, f->Kx, N, f->Ky * f->Kz);  // Bbar
-  launch_axis(f, f->B, f->A, f->Eyi, C * N, f->Ky, N, f->Kz);       // Abar
-  launch_z_inv(f, f->A, hin_bar, f->Gza, 1);
+  synthesise_yz(f, hin_bar, f->Gza, 1);
+  f->launches += 3;
 }
 
 template <int C>
@@ -1142,20 +1682,20 @@ void project(deft_fno *f, float *zq, const float *target, const float *w, float 
 // backward pass reads.
 int forward(deft_fno *f, float eta, bool train) {
   const int C = f->C;
-  f->launches += 1 + 8 * f->L;  // lift; per layer 7 spectral launches and the pointwise one
+  f->launches++;  // lift
   k_lift<<<grid_for(f->NR), kT, 0, f->stream>>>(f->mask, eta, f->pb + f->oP, f->pb + f->op, f->h[0],
                                                C, f->NR);
   for (int l = 0; l < f->L; l++) {
+    spectral_fwd(f, l, f->h[l]);
     if (!train) {
-      // inference: no z field for a backward pass; one launch fewer per layer
-      spectral_fwd(f, l, f->h[l], nullptr);
-      f->launches--;
-      if (C == 16) launch_layer_synth_pw<16>(f, l);
-      else if (C == 8) launch_layer_synth_pw<8>(f, l);
-      else launch_layer_synth_pw<4>(f, l);
+      // inference: no z field for a backward pass
+      if (C == 16) launch_layer_synth<16>(f, l);
+      else if (C == 8) launch_layer_synth<8>(f, l);
+      else launch_layer_synth<4>(f, l);
       continue;
     }
-    spectral_fwd(f, l, f->h[l], f->z[l]);
+    synthesise_yz(f, f->z[l], f->Gzi, 0);
+    f->launches++;
     if (C == 16) launch_layer_pw<16>(f, l, 1);
     else if (C == 8) launch_layer_pw<8>(f, l, 1);
     else launch_layer_pw<4>(f, l, 1);
@@ -1263,6 +1803,11 @@ int deft_fno_create(int device, int N, int channels, int modes, int layers, unsi
   dev(&f->Eyi, sizeof(float2) * eyi.size());
   dev(&f->Exf, sizeof(float2) * exf.size());
   dev(&f->Exi, sizeof(float2) * exi.size());
+  f->slab = slab_ok(N, modes);
+  std::vector<float2> yc((size_t)N * (modes + 1));
+  for (int n = 0; n < N; n++)
+    for (int k = 0; k <= modes; k++) yc[(size_t)n * (modes + 1) + k] = cexp(tp * (double)((long long)k * n % N) / N);
+  dev(&f->Yc, sizeof(float2) * yc.size());
   const size_t act = sizeof(float) * C * f->NR;
   f->h.resize(layers + 1);
   f->z.resize(layers);
@@ -1312,6 +1857,7 @@ int deft_fno_create(int device, int N, int channels, int modes, int layers, unsi
   cudaMemcpy(f->Eyi, eyi.data(), sizeof(float2) * eyi.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(f->Exf, exf.data(), sizeof(float2) * exf.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(f->Exi, exi.data(), sizeof(float2) * exi.size(), cudaMemcpyHostToDevice);
+  cudaMemcpy(f->Yc, yc.data(), sizeof(float2) * yc.size(), cudaMemcpyHostToDevice);
   const size_t zf = smem_z_fwd(N, f->Kz);
   cudaFuncSetAttribute(k_dft_z_fwd<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zf);
   cudaFuncSetAttribute(k_dft_z_fwd<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zf);
@@ -1335,7 +1881,7 @@ int deft_fno_destroy(deft_fno *f) {
   if (f->stream) cudaStreamSynchronize(f->stream);
   for (void *q : {(void *)f->p, (void *)f->g, (void *)f->am, (void *)f->av, (void *)f->pb,
                   (void *)f->Ezf, (void *)f->Ezb, (void *)f->Gzi, (void *)f->Gza, (void *)f->Eyf,
-                  (void *)f->Eyi, (void *)f->Exf, (void *)f->Exi, (void *)f->zq, (void *)f->y,
+                  (void *)f->Eyi, (void *)f->Exf, (void *)f->Exi, (void *)f->Yc, (void *)f->zq, (void *)f->y,
                   (void *)f->mask, (void *)f->target, (void *)f->wt, (void *)f->A, (void *)f->B,
                   (void *)f->S, (void *)f->S2, (void *)f->hb0, (void *)f->hb1, (void *)f->zb,
                   (void *)f->part, (void *)f->loss_d, (void *)f->bulk, (void *)f->part_d})
@@ -1416,7 +1962,7 @@ int eval_impl(deft_fno *f, const float *mask, float eta, const float *target, cu
   }
   if (y_out) cudaMemcpyAsync(y_out, f->y, rb, kout, f->stream);
   if (want_grad && target) {
-    f->launches += 4 + 9 * f->L;  // projection, lift and layer backward passes with their sums
+    f->launches += 4 + 2 * f->L;  // projection, lift and pointwise backward passes with their sums
     cudaMemsetAsync(f->g, 0, sizeof(float) * f->nparam, f->stream);
     // projection
     if (C == 16) project_bwd<16>(f);
