@@ -79,12 +79,17 @@ __device__ __forceinline__ float d2f_small(double d) {
     const unsigned rh = (hi & 0x7fffffffu) + (rl < lo ? 1u : 0u);
     return __uint_as_float((__funnelshift_r(rl, rh, 29) - (384u << 23)) | sign);
   }
+  if (((hi & 0x7fffffffu) | lo) == 0) return __uint_as_float(sign);
   return (float)d;
 }
-// A real of the transforms' type from FP64 data.
+// A real of the transforms' type from FP64 data (or from FP32: widening or a
+// copy), and the way back; none of the common cases runs on the FP64 pipe.
 template <typename T> __device__ __forceinline__ T real_from(double d) { return T(d); }
 template <> __device__ __forceinline__ dfl real_from<dfl>(double d) { return df_from(d); }
+template <> __device__ __forceinline__ float real_from<float>(double d) { return d2f_small(d); }
 template <typename T> __device__ __forceinline__ T real_from(dfl d) { return T(d); }
+template <typename T> __device__ __forceinline__ T real_from(float f) { return T(f); }
+template <> __device__ __forceinline__ double real_from<double>(float f) { return f2d(f); }
 
 // Knuth's TwoSum: s + e == a + b exactly.
 __device__ __forceinline__ dfl df_two_sum(float a, float b) {

@@ -8,7 +8,8 @@
 // exp(-2 pi i t / L), runs a register DFT of length r and writes the
 // self-sorted result into the other buffer (ping-pong), so no bit-reversal
 // pass is needed.  Radices 2, 3, 4, 5 and 8 are hand-written; 7, 11 and 13 are
-// folded DFTs with compile-time roots (dft_prime).
+// folded DFTs with compile-time roots (dft_prime); FP32 plans also run pairs
+// of small radices as one pass of 10, 12 or 16 (fuse_passes).
 //
 // Sign convention (FFTW's, which the reference links): SIGN = -1 forward,
 // +1 backward, both unnormalised.
@@ -45,6 +46,8 @@ struct FftPlan {
   FastDiv ns[kMaxPasses];  // product of the radices of the earlier passes
   const void *tw;          // device table, n entries of Cplx<T>
   int reg;                 // 1: register-resident two-stage transform (radix order 16, n/16)
+  int nord;                // FP32: the chosen radix order the passes were fused from
+  signed char order[kMaxPasses];
 };
 
 // Whether a plan has a pass of radix 7, 11 or 13.
@@ -61,6 +64,27 @@ inline void plan_fill_ns(FftPlan &p) {
     p.ns[i] = make_fastdiv(Ns);
     Ns *= (unsigned)p.radix[i];
   }
+}
+
+// FP32 plans: neighbouring radices (4, 4), (4, 3), (3, 4), (2, 5) and (5, 2) of
+// the chosen order run as one pass of 16, 12 or 10, which keeps the inner
+// transform in registers: one crossing of shared memory and one set of
+// twiddles less.  128 = 8 x 16 and 96 = 8 x 12 take two passes instead of
+// three.  (Double-float passes hold twice the registers and are bound by
+// their arithmetic: they keep the small radices.)
+inline void fuse_passes(FftPlan &p) {
+  p.nord = p.npass;
+  for (int i = 0; i < p.npass; i++) p.order[i] = (signed char)p.radix[i];
+  int k = 0;
+  for (int i = 0; i < p.nord; i++) {
+    const int a = p.order[i], b = i + 1 < p.nord ? p.order[i + 1] : 0;
+    const bool fuse = (a == 4 && (b == 4 || b == 3)) || (a == 3 && b == 4) ||
+                      (a == 2 && b == 5) || (a == 5 && b == 2);
+    p.radix[k++] = fuse ? a * b : a;
+    i += fuse;
+  }
+  p.npass = k;
+  plan_fill_ns(p);
 }
 
 template <typename C> __device__ __forceinline__ C c_add(C a, C b) { return C{a.x + b.x, a.y + b.y}; }
@@ -229,43 +253,6 @@ template <int SIGN, typename C> __device__ __forceinline__ C tw_load(const C *tw
   return w;
 }
 
-// One radix-R pass over a tile: src -> dst.
-template <typename T, int SIGN, int R>
-__device__ __forceinline__ void fft_pass(const typename Cplx<T>::type *__restrict__ src,
-                                         typename Cplx<T>::type *__restrict__ dst,
-                                         const FastDiv &bd, int L, const FastDiv &nsd,
-                                         const typename Cplx<T>::type *__restrict__ tw) {
-  using C = typename Cplx<T>::type;
-  const int B = (int)bd.d, Ns = (int)nsd.d;
-  const int m = L / R;
-  const int twstep = L / (Ns * R);
-  const int total = m * B;
-  for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-    int j, bl, q, k;
-    fdivmod(idx, bd, j, bl);
-    fdivmod(j, nsd, q, k);
-    C v[R];
-#pragma unroll
-    for (int s = 0; s < R; ++s) v[s] = src[(j + s * m) * B + bl];
-    if (k) {
-#pragma unroll
-      for (int s = 1; s < R; ++s) v[s] = c_mul(v[s], tw_load<SIGN>(tw, s * k * twstep));
-    }
-    const int base = q * Ns * R + k;
-    if constexpr (R > 5 && R != 8) {
-      dft_prime<SIGN, T, C, R>(v, [&](int o, C x) { dst[(base + o * Ns) * B + bl] = x; });
-    } else {
-      if constexpr (R == 2) dft2<SIGN>(v[0], v[1]);
-      else if constexpr (R == 4) dft4<SIGN>(v[0], v[1], v[2], v[3]);
-      else if constexpr (R == 8) dft8<SIGN, T>(v);
-      else if constexpr (R == 3) dft3<SIGN, T>(v);
-      else dft5<SIGN, T>(v);
-#pragma unroll
-      for (int s = 0; s < R; ++s) dst[(base + s * Ns) * B + bl] = v[s];
-    }
-  }
-}
-
 // (x + iy) (cr + i ci)
 template <typename C, typename T> __device__ __forceinline__ C c_mulc(C a, T cr, T ci) {
   return C{a.x * cr - a.y * ci, a.x * ci + a.y * cr};
@@ -310,6 +297,76 @@ template <int SIGN, typename T, typename C, int M> __device__ __forceinline__ vo
   else if constexpr (M == 5) dft5<SIGN, T>(v);
   else if constexpr (M == 8) dft8<SIGN, T>(v);
   else dft16<SIGN, T>(v);
+}
+
+// DFT of length R1 R2 (coprime) in registers, natural order in and out, by the
+// prime-factor map (Good 1958): with n = R2 n1 + R1 n2 and k = A k1 + B k2 mod R
+// (A = 1 mod R1 and 0 mod R2, B the other way round) the two stages need no
+// factors between them.
+template <int R1, int R2> __host__ __device__ constexpr int pfa_idem() {
+  for (int a = 0; a < R1 * R2; a += R2)
+    if (a % R1 == 1) return a;
+  return 0;
+}
+template <int SIGN, typename T, typename C, int R1, int R2>
+__device__ __forceinline__ void dft_pfa(C *v) {
+  constexpr int R = R1 * R2, A = pfa_idem<R1, R2>(), B = pfa_idem<R2, R1>();
+  C t[R];
+#pragma unroll
+  for (int n2 = 0; n2 < R2; n2++) {
+    C u[R1];
+#pragma unroll
+    for (int n1 = 0; n1 < R1; n1++) u[n1] = v[(R2 * n1 + R1 * n2) % R];
+    dft_m<SIGN, T, C, R1>(u);
+#pragma unroll
+    for (int k1 = 0; k1 < R1; k1++) t[k1 * R2 + n2] = u[k1];
+  }
+#pragma unroll
+  for (int k1 = 0; k1 < R1; k1++) {
+    dft_m<SIGN, T, C, R2>(&t[k1 * R2]);
+#pragma unroll
+    for (int k2 = 0; k2 < R2; k2++) v[(A * k1 + B * k2) % R] = t[k1 * R2 + k2];
+  }
+}
+
+// One radix-R pass over a tile: src -> dst.
+template <typename T, int SIGN, int R>
+__device__ __forceinline__ void fft_pass(const typename Cplx<T>::type *__restrict__ src,
+                                         typename Cplx<T>::type *__restrict__ dst,
+                                         const FastDiv &bd, int L, const FastDiv &nsd,
+                                         const typename Cplx<T>::type *__restrict__ tw) {
+  using C = typename Cplx<T>::type;
+  const int B = (int)bd.d, Ns = (int)nsd.d;
+  const int m = L / R;
+  const int twstep = L / (Ns * R);
+  const int total = m * B;
+  for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+    int j, bl, q, k;
+    fdivmod(idx, bd, j, bl);
+    fdivmod(j, nsd, q, k);
+    C v[R];
+#pragma unroll
+    for (int s = 0; s < R; ++s) v[s] = src[(j + s * m) * B + bl];
+    if (k) {
+#pragma unroll
+      for (int s = 1; s < R; ++s) v[s] = c_mul(v[s], tw_load<SIGN>(tw, s * k * twstep));
+    }
+    const int base = q * Ns * R + k;
+    if constexpr (R == 7 || R == 11 || R == 13) {
+      dft_prime<SIGN, T, C, R>(v, [&](int o, C x) { dst[(base + o * Ns) * B + bl] = x; });
+    } else {
+      if constexpr (R == 2) dft2<SIGN>(v[0], v[1]);
+      else if constexpr (R == 4) dft4<SIGN>(v[0], v[1], v[2], v[3]);
+      else if constexpr (R == 8) dft8<SIGN, T>(v);
+      else if constexpr (R == 3) dft3<SIGN, T>(v);
+      else if constexpr (R == 5) dft5<SIGN, T>(v);
+      else if constexpr (R == 10) dft_pfa<SIGN, T, C, 2, 5>(v);
+      else if constexpr (R == 12) dft_pfa<SIGN, T, C, 4, 3>(v);
+      else dft16<SIGN, T>(v);
+#pragma unroll
+      for (int s = 0; s < R; ++s) dst[(base + s * Ns) * B + bl] = v[s];
+    }
+  }
 }
 
 // Register-resident transform of the B lines of an element-major tile
@@ -429,6 +486,20 @@ __device__ typename Cplx<T>::type *fft_tile(typename Cplx<T>::type *a, typename 
       case 5: fft_pass<T, SIGN, 5>(src, dst, bd, p.n, nsd, tw); break;
       case 8: fft_pass<T, SIGN, 8>(src, dst, bd, p.n, nsd, tw); break;
       default:
+        if constexpr (std::is_same<T, float>::value) {
+          if (r == 16) {
+            fft_pass<T, SIGN, 16>(src, dst, bd, p.n, nsd, tw);
+            break;
+          }
+          if (r == 12) {
+            fft_pass<T, SIGN, 12>(src, dst, bd, p.n, nsd, tw);
+            break;
+          }
+          if (r == 10) {
+            fft_pass<T, SIGN, 10>(src, dst, bd, p.n, nsd, tw);
+            break;
+          }
+        }
         if constexpr (RN < 0 || !std::is_same<T, dfl>::value) {
           if (r == 7) fft_pass<T, SIGN, 7>(src, dst, bd, p.n, nsd, tw);
           else if (r == 11) fft_pass<T, SIGN, 11>(src, dst, bd, p.n, nsd, tw);

@@ -28,7 +28,9 @@
 #include "warp_fft.cuh"
 #include "wb_phi.cuh"
 
+#include <algorithm>
 #include <cmath>
+#include <functional>
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
@@ -235,20 +237,17 @@ __device__ __forceinline__ void unpack_r2c_store(const typename Cplx<T>::type *r
                                                  const Geom &g, int p0, int P, T s) {
   using C = typename Cplx<T>::type;
   const int Nz = g.Nz, NzH = g.NzH;
+  const T h = T(0.5) * s;
   #pragma unroll 4
-  for (int idx = threadIdx.x; idx < 2 * P * NzH; idx += blockDim.x) {
-    int ll, k;
-    fdivmod(idx, g.fNzH, ll, k);
-    const int line = 2 * p0 + ll;
-    if (line >= g.lines) continue;
-    const int pb = ll >> 1;
+  for (int idx = threadIdx.x; idx < P * NzH; idx += blockDim.x) {
+    int pb, k;
+    fdivmod(idx, g.fNzH, pb, k);
+    const int line = 2 * (p0 + pb);
     const C zk = res[k * P + pb];
     const C zm = res[(k == 0 ? 0 : Nz - k) * P + pb];
-    const T h = T(0.5) * s;
-    C o;
-    if ((ll & 1) == 0) o = C{h * (zk.x + zm.x), h * (zk.y - zm.y)};
-    else o = C{h * (zk.y + zm.y), -h * (zk.x - zm.x)};
-    out[(size_t)line * NzH + k] = o;
+    C *o = out + (size_t)line * NzH + k;
+    if (line < g.lines) o[0] = C{h * (zk.x + zm.x), h * (zk.y - zm.y)};
+    if (line + 1 < g.lines) o[NzH] = C{h * (zk.y + zm.y), -h * (zk.x - zm.x)};
   }
 }
 
@@ -389,6 +388,28 @@ struct LocalArgs {
   // with h the Hessian of phi at the bulk weighted densities (0: off).
   float pc_inv_nb, pc_h33, pc_h32x2, pc_h22, pc_hvv, pc_inv_kTdV;
   DfPhiConst dfk;  // the FP64 form's double-float Phi
+  // FP32 copies for the mixed form's kernels: converted in the kernels they
+  // cost up to four FP64-pipe instructions a point (the compiler does not
+  // hoist them out of the terms' branches)
+  float kTf, muf, inv_nQf, dVf, cf;  // cf = dV kT
+  void set_floats() {
+    kTf = (float)kT;
+    muf = (float)mu;
+    inv_nQf = (float)inv_nQ;
+    dVf = (float)dV;
+    cf = (float)(dV * kT);
+  }
+};
+// The local terms' constants in U.
+template <typename U> struct LocalConsts {
+  U kT, mu, inv_nQ, dV, c;
+  __device__ __forceinline__ explicit LocalConsts(const LocalArgs &a) {
+    if constexpr (sizeof(U) == 4) {
+      kT = a.kTf, mu = a.muf, inv_nQ = a.inv_nQf, dV = a.dVf, c = a.cf;
+    } else {
+      kT = U(a.kT), mu = U(a.mu), inv_nQ = U(a.inv_nQ), dV = U(a.dV), c = U(a.dV * a.kT);
+    }
+  }
 };
 
 // The bulk density nb in equilibrium with the chemical-potential term of f
@@ -452,9 +473,7 @@ double bulk_density_of(double R, double kT, double mu, int hs) {
   memset(&la, 0, sizeof(la));
   la.dV = 1.0;
   WbRadius wr;
-  wr.inv_4piR = 1.0 / (4 * M_PI * R);
-  wr.inv_4piR2 = 1.0 / (4 * M_PI * R * R);
-  wr.kind = hs;
+  wb_radius(wr, R, hs);
   return bulk_structure(f, nQ_of(kT), wr, la);
 }
 
@@ -1278,35 +1297,33 @@ __device__ __forceinline__ dfl half_of(dfl x) { return df_ldexp(x, 0.5f); }
 template <typename T, int RN = 0>
 __device__ void z_r2c_store5(typename Cplx<T>::type *res, typename Cplx<T>::type *other,
                              typename Cplx<T>::type *__restrict__ S5, const Geom &g,
-                             const FftPlan &pz, const FastDiv &fP, const FastDiv &f2P,
-                             const FastDiv &f5P, int p0) {
+                             const FftPlan &pz, const FastDiv &fP, const FastDiv &f5P, int p0) {
   using C = typename Cplx<T>::type;
   const int P = (int)fP.d, P5 = 5 * P, Nz = g.Nz, NzH = g.NzH;
   const C *out = fft_tile<T, -1, RN>(res, other, f5P, pz);
   #pragma unroll 4
-  for (int idx = threadIdx.x; idx < 10 * P * NzH; idx += blockDim.x) {
-    int lb, k, a, ll;
-    fdivmod(idx, g.fNzH, lb, k);
-    fdivmod(lb, f2P, a, ll);
-    const int line = 2 * p0 + ll;
-    if (line >= g.lines) continue;
-    const int b = a * P + (ll >> 1);
+  for (int idx = threadIdx.x; idx < P5 * NzH; idx += blockDim.x) {
+    int b, k, a, pb;
+    fdivmod(idx, g.fNzH, b, k);
+    fdivmod(b, fP, a, pb);
+    const int line = 2 * (p0 + pb);
     const C zk = out[k * P5 + b];
     const C zm = out[(k == 0 ? 0 : Nz - k) * P5 + b];
-    C o;
-    if ((ll & 1) == 0) o = C{half_of(zk.x + zm.x), half_of(zk.y - zm.y)};
-    else o = C{half_of(zk.y + zm.y), half_of(zm.x - zk.x)};
-    S5[(size_t)a * g.NC + (size_t)line * NzH + k] = o;
+    C *o = S5 + (size_t)a * g.NC + (size_t)line * NzH + k;
+    if (line < g.lines) o[0] = C{half_of(zk.x + zm.x), half_of(zk.y - zm.y)};
+    if (line + 1 < g.lines) o[NzH] = C{half_of(zk.y + zm.y), half_of(zm.x - zk.x)};
   }
 }
 
 // c2r of the five weighted densities, phi and local terms, per-block
 // energies, and (GRAD) r2c of the five partials dV kT dphi/dn_a in place.
-// The shared-memory FP32 form asks for 5 blocks per SM (48 registers, 20 B
-// of spills): 88 us at 128^3 against 92 us with ptxas's own choice (64
-// registers).  A 6-block cap spills 76 B.
+// Issue-bound (FP32: 680 instructions a point at 96^3); the FP32 form asks for 3
+// blocks per SM (80 registers, what its shared memory leaves room for): with 4
+// the radix-16 passes spill 44 B, with 5 (48 registers) 72 B.  128^3 in FP32:
+// 73 us with single radices and 5 blocks, 64 with the density read one round
+// ahead and conversions off the FP64 pipe, 55 with passes of 8 x 16.
 #ifndef DEFT_Z_PHI_MIN_BLOCKS
-#define DEFT_Z_PHI_MIN_BLOCKS 5
+#define DEFT_Z_PHI_MIN_BLOCKS 3
 #endif
 // The pointwise logarithm of the FP64 forms: by table (logtab.cuh) beside the
 // double-float transforms.
@@ -1322,8 +1339,7 @@ __global__ void __launch_bounds__(kThreads,
     k_z_phi(typename Cplx<T>::type *S5,
                                                     const R *__restrict__ n,
                                                     const R *__restrict__ V, Geom g,
-                                                    FftPlan pz, FastDiv fP, FastDiv f2P,
-                                                    FastDiv f5P, const LocalArgs *__restrict__ lap,
+                                                    FftPlan pz, FastDiv fP, FastDiv f5P, const LocalArgs *__restrict__ lap,
                                                     double *partials, double *__restrict__ lnq) {
   const LocalArgs la = *lap;
   const int P = (int)fP.d;
@@ -1340,19 +1356,24 @@ __global__ void __launch_bounds__(kThreads,
   using U = Acc<T>;
   U tacc[kNumTerms] = {0, 0, 0, 0, 0, 0};
   const bool hs = la.terms & kTermHS;
-  const U inv_nQ = U(la.inv_nQ);
-  const U c = U(la.dV * la.kT);
-  #pragma unroll (is_df<T> ? 1 : 4)
-  for (int idx = threadIdx.x; idx < 2 * P * Nz; idx += blockDim.x) {
+  const LocalConsts<U> lc(la);
+  const U inv_nQ = lc.inv_nQ, c = lc.c;
+  // the tile's lines are contiguous in the fields; the density is read one
+  // round ahead
+  const size_t r0 = (size_t)2 * p0 * Nz;
+  const int total = 2 * P * Nz, valid = (g.lines - 2 * p0) * Nz;
+  R nnext = (int)threadIdx.x < valid ? n[r0 + threadIdx.x] : R(0);
+  #pragma unroll 1
+  for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
     int ll, z;
     fdivmod(idx, g.fNz, ll, z);
-    const int line = 2 * p0 + ll;
     T *cell = reinterpret_cast<T *>(res + z * P5 + (ll >> 1)) + (ll & 1);  // field 0
     const int fstride = 2 * P;  // T elements between fields
     T d[5] = {0, 0, 0, 0, 0};
-    if (line < g.lines) {
-      const size_t r = (size_t)line * Nz + z;
-      const U nv = U(n[r]);
+    const U nv = real_from<U>(nnext);
+    if (idx + (int)blockDim.x < valid) nnext = n[r0 + idx + blockDim.x];
+    if (idx < valid) {
+      const size_t r = r0 + idx;
       if (hs) {
         T w[5];
 #pragma unroll
@@ -1377,7 +1398,7 @@ __global__ void __launch_bounds__(kThreads,
         if (lnq) lnq[r] = double(lg);
       }
       if (la.terms & kTermMu) tacc[4] += nv;
-      if (la.terms & kTermVext) tacc[5] += U(V[r]) * nv;
+      if (la.terms & kTermVext) tacc[5] += real_from<U>(V[r]) * nv;
     }
     if (GRAD) {
 #pragma unroll
@@ -1392,7 +1413,7 @@ __global__ void __launch_bounds__(kThreads,
   block_reduce_terms<U>(tacc, la, red, partials);
   if (!GRAD) return;
   __syncthreads();
-  z_r2c_store5<T, RN>(res, res == A ? Bf : A, S5, g, pz, fP, f2P, f5P, p0);
+  z_r2c_store5<T, RN>(res, res == A ? Bf : A, S5, g, pz, fP, f5P, p0);
 }
 
 // c2r of the adjoint sum, + local gradient terms, masked.
@@ -1415,39 +1436,67 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_grad(const typename Cplx<T>::type *__res
   const bool hs = la.terms & kTermHS;
   const C *res = nullptr;
   using U = Acc<T>;
+  const LocalConsts<U> lc(la);
   U dacc[3] = {0, 0, 0};
   if (hs) {
     pack_c2r<T>(in, buf0, g, p0, P);
     res = fft_tile<T, +1, RN>(buf0, buf1, fP, pz);
   }
-  #pragma unroll 4
-  for (int idx = threadIdx.x; idx < 2 * P * g.Nz; idx += blockDim.x) {
-    int ll, z;
-    fdivmod(idx, g.fNz, ll, z);
-    const int line = 2 * p0 + ll;
-    if (line >= g.lines) continue;
-    const size_t r = (size_t)line * g.Nz + z;
-    U conv = 0;
-    if (hs) {
-      const C v = res[z * P + (ll >> 1)];
-      conv = U((ll & 1) ? v.y : v.x);
+  // four points a thread and round, each input's loads under one test of its
+  // term (a test per point puts every load behind the previous point's
+  // logarithm)
+  constexpr int Q = 4;
+  const int total = 2 * P * g.Nz, valid = (g.lines - 2 * p0) * g.Nz;
+  const int end = total < valid ? total : valid;
+  const size_t r0 = (size_t)2 * p0 * g.Nz;  // the tile's lines are contiguous
+  const bool ideal = la.terms & kTermIdeal, vext = la.terms & kTermVext,
+             masked = la.terms & kTermMask;
+  for (int i0 = threadIdx.x; i0 < end; i0 += Q * blockDim.x) {
+    U loc[Q], conv[Q], vv[Q], mv[Q];
+    auto each = [&](auto f) {
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        const int idx = i0 + q * blockDim.x;
+        if (idx < end) f(q, idx);
+      }
+    };
+#pragma unroll
+    for (int q = 0; q < Q; q++) loc[q] = conv[q] = vv[q] = U(0), mv[q] = U(1);
+    if (ideal) {
+      if (lnq) each([&](int q, int i) { loc[q] = U(lnq[r0 + i]); });
+      else each([&](int q, int i) { loc[q] = real_from<U>(n[r0 + i]); });
     }
-    U loc = 0;
-    if (la.terms & kTermIdeal)
-      loc += U(la.kT) * (lnq ? U(lnq[r]) : local_log<T>(U(n[r]) * U(la.inv_nQ)));
-    if (la.terms & kTermMu) loc += U(la.mu);
-    if (la.terms & kTermVext) loc += U(V[r]);
-    U gr = conv + U(la.dV) * loc;
-    if (la.terms & kTermMask) {
-      const U m = U(mask[r]);
-      gr = m == U(0) ? U(0) : m * gr;
-    }
-    grad[r] = double(gr);
+    if (vext) each([&](int q, int i) { vv[q] = real_from<U>(V[r0 + i]); });
+    if (masked) each([&](int q, int i) { mv[q] = real_from<U>(mask[r0 + i]); });
+    if (hs)
+      each([&](int q, int i) {
+        int ll, z;
+        fdivmod(i, g.fNz, ll, z);
+        const C v = res[z * P + (ll >> 1)];
+        conv[q] = U((ll & 1) ? v.y : v.x);
+      });
+    each([&](int q, int i) {
+      U lo = 0;
+      if (ideal) lo += lc.kT * (lnq ? loc[q] : local_log<T>(loc[q] * lc.inv_nQ));
+      if (la.terms & kTermMu) lo += lc.mu;
+      if (vext) lo += vv[q];
+      U gr = conv[q] + lc.dV * lo;
+      if (masked) gr = mv[q] == U(0) ? U(0) : mv[q] * gr;
+      conv[q] = gr;
+      grad[r0 + i] = real_from<double>(gr);
+    });
     // per-thread sums in U (a dozen terms; FP32 products of the FP32
     // gradient), the block and grid sums in FP64
 #pragma unroll
-    for (int i = 0; i < 3; i++)
-      if (i < gd.k) dacc[i] += gr * (gd.b[i] ? U(gd.b[i][r]) : gr);
+    for (int i = 0; i < 3; i++) {
+      if (i >= gd.k) continue;
+      if (gd.b[i]) {
+        each([&](int q, int j) { vv[q] = real_from<U>(gd.b[i][r0 + j]); });
+        each([&](int q, int) { dacc[i] += conv[q] * vv[q]; });
+      } else {
+        each([&](int q, int) { dacc[i] += conv[q] * conv[q]; });
+      }
+    }
   }
   if (gd.k > 0) {
     __shared__ double dred[32 * 3];
@@ -1506,10 +1555,9 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_hess(const typename Cplx<T>::type *__res
 // perturbations dw, dP = dV kT J dw with the stored blocks, r2c of dP in place.
 template <typename T, int RN = 0>
 __global__ void DEFT_FFT_BOUNDS(RN) k_z_jac(typename Cplx<T>::type *S5, Geom g, FftPlan pz,
-                                                    FastDiv fP, FastDiv f2P, FastDiv f5P,
+                                                    FastDiv fP, FastDiv f5P,
                                                     const LocalArgs *__restrict__ lap,
                                                     const float *__restrict__ hess) {
-  const double c = lap->dV * lap->kT;
   const int P = (int)fP.d;
   using C = typename Cplx<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1518,7 +1566,7 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_jac(typename Cplx<T>::type *S5, Geom g, 
   const int Nz = g.Nz, P5 = 5 * P;
   const int p0 = blockIdx.x * P;
   C *res = z_load5_c2r<T, RN>(S5, A, Bf, g, pz, fP, f5P, p0);
-  const T cc = T(c);
+  const T cc = LocalConsts<T>(*lap).c;
   #pragma unroll 4
   for (int idx = threadIdx.x; idx < 2 * P * Nz; idx += blockDim.x) {
     int ll, z;
@@ -1544,7 +1592,7 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_jac(typename Cplx<T>::type *S5, Geom g, 
     for (int a = 0; a < 5; a++) cell[a * fs] = cc * o[a];
   }
   __syncthreads();
-  z_r2c_store5<T, RN>(res, res == A ? Bf : A, S5, g, pz, fP, f2P, f5P, p0);
+  z_r2c_store5<T, RN>(res, res == A ? Bf : A, S5, g, pz, fP, f5P, p0);
 }
 
 // Hessian-vector product, last stage: c2r of the adjoint sum plus the
@@ -1556,6 +1604,7 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_hvp_out(
     Geom g, FftPlan pz, FastDiv fP, const LocalArgs *__restrict__ lap, double *dpart,
     unsigned int *counter, double *dout) {
   const LocalArgs la = *lap;
+  const LocalConsts<T> lc(la);
   T pq[1] = {0};  // per-thread sum in T (a dozen terms), block and grid sums in FP64
   const int P = (int)fP.d;
   using C = typename Cplx<T>::type;
@@ -1569,27 +1618,36 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_hvp_out(
     pack_c2r<T>(in, buf0, g, p0, P);
     res = fft_tile<T, +1, RN>(buf0, buf1, fP, pz);
   }
-  #pragma unroll 4
-  for (int idx = threadIdx.x; idx < 2 * P * g.Nz; idx += blockDim.x) {
-    int ll, z;
-    fdivmod(idx, g.fNz, ll, z);
-    const int line = 2 * p0 + ll;
-    if (line >= g.lines) continue;
-    const size_t r = (size_t)line * g.Nz + z;
-    T conv = 0;
-    if (hs) {
-      const C v = res[z * P + (ll >> 1)];
-      conv = (ll & 1) ? v.y : v.x;
-    }
-    const double dxv = dx[r];
-    const T dxt = T(dxv);
-    T o = conv + T(la.dV) * T(hloc[r]) * dxt;
-    if (la.terms & kTermMask) {
-      const T m = T(mask[r]);
-      o = m == T(0) ? T(0) : m * o;
-    }
-    out[r] = double(o);
-    pq[0] += dxt * o;
+  constexpr int Q = 4;  // points a thread and round, as in k_z_grad
+  const int total = 2 * P * g.Nz, valid = (g.lines - 2 * p0) * g.Nz;
+  const int end = total < valid ? total : valid;
+  const size_t r0 = (size_t)2 * p0 * g.Nz;
+  const bool masked = la.terms & kTermMask;
+  for (int i0 = threadIdx.x; i0 < end; i0 += Q * blockDim.x) {
+    T dxt[Q], hl[Q], mv[Q];
+    auto each = [&](auto f) {
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        const int idx = i0 + q * blockDim.x;
+        if (idx < end) f(q, idx);
+      }
+    };
+    each([&](int q, int i) { dxt[q] = real_from<T>(dx[r0 + i]); });
+    each([&](int q, int i) { hl[q] = T(hloc[r0 + i]); });
+    if (masked) each([&](int q, int i) { mv[q] = real_from<T>(mask[r0 + i]); });
+    each([&](int q, int i) {
+      T conv = 0;
+      if (hs) {
+        int ll, z;
+        fdivmod(i, g.fNz, ll, z);
+        const C v = res[z * P + (ll >> 1)];
+        conv = (ll & 1) ? v.y : v.x;
+      }
+      T o = conv + lc.dV * hl[q] * dxt[q];
+      if (masked) o = mv[q] == T(0) ? T(0) : mv[q] * o;
+      out[r0 + i] = real_from<double>(o);
+      pq[0] += dxt[q] * o;
+    });
   }
   // dout: dx.out by the last block to finish, in block order
   if (dout) {
@@ -1678,7 +1736,7 @@ __global__ void __launch_bounds__(32 * kZWarps)
 #pragma unroll
   for (int m = 0; m < E; m++) {
     const size_t r = (size_t)l0 * N + lane + 32 * m;
-    v[m] = make_float2(a0 ? float(in[r]) : 0.f, a1 ? float(in[r + N]) : 0.f);
+    v[m] = make_float2(a0 ? real_from<float>(in[r]) : 0.f, a1 ? real_from<float>(in[r + N]) : 0.f);
   }
   warp_n2s<-1, E>(v, lane, tw, w);
   warp_unpack_store<E>(v, lane, s, wb, out + (size_t)l0 * NzH, zwarp_nvalid(l0, g));
@@ -1699,29 +1757,46 @@ __global__ void __launch_bounds__(32 * kZWarps)
   float2 *wb = reinterpret_cast<float2 *>(smem_raw) + warp * warp_buf_elems<E>();
   const int l0 = 2 * (blockIdx.x * kZWarps + warp);
   const bool hs = la.terms & kTermHS;
-  // the pointwise inputs (and the local gradient terms) first, so their
-  // loads are in flight while the line is transformed
+  // the pointwise inputs first, so their loads are in flight while the line
+  // is transformed; each input's 2 E loads under one test of its term (a test
+  // per point puts every load behind the previous point's logarithm: 36 us a
+  // gradient at 128^3 against 18.6)
   float loc[2][E], mk[2][E], bv[3][2][E];
-#pragma unroll
-  for (int half = 0; half < 2; half++) {
-    const bool ok = l0 + half < g.lines;
+  const bool ok0 = l0 < g.lines, ok1 = l0 + 1 < g.lines;
+  auto load2 = [&](const R *src, float (&dst)[2][E], float other) {
+    const R *q = src + (size_t)l0 * N + lane;
+    R t[2][E];
 #pragma unroll
     for (int m = 0; m < E; m++) {
-      const size_t r = (size_t)(l0 + half) * N + lane + 32 * m;
-      float lc = 0, mv = 1;
-      if (ok) {
-        if (la.terms & kTermIdeal)
-          lc += float(la.kT) * wb_log<float>(float(n[r]) * float(la.inv_nQ));
-        if (la.terms & kTermMu) lc += float(la.mu);
-        if (la.terms & kTermVext) lc += float(V[r]);
-        if (la.terms & kTermMask) mv = float(mask[r]);
-      }
-      loc[half][m] = lc;
-      mk[half][m] = mv;
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-        bv[i][half][m] = (ok && i < gd.k && gd.b[i]) ? float(gd.b[i][r]) : 0.f;
+      t[0][m] = ok0 ? q[32 * m] : R(0);
+      t[1][m] = ok1 ? q[N + 32 * m] : R(0);
     }
+#pragma unroll
+    for (int m = 0; m < E; m++) {
+      dst[0][m] = ok0 ? real_from<float>(t[0][m]) : other;
+      dst[1][m] = ok1 ? real_from<float>(t[1][m]) : other;
+    }
+  };
+  const bool ideal = la.terms & kTermIdeal, vext = la.terms & kTermVext;
+  if (ideal) load2(n, loc, 1.f);
+  if (vext) load2(V, bv[0], 0.f);  // folded into loc before the dots' vectors are read
+  if (la.terms & kTermMask) load2(mask, mk, 1.f);
+  else
+#pragma unroll
+    for (int m = 0; m < E; m++) mk[0][m] = mk[1][m] = 1.f;
+#pragma unroll
+  for (int half = 0; half < 2; half++) {
+#pragma unroll
+    for (int m = 0; m < E; m++) {
+      float lc = ideal ? la.kTf * wb_log<float>(loc[half][m] * la.inv_nQf) : 0.f;
+      if (la.terms & kTermMu) lc += la.muf;
+      if (vext) lc += bv[0][half][m];
+      loc[half][m] = lc;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    if (i < gd.k && gd.b[i]) load2(gd.b[i], bv[i], 0.f);
   }
   float2 v[E];
   if (hs) {
@@ -1742,9 +1817,9 @@ __global__ void __launch_bounds__(32 * kZWarps)
     for (int m = 0; m < E; m++) {
       const size_t r = (size_t)line * N + lane + 32 * m;
       const float conv = half ? v[m].y : v[m].x;
-      float gr = conv + float(la.dV) * loc[half][m];
+      float gr = conv + la.dVf * loc[half][m];
       if (la.terms & kTermMask) gr = mk[half][m] == 0.f ? 0.f : mk[half][m] * gr;
-      grad[r] = R(gr);
+      grad[r] = real_from<R>(gr);
 #pragma unroll
       for (int i = 0; i < 3; i++)
         if (i < gd.k) dacc[i] += gr * (gd.b[i] ? bv[i][half][m] : gr);
@@ -1791,17 +1866,28 @@ __global__ void __launch_bounds__(32 * kZWarps)
   for (int half = 0; half < 2; half++) {
     const int line = l0 + half;
     if (line >= g.lines) continue;
+    const size_t r0 = (size_t)line * N + lane;
+    R dxr[E], mr[E];  // a line's loads together, as in k_pc_out_warp
+    float hl[E];
 #pragma unroll
     for (int m = 0; m < E; m++) {
-      const size_t r = (size_t)line * N + lane + 32 * m;
+      dxr[m] = dx[r0 + 32 * m];
+      hl[m] = hloc[r0 + 32 * m];
+    }
+    if (la.terms & kTermMask) {
+#pragma unroll
+      for (int m = 0; m < E; m++) mr[m] = mask[r0 + 32 * m];
+    }
+#pragma unroll
+    for (int m = 0; m < E; m++) {
       const float conv = half ? v[m].y : v[m].x;
-      const float dxt = float(dx[r]);
-      float o = conv + float(la.dV) * hloc[r] * dxt;
+      const float dxt = real_from<float>(dxr[m]);
+      float o = conv + la.dVf * hl[m] * dxt;
       if (la.terms & kTermMask) {
-        const float mk = float(mask[r]);
+        const float mk = real_from<float>(mr[m]);
         o = mk == 0.f ? 0.f : mk * o;
       }
-      out[r] = R(o);
+      out[r0 + 32 * m] = real_from<R>(o);
       pq += dxt * o;
     }
   }
@@ -1828,16 +1914,36 @@ __global__ void __launch_bounds__(32 * kZWarps)
   float2 w[4];
   warp_stage_tw<-1, E>(tw, lane, w);
   const bool a0 = l0 < g.lines, a1 = l0 + 1 < g.lines;
+  const size_t r0 = (size_t)l0 * N + lane;
+  R nr[2][E], rr[2][E], mr[2][E];  // all loads first
+#pragma unroll
+  for (int half = 0; half < 2; half++) {
+    const bool ok = half ? a1 : a0;
+#pragma unroll
+    for (int m = 0; m < E; m++) {
+      nr[half][m] = ok ? n[r0 + half * N + 32 * m] : R(0);
+      rr[half][m] = ok ? rv[r0 + half * N + 32 * m] : R(0);
+    }
+  }
+  if (mask) {
+#pragma unroll
+    for (int m = 0; m < E; m++) {
+      mr[0][m] = a0 ? mask[r0 + 32 * m] : R(0);
+      mr[1][m] = a1 ? mask[r0 + N + 32 * m] : R(0);
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < E; m++) mr[0][m] = mr[1][m] = R(1);
+  }
   float2 v[E];
 #pragma unroll
   for (int m = 0; m < E; m++) {
-    const size_t r = (size_t)l0 * N + lane + 32 * m;
-    float u0 = 0.f, u1 = 0.f;
-    if (a0) u0 = pc_point_scale(mask ? float(mask[r]) : 1.f, float(n[r]), inv_nb) * float(rv[r]);
-    if (a1)
-      u1 = pc_point_scale(mask ? float(mask[r + N]) : 1.f, float(n[r + N]), inv_nb) *
-           float(rv[r + N]);
-    v[m] = make_float2(u0, u1);
+    float u[2];
+#pragma unroll
+    for (int half = 0; half < 2; half++)
+      u[half] = pc_point_scale(real_from<float>(mr[half][m]), real_from<float>(nr[half][m]), inv_nb) *
+                real_from<float>(rr[half][m]);
+    v[m] = make_float2(a0 ? u[0] : 0.f, a1 ? u[1] : 0.f);
   }
   warp_n2s<-1, E>(v, lane, tw, w);
   warp_unpack_store<E>(v, lane, 1.0f, wb, out + (size_t)l0 * NzH, zwarp_nvalid(l0, g));
@@ -1870,15 +1976,35 @@ __global__ void __launch_bounds__(32 * kZWarps)
   for (int half = 0; half < 2; half++) {
     const int line = l0 + half;
     if (line >= g.lines) continue;
+    // a line's loads together, after the transform: held across it they cost
+    // a third of the resident warps (23 us at 128^3 against 16)
+    const size_t r0 = (size_t)line * N + lane;
+    R nr[E], ar[E], br[E], mr[E];
 #pragma unroll
     for (int m = 0; m < E; m++) {
-      const size_t r = (size_t)line * N + lane + 32 * m;
-      const float s = pc_point_scale(mask ? float(mask[r]) : 1.f, float(n[r]), inv_nb);
+      nr[m] = n[r0 + 32 * m];
+      ar[m] = a[r0 + 32 * m];
+    }
+    if (b) {
+#pragma unroll
+      for (int m = 0; m < E; m++) br[m] = b[r0 + 32 * m];
+    }
+    if (mask) {
+#pragma unroll
+      for (int m = 0; m < E; m++) mr[m] = mask[r0 + 32 * m];
+    } else {
+#pragma unroll
+      for (int m = 0; m < E; m++) mr[m] = R(1);
+    }
+#pragma unroll
+    for (int m = 0; m < E; m++) {
+      const float s =
+          pc_point_scale(real_from<float>(mr[m]), real_from<float>(nr[m]), inv_nb);
       const float zv = s * (half ? v[m].y : v[m].x);
-      z[r] = R(zv);
-      const float av = float(a[r]);
+      z[r0 + 32 * m] = real_from<R>(zv);
+      const float av = real_from<float>(ar[m]);
       acc[0] += zv * av;
-      if (b) acc[1] += zv * float(b[r]);
+      if (b) acc[1] += zv * real_from<float>(br[m]);
       acc[2] += av * av;
     }
   }
@@ -1907,8 +2033,7 @@ __global__ void __launch_bounds__(32 * kZWarps, DEFT_ZWARP5_MIN_BLOCKS)
   float2 v[5][E];
   if (hs) warp_load5_c2r<E>(S5, g, l0, nvalid, wb, lane, tw, v);
   float tacc[kNumTerms] = {0, 0, 0, 0, 0, 0};
-  const float inv_nQ = float(la.inv_nQ);
-  const float c = float(la.dV * la.kT);
+  const float inv_nQ = la.inv_nQf, c = la.cf;
 #pragma unroll
   for (int half = 0; half < 2; half++) {
     const int line = l0 + half;
@@ -1928,10 +2053,10 @@ __global__ void __launch_bounds__(32 * kZWarps, DEFT_ZWARP5_MIN_BLOCKS)
           tacc[1] += phi[1];
           tacc[2] += phi[2];
         }
-        const float nv = float(n[r]);
+        const float nv = real_from<float>(n[r]);
         if (la.terms & kTermIdeal) tacc[3] += ideal_energy_t<float>(nv, inv_nQ);
         if (la.terms & kTermMu) tacc[4] += nv;
-        if (la.terms & kTermVext) tacc[5] += float(V[r]) * nv;
+        if (la.terms & kTermVext) tacc[5] += real_from<float>(V[r]) * nv;
       }
       if (GRAD && hs) {
 #pragma unroll
@@ -1954,7 +2079,7 @@ __global__ void __launch_bounds__(32 * kZWarps, DEFT_ZWARP5_MIN_BLOCKS)
     k_z_jac_warp(float2 *S5, Geom g, const float2 *__restrict__ tw,
                  const LocalArgs *__restrict__ lap, const float *__restrict__ hess) {
   constexpr int N = 32 * E;
-  const float cc = float(lap->dV * lap->kT);
+  const float cc = lap->cf;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float2 *wb = reinterpret_cast<float2 *>(smem_raw) + warp * 5 * warp_buf_elems<E>();
@@ -2346,15 +2471,15 @@ __global__ void k_to_f32(const double *__restrict__ a, float *__restrict__ b, in
   DEFT_V4_LOOP(n) {
     const double2 u = reinterpret_cast<const double2 *>(a)[2 * i4];
     const double2 v = reinterpret_cast<const double2 *>(a)[2 * i4 + 1];
-    reinterpret_cast<float4 *>(b)[i4] = make_float4((float)u.x, (float)u.y, (float)v.x, (float)v.y);
+    reinterpret_cast<float4 *>(b)[i4] = make_float4(d2f_small(u.x), d2f_small(u.y), d2f_small(v.x), d2f_small(v.y));
   }
-  DEFT_V4_TAIL(n) b[i] = (float)a[i];
+  DEFT_V4_TAIL(n) b[i] = d2f_small(a[i]);
 }
 __global__ void k_to_f64(const float *__restrict__ a, double *__restrict__ b, int n) {
   DEFT_V4_LOOP(n) {
     const float4 u = reinterpret_cast<const float4 *>(a)[i4];
-    reinterpret_cast<double2 *>(b)[2 * i4] = make_double2(u.x, u.y);
-    reinterpret_cast<double2 *>(b)[2 * i4 + 1] = make_double2(u.z, u.w);
+    reinterpret_cast<double2 *>(b)[2 * i4] = make_double2(f2d(u.x), f2d(u.y));
+    reinterpret_cast<double2 *>(b)[2 * i4 + 1] = make_double2(f2d(u.z), f2d(u.w));
   }
   DEFT_V4_TAIL(n) b[i] = (double)a[i];
 }
@@ -2613,6 +2738,47 @@ bool factorize(int n, FftPlan &p) {
   return n == 1;
 }
 
+// The FP32 plan's order: the fewest passes of the radices fuse_passes can make
+// (16, 12, 10 beside the plain ones), the smallest largest radix among those
+// (80 = 10 x 8 rather than 16 x 5), written out in plain radices.
+bool factorize_f32(int n, FftPlan &p) {
+  static const int cand[] = {16, 13, 12, 11, 10, 8, 7, 5, 4, 3, 2};
+  int best[kMaxPasses], nbest = kMaxPasses + 1, cur[kMaxPasses];
+  std::function<void(int, int, int)> go = [&](int rest, int from, int k) {
+    if (rest == 1) {
+      // candidates run from the largest first radix down: an equal count with
+      // a smaller largest radix comes later and wins
+      if (k <= nbest) {
+        nbest = k;
+        std::copy(cur, cur + k, best);
+      }
+      return;
+    }
+    if (k + 1 > nbest || k >= kMaxPasses) return;
+    for (int i = from; i < (int)(sizeof(cand) / sizeof(cand[0])); i++)
+      if (rest % cand[i] == 0) {
+        cur[k] = cand[i];
+        go(rest / cand[i], i, k + 1);
+      }
+  };
+  go(n, 0, 0);
+  if (nbest > kMaxPasses) return false;
+  int k = 0;
+  for (int i = 0; i < nbest; i++) {
+    const int r = best[i];
+    if (k + 2 > kMaxPasses) return false;
+    if (r == 16 || r == 12 || r == 10) {
+      p.radix[k++] = r == 10 ? 2 : 4;
+      p.radix[k++] = r == 16 ? 4 : r == 12 ? 3 : 5;
+    } else {
+      p.radix[k++] = r;
+    }
+  }
+  p.npass = k;
+  fuse_passes(p);
+  return true;
+}
+
 double det3(const double m[9]) {
   return m[0] * (m[4] * m[8] - m[5] * m[7]) - m[1] * (m[3] * m[8] - m[5] * m[6]) +
          m[2] * (m[3] * m[7] - m[4] * m[6]);
@@ -2651,7 +2817,7 @@ double bulk_density(double R, double kT, double mu, int hs) {
 // (cs = bytes of one complex element).
 struct Tiles {
   int By = 1, Bx = 1, Bxf = 1, Bxc = 1, Pz = 1, Pphi = 1;
-  FastDiv fBy{}, fBx{}, fBxf{}, fBxc{}, f5Bxc{}, fPz{}, fPphi{}, f2Pphi{}, f5Pphi{};
+  FastDiv fBy{}, fBx{}, fBxf{}, fBxc{}, f5Bxc{}, fPz{}, fPphi{}, f5Pphi{};
   size_t smem_y = 0, smem_x2 = 0, smem_xf = 0, smem_xc = 0, smem_z = 0, smem_phi = 0;
   size_t smem_max() const {
     size_t m = smem_y;
@@ -2675,7 +2841,6 @@ void finish_tiles(Tiles &t, const Geom &g, size_t cs) {
   t.f5Bxc = make_fastdiv(5 * t.Bxc);
   t.fPz = make_fastdiv(t.Pz);
   t.fPphi = make_fastdiv(t.Pphi);
-  t.f2Pphi = make_fastdiv(2 * t.Pphi);
   t.f5Pphi = make_fastdiv(5 * t.Pphi);
   t.smem_y = 2 * (size_t)g.Ny * t.By * cs;
   t.smem_x2 = 2 * (size_t)g.Nx * t.Bx * cs;
@@ -2683,6 +2848,37 @@ void finish_tiles(Tiles &t, const Geom &g, size_t cs) {
   t.smem_xc = 10 * (size_t)g.Nx * t.Bxc * cs;
   t.smem_z = 2 * (size_t)g.Nz * t.Pz * cs;
   t.smem_phi = 10 * (size_t)g.Nz * t.Pphi * cs;
+}
+
+// Groups (line pairs or columns) of five fields a block of the FP32 kernels
+// takes, of `count`, in the length n of plan p.  A block's time is modelled as
+// 12 + sum over the passes of rounds x radix (a round: 256 threads, a butterfly
+// each), a launch's as that times ceil(L / R) + L / 10, with L blocks an SM of
+// which R = 3 are resident (registers) or fewer (shared memory).  Measured
+// against the widest tiles of the budget: Phi 128^3 6 pairs 59 us against 66
+// with 9, 96^3 6 pairs 32.7 against 34.8 with 9, 64^3 5 pairs 14.3 against 20.4
+// with 13, 48^3 4 pairs 12.2 against 16.6 with 15; adjoint convolution 96^3 6
+// columns 27.2 against 33.1 with 9, 80^3 8 columns 16.4 against 18.4 with 11,
+// 48^3 4 columns 12.3 against 16.4 with 16.
+int five_field_tile(const FftPlan &p, int n, int count, size_t budget, int sms) {
+  int best = 1;
+  double best_cost = 0;
+  for (int P = 1; P <= 16 && P <= count; P++) {
+    const size_t smem = 10 * (size_t)n * P * sizeof(float2);
+    if (P > 1 && smem > budget) break;
+    int work = 12;
+    for (int i = 0; i < p.npass; i++)
+      work += (5 * P * (n / p.radix[i]) + kThreads - 1) / kThreads * p.radix[i];
+    const int fit = (int)(220 * 1024 / smem), R = fit < 1 ? 1 : fit < 3 ? fit : 3;
+    const int blocks = (count + P - 1) / P, L = (blocks + sms - 1) / sms;
+    const double cost = work * ((L + R - 1) / R + 0.1 * L);
+    // equal costs: odd counts, whose z-strided shared accesses are free of conflicts
+    if (P == 1 || cost < best_cost || (cost == best_cost && P % 2 == 1)) {
+      best = P;
+      best_cost = cost;
+    }
+  }
+  return best;
 }
 
 // Built-in rule: the widest tiles within `budget` bytes of shared memory (at
@@ -2725,6 +2921,11 @@ Tiles make_tiles(const Geom &g, size_t cs, size_t budget, const TileChoice *ov =
       for (int i = 0; i < px.npass; i++) rmin = least(rmin, px.radix[i]);
     t.Bxf = least(t.Bxf, most(4, 256 * rmin / g.Nx));
     t.Bxc = least(t.Bxc, 4);
+  } else {
+    constexpr int kSms = 152;
+    FftPlan px, pz;
+    if (factorize_f32(g.Nx, px)) t.Bxc = five_field_tile(px, g.Nx, g.Ny * g.NzH, budget, kSms);
+    if (factorize_f32(g.Nz, pz)) pm = five_field_tile(pz, g.Nz, pairs, budget, kSms);
   }
   t.Pphi = pm < pairs ? pm : pairs;
   if (ov) {
@@ -2754,6 +2955,7 @@ bool set_radix_order(FftPlan &p, const int *r) {
   }
   if (k == 0 || prod != p.n) return false;
   p.npass = k;
+  p.nord = 0;
   for (int i = 0; i < k; i++) p.radix[i] = tmp[i];
   plan_fill_ns(p);
   p.reg = 0;
@@ -2766,6 +2968,7 @@ bool set_reg_order(FftPlan &p, const int *r) {
   if (!(r[0] == 16 && r[1] > 0 && r[2] == 0 && 16 * r[1] == p.n && reg_fft_length(p.n)))
     return false;
   p.reg = 1;
+  p.nord = 0;
   p.npass = 2;
   p.radix[0] = 16;
   p.radix[1] = r[1];
@@ -2966,6 +3169,7 @@ class EngineImpl {
     }
     plan_fill_ns(p);
     pf = p;
+    if (!factorize_f32(n, pf)) pf = p;
     pd = p;
     std::vector<double2> h(n);
     std::vector<float2> hf(n);
@@ -3254,11 +3458,12 @@ class EngineImpl {
     }
     FftPlan np[3] = {f32 ? pxf : px, f32 ? pyf : py, f32 ? pzf : pz};
     for (int a = 0; a < 3; a++) {
-      if (c.radix[a][0] && !(f32 && set_reg_order(np[a], c.radix[a])) &&
-          !set_radix_order(np[a], c.radix[a])) {
+      if (!c.radix[a][0] || (f32 && set_reg_order(np[a], c.radix[a]))) continue;
+      if (!set_radix_order(np[a], c.radix[a])) {
         err = "radix order does not factor axis " + std::to_string(a);
         return -1;
       }
+      if (f32) fuse_passes(np[a]);
     }
     const int need = pairs_tiles(t.Pphi);
     if (need > max_blocks) {
@@ -3305,7 +3510,10 @@ class EngineImpl {
     c->Pphi = t.Pphi;
     const FftPlan *pl[3] = {f32 ? &pxf : &px, f32 ? &pyf : &py, f32 ? &pzf : &pz};
     for (int a = 0; a < 3; a++)
-      for (int i = 0; i < 8; i++) c->radix[a][i] = i < pl[a]->npass ? pl[a]->radix[i] : 0;
+      for (int i = 0; i < 8; i++) {
+        if (pl[a]->nord) c->radix[a][i] = i < pl[a]->nord ? pl[a]->order[i] : 0;
+        else c->radix[a][i] = i < pl[a]->npass ? pl[a]->radix[i] : 0;
+      }
   }
 
   // Pencil kernels for the FP32 and double-float x and y transforms of
@@ -3561,9 +3769,8 @@ class EngineImpl {
     la.nQ = nQ_of(f.kT);
     la.inv_nQ = 1.0 / la.nQ;
     la.dV = g.dV;
-    la.wr.inv_4piR = 1.0 / (4 * M_PI * f.R);
-    la.wr.inv_4piR2 = 1.0 / (4 * M_PI * f.R * f.R);
-    la.wr.kind = f.hs;
+    wb_radius(la.wr, f.R, f.hs);
+    la.set_floats();
     la.terms = f.terms;
     la.dfk = df_phi_const(la.wr, g.dV * f.kT);
     if (f.terms & kTermHS) {
@@ -3834,11 +4041,11 @@ class EngineImpl {
           constexpr int RN = decltype(rn)::value;
           if (grad)
             k_z_phi<T, true, RN, R><<<nblk, kThreads, t.smem_phi, stream>>>(
-                spec5<T>(), n, V, g, plan<T>(2), t.fPphi, t.f2Pphi, t.f5Pphi, la_dev, partials,
+                spec5<T>(), n, V, g, plan<T>(2), t.fPphi, t.f5Pphi, la_dev, partials,
                 lnq_for<T>(f));
           else
             k_z_phi<T, false, RN, R><<<nblk, kThreads, t.smem_phi, stream>>>(
-                spec5<T>(), n, V, g, plan<T>(2), t.fPphi, t.f2Pphi, t.f5Pphi, la_dev, partials,
+                spec5<T>(), n, V, g, plan<T>(2), t.fPphi, t.f5Pphi, la_dev, partials,
                 nullptr);
         });
       }
@@ -4063,7 +4270,7 @@ class EngineImpl {
         with_rn<float>(plan<float>(2), [&](auto rn) {
           k_z_jac<float, decltype(rn)::value><<<pairs_tiles(t32.Pphi), kThreads, t32.smem_phi,
                                                 stream>>>(spec5<float>(), g, plan<float>(2),
-                                                          t32.fPphi, t32.f2Pphi, t32.f5Pphi,
+                                                          t32.fPphi, t32.f5Pphi,
                                                           la_dev, hess);
         });
       }
@@ -4821,9 +5028,8 @@ int noalloc_energy_grad(const GridSpec &s, const FmtSpec &f, const double *n, co
   la.nQ = nQ_of(f.kT);
   la.inv_nQ = 1.0 / la.nQ;
   la.dV = g.dV;
-  la.wr.inv_4piR = 1.0 / (4 * M_PI * f.R);
-  la.wr.inv_4piR2 = 1.0 / (4 * M_PI * f.R * f.R);
-  la.wr.kind = f.hs;
+  wb_radius(la.wr, f.R, f.hs);
+  la.set_floats();
   la.terms = f.terms;
   // the kernels read it from the scratch array (pageable source, consumed on return)
   e = cudaMemcpyAsync(la_dev, &la, sizeof(la), cudaMemcpyHostToDevice, stream);
@@ -4846,7 +5052,7 @@ int noalloc_energy_grad(const GridSpec &s, const FmtSpec &f, const double *n, co
         S0, S5, w3, w2, wv, g, px, t.fBxf, la_dev);
     k_y_fft<double, +1><<<ygrid5, kThreads, t.smem_y, stream>>>(S5, g, py, t.fBy);
     k_z_phi<double, true><<<nblk_phi, kThreads, t.smem_phi, stream>>>(
-        S5, n, V, g, pz, t.fPphi, t.f2Pphi, t.f5Pphi, la_dev, partials, nullptr);
+        S5, n, V, g, pz, t.fPphi, t.f5Pphi, la_dev, partials, nullptr);
     k_y_fft<double, -1><<<ygrid5, kThreads, t.smem_y, stream>>>(S5, g, py, t.fBy);
     k_x_conv_adj<double><<<xt, kThreads, t.smem_xc, stream>>>(S5, S0, w3, w2, wv, g, px, t.fBxc,
                                                               t.f5Bxc, la_dev);

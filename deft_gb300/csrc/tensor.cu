@@ -315,9 +315,7 @@ int tensor_hs(Engine *e, const FmtSpec &f, const double *n, double *scratch, dou
     for (int c = 0; c < 3; c++) fw.add(kWtXY + c, nullptr, tb);
     if (e->spectrum(n) || e->fan_out(fw, 1, spec, w)) return fail(e->last_error());
     WbRadius wr;
-    wr.inv_4piR = 1 / (4 * kPi * f.R);
-    wr.inv_4piR2 = 1 / (4 * kPi * f.R * f.R);
-    wr.kind = kind == 1 ? kHsRosenfeld : kHsWhiteBear;
+    wb_radius(wr, f.R, kind == 1 ? kHsRosenfeld : kHsWhiteBear);
     const double c = g.dV * f.kT;
     k_tensor_phi_df<<<kBlocks, kThreads, 0, s>>>(kind, f.R, f.kT, c, df_phi_const(wr, c), n, w, NR,
                                                  grad != nullptr, partials);

@@ -128,9 +128,16 @@ template <int E> constexpr int warp_buf_elems() {
 template <int E>
 __device__ __forceinline__ void warp_stage_load(const float2 *__restrict__ src, int nvalid,
                                                 float2 *wb, int lane) {
-  constexpr int NzH = 16 * E + 1;
-  for (int i = lane; i < 2 * NzH; i += 32)
-    wb[wslot(i)] = i < nvalid ? src[i] : make_float2(0.f, 0.f);
+  // all loads first: with each stored as it arrives the lane waits for
+  // memory once per 32 values
+  constexpr int NV = 2 * (16 * E + 1), M = (NV + 31) / 32;
+  float2 t[M];
+#pragma unroll
+  for (int m = 0; m < M; m++)
+    t[m] = lane + 32 * m < nvalid ? src[lane + 32 * m] : make_float2(0.f, 0.f);
+#pragma unroll
+  for (int m = 0; m < M; m++)
+    if (lane + 32 * m < NV) wb[wslot(lane + 32 * m)] = t[m];
 }
 // The Hermitian-packed line Z = A + iB of full length, in spectral order,
 // from a staged buffer (only the real parts of the kz = 0 and Nyquist
@@ -186,7 +193,9 @@ __device__ __forceinline__ void warp_unpack_store(const float2 (&v)[E], int lane
     }
   }
   __syncwarp();
-  for (int i = lane; i < nvalid; i += 32) dst[i] = wb[wslot(i)];
+#pragma unroll
+  for (int m = 0; m < (2 * NzH + 31) / 32; m++)
+    if (lane + 32 * m < nvalid) dst[lane + 32 * m] = wb[wslot(lane + 32 * m)];
   __syncwarp();
 }
 

@@ -190,13 +190,30 @@ struct WbRadius {
   double inv_4piR;   // 1 / (4 pi R)
   double inv_4piR2;  // 1 / (4 pi R^2)
   int kind;          // kHs*
+  float inv_4piRf, inv_4piR2f;  // FP32 copies (a conversion a point is FP64-pipe work)
 };
+inline void wb_radius(WbRadius &r, double R, int kind) {
+  const double pi = 3.14159265358979323846;
+  r.inv_4piR = 1 / (4 * pi * R);
+  r.inv_4piR2 = 1 / (4 * pi * R * R);
+  r.kind = kind;
+  r.inv_4piRf = (float)r.inv_4piR;
+  r.inv_4piR2f = (float)r.inv_4piR2;
+}
+template <typename T> __host__ __device__ __forceinline__ T wb_a1(const WbRadius &r) {
+  if constexpr (sizeof(T) == 4) return r.inv_4piR2f;
+  else return T(r.inv_4piR2);
+}
+template <typename T> __host__ __device__ __forceinline__ T wb_a2(const WbRadius &r) {
+  if constexpr (sizeof(T) == 4) return r.inv_4piRf;
+  else return T(r.inv_4piR);
+}
 
 // phi = (phi3, phi1, phi2); d = d phi / d(n3, n2, vx, vy, vz).
 template <typename T>
 __host__ __device__ __forceinline__ void wb_phi(const WbRadius &r, T n3, T n2, T vx, T vy, T vz, T phi[3],
                                        T d[5]) {
-  const T a1 = T(r.inv_4piR2), a2 = T(r.inv_4piR);
+  const T a1 = wb_a1<T>(r), a2 = wb_a2<T>(r);
   const T v2 = vx * vx + vy * vy + vz * vz;
   const T u = T(1) / (T(1) - n3);
   const T l = wb_log<T>(T(1) - n3);
@@ -221,7 +238,7 @@ __host__ __device__ __forceinline__ void wb_phi(const WbRadius &r, T n3, T n2, T
 constexpr int kHessPacked = 10;  // h33 h32 h3x h3y h3z h22 h2x h2y h2z hvv
 template <typename T>
 __host__ __device__ __forceinline__ void wb_hess(const WbRadius &r, T n3, T n2, T vx, T vy, T vz, T h[10]) {
-  const T a1 = T(r.inv_4piR2), a2 = T(r.inv_4piR);
+  const T a1 = wb_a1<T>(r), a2 = wb_a2<T>(r);
   const T v2 = vx * vx + vy * vy + vz * vz;
   const T u = T(1) / (T(1) - n3);
   T f2[3], f3[3];
