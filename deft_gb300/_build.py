@@ -1,6 +1,6 @@
 """Builds the in-tree CUDA library deft_gb300/libdeft_gb300.so for sm_103a.
 
-Two translation units (the engine and the C ABI) compile in parallel with
+The translation units compile in parallel with
 nvcc and link into one shared object with the CUDA runtime linked
 statically, so the library loads without any path setup.
 """
@@ -17,7 +17,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libdeft_gb300.so")
 
 SOURCES = ["fmt_engine.cu", "deft_capi.cu", "batch.cu", "fno.cu", "contact.cu", "tensor.cu", "saft.cu",
-           "devcg.cu"]
+           "devcg.cu", "two_pass.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
          "--expt-relaxed-constexpr", "-I" + os.path.join(ROOT, "include")]

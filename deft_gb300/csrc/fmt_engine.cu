@@ -25,8 +25,10 @@
 #include "fft_smem.cuh"
 #include "fmt_engine.h"
 #include "pencil_fft.cuh"
+#include "two_pass.h"
 #include "warp_fft.cuh"
 #include "wb_phi.cuh"
+#include "weights_f.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -52,8 +54,6 @@ template <typename T> using Acc = std::conditional_t<is_df<T>, double, T>;
 
 // ---------------------------------------------------------------------------
 // Device helpers
-
-__device__ __forceinline__ int wrapm(int i, int N) { return i > N / 2 ? i - N : i; }
 
 __device__ __forceinline__ double kcomp(const Geom &g, int c, int x, int y, int z) {
   return g.Bm[3 * c] * wrapm(x, g.Nx) + g.Bm[3 * c + 1] * wrapm(y, g.Ny) + g.Bm[3 * c + 2] * z;
@@ -94,35 +94,6 @@ __device__ void weights_at(double k2, double R, double dr, double &w3, double &w
          (-kR2 * kR2 * kR2 * (1.0 / 120 / 6 / 7) + kR2 * kR2 * (1.0 / 120) - kR2 * (1.0 / 6) + 1);
     wv = (4 * M_PI) * R * R * R *
          (kR2 * kR2 * (1.0 / 5040 - 1.0 / 720) + kR2 * (1.0 / 24 - 1.0 / 120) - 1.0 / 3);
-  }
-}
-
-// The same weights in FP32, evaluated on the fly in the convolution kernels
-// (scale = dV/V folded in).  Below kR = 0.5 the closed forms lose digits to
-// cancellation in FP32, so the Taylor series of the reference's small-kR
-// branch is used there, times the smear factor (which is not 1 to FP32
-// precision at that threshold; at kR <= 1e-3, where the FP64 branch omits it,
-// the two differ by at most 6 (k dr)^2 < 3e-7).
-__device__ __forceinline__ void weights_at_f(float k2, float R, float dr, float scale, float &w3,
-                                             float &w2, float &wv) {
-  const float kk = sqrtf(k2);
-  const float kR = kk * R;
-  const float kdr = kk * dr;
-  const float smear = expf(-6.0f * kdr * kdr) * scale;
-  const float fpi = 12.566370614359172954f;
-  if (kR > 0.5f) {
-    float sn, cs;
-    sincosf(kR, &sn, &cs);
-    const float ik = 1.0f / kk;
-    w3 = smear * fpi * (sn - kR * cs) * ik * ik * ik;
-    w2 = smear * fpi * R * sn * ik;
-    wv = smear * fpi * ik * ik * (R * cs - sn * ik);
-  } else {
-    const float x = kR * kR, R3 = R * R * R;
-    w3 = smear * (fpi / 3) * R3 * (((-1.0f / 15120) * x + 1.0f / 280) * x - 0.1f) * x + smear * (fpi / 3) * R3;
-    w2 = smear * fpi * R * R * ((((-1.0f / 5040) * x + 1.0f / 120) * x - 1.0f / 6) * x + 1.0f);
-    wv = smear * fpi * R3 * (((1.0f / 5040 - 1.0f / 720) * x + (1.0f / 24 - 1.0f / 120)) * x -
-                             1.0f / 3);
   }
 }
 
@@ -830,35 +801,33 @@ __global__ void k_radial_table(int kind, Geom g, double R, dfl *__restrict__ out
 }
 
 // ---------------------------------------------------------------------------
-// Pencil kernels (FP32, lengths 32/64/128/256): register-resident transforms
-// of 32 adjacent columns per W warps (pencil_fft.cuh), loading and storing
-// global memory directly in 256-byte rows.
+// Pencil kernels (lengths 32/64/128/256): register-resident transforms of 32
+// adjacent columns per W warps (pencil_fft.cuh), loading and storing global
+// memory directly.
 
 // FFT along y of nf complex fields in place.  Columns c = x NzH + kz (all x
 // planes back to back); element y of column c at x Ny NzH + y NzH + kz.
 // grid = (column groups, fields).
-// T = dfl: 128 registers, i.e. 16 warps per SM.  Mean of a one-field and a
+// 128 registers, i.e. 16 warps per SM.  Mean of a one-field and a
 // five-field launch against the shared-memory passes: 128^3 53 -> 31 us, 256^3
 // 520 -> 300 us.
-template <int SIGN, int W, typename T = float>
-__global__ void __launch_bounds__(is_df<T> ? 32 * W : pencil_threads<W>(), is_df<T> ? 16 / W : 0)
-    k_y_pencil(typename Cplx<T>::type *data, Geom g,
-               const typename Cplx<T>::type *__restrict__ tw) {
-  using C = typename Cplx<T>::type;
-  constexpr int G = is_df<T> ? 1 : pencil_groups<W>(), P = 16 / W;
+template <int SIGN, int W>
+__global__ void __launch_bounds__(32 * W, 16 / W)
+    k_y_pencil(dfc *data, Geom g, const dfc *__restrict__ tw) {
+  constexpr int P = 16 / W;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w = warp % W, grp = warp / W;
-  auto *xs = reinterpret_cast<typename PencilXs<T>::type *>(smem_raw) + grp * pencil_xs_elems<W>();
-  const int c = (blockIdx.x * G + grp) * 32 + lane;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  dfl *xs = reinterpret_cast<dfl *>(smem_raw);
+  const int c = blockIdx.x * 32 + lane;
   const bool act = c < g.Nx * g.NzH;
   int x, kz;
   fdivmod(act ? c : 0, g.fNzH, x, kz);
-  C *base = data + (size_t)blockIdx.y * g.NC + (size_t)x * g.Ny * g.NzH + kz;
+  dfc *base = data + (size_t)blockIdx.y * g.NC + (size_t)x * g.Ny * g.NzH + kz;
   const int st = g.NzH;
-  C v[16];
+  dfc v[16];
 #pragma unroll
-  for (int m = 0; m < 16; m++) v[m] = act ? base[(w + W * m) * st] : C{0, 0};
-  pencil_n2s<T, SIGN, W>(v, xs, w, lane, tw);
+  for (int m = 0; m < 16; m++) v[m] = act ? base[(w + W * m) * st] : dfc{0, 0};
+  pencil_n2s<dfl, SIGN, W>(v, xs, w, lane, tw);
   if (act) {
 #pragma unroll
     for (int i = 0; i < P; i++)
@@ -867,151 +836,8 @@ __global__ void __launch_bounds__(is_df<T> ? 32 * W : pencil_threads<W>(), is_df
   }
 }
 
-// Shared weight slots of the pencil convolutions: three FP32 weights (w3,
-// w2, wv; dV/V folded in) for each of a thread's 16 spectral slots,
-// thread-private and conflict-free.
-__device__ __forceinline__ float &pencil_wt(float *wts, int q, int a) {
-  return wts[(q * 3 + a) * blockDim.x + threadIdx.x];
-}
-
-// Weights at the 16 x-frequencies a thread holds of column (y, kz).
-template <int W>
-__device__ __forceinline__ void pencil_weights(float *wts, const Geom &g, int w, int y, int kz,
-                                               float R, float (&kc)[3]) {
-  const float yw = (float)wrapm(y, g.Ny), zf = (float)kz;
-#pragma unroll
-  for (int c = 0; c < 3; c++) kc[c] = g.Bmf[3 * c + 1] * yw + g.Bmf[3 * c + 2] * zf;
-#pragma unroll 1
-  for (int q = 0; q < 16; q++) {
-    const float xw = (float)wrapm(pencil_freq<W>(w, q), g.Nx);
-    const float kx = g.Bmf[0] * xw + kc[0], ky = g.Bmf[3] * xw + kc[1], kzz = g.Bmf[6] * xw + kc[2];
-    float a3, a2, av;
-    weights_at_f(kx * kx + ky * ky + kzz * kzz, R, (float)g.dr, (float)g.scale, a3, a2, av);
-    pencil_wt(wts, q, 0) = a3;
-    pencil_wt(wts, q, 1) = a2;
-    pencil_wt(wts, q, 2) = av;
-  }
-}
-
-// Forward convolution along x (pencil form of k_x_conv_fwd): x-FFT of n^,
-// times the five weights (w3, w2, i k_c wv), five inverse x-FFTs.  Columns
-// j = y NzH + kz < Ny NzH; element x at x Ny NzH + j.
-template <int W>
-__global__ void __launch_bounds__(pencil_threads<W>(), W >= 16 ? 1 : 2)
-    k_x_conv_fwd_pencil(const float2 *__restrict__ in, float2 *__restrict__ out5, Geom g,
-                        const float2 *__restrict__ tw, const LocalArgs *__restrict__ lap) {
-  constexpr int G = pencil_groups<W>();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w = warp % W, grp = warp / W;
-  float2 *xs = reinterpret_cast<float2 *>(smem_raw) + grp * pencil_xs_elems<W>();
-  float2 *spec = reinterpret_cast<float2 *>(smem_raw) + G * pencil_xs_elems<W>();
-  float *wts = reinterpret_cast<float *>(spec + 16 * pencil_threads<W>());
-  const int J = g.Ny * g.NzH;
-  const int j = (blockIdx.x * G + grp) * 32 + lane;
-  const bool act = j < J;
-  int y, kz;
-  fdivmod(act ? j : 0, g.fNzH, y, kz);
-  {
-    float2 v[16];
-    const float2 *src = in + j + w * J;
-    const int sW = W * J;
-#pragma unroll
-    for (int m = 0; m < 16; m++) v[m] = act ? src[m * sW] : make_float2(0.f, 0.f);
-    pencil_n2s<float, -1, W>(v, xs, w, lane, tw);
-    // the spectrum waits in thread-private shared slots while the five
-    // weighted copies are transformed back
-#pragma unroll
-    for (int q = 0; q < 16; q++) spec[q * blockDim.x + threadIdx.x] = v[q];
-  }
-  float kc[3];
-  pencil_weights<W>(wts, g, w, y, kz, (float)lap->R, kc);
-#pragma unroll 1
-  for (int a = 0; a < 5; a++) {
-    const float kca = a == 2 ? kc[0] : a == 3 ? kc[1] : kc[2];
-    const float bx = a == 2 ? g.Bmf[0] : a == 3 ? g.Bmf[3] : g.Bmf[6];
-    float2 u[16];
-#pragma unroll
-    for (int q = 0; q < 16; q++) {
-      const float2 v = spec[q * blockDim.x + threadIdx.x];
-      if (a < 2) {
-        const float wt = pencil_wt(wts, q, a);
-        u[q] = make_float2(v.x * wt, v.y * wt);
-      } else {
-        const float xw = (float)wrapm(pencil_freq<W>(w, q), g.Nx);
-        const float wk = (bx * xw + kca) * pencil_wt(wts, q, 2);
-        u[q] = make_float2(-v.y * wk, v.x * wk);  // times i wk
-      }
-    }
-    pencil_s2n<float, +1, W>(u, xs, w, lane, tw);
-    if (act) {
-      float2 *dst = out5 + (size_t)a * g.NC + j + w * J;
-      const int sW = W * J;
-#pragma unroll
-      for (int m = 0; m < 16; m++) dst[m * sW] = u[m];
-    }
-  }
-}
-
-// Adjoint convolution along x (pencil form of k_x_conv_adj): x-FFT of each
-// of the five partial spectra, times its adjoint weight (odd ones negated),
-// summed, one inverse x-FFT.
-template <int W>
-__global__ void __launch_bounds__(pencil_threads<W>(), W >= 16 ? 1 : 2)
-    k_x_conv_adj_pencil(const float2 *__restrict__ in5, float2 *__restrict__ out, Geom g,
-                        const float2 *__restrict__ tw, const LocalArgs *__restrict__ lap) {
-  constexpr int G = pencil_groups<W>();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w = warp % W, grp = warp / W;
-  float2 *xs = reinterpret_cast<float2 *>(smem_raw) + grp * pencil_xs_elems<W>();
-  float2 *sum = reinterpret_cast<float2 *>(smem_raw) + G * pencil_xs_elems<W>();
-  float *wts = reinterpret_cast<float *>(sum + 16 * pencil_threads<W>());
-  const int J = g.Ny * g.NzH;
-  const int j = (blockIdx.x * G + grp) * 32 + lane;
-  const bool act = j < J;
-  int y, kz;
-  fdivmod(act ? j : 0, g.fNzH, y, kz);
-  float kc[3];
-  pencil_weights<W>(wts, g, w, y, kz, (float)lap->R, kc);
-  // the weighted sum accumulates in thread-private shared slots
-#pragma unroll 1
-  for (int a = 0; a < 5; a++) {
-    float2 v[16];
-    const float2 *src = in5 + (size_t)a * g.NC + j + w * J;
-    const int sW = W * J;
-#pragma unroll
-    for (int m = 0; m < 16; m++) v[m] = act ? src[m * sW] : make_float2(0.f, 0.f);
-    pencil_n2s<float, -1, W>(v, xs, w, lane, tw);
-    const float kca = a == 2 ? kc[0] : a == 3 ? kc[1] : kc[2];
-    const float bx = a == 2 ? g.Bmf[0] : a == 3 ? g.Bmf[3] : g.Bmf[6];
-#pragma unroll
-    for (int q = 0; q < 16; q++) {
-      float2 o = a == 0 ? make_float2(0.f, 0.f) : sum[q * blockDim.x + threadIdx.x];
-      if (a < 2) {
-        const float wt = pencil_wt(wts, q, a);
-        o.x += v[q].x * wt;
-        o.y += v[q].y * wt;
-      } else {
-        const float xw = (float)wrapm(pencil_freq<W>(w, q), g.Nx);
-        const float wk = (bx * xw + kca) * pencil_wt(wts, q, 2);
-        o.x += v[q].y * wk;  // times -i wk
-        o.y -= v[q].x * wk;
-      }
-      sum[q * blockDim.x + threadIdx.x] = o;
-    }
-  }
-  float2 acc[16];
-#pragma unroll
-  for (int q = 0; q < 16; q++) acc[q] = sum[q * blockDim.x + threadIdx.x];
-  pencil_s2n<float, +1, W>(acc, xs, w, lane, tw);
-  if (act) {
-    float2 *dst = out + j + w * J;
-    const int sW = W * J;
-#pragma unroll
-    for (int m = 0; m < 16; m++) dst[m * sW] = acc[m];
-  }
-}
-
-// The double-float forms of the two convolutions, one column group a block.
+// The double-float pencil forms of the two convolutions, one column group a
+// block; columns j = y NzH + kz < Ny NzH, element x at x Ny NzH + j.
 // The weights come from the table (three reads a k-point).  Bound by the
 // double-float arithmetic, about 200 FP32 operations a complex point and
 // transform.  SPLIT false: a block takes all five fields one after another,
@@ -1229,12 +1055,9 @@ __global__ void k_pc_table(float *__restrict__ P, Geom g, const LocalArgs *__res
   }
 }
 
-// Shared memory of the pencil kernels: the exchange buffers, plus, for the
-// convolutions, a spectrum (or sum) slot and three weight slots per
-// frequency a thread holds.
-template <int W> constexpr size_t pencil_smem(bool conv) {
-  return sizeof(float2) * pencil_groups<W>() * pencil_xs_elems<W>() +
-         (conv ? (sizeof(float2) * 16 + sizeof(float) * 48) * pencil_threads<W>() : 0);
+// Shared memory of the FP32 pencil kernel (the exchange buffers).
+template <int W> constexpr size_t pencil_smem() {
+  return sizeof(float2) * pencil_groups<W>() * pencil_xs_elems<W>();
 }
 // Double-float: half-width exchange buffers, and the spectrum or sum slots.
 template <int W> constexpr size_t pencil_smem_df(bool conv) {
@@ -3332,13 +3155,9 @@ class EngineImpl {
     };
     auto smemp = [&](auto wc) {
       constexpr int W = decltype(wc)::value;
-      set_smem(k_y_pencil<-1, W>, pencil_smem<W>(false));
-      set_smem(k_y_pencil<+1, W>, pencil_smem<W>(false));
-      set_smem(k_x_conv_fwd_pencil<W>, pencil_smem<W>(true));
-      set_smem(k_x_conv_adj_pencil<W>, pencil_smem<W>(true));
-      set_smem(k_x_pc_pencil<W>, pencil_smem<W>(false));
-      set_smem(k_y_pencil<-1, W, dfl>, pencil_smem_df<W>(false));
-      set_smem(k_y_pencil<+1, W, dfl>, pencil_smem_df<W>(false));
+      set_smem(k_x_pc_pencil<W>, pencil_smem<W>());
+      set_smem(k_y_pencil<-1, W>, pencil_smem_df<W>(false));
+      set_smem(k_y_pencil<+1, W>, pencil_smem_df<W>(false));
       set_smem(k_x_conv_fwd_pencil_df<W, false>, pencil_smem_df<W>(true));
       set_smem(k_x_conv_adj_pencil_df<W, false>, pencil_smem_df<W>(true));
       set_smem(k_x_conv_fwd_pencil_df<W, true>, pencil_smem_df<W>(false));
@@ -3376,6 +3195,7 @@ class EngineImpl {
       ev = getenv("DEFT_ZWARP");
       if (ev) zwarp_mask = atoi(ev) & 3;
     }
+    two_pass_setup(g.Nx);
     smem32(std::integral_constant<int, 0>());
     smem32(std::integral_constant<int, 32>());
     smem32(std::integral_constant<int, 64>());
@@ -3516,10 +3336,11 @@ class EngineImpl {
       }
   }
 
-  // Pencil kernels for the FP32 and double-float x and y transforms of
-  // lengths 32..256 (DEFT_PENCIL=0 in the environment at grid creation
-  // selects the shared-memory Stockham kernels instead, which are also what
-  // every other length takes).  Double-float ones also need a warp for every
+  // Pencil kernels for the double-float x and y transforms of lengths 32..256
+  // and the FP32 preconditioner's x transforms (DEFT_PENCIL=0 in the environment at grid creation
+  // selects the shared-memory Stockham kernels instead, here and in place of
+  // the two-pass and warp kernels; they are also what lengths without any of
+  // these take).  Double-float ones also need a warp for every
   // SM: their straight-line code (some 3000 instructions a transform) is
   // fetched once per warp, and with fewer warps the fetches are what a launch
   // takes (one field at 32^3, 34 warps: 6 us against 4 us).
@@ -3529,6 +3350,12 @@ class EngineImpl {
     if (std::is_same<T, double>::value || !pencil_on || pencil_w(L) == 0) return false;
     const int cols = axis == 0 ? g.Ny * g.NzH : g.Nx * g.NzH;
     return !is_df<T> || (cols + 31) / 32 * (L / 16) >= sms;
+  }
+  // Two-pass FP32 kernels of the y and x axes (two_pass.cu), under the same
+  // switch; they take their lengths whatever radix order is set, as the pencils
+  // do.
+  bool two_pass(int axis) const {
+    return pencil_on && two_pass_length(axis == 0 ? g.Nx : g.Ny);
   }
   // The double-float x convolutions run a block per column group and field
   // where the column groups alone leave the SMs fewer than eight warps each
@@ -3573,21 +3400,24 @@ class EngineImpl {
     dim3 grid((g.NzH + t.By - 1) / t.By, g.Nx, nf);
     const int kid = kslot<T>(nf == 1 ? kK_y_fft1 : kK_y_fft5);
     pre(kid);
-    if constexpr (!std::is_same<T, double>::value) {
+    if constexpr (is_df<T>) {
       if (pencil<T>(1)) {
         with_w(g.Ny, [&](auto wc) {
           constexpr int W = decltype(wc)::value;
-          const int cols = 32 * (is_df<T> ? 1 : pencil_groups<W>());
-          const int threads = is_df<T> ? 32 * W : pencil_threads<W>();
-          const dim3 pg((g.Nx * g.NzH + cols - 1) / cols, nf);
-          using C = typename Cplx<T>::type;
-          const C *tw = reinterpret_cast<const C *>(plan<T>(1).tw);
-          const size_t sm = is_df<T> ? pencil_smem_df<W>(false) : pencil_smem<W>(false);
+          const dim3 pg((g.Nx * g.NzH + 31) / 32, nf);
+          const size_t sm = pencil_smem_df<W>(false);
           if (sign < 0)
-            k_y_pencil<-1, W, T><<<pg, threads, sm, stream>>>(data, g, tw);
+            k_y_pencil<-1, W><<<pg, 32 * W, sm, stream>>>(data, g, tw_yd);
           else
-            k_y_pencil<+1, W, T><<<pg, threads, sm, stream>>>(data, g, tw);
+            k_y_pencil<+1, W><<<pg, 32 * W, sm, stream>>>(data, g, tw_yd);
         });
+        post(kid);
+        return;
+      }
+    }
+    if constexpr (std::is_same<T, float>::value) {
+      if (two_pass(1)) {
+        two_pass_y(data, g, nf, sign, reinterpret_cast<const float2 *>(pyf.tw), stream);
         post(kid);
         return;
       }
@@ -3606,11 +3436,10 @@ class EngineImpl {
   // Queues the adjoint x convolution: spec5 -> spec0.
   template <typename T> void x_conv_adj() {
     const Tiles &t = tl<T>();
-    if (pencil<T>(0)) {
-      with_w(g.Nx, [&](auto wc) {
-        constexpr int W = decltype(wc)::value;
-        const int blocks = (g.Ny * g.NzH + 32 * pencil_groups<W>() - 1) / (32 * pencil_groups<W>());
-        if constexpr (is_df<T>) {
+    if constexpr (is_df<T>) {
+      if (pencil<T>(0)) {
+        with_w(g.Nx, [&](auto wc) {
+          constexpr int W = decltype(wc)::value;
           const int groups = (g.Ny * g.NzH + 31) / 32;
           if (split_x_df<W>()) {
             k_x_conv_adj_pencil_df<W, true><<<dim3(groups, 5), 32 * W, pencil_smem_df<W>(false),
@@ -3624,10 +3453,13 @@ class EngineImpl {
             k_x_conv_adj_pencil_df<W, false><<<groups, 32 * W, pencil_smem_df<W>(true), stream>>>(
                 spec5<T>(), spec0<T>(), w3d, w2d, wvd, g, tw_xd, la_dev);
           }
-        } else if constexpr (std::is_same<T, float>::value)
-          k_x_conv_adj_pencil<W><<<blocks, pencil_threads<W>(), pencil_smem<W>(true), stream>>>(
-              spec5<T>(), spec0<T>(), g, reinterpret_cast<const float2 *>(plan<T>(0).tw), la_dev);
-      });
+        });
+        return;
+      }
+    }
+    if (std::is_same<T, float>::value && two_pass(0)) {
+      two_pass_x_adj(spec5<float>(), spec0<float>(), g, reinterpret_cast<const float2 *>(pxf.tw),
+                     &la_dev->R, stream);
       return;
     }
     with_rn<T>(plan<T>(0), [&](auto rn) {
@@ -3731,11 +3563,10 @@ class EngineImpl {
     z_r2c_spec0<T, R>(n);
     y_fft<T>(spec0<T>(), 1, -1);
     pre(kslot<T>(kK_x_conv_fwd));
-    if (pencil<T>(0)) {
-      with_w(g.Nx, [&](auto wc) {
-        constexpr int W = decltype(wc)::value;
-        const int blocks = (g.Ny * g.NzH + 32 * pencil_groups<W>() - 1) / (32 * pencil_groups<W>());
-        if constexpr (is_df<T>) {
+    if (is_df<T> && pencil<T>(0)) {
+      if constexpr (is_df<T>)
+        with_w(g.Nx, [&](auto wc) {
+          constexpr int W = decltype(wc)::value;
           const int groups = (g.Ny * g.NzH + 31) / 32;
           if (split_x_df<W>())
             k_x_conv_fwd_pencil_df<W, true><<<dim3(groups, 5), 32 * W, pencil_smem_df<W>(false),
@@ -3744,10 +3575,10 @@ class EngineImpl {
           else
             k_x_conv_fwd_pencil_df<W, false><<<groups, 32 * W, pencil_smem_df<W>(true), stream>>>(
                 spec0<T>(), spec5<T>(), w3d, w2d, wvd, g, tw_xd, la_dev);
-        } else if constexpr (std::is_same<T, float>::value)
-          k_x_conv_fwd_pencil<W><<<blocks, pencil_threads<W>(), pencil_smem<W>(true), stream>>>(
-              spec0<T>(), spec5<T>(), g, reinterpret_cast<const float2 *>(plan<T>(0).tw), la_dev);
-      });
+        });
+    } else if (std::is_same<T, float>::value && two_pass(0)) {
+      two_pass_x_fwd(spec0<float>(), spec5<float>(), g, reinterpret_cast<const float2 *>(pxf.tw),
+                     &la_dev->R, stream);
     } else {
       with_rn<T>(plan<T>(0), [&](auto rn) {
         k_x_conv_fwd<T, decltype(rn)::value><<<x_tiles(t.Bxf), kThreads, t.smem_xf, stream>>>(
@@ -4169,7 +4000,7 @@ class EngineImpl {
         constexpr int W = decltype(wc)::value;
         const int cols = 32 * pencil_groups<W>();
         k_x_pc_pencil<W><<<(g.Ny * g.NzH + cols - 1) / cols, pencil_threads<W>(),
-                           pencil_smem<W>(false), stream>>>(
+                           pencil_smem<W>(), stream>>>(
             w, g, reinterpret_cast<const float2 *>(plan<float>(0).tw), pc_table);
       });
       post(kslot<float>(kK_struct_pc));

@@ -1,7 +1,9 @@
-"""FP32 plans that run pairs of small radices as one pass of 10, 12 or 16, and
-the z kernels that read their pointwise inputs in rounds of four: the mixed
-form's energy and gradient against the FP64 form of the same state, and against
-orders in which no pair is fused.
+"""The FP32 transforms: plans that run pairs of small radices as one pass of 10,
+12 or 16, the two-pass kernels of the y and x axes (every length they take, and
+column counts that leave part of the last block empty), and the z kernels that
+read their pointwise inputs in rounds of four.  The mixed form's energy and
+gradient against the FP64 form of the same state, by the built-in kernels, by
+the shared-memory passes, and by orders in which no pair is fused.
 
 Tolerance: an FP32 transform of N = Nx Ny Nz points rounds with a relative rms
 of about 2^-24 sqrt(log2 N) < 3e-7 of its largest output, five times in a row
@@ -49,7 +51,8 @@ def _orders(g):
     ((3, 100, 36), ([3], [5, 4, 5], [3, 3, 4])),
     ((2, 3, 480), ([2], [3], [8, 3, 4, 5])),
 ])
-def test_fused_passes(shape, plain):
+def test_fused_passes(shape, plain, monkeypatch):
+    monkeypatch.setenv("DEFT_PENCIL", "0")  # the shared-memory passes on every axis
     tol = 1.5e-5
     ctx, g, f, n = _state(shape, 0)
     try:
@@ -75,3 +78,23 @@ def test_fused_passes(shape, plain):
             assert np.abs(gr - g64).max() <= tol * np.abs(g64).max()
     finally:
         f.close(), g.close(), ctx.close()
+
+
+@pytest.mark.parametrize("n", [32, 36, 40, 48, 50, 60, 64, 72, 80, 96, 100, 120, 128, 144, 160,
+                               192, 256])
+@pytest.mark.parametrize("axis", [0, 1])
+def test_two_pass_lengths(n, axis):
+    tol = 1.5e-5
+    shape = [3, 5, 6]  # 20 or 12 columns: fewer than a block's
+    shape[axis] = n
+    if n == 48:
+        shape[1 - axis] = 11  # 44 columns: two blocks of 32, the second part full
+    out = []
+    for precision in (0, 1):
+        ctx, g, f, x = _state(tuple(shape), precision)
+        try:
+            out.append(f.energy_grad(x))
+        finally:
+            f.close(), g.close(), ctx.close()
+    assert abs(out[1][0] / out[0][0] - 1) < tol
+    assert np.abs(out[1][1] - out[0][1]).max() <= tol * np.abs(out[0][1]).max()
