@@ -1,7 +1,9 @@
-// Fixed-order FP64 sums over warps and blocks.
+// Fixed-order FP64 and double-float sums over warps and blocks.
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include "dfloat.cuh"
 
 namespace deft {
 
@@ -70,6 +72,36 @@ __device__ __forceinline__ void block_reduce(double (&v)[K], double *smem /* 32*
       for (int w = 0; w < nw; w++) s += smem[w * K + lane];
 #pragma unroll
     for (int k = 0; k < K; k++) v[k] = __shfl_sync(0xffffffffu, s, k);
+  }
+}
+
+// The same for the FP32 kernels' per-thread sums, in double-float (2^-47 a step
+// against the terms' own 2^-24): no FP64 addition but the last one.  Three
+// values over a warp are about 170 issue slots instead of 10 x 64 cycles of
+// FP64 pipe; the Hessian product's last stage at 96^3 (its dot in FP64) spent 2
+// of 17 us there, the gradient with two dots 4 of 22.
+template <int K>
+__device__ __forceinline__ void block_reduce(const float (&x)[K], double (&v)[K],
+                                             double *smem /* 32*K */) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  dfl *part = reinterpret_cast<dfl *>(smem);
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    dfl r = df_two_sum(x[k], __shfl_xor_sync(0xffffffffu, x[k], 16));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+      r += dfl(__shfl_xor_sync(0xffffffffu, r.hi, o), __shfl_xor_sync(0xffffffffu, r.lo, o));
+    if (lane == 0) part[warp * K + k] = r;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const int nw = (blockDim.x + 31) >> 5;
+    dfl s(0.f, 0.f);
+    if (lane < K)
+      for (int w = 0; w < nw; w++) s += part[w * K + lane];
+    const double d = double(s);
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = __shfl_sync(0xffffffffu, d, k);
   }
 }
 

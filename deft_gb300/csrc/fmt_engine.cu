@@ -483,6 +483,9 @@ using GradDots = GradDotsT<double>;
 template <int K>
 __device__ void finish_dots(double (&acc)[K], double *red, double *partials,
                             unsigned int *counter, double *out);
+template <int K>
+__device__ void finish_dots(const float (&acc)[K], double *red, double *partials,
+                            unsigned int *counter, double *out);
 
 // The double-float form's k = 0 entries, weighted in FP64: the table's
 // rounding of w(0) to a double-float would scale the mean of a field, and
@@ -1265,66 +1268,68 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_grad(const typename Cplx<T>::type *__res
     pack_c2r<T>(in, buf0, g, p0, P);
     res = fft_tile<T, +1, RN>(buf0, buf1, fP, pz);
   }
-  // four points a thread and round, each input's loads under one test of its
-  // term (a test per point puts every load behind the previous point's
-  // logarithm)
-  constexpr int Q = 4;
+  // Two points a thread and round, all their inputs read before any is used or
+  // converted (a test of its term or a conversion's slow path between two loads
+  // makes the second wait for the first).
+  constexpr int Q = 2;
   const int total = 2 * P * g.Nz, valid = (g.lines - 2 * p0) * g.Nz;
   const int end = total < valid ? total : valid;
   const size_t r0 = (size_t)2 * p0 * g.Nz;  // the tile's lines are contiguous
   const bool ideal = la.terms & kTermIdeal, vext = la.terms & kTermVext,
              masked = la.terms & kTermMask;
+  const double *logs = lnq ? lnq : n;  // ln(n/nQ), or n
   for (int i0 = threadIdx.x; i0 < end; i0 += Q * blockDim.x) {
-    U loc[Q], conv[Q], vv[Q], mv[Q];
-    auto each = [&](auto f) {
+    double lr[Q], vr[Q], mr[Q], br[3][Q];
+    bool ok[Q];
 #pragma unroll
-      for (int q = 0; q < Q; q++) {
-        const int idx = i0 + q * blockDim.x;
-        if (idx < end) f(q, idx);
-      }
-    };
+    for (int q = 0; q < Q; q++) {
+      const int i = i0 + q * blockDim.x;
+      ok[q] = i < end;
+      lr[q] = ok[q] && ideal ? logs[r0 + i] : 1.0;
+      vr[q] = ok[q] && vext ? V[r0 + i] : 0.0;
+      mr[q] = ok[q] && masked ? mask[r0 + i] : 1.0;
 #pragma unroll
-    for (int q = 0; q < Q; q++) loc[q] = conv[q] = vv[q] = U(0), mv[q] = U(1);
-    if (ideal) {
-      if (lnq) each([&](int q, int i) { loc[q] = U(lnq[r0 + i]); });
-      else each([&](int q, int i) { loc[q] = real_from<U>(n[r0 + i]); });
+      for (int k = 0; k < 3; k++)
+        br[k][q] = ok[q] && k < gd.k && gd.b[k] ? gd.b[k][r0 + i] : 0.0;
     }
-    if (vext) each([&](int q, int i) { vv[q] = real_from<U>(V[r0 + i]); });
-    if (masked) each([&](int q, int i) { mv[q] = real_from<U>(mask[r0 + i]); });
-    if (hs)
-      each([&](int q, int i) {
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      if (!ok[q]) continue;
+      const int i = i0 + q * blockDim.x;
+      U conv = 0, loc = 0;
+      if (hs) {
         int ll, z;
         fdivmod(i, g.fNz, ll, z);
         const C v = res[z * P + (ll >> 1)];
-        conv[q] = U((ll & 1) ? v.y : v.x);
-      });
-    each([&](int q, int i) {
-      U lo = 0;
-      if (ideal) lo += lc.kT * (lnq ? loc[q] : local_log<T>(loc[q] * lc.inv_nQ));
-      if (la.terms & kTermMu) lo += lc.mu;
-      if (vext) lo += vv[q];
-      U gr = conv[q] + lc.dV * lo;
-      if (masked) gr = mv[q] == U(0) ? U(0) : mv[q] * gr;
-      conv[q] = gr;
-      grad[r0 + i] = real_from<double>(gr);
-    });
-    // per-thread sums in U (a dozen terms; FP32 products of the FP32
-    // gradient), the block and grid sums in FP64
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      if (i >= gd.k) continue;
-      if (gd.b[i]) {
-        each([&](int q, int j) { vv[q] = real_from<U>(gd.b[i][r0 + j]); });
-        each([&](int q, int) { dacc[i] += conv[q] * vv[q]; });
-      } else {
-        each([&](int q, int) { dacc[i] += conv[q] * conv[q]; });
+        conv = U((ll & 1) ? v.y : v.x);
       }
+      if (ideal)
+        loc += lc.kT * (lnq ? U(lr[q]) : local_log<T>(real_from<U>(lr[q]) * lc.inv_nQ));
+      if (la.terms & kTermMu) loc += lc.mu;
+      if (vext) loc += real_from<U>(vr[q]);
+      U gr = conv + lc.dV * loc;
+      if (masked) {
+        const U m = real_from<U>(mr[q]);
+        gr = m == U(0) ? U(0) : m * gr;
+      }
+      grad[r0 + i] = real_from<double>(gr);
+      // per-thread sums in U (a dozen terms; FP32 products of the FP32
+      // gradient), the block and grid sums in FP64
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        if (k < gd.k) dacc[k] += gr * (gd.b[k] ? real_from<U>(br[k][q]) : gr);
     }
   }
   if (gd.k > 0) {
     __shared__ double dred[32 * 3];
-    double dsum[3] = {double(dacc[0]), double(dacc[1]), double(dacc[2])};
-    block_reduce<3>(dsum, dred);
+    double dsum[3];
+    if constexpr (sizeof(dacc[0]) == 4) {
+      block_reduce<3>(dacc, dsum, dred);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 3; i++) dsum[i] = dacc[i];
+      block_reduce<3>(dsum, dred);
+    }
     if (threadIdx.x == 0)
       for (int i = 0; i < 3; i++) gd.partials[(size_t)blockIdx.x * 3 + i] = dsum[i];
   }
@@ -1428,7 +1433,7 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_hvp_out(
     unsigned int *counter, double *dout) {
   const LocalArgs la = *lap;
   const LocalConsts<T> lc(la);
-  T pq[1] = {0};  // per-thread sum in T (a dozen terms), block and grid sums in FP64
+  T pq[1] = {0};  // per-thread sum in T (a dozen terms)
   const int P = (int)fP.d;
   using C = typename Cplx<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1441,24 +1446,27 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_hvp_out(
     pack_c2r<T>(in, buf0, g, p0, P);
     res = fft_tile<T, +1, RN>(buf0, buf1, fP, pz);
   }
-  constexpr int Q = 4;  // points a thread and round, as in k_z_grad
+  constexpr int Q = 4;  // points a thread and round, read as in k_z_grad
   const int total = 2 * P * g.Nz, valid = (g.lines - 2 * p0) * g.Nz;
   const int end = total < valid ? total : valid;
   const size_t r0 = (size_t)2 * p0 * g.Nz;
   const bool masked = la.terms & kTermMask;
   for (int i0 = threadIdx.x; i0 < end; i0 += Q * blockDim.x) {
-    T dxt[Q], hl[Q], mv[Q];
-    auto each = [&](auto f) {
+    double dr[Q], mr[Q];
+    float hl[Q];
+    bool ok[Q];
 #pragma unroll
-      for (int q = 0; q < Q; q++) {
-        const int idx = i0 + q * blockDim.x;
-        if (idx < end) f(q, idx);
-      }
-    };
-    each([&](int q, int i) { dxt[q] = real_from<T>(dx[r0 + i]); });
-    each([&](int q, int i) { hl[q] = T(hloc[r0 + i]); });
-    if (masked) each([&](int q, int i) { mv[q] = real_from<T>(mask[r0 + i]); });
-    each([&](int q, int i) {
+    for (int q = 0; q < Q; q++) {
+      const int i = i0 + q * blockDim.x;
+      ok[q] = i < end;
+      dr[q] = ok[q] ? dx[r0 + i] : 0.0;
+      hl[q] = ok[q] ? hloc[r0 + i] : 0.f;
+      mr[q] = ok[q] && masked ? mask[r0 + i] : 1.0;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      if (!ok[q]) continue;
+      const int i = i0 + q * blockDim.x;
       T conv = 0;
       if (hs) {
         int ll, z;
@@ -1466,17 +1474,20 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_hvp_out(
         const C v = res[z * P + (ll >> 1)];
         conv = (ll & 1) ? v.y : v.x;
       }
-      T o = conv + lc.dV * hl[q] * dxt[q];
-      if (masked) o = mv[q] == T(0) ? T(0) : mv[q] * o;
+      const T dxt = real_from<T>(dr[q]);
+      T o = conv + lc.dV * T(hl[q]) * dxt;
+      if (masked) {
+        const T m = real_from<T>(mr[q]);
+        o = m == T(0) ? T(0) : m * o;
+      }
       out[r0 + i] = real_from<double>(o);
-      pq[0] += dxt[q] * o;
-    });
+      pq[0] += dxt * o;
+    }
   }
   // dout: dx.out by the last block to finish, in block order
   if (dout) {
     __shared__ double red[32];
-    double pqd[1] = {double(pq[0])};
-    finish_dots<1>(pqd, red, dpart, counter, dout);
+    finish_dots<1>(pq, red, dpart, counter, dout);
   }
 }
 
@@ -1650,8 +1661,14 @@ __global__ void __launch_bounds__(32 * kZWarps)
   }
   if (gd.k > 0) {
     __shared__ double dred[32 * 3];
-    double dsum[3] = {double(dacc[0]), double(dacc[1]), double(dacc[2])};
-    block_reduce<3>(dsum, dred);
+    double dsum[3];
+    if constexpr (sizeof(dacc[0]) == 4) {
+      block_reduce<3>(dacc, dsum, dred);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 3; i++) dsum[i] = dacc[i];
+      block_reduce<3>(dsum, dred);
+    }
     if (threadIdx.x == 0)
       for (int i = 0; i < 3; i++) gd.partials[(size_t)blockIdx.x * 3 + i] = dsum[i];
   }
@@ -1716,7 +1733,7 @@ __global__ void __launch_bounds__(32 * kZWarps)
   }
   if (dout) {
     __shared__ double red[32];
-    double pqd[1] = {double(pq)};
+    const float pqd[1] = {pq};
     finish_dots<1>(pqd, red, dpart, counter, dout);
   }
 }
@@ -1832,8 +1849,7 @@ __global__ void __launch_bounds__(32 * kZWarps)
     }
   }
   __shared__ double red[32 * 3];
-  double accd[3] = {acc[0], acc[1], acc[2]};
-  finish_dots<3>(accd, red, partials, counter, out);
+  finish_dots<3>(acc, red, partials, counter, out);
 }
 
 // Warp form of k_z_phi: c2r of the five weighted densities of the pair, phi
@@ -2141,10 +2157,9 @@ __global__ void k_dots(int k, const double *a0, const double *b0, const double *
 // partials, the last block to arrive sums them into out[0..K) and resets
 // the counter.
 template <int K>
-__device__ void finish_dots(double (&acc)[K], double *red, double *partials,
-                            unsigned int *counter, double *out) {
+__device__ void finish_block_sums(const double (&acc)[K], double *red, double *partials,
+                                  unsigned int *counter, double *out) {
   __shared__ bool last;
-  block_reduce<K>(acc, red);
   if (threadIdx.x == 0) {
     for (int t = 0; t < K; t++) partials[(size_t)blockIdx.x * K + t] = acc[t];
     __threadfence();
@@ -2164,6 +2179,21 @@ __device__ void finish_dots(double (&acc)[K], double *red, double *partials,
     for (int t = 0; t < K; t++) out[t] = s[t];
     *counter = 0;
   }
+}
+
+template <int K>
+__device__ void finish_dots(double (&acc)[K], double *red, double *partials,
+                            unsigned int *counter, double *out) {
+  block_reduce<K>(acc, red);
+  finish_block_sums<K>(acc, red, partials, counter, out);
+}
+// ... of FP32 per-thread sums.
+template <int K>
+__device__ void finish_dots(const float (&acc)[K], double *red, double *partials,
+                            unsigned int *counter, double *out) {
+  double sum[K];
+  block_reduce<K>(acc, sum, red);
+  finish_block_sums<K>(sum, red, partials, counter, out);
 }
 
 // The density preconditioner of the secant CG with its two dot products in
@@ -2238,8 +2268,7 @@ __global__ void k_precond_dots32(const float *__restrict__ n, const float *__res
     acc[0] += zv * gv;
     acc[1] += zv * h[i];
   }
-  double accd[2] = {acc[0], acc[1]};
-  finish_dots<2>(accd, red, partials, counter, out);
+  finish_dots<2>(acc, red, partials, counter, out);
 }
 __global__ void k_scal_add32(float beta, float *__restrict__ d, float alpha,
                              const float *__restrict__ g, int n) {
@@ -2275,7 +2304,7 @@ __global__ void k_scal_add_dot32(float beta, float *__restrict__ d, float alpha,
     d[i] = dv;
     acc += h[i] * dv;
   }
-  double accd[1] = {acc};
+  const float accd[1] = {acc};
   finish_dots<1>(accd, red, partials, counter, out);
 }
 __global__ void k_axpy32(float alpha, const float *__restrict__ x, float *__restrict__ y, int n) {
@@ -2346,7 +2375,7 @@ __global__ void k_diag_precond_dot32(const float *__restrict__ n, const float *_
     z[i] = zv;
     acc += rv * zv;
   }
-  double accd[1] = {acc};
+  const float accd[1] = {acc};
   finish_dots<1>(accd, red, partials, counter, out);
 }
 __global__ void k_newton_update32(float alpha, const float *__restrict__ p,
@@ -2390,8 +2419,7 @@ __global__ void k_newton_update32(float alpha, const float *__restrict__ p,
     acc[0] += rv * rv;
     acc[1] += rv * zv;
   }
-  double accd[2] = {acc[0], acc[1]};
-  finish_dots<2>(accd, red, partials, counter, out);
+  finish_dots<2>(acc, red, partials, counter, out);
 }
 // The linear CG update before a structure-preconditioner application:
 // dx += alpha p, r -= alpha q.
@@ -2898,11 +2926,9 @@ class EngineImpl {
   double2 *S0 = nullptr, *S5 = nullptr;
   double *w3 = nullptr, *w2 = nullptr, *wv = nullptr;
   double table_R = -1;
-  // mixed form: FP32 twiddles and weight table (spectra share S0/S5)
+  // mixed form: FP32 twiddles (spectra share S0/S5)
   FftPlan pxf{}, pyf{}, pzf{};
   float2 *tw_xf = nullptr, *tw_yf = nullptr, *tw_zf = nullptr;
-  float *w3f = nullptr, *w2f = nullptr, *wvf = nullptr;
-  double table_Rf = -1;
   // the FP64 form's double-float transforms (DEFT_FP64_TRANSFORMS=fp64 in
   // the environment at grid creation keeps FP64 arithmetic instead)
   bool df_on = true;
@@ -2943,9 +2969,6 @@ class EngineImpl {
     cudaFree(w3d);
     cudaFree(w2d);
     cudaFree(wvd);
-    cudaFree(w3f);
-    cudaFree(w2f);
-    cudaFree(wvf);
     cudaFree(hess);
     cudaFree(pc_table);
     cudaFree(lnq);
@@ -3035,7 +3058,7 @@ class EngineImpl {
     return reinterpret_cast<typename Cplx<T>::type *>(S5);
   }
   template <typename T> const T *table(int which) const {
-    if constexpr (std::is_same<T, float>::value) return which == 0 ? w3f : which == 1 ? w2f : wvf;
+    if constexpr (sizeof(T) == 4) return nullptr;  // the FP32 kernels evaluate their weights
     else if constexpr (is_df<T>) return which == 0 ? w3d : which == 1 ? w2d : wvd;
     else return which == 0 ? w3 : which == 1 ? w2 : wv;
   }
@@ -3235,16 +3258,7 @@ class EngineImpl {
   template <typename T> int ensure_table(double R) {
     const int blocks = (g.NC + kThreads - 1) / kThreads;
     const int nb = blocks < 4096 ? blocks : 4096;
-    if constexpr (std::is_same<T, float>::value) {
-      if (R == table_Rf) return 0;
-      if (!w3f && (alloc(&w3f, sizeof(float) * g.NC) || alloc(&w2f, sizeof(float) * g.NC) ||
-                   alloc(&wvf, sizeof(float) * g.NC)))
-        return -1;
-      pre(kslot<float>(kK_weight_table));
-      k_weight_table<float><<<nb, kThreads, 0, stream>>>(g, R, w3f, w2f, wvf);
-      post(kslot<float>(kK_weight_table));
-      table_Rf = R;
-    } else if constexpr (is_df<T>) {
+    if constexpr (is_df<T>) {
       if (R == table_Rd) return 0;
       if (!w3d && (alloc(&w3d, sizeof(dfl) * g.NC) || alloc(&w2d, sizeof(dfl) * g.NC) ||
                    alloc(&wvd, sizeof(dfl) * g.NC)))
@@ -3774,7 +3788,7 @@ class EngineImpl {
   int eval(const FmtSpec &f, const double *n, const double *V, const double *mask, double *grad,
            double *E_host, double *terms_host, int kd = 0, const double *const *da = nullptr,
            const double *const *db = nullptr, double *dots_host = nullptr) {
-    if ((f.terms & kTermHS) && ensure_table<T>(f.R)) return -1;
+    if (sizeof(T) != 4 && (f.terms & kTermHS) && ensure_table<T>(f.R)) return -1;
     if (sizeof(T) != 4 && grad && (is_df<T> || (f.terms & kTermHS)) && ensure_lnq()) return -1;
     if (upload_args(f)) return -1;
     const GraphKey key =
@@ -3806,7 +3820,7 @@ class EngineImpl {
       err = "FP32 vectors: not for this functional or grid";
       return -1;
     }
-    if (ensure_table<float>(f.R) || upload_args(f)) return -1;
+    if (upload_args(f)) return -1;
     const double *ka[3] = {nullptr, nullptr, nullptr}, *kb[3] = {nullptr, nullptr, nullptr};
     GradDotsT<float> gd{};
     for (int i = 0; i < kd; i++) {
@@ -4047,7 +4061,7 @@ class EngineImpl {
       return -1;
     if (upload_args(f)) return -1;
     if (f.terms & kTermHS) {
-      if (ensure_table<float>(f.R) || forward_weighted<float>(f, n)) return -1;
+      if (forward_weighted<float>(f, n)) return -1;
     }
     pre(kslot<float>(kK_z_hess));
     if (zwarp<float>(5)) {
@@ -4077,7 +4091,6 @@ class EngineImpl {
       err = "FP32 vectors: not for this functional or grid";
       return -1;
     }
-    if ((f.terms & kTermHS) && ensure_table<float>(f.R)) return -1;
     if (upload_args(f)) return -1;
     const GraphKey key = graph_key(r64 ? (pq_host ? 3 : 2) : (pq_host ? 7 : 6), 4, f, dx, mask,
                                    out, hess);
@@ -4270,7 +4283,7 @@ int Engine::fan_in(const FieldWeights &w, int sgn, const dfl *in, dfc *spec, dfl
 int Engine::weighted(const FmtSpec &f, const double *n, double *out5, Arith a) {
   EngineImpl &e = *impl_;
   if (f.precision == kPrecisionMixed) {
-    if (e.upload_args(f) || e.ensure_table<float>(f.R) || e.forward_weighted<float>(f, n))
+    if (e.upload_args(f) || e.forward_weighted<float>(f, n))
       return -1;
     e.pre(kslot<float>(kK_z_c2r));
     k_z_c2r<float><<<dim3(e.pairs_tiles(e.t32.Pz), 5), kThreads, e.t32.smem_z, e.stream>>>(
@@ -4520,7 +4533,6 @@ int Engine::scal_add_dot(double beta, double *d, double alpha, const double *g, 
 int Engine::dev_prepare(const FmtSpec &f, bool structure) {
   EngineImpl &e = *impl_;
   if (f.terms & kTermHS) {
-    if (e.ensure_table<float>(f.R)) return -1;
     if (e.df_on ? e.ensure_table<dfl>(f.R) : e.ensure_table<double>(f.R)) return -1;
   }
   if (e.upload_args(f)) return -1;
