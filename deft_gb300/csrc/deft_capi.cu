@@ -5,6 +5,7 @@
 // scalars (energies and dot products) come back.
 #include "../../include/deft_gb300.h"
 #include "contact.h"
+#include "dev_mem.h"
 #include "devcg.h"
 #include "fmt_engine.h"
 #include "saft.h"
@@ -194,13 +195,13 @@ int engine_precision(int p) {
 
 int set_field(deft_fmt *f, double **slot, const double *src, int on_device) {
   if (!src) {
-    cudaFree(*slot);
+    deft::dev_free(*slot);
     *slot = nullptr;
     return DEFT_OK;
   }
   cudaSetDevice(f->grid->ctx->device);
   if (!*slot) {
-    cudaError_t e = cudaMalloc((void **)slot, sizeof(double) * nr(f->grid));
+    cudaError_t e = deft::dev_malloc((void **)slot, sizeof(double) * nr(f->grid));
     if (e != cudaSuccess) return cuda_err(e, "cudaMalloc");
   }
   cudaError_t e = cudaMemcpyAsync(*slot, src, sizeof(double) * nr(f->grid),
@@ -297,9 +298,9 @@ int deft_grid_create(deft_ctx *c, const double lat[9], int Nx, int Ny, int Nz, d
         eng->set_tiles(engine_precision(t.precision), t.choice);  // invalid entries are skipped
   }
   const deft::Geom &ge = eng->geom();
-  cudaError_t e = cudaMalloc((void **)&g->in_buf, sizeof(double) * ge.NR);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&g->out_buf, sizeof(double) * ge.NR);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&g->c_buf, sizeof(double2) * ge.NC);
+  cudaError_t e = deft::dev_malloc((void **)&g->in_buf, sizeof(double) * ge.NR);
+  if (e == cudaSuccess) e = deft::dev_malloc((void **)&g->out_buf, sizeof(double) * ge.NR);
+  if (e == cudaSuccess) e = deft::dev_malloc((void **)&g->c_buf, sizeof(double2) * ge.NC);
   if (e != cudaSuccess) {
     deft_grid_destroy(g);
     return cuda_err(e, "cudaMalloc");
@@ -323,9 +324,9 @@ int deft_grid_destroy(deft_grid *g) {
   if (!g) return DEFT_OK;
   cudaSetDevice(g->ctx->device);
   cudaStreamSynchronize(g->ctx->stream);
-  cudaFree(g->in_buf);
-  cudaFree(g->out_buf);
-  cudaFree(g->c_buf);
+  deft::dev_free(g->in_buf);
+  deft::dev_free(g->out_buf);
+  deft::dev_free(g->c_buf);
   delete g->eng;
   delete g;
   return DEFT_OK;
@@ -468,7 +469,7 @@ int deft_fmt_create(deft_grid *g, const deft_fmt_params *p, deft_fmt **out) {
   deft_fmt *f = new deft_fmt();
   f->grid = g;
   f->p = *p;
-  cudaError_t e = cudaMalloc((void **)&f->g_buf, sizeof(double) * nr(g));
+  cudaError_t e = deft::dev_malloc((void **)&f->g_buf, sizeof(double) * nr(g));
   if (e != cudaSuccess) {
     delete f;
     return cuda_err(e, "cudaMalloc");
@@ -481,14 +482,14 @@ int deft_fmt_destroy(deft_fmt *f) {
   if (!f) return DEFT_OK;
   cudaSetDevice(f->grid->ctx->device);
   cudaStreamSynchronize(f->grid->ctx->stream);
-  cudaFree(f->V);
-  cudaFree(f->mask);
-  cudaFree(f->g_buf);
-  cudaFree(f->w_buf);
-  cudaFree(f->t_buf);
-  cudaFree(f->s_buf);
-  cudaFree(f->n_veff);
-  cudaFree(f->gn_veff);
+  deft::dev_free(f->V);
+  deft::dev_free(f->mask);
+  deft::dev_free(f->g_buf);
+  deft::dev_free(f->w_buf);
+  deft::dev_free(f->t_buf);
+  deft::dev_free(f->s_buf);
+  deft::dev_free(f->n_veff);
+  deft::dev_free(f->gn_veff);
   delete f;
   return DEFT_OK;
 }
@@ -536,10 +537,10 @@ namespace {
 int veff_buffers(deft_fmt *f) {
   if (f->n_veff) return DEFT_OK;
   const size_t bytes = sizeof(double) * nr(f->grid);
-  cudaError_t e = cudaMalloc((void **)&f->n_veff, bytes);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&f->gn_veff, bytes);
+  cudaError_t e = deft::dev_malloc((void **)&f->n_veff, bytes);
+  if (e == cudaSuccess) e = deft::dev_malloc((void **)&f->gn_veff, bytes);
   if (e != cudaSuccess) {
-    cudaFree(f->n_veff);
+    deft::dev_free(f->n_veff);
     f->n_veff = nullptr;
     f->gn_veff = nullptr;
     return cuda_err(e, "cudaMalloc");
@@ -583,7 +584,7 @@ int density_eval(deft_fmt *f, const deft::FmtSpec &spec_in, const double *n, dou
   Engine *e = f->grid->eng;
   if (!f->s_buf) {
     const size_t ns = deft::saft_scratch_doubles(e->geom());
-    cudaError_t ce = cudaMalloc((void **)&f->s_buf, sizeof(double) * (ns + nr(f->grid)));
+    cudaError_t ce = deft::dev_malloc((void **)&f->s_buf, sizeof(double) * (ns + nr(f->grid)));
     if (ce != cudaSuccess) {
       f->s_buf = nullptr;
       return cuda_err(ce, "cudaMalloc");
@@ -614,7 +615,7 @@ int density_eval_fmt(deft_fmt *f, const deft::FmtSpec &spec, const double *n, do
   deft_grid *g = f->grid;
   if (!f->t_buf) {
     const size_t nd = deft::tensor_scratch_doubles(e->geom()) + nr(g);
-    cudaError_t ce = cudaMalloc((void **)&f->t_buf, sizeof(double) * nd);
+    cudaError_t ce = deft::dev_malloc((void **)&f->t_buf, sizeof(double) * nd);
     if (ce != cudaSuccess) {
       f->t_buf = nullptr;
       return cuda_err(ce, "cudaMalloc");
@@ -685,7 +686,7 @@ int deft_fmt_energy_grad_pgrad(deft_fmt *f, const double *n, int on_device, doub
   double *pdst = pgrad;
   if (pgrad && !on_device) {
     if (!f->w_buf) {
-      cudaError_t e = cudaMalloc((void **)&f->w_buf, 5 * sizeof(double) * nr(g));
+      cudaError_t e = deft::dev_malloc((void **)&f->w_buf, 5 * sizeof(double) * nr(g));
       if (e != cudaSuccess) return cuda_err(e, "cudaMalloc");
     }
     pdst = f->w_buf;
@@ -718,7 +719,7 @@ int deft_fmt_weighted(deft_fmt *f, const double *n, int on_device, double *out5)
   double *dst = out5;
   if (!on_device) {
     if (!f->w_buf) {
-      cudaError_t e = cudaMalloc((void **)&f->w_buf, 5 * sizeof(double) * nr(g));
+      cudaError_t e = deft::dev_malloc((void **)&f->w_buf, 5 * sizeof(double) * nr(g));
       if (e != cudaSuccess) return cuda_err(e, "cudaMalloc");
     }
     dst = f->w_buf;
@@ -751,7 +752,7 @@ int deft_fmt_contact(deft_fmt *f, const double *n, int on_device, int which, dou
   if (int s = fmt_density(f, spec, src, &dens)) return s;
   const size_t ns = deft::contact_scratch_doubles(g->eng->geom(), which);
   double *scratch = nullptr;
-  cudaError_t ce = cudaMalloc((void **)&scratch, sizeof(double) * (ns + (on_device ? 0 : nr(g))));
+  cudaError_t ce = deft::dev_malloc((void **)&scratch, sizeof(double) * (ns + (on_device ? 0 : nr(g))));
   if (ce != cudaSuccess) return cuda_err(ce, "cudaMalloc");
   double *dst = on_device ? out : scratch + ns;
   std::string err;
@@ -759,7 +760,7 @@ int deft_fmt_contact(deft_fmt *f, const double *n, int on_device, int which, dou
   if (!r && !on_device)
     ce = cudaMemcpyAsync(out, dst, sizeof(double) * nr(g), cudaMemcpyDeviceToHost, g->ctx->stream);
   const int sr = sync(g->ctx);
-  cudaFree(scratch);
+  deft::dev_free(scratch);
   if (r) return set_err(DEFT_ERR_CUDA, err);
   if (ce != cudaSuccess) return cuda_err(ce, "device-to-host copy");
   return sr;
@@ -940,11 +941,11 @@ int deft_cg_create(deft_fmt *f, const deft_cg_params *p, deft_cg **out) {
   c->alpha = p->step;
   c->err_est = std::fmax(1.0, 2 * p->precision);
   const size_t bytes = sizeof(double) * nr(f->grid);
-  cudaError_t e = cudaMalloc((void **)&c->x, bytes);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&c->g, bytes);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&c->d, bytes);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&c->gold, bytes);
-  if (e == cudaSuccess && p->preconditioned) e = cudaMalloc((void **)&c->pg, bytes);
+  cudaError_t e = deft::dev_malloc((void **)&c->x, bytes);
+  if (e == cudaSuccess) e = deft::dev_malloc((void **)&c->g, bytes);
+  if (e == cudaSuccess) e = deft::dev_malloc((void **)&c->d, bytes);
+  if (e == cudaSuccess) e = deft::dev_malloc((void **)&c->gold, bytes);
+  if (e == cudaSuccess && p->preconditioned) e = deft::dev_malloc((void **)&c->pg, bytes);
   if (e == cudaSuccess) e = cudaMemsetAsync(c->d, 0, bytes, f->grid->ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(c->gold, 0, bytes, f->grid->ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(c->x, 0, bytes, f->grid->ctx->stream);
@@ -961,14 +962,14 @@ int deft_cg_set_params(deft_cg *c, const deft_cg_params *p) {
   if (int s = check_cg_params(c->f, p)) return s;
   cudaSetDevice(c->f->grid->ctx->device);
   if (p->preconditioned && !c->pg) {
-    cudaError_t e = cudaMalloc((void **)&c->pg, sizeof(double) * nr(c->f->grid));
+    cudaError_t e = deft::dev_malloc((void **)&c->pg, sizeof(double) * nr(c->f->grid));
     if (e != cudaSuccess) {
       c->pg = nullptr;
       return cuda_err(e, "cudaMalloc");
     }
   } else if (!p->preconditioned && c->pg) {
     cudaStreamSynchronize(c->f->grid->ctx->stream);
-    cudaFree(c->pg);
+    deft::dev_free(c->pg);
     c->pg = nullptr;
   }
   c->p = *p;
@@ -980,14 +981,14 @@ int deft_cg_destroy(deft_cg *c) {
   if (!c) return DEFT_OK;
   cudaSetDevice(c->f->grid->ctx->device);
   cudaStreamSynchronize(c->f->grid->ctx->stream);
-  cudaFree(c->x);
-  cudaFree(c->g);
-  cudaFree(c->d);
-  cudaFree(c->gold);
-  cudaFree(c->pg);
-  cudaFree(c->q);
-  cudaFree(c->dxv);
-  cudaFree(c->x32);  // the block holding all nine FP32 vectors
+  deft::dev_free(c->x);
+  deft::dev_free(c->g);
+  deft::dev_free(c->d);
+  deft::dev_free(c->gold);
+  deft::dev_free(c->pg);
+  deft::dev_free(c->q);
+  deft::dev_free(c->dxv);
+  deft::dev_free(c->x32);  // the block holding all nine FP32 vectors
   if (c->log) fclose(c->log);
   deft::dcg_free(c->dgraph);
   delete c;
@@ -1313,7 +1314,7 @@ int f32_buffers(deft_cg *c) {
     // of minimisers pays one cudaMalloc each instead of nine
     const size_t stride = (n + 63) / 64 * 64;
     float *block = nullptr;
-    cudaError_t ce = cudaMalloc((void **)&block, sizeof(float) * stride * 9);
+    cudaError_t ce = deft::dev_malloc((void **)&block, sizeof(float) * stride * 9);
     if (ce != cudaSuccess) return cuda_err(ce, "cudaMalloc");
     float **vs[9] = {&c->x32, &c->g32, &c->d32, &c->gold32, &c->pg32, &c->V32, &c->mask32,
                      &c->q32, &c->dx32};
@@ -1559,8 +1560,8 @@ int step_newton(deft_cg *c, deft_cg_status *st, const deft::FmtSpec &spec) {
   const size_t bytes = sizeof(double) * nr(c->f->grid);
   cudaStream_t stream = c->f->grid->ctx->stream;
   if (!c->q) {
-    cudaError_t ce = cudaMalloc((void **)&c->q, bytes);
-    if (ce == cudaSuccess) ce = cudaMalloc((void **)&c->dxv, bytes);
+    cudaError_t ce = deft::dev_malloc((void **)&c->q, bytes);
+    if (ce == cudaSuccess) ce = deft::dev_malloc((void **)&c->dxv, bytes);
     if (ce != cudaSuccess) return cuda_err(ce, "cudaMalloc");
   }
   if (!c->have_g || c->last_eval_mixed) {
@@ -2115,8 +2116,8 @@ int device_problem(deft_cg *c, deft::DcgProblem *p) {
                    "device-driven solves take the fused functionals in the density variable");
   const size_t bytes = sizeof(double) * nr(f->grid);
   if (!c->q) {
-    cudaError_t ce = cudaMalloc((void **)&c->q, bytes);
-    if (ce == cudaSuccess) ce = cudaMalloc((void **)&c->dxv, bytes);
+    cudaError_t ce = deft::dev_malloc((void **)&c->q, bytes);
+    if (ce == cudaSuccess) ce = deft::dev_malloc((void **)&c->dxv, bytes);
     if (ce != cudaSuccess) return cuda_err(ce, "cudaMalloc");
   }
   const deft::FmtSpec spec = spec_of(f);

@@ -21,6 +21,7 @@
 // analytically once per (grid, R) into a table, with the convolution
 // normalisation dV/V folded in.
 #include "block_sum.cuh"
+#include "dev_mem.h"
 #include "df_phi.cuh"
 #include "fft_smem.cuh"
 #include "fmt_engine.h"
@@ -2957,35 +2958,35 @@ class EngineImpl {
       cudaEventDestroy(p.second.second);
     }
     for (cudaEvent_t e : pool) cudaEventDestroy(e);
-    cudaFree(tw_x);
-    cudaFree(tw_y);
-    cudaFree(tw_z);
-    cudaFree(tw_xf);
-    cudaFree(tw_yf);
-    cudaFree(tw_zf);
-    cudaFree(tw_xd);
-    cudaFree(tw_yd);
-    cudaFree(tw_zd);
-    cudaFree(w3d);
-    cudaFree(w2d);
-    cudaFree(wvd);
-    cudaFree(hess);
-    cudaFree(pc_table);
-    cudaFree(lnq);
-    for (Radial &r : radials) cudaFree(r.tab);
+    dev_free(tw_x);
+    dev_free(tw_y);
+    dev_free(tw_z);
+    dev_free(tw_xf);
+    dev_free(tw_yf);
+    dev_free(tw_zf);
+    dev_free(tw_xd);
+    dev_free(tw_yd);
+    dev_free(tw_zd);
+    dev_free(w3d);
+    dev_free(w2d);
+    dev_free(wvd);
+    dev_free(hess);
+    dev_free(pc_table);
+    dev_free(lnq);
+    for (Radial &r : radials) dev_free(r.tab);
     clear_graphs();
-    cudaFree(la_dev);
-    cudaFree(hloc);
-    cudaFree(S0);
-    cudaFree(S5);
-    cudaFree(w3);
-    cudaFree(w2);
-    cudaFree(wv);
-    cudaFree(partials);
-    cudaFree(results);
-    cudaFree(dot_partials);
-    cudaFree(grad_partials);
-    cudaFree(dot_counter);
+    dev_free(la_dev);
+    dev_free(hloc);
+    dev_free(S0);
+    dev_free(S5);
+    dev_free(w3);
+    dev_free(w2);
+    dev_free(wv);
+    dev_free(partials);
+    dev_free(results);
+    dev_free(dot_partials);
+    dev_free(grad_partials);
+    dev_free(dot_counter);
     cudaFreeHost(results_host);
   }
 
@@ -3001,7 +3002,7 @@ class EngineImpl {
 
   template <typename P>
   int alloc(P **p, size_t n) {
-    cudaError_t e = cudaMalloc((void **)p, n);
+    cudaError_t e = dev_malloc((void **)p, n);
     if (e != cudaSuccess) return fail("cudaMalloc", e);
     bytes += n;
     return 0;
@@ -3029,9 +3030,10 @@ class EngineImpl {
     };
     for (int t = 0; t < n; t++) {
       const long double a = twopi * (long double)t / (long double)n;
-      h[t] = make_double2((double)cosl(a), (double)-sinl(a));
-      hf[t] = make_float2((float)cosl(a), (float)-sinl(a));
-      hd[t] = dfc{split(cosl(a)), split(-sinl(a))};
+      const long double c = cosl(a), sn = -sinl(a);  // software arithmetic on aarch64: once
+      h[t] = make_double2((double)c, (double)sn);
+      hf[t] = make_float2((float)c, (float)sn);
+      hd[t] = dfc{split(c), split(sn)};
     }
     if (alloc(tw, sizeof(double2) * n) || alloc(twf, sizeof(float2) * n) ||
         alloc(twd, sizeof(dfc) * n))
@@ -3303,11 +3305,11 @@ class EngineImpl {
     if (need > max_blocks) {
       cudaStreamSynchronize(stream);
       double *np2 = nullptr;
-      if (cudaMalloc((void **)&np2, sizeof(double) * kNumTerms * need) != cudaSuccess) {
+      if (dev_malloc((void **)&np2, sizeof(double) * kNumTerms * need) != cudaSuccess) {
         err = "cudaMalloc (energy partials)";
         return -1;
       }
-      cudaFree(partials);
+      dev_free(partials);
       partials = np2;
       max_blocks = need;
     }
