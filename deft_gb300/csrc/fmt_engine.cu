@@ -1269,10 +1269,12 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_grad(const typename Cplx<T>::type *__res
     pack_c2r<T>(in, buf0, g, p0, P);
     res = fft_tile<T, +1, RN>(buf0, buf1, fP, pz);
   }
-  // Two points a thread and round, all their inputs read before any is used or
-  // converted (a test of its term or a conversion's slow path between two loads
-  // makes the second wait for the first).
-  constexpr int Q = 2;
+  // A few points a thread and round.  FP32: all their inputs are read before any
+  // is used or converted (a test of its term or a conversion's slow path
+  // between two loads makes the second wait for the first).  FP64 and
+  // double-float need no conversions and would spill: an input at a time
+  // (128^3: 47 us against 57 with the FP32 form's order).
+  constexpr int Q = sizeof(U) == 4 ? 2 : 4;
   const int total = 2 * P * g.Nz, valid = (g.lines - 2 * p0) * g.Nz;
   const int end = total < valid ? total : valid;
   const size_t r0 = (size_t)2 * p0 * g.Nz;  // the tile's lines are contiguous
@@ -1280,45 +1282,80 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_z_grad(const typename Cplx<T>::type *__res
              masked = la.terms & kTermMask;
   const double *logs = lnq ? lnq : n;  // ln(n/nQ), or n
   for (int i0 = threadIdx.x; i0 < end; i0 += Q * blockDim.x) {
-    double lr[Q], vr[Q], mr[Q], br[3][Q];
-    bool ok[Q];
+    auto each = [&](auto f) {
 #pragma unroll
-    for (int q = 0; q < Q; q++) {
-      const int i = i0 + q * blockDim.x;
-      ok[q] = i < end;
-      lr[q] = ok[q] && ideal ? logs[r0 + i] : 1.0;
-      vr[q] = ok[q] && vext ? V[r0 + i] : 0.0;
-      mr[q] = ok[q] && masked ? mask[r0 + i] : 1.0;
-#pragma unroll
-      for (int k = 0; k < 3; k++)
-        br[k][q] = ok[q] && k < gd.k && gd.b[k] ? gd.b[k][r0 + i] : 0.0;
-    }
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-      if (!ok[q]) continue;
-      const int i = i0 + q * blockDim.x;
-      U conv = 0, loc = 0;
-      if (hs) {
-        int ll, z;
-        fdivmod(i, g.fNz, ll, z);
-        const C v = res[z * P + (ll >> 1)];
-        conv = U((ll & 1) ? v.y : v.x);
+      for (int q = 0; q < Q; q++) {
+        const int i = i0 + q * blockDim.x;
+        if (i < end) f(q, i);
       }
-      if (ideal)
-        loc += lc.kT * (lnq ? U(lr[q]) : local_log<T>(real_from<U>(lr[q]) * lc.inv_nQ));
-      if (la.terms & kTermMu) loc += lc.mu;
-      if (vext) loc += real_from<U>(vr[q]);
-      U gr = conv + lc.dV * loc;
-      if (masked) {
-        const U m = real_from<U>(mr[q]);
-        gr = m == U(0) ? U(0) : m * gr;
-      }
-      grad[r0 + i] = real_from<double>(gr);
-      // per-thread sums in U (a dozen terms; FP32 products of the FP32
-      // gradient), the block and grid sums in FP64
+    };
+    U gr[Q];  // the local terms, then the gradient
+    auto convolved = [&](int i) {
+      int ll, z;
+      fdivmod(i, g.fNz, ll, z);
+      const C v = res[z * P + (ll >> 1)];
+      return U((ll & 1) ? v.y : v.x);
+    };
+    if constexpr (sizeof(U) == 4) {
+      double lr[Q], vr[Q], mr[Q], br[3][Q];
 #pragma unroll
-      for (int k = 0; k < 3; k++)
-        if (k < gd.k) dacc[k] += gr * (gd.b[k] ? real_from<U>(br[k][q]) : gr);
+      for (int q = 0; q < Q; q++) {
+        const int i = i0 + q * blockDim.x;
+        const bool ok = i < end;
+        lr[q] = ok && ideal ? logs[r0 + i] : 1.0;
+        vr[q] = ok && vext ? V[r0 + i] : 0.0;
+        mr[q] = ok && masked ? mask[r0 + i] : 1.0;
+#pragma unroll
+        for (int k = 0; k < 3; k++) br[k][q] = ok && k < gd.k && gd.b[k] ? gd.b[k][r0 + i] : 0.0;
+      }
+      each([&](int q, int i) {
+        U loc = 0;
+        if (ideal)
+          loc += lc.kT * (lnq ? U(lr[q]) : local_log<T>(real_from<U>(lr[q]) * lc.inv_nQ));
+        if (la.terms & kTermMu) loc += lc.mu;
+        if (vext) loc += real_from<U>(vr[q]);
+        gr[q] = (hs ? convolved(i) : U(0)) + lc.dV * loc;
+        if (masked) {
+          const U m = real_from<U>(mr[q]);
+          gr[q] = m == U(0) ? U(0) : m * gr[q];
+        }
+        grad[r0 + i] = real_from<double>(gr[q]);
+        // per-thread sums in U (a dozen terms; FP32 products of the FP32
+        // gradient)
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+          if (k < gd.k) dacc[k] += gr[q] * (gd.b[k] ? real_from<U>(br[k][q]) : gr[q]);
+      });
+    } else {
+      U mv[Q];
+#pragma unroll
+      for (int q = 0; q < Q; q++) gr[q] = U(0), mv[q] = U(1);
+      if (ideal) {
+        each([&](int q, int i) { gr[q] = U(logs[r0 + i]); });
+        each([&](int q, int) { gr[q] = lc.kT * (lnq ? gr[q] : local_log<T>(gr[q] * lc.inv_nQ)); });
+      }
+      if (la.terms & kTermMu) each([&](int q, int) { gr[q] += lc.mu; });
+      if (vext) {
+        U vv[Q];
+        each([&](int q, int i) { vv[q] = U(V[r0 + i]); });
+        each([&](int q, int) { gr[q] += vv[q]; });
+      }
+      if (masked) each([&](int q, int i) { mv[q] = U(mask[r0 + i]); });
+      each([&](int q, int i) {
+        gr[q] = (hs ? convolved(i) : U(0)) + lc.dV * gr[q];
+        if (masked) gr[q] = mv[q] == U(0) ? U(0) : mv[q] * gr[q];
+        grad[r0 + i] = double(gr[q]);
+      });
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        if (k >= gd.k) continue;
+        if (gd.b[k]) {
+          each([&](int q, int i) { mv[q] = U(gd.b[k][r0 + i]); });
+          each([&](int q, int) { dacc[k] += gr[q] * mv[q]; });
+        } else {
+          each([&](int q, int) { dacc[k] += gr[q] * gr[q]; });
+        }
+      }
     }
   }
   if (gd.k > 0) {
@@ -1578,9 +1615,11 @@ __global__ void __launch_bounds__(32 * kZWarps)
 }
 
 // Warp form of k_z_grad: c2r of the adjoint sum, + local gradient terms,
-// masked, optional dot products of the new gradient.
+// masked, optional dot products of the new gradient.  Bound by the latency of
+// its loads: four blocks an SM (64 registers) instead of three 18.8 -> 15.5 us
+// at 128^3.
 template <int E, typename R = double>
-__global__ void __launch_bounds__(32 * kZWarps)
+__global__ void __launch_bounds__(32 * kZWarps, E <= 4 ? 4 : 0)
     k_z_grad_warp(const float2 *__restrict__ in, const R *__restrict__ n,
                   const R *__restrict__ V, const R *__restrict__ mask,
                   R *__restrict__ grad, Geom g, const float2 *__restrict__ tw,
@@ -1595,7 +1634,7 @@ __global__ void __launch_bounds__(32 * kZWarps)
   // the pointwise inputs first, so their loads are in flight while the line
   // is transformed; each input's 2 E loads under one test of its term (a test
   // per point puts every load behind the previous point's logarithm: 36 us a
-  // gradient at 128^3 against 18.6)
+  // gradient at 128^3 against 15.5)
   float loc[2][E], mk[2][E], bv[3][2][E];
   const bool ok0 = l0 < g.lines, ok1 = l0 + 1 < g.lines;
   auto load2 = [&](const R *src, float (&dst)[2][E], float other) {
