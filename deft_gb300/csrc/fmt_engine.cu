@@ -501,7 +501,10 @@ __device__ __forceinline__ dfc dc_weight(dfc v, double w) {
 
 // x-FFT of n^, multiplication by the five weights, and the five inverse
 // x-FFTs one field at a time (three tiles of B lines: the forward result and
-// a ping-pong pair), which keeps B wide for coalesced column runs.
+// a ping-pong pair), which keeps B wide for coalesced column runs.  With
+// gridDim.y = 5 a block does one field (blockIdx.y) and its own forward
+// transform: two transforms in a row instead of six, for grids whose tiles
+// are too few to fill the chip (split_x).
 template <typename T, int RN = 0>
 __global__ void DEFT_FFT_BOUNDS(RN) k_x_conv_fwd(
     const typename Cplx<T>::type *__restrict__ in, typename Cplx<T>::type *__restrict__ out5,
@@ -539,7 +542,8 @@ __global__ void DEFT_FFT_BOUNDS(RN) k_x_conv_fwd(
   const C *R0 = fft_tile<T, -1, RN>(bufA, bufB, fB, px);
   C *F1 = (R0 == bufA) ? bufB : bufA;
   C *F2 = bufC;
-  for (int a = 0; a < 5; a++) {
+  const int a0 = gridDim.y > 1 ? blockIdx.y : 0, a1 = gridDim.y > 1 ? a0 + 1 : 5;
+  for (int a = a0; a < a1; a++) {
     #pragma unroll 4
     for (int idx = threadIdx.x; idx < g.Nx * B; idx += blockDim.x) {
       int e, j;
@@ -979,20 +983,26 @@ __global__ void __launch_bounds__(32 * W, 16 / W)
   dfl *xs = reinterpret_cast<dfl *>(smem_raw);
   const int J = g.Ny * g.NzH;
   const int j = blockIdx.x * 32 + lane;
+  // Columns past the end read the last one: without a test a slot the loads of
+  // several slots are in flight (64^3: 13.1 us,
+  // 8.6 like this).
+  const int jc = j < J ? j : J - 1;
   dfc v[16];
 #pragma unroll
-  for (int q = 0; q < 16; q++) {
-    dfc o = dfc{0, 0};
-    if (j < J) {
-      const dfc *src = in5 + (size_t)(w * 16 + q) * J + j;
-      o = src[0];
+  for (int q0 = 0; q0 < 16; q0 += 2) {
+    dfc t[2][5];
 #pragma unroll
-      for (int a = 1; a < 5; a++) {
-        const dfc t = src[(size_t)a * g.NC];
-        o = dfc{o.x + t.x, o.y + t.y};
-      }
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int a = 0; a < 5; a++)
+        t[i][a] = ldg_c(in5 + (size_t)a * g.NC + (size_t)(w * 16 + q0 + i) * J + jc);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      dfc o = t[i][0];
+#pragma unroll
+      for (int a = 1; a < 5; a++) o = dfc{o.x + t[i][a].x, o.y + t[i][a].y};
+      v[q0 + i] = o;
     }
-    v[q] = o;
   }
   pencil_s2n<dfl, +1, W>(v, xs, w, lane, tw);
   pencil_store<W>(v, out, w, j, J);
@@ -3487,6 +3497,12 @@ class EngineImpl {
     post(kid);
   }
   int x_tiles(int B) const { return (g.Ny * g.NzH + B - 1) / B; }
+  // A block per tile and field where the tiles alone are no more than the SMs:
+  // ten transforms in all instead of six, but two in a row.  Double-float, with
+  // events: 32^3 (34 tiles) 22.8 -> 13.8 us, 48^3 (75) 27.3 -> 16.5, 56^3 (102)
+  // 40.6 -> 33.7; beyond the line 72^3 (267) 38.9 -> 44.5, 96^3 (588) 58.3 -> 83.9.
+  // FP32: 24^3 14.5 -> 9.7, 56^3 18.9 -> 13.5; 77^3 (189) 23.8 -> 24.5.
+  bool split_x(int B) const { return x_tiles(B) <= sms; }
 
   // Queues the adjoint x convolution: spec5 -> spec0.
   template <typename T> void x_conv_adj() {
@@ -3636,7 +3652,8 @@ class EngineImpl {
                      &la_dev->R, stream);
     } else {
       with_rn<T>(plan<T>(0), [&](auto rn) {
-        k_x_conv_fwd<T, decltype(rn)::value><<<x_tiles(t.Bxf), kThreads, t.smem_xf, stream>>>(
+        k_x_conv_fwd<T, decltype(rn)::value><<<dim3(x_tiles(t.Bxf), split_x(t.Bxf) ? 5 : 1),
+                                               kThreads, t.smem_xf, stream>>>(
             spec0<T>(), spec5<T>(), table<T>(0), table<T>(1), table<T>(2), g, plan<T>(0), t.fBxf,
             la_dev);
       });
