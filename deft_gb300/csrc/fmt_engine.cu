@@ -2269,7 +2269,7 @@ __global__ void k_precond_dots(const double *__restrict__ n, const double *__res
 // FP32-vector forms for the mixed form's FP32 stage: z = g n / (kT dV) on
 // the active points (mask != 0, n > 0) with (z.g, z.h) summed in FP64;
 // d = alpha g + beta d; y += alpha x; conversions.  Four elements per
-// thread and step (16-byte accesses; the vectors come from cudaMalloc),
+// thread and step (16-byte accesses; the vectors are 256-byte aligned),
 // a scalar tail when the length is not a multiple of 4; per-thread sums in
 // FP32, FP64 across threads and blocks.
 #define DEFT_V4_LOOP(n)                                                              \
@@ -2552,7 +2552,7 @@ __global__ void k_scal_add_dot(double beta, double *__restrict__ d, double alpha
 }
 
 // Vector kernels: two doubles per thread per step (16-byte accesses); the
-// vectors come from cudaMalloc (256-byte aligned), n odd leaves a tail.
+// vectors are 256-byte aligned, n odd leaves a tail.
 __global__ void k_axpy(double alpha, const double *x, double *y, int n) {
   const int n2 = n >> 1;
   const double2 *x2 = reinterpret_cast<const double2 *>(x);
