@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cstring>
 #include <mutex>
 #include <numeric>
@@ -103,9 +104,17 @@ extern "C" int deft_batch_solve(int device, int count, const deft_batch_problem 
   int workers = bp->workers > 0 ? bp->workers : 8;
   if (workers > count) workers = count > 0 ? count : 1;
   std::atomic<int> next(0);
-  std::atomic<int> first_error(DEFT_OK);
-  std::mutex msg_mu;
+  // the first failing problem of the list, whatever order they ran in
+  std::mutex err_mu;
+  int first_index = INT_MAX, first_error = DEFT_OK;
   std::string first_msg;
+  auto failed = [&](int index, int status, const std::string &msg) {
+    std::lock_guard<std::mutex> lock(err_mu);
+    if (index >= first_index) return;
+    first_index = index;
+    first_error = status;
+    first_msg = msg;
+  };
   // largest first (a large one started last would run alone at the end)
   std::vector<int> order(count);
   std::iota(order.begin(), order.end(), 0);
@@ -130,8 +139,7 @@ extern "C" int deft_batch_solve(int device, int count, const deft_batch_problem 
       } scope;
       Worker w;
       if (deft_ctx_create(device, &w.ctx) != DEFT_OK) {
-        int expect = DEFT_OK;
-        first_error.compare_exchange_strong(expect, DEFT_ERR_CUDA);
+        failed(-1, DEFT_ERR_CUDA, deft_last_error());
         return;
       }
       deft::thread_pool = {pool, static_cast<cudaStream_t>(deft_ctx_stream(w.ctx))};
@@ -143,18 +151,12 @@ extern "C" int deft_batch_solve(int device, int count, const deft_batch_problem 
         memset(&st, 0, sizeof(st));
         const int s = solve_one(w, probs[i], bp->cg, &st);
         st.status = s;
-        if (s) {
-          int expect = DEFT_OK;
-          if (first_error.compare_exchange_strong(expect, s)) {
-            std::lock_guard<std::mutex> lock(msg_mu);
-            first_msg = "problem " + std::to_string(i) + ": " + deft_last_error();
-          }
-        }
+        if (s) failed(i, s, "problem " + std::to_string(i) + ": " + deft_last_error());
       }
     });
   }
   for (auto &th : threads) th.join();
   if (pool) cudaMemPoolDestroy(pool);
-  if (first_error.load() != DEFT_OK) deft::set_last_error_message(first_msg);
-  return first_error.load();
+  if (first_error != DEFT_OK) deft::set_last_error_message(first_msg);
+  return first_error;
 }
