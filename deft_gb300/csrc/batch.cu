@@ -123,14 +123,10 @@ extern "C" int deft_batch_solve(int device, int count, const deft_batch_problem 
   };
   std::stable_sort(order.begin(), order.end(),
                    [&](int a, int b) { return points(a) > points(b); });
-  int devices = 0, before = 0;
+  // made by the first worker: the calling thread keeps its device, and gets no
+  // context on another
+  std::once_flag pool_made;
   cudaMemPool_t pool = nullptr;
-  if (cudaGetDeviceCount(&devices) == cudaSuccess && device >= 0 && device < devices &&
-      cudaGetDevice(&before) == cudaSuccess) {
-    cudaSetDevice(device);
-    pool = deft::make_call_pool(device);
-    cudaSetDevice(before);
-  }
   std::vector<std::thread> threads;
   for (int t = 0; t < workers; t++) {
     threads.emplace_back([&]() {
@@ -142,6 +138,7 @@ extern "C" int deft_batch_solve(int device, int count, const deft_batch_problem 
         failed(-1, DEFT_ERR_CUDA, deft_last_error());
         return;
       }
+      std::call_once(pool_made, [&]() { pool = deft::make_call_pool(device); });
       deft::thread_pool = {pool, static_cast<cudaStream_t>(deft_ctx_stream(w.ctx))};
       for (;;) {
         const int k = next.fetch_add(1);

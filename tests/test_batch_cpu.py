@@ -1,5 +1,6 @@
 """The host side of a batch (csrc/batch.cu, csrc/dev_mem.h) against a model of
-the CUDA runtime: which error a batch reports.  The sources are compiled with
+the CUDA runtime: which error a batch reports, and that the calling thread
+keeps its device.  The sources are compiled with
 g++ against the few calls they make; no GPU."""
 import os
 import subprocess
@@ -151,10 +152,17 @@ static int errors() {
   }
   return 0;
 }
+static int caller_device() {
+  // a batch on another device than the caller's leaves the caller's thread alone
+  std::vector<deft_cg_status> st;
+  WANT(batch({problem(8, 0, 10)}, 1, st, 1) == DEFT_OK);
+  WANT(set_device_calls == 0);
+  return 0;
+}
 int main(int argc, char **argv) {
   caller = true;
   const std::string s = argv[1];
-  return s == "errors" ? errors() : 2;
+  return s == "errors" ? errors() : s == "caller_device" ? caller_device() : 2;
 }
 """
 
@@ -170,7 +178,7 @@ def program(tmp_path_factory):
     return str(d / "main")
 
 
-@pytest.mark.parametrize("scenario", ["errors"])
+@pytest.mark.parametrize("scenario", ["errors", "caller_device"])
 def test_batch_host(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
