@@ -148,12 +148,14 @@ extern "C" int deft_batch_solve(int device, int count, const deft_batch_problem 
         memset(&st, 0, sizeof(st));
         const int s = solve_one(w, probs[i], bp->cg, &st);
         st.status = s;
+        // what it freed is there for the other workers from here on
+        cudaStreamSynchronize(deft::thread_pool.stream);
         if (s) failed(i, s, "problem " + std::to_string(i) + ": " + deft_last_error());
       }
     });
   }
   for (auto &th : threads) th.join();
-  if (pool) cudaMemPoolDestroy(pool);
+  deft::end_call_pool(pool);
   if (first_error != DEFT_OK) deft::set_last_error_message(first_msg);
   return first_error;
 }

@@ -26,6 +26,7 @@
 // out of its 40 trials ends the FP32 stage at once (the host first retries
 // once along steepest descent), and the loop budget ends a solve with
 // DEFT_ERR_TIMEOUT instead of running on.
+#include "dev_mem.h"
 #include "devcg.h"
 
 #include <cmath>
@@ -875,8 +876,8 @@ void dcg_free(DcgGraph *gr) {
   if (gr->exec) cudaGraphExecDestroy(gr->exec);
   if (gr->graph) cudaGraphDestroy(gr->graph);
   for (Solve &s : gr->solves) {
-    cudaFree(s.st);
-    cudaFree(s.partials);
+    dev_free(s.st);
+    dev_free(s.partials);
   }
   if (gr->host) cudaFreeHost(gr->host);
   delete gr;
@@ -904,9 +905,9 @@ DcgGraph *dcg_build(const DcgProblem *p, int count, std::string *err) {
   for (int i = 0; i < count && r == cudaSuccess; i++) {
     Solve &sv = gr->solves[i];
     sv.p = p[i];
-    r = cudaMalloc((void **)&sv.st, sizeof(DcgState));
+    r = dev_malloc((void **)&sv.st, sizeof(DcgState));
     if (r == cudaSuccess)
-      r = cudaMalloc((void **)&sv.partials, sizeof(double) * 2 * sv.p.eng->vector_blocks());
+      r = dev_malloc((void **)&sv.partials, sizeof(double) * 2 * sv.p.eng->vector_blocks());
     if (r == cudaSuccess) r = cudaMemset(sv.st, 0, sizeof(DcgState));
   }
   if (r != cudaSuccess) {

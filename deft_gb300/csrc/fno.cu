@@ -18,6 +18,7 @@
 // pass reads BF16 copies (round-to-nearest-even of the masters) and
 // accumulates in FP32.
 #include "../../include/deft_gb300.h"
+#include "dev_mem.h"
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -1787,7 +1788,7 @@ int deft_fno_create(int device, int N, int channels, int modes, int layers, unsi
     }
   bool ok = true;
   auto dev = [&](auto **ptr, size_t bytes) {
-    if (ok && cudaMalloc((void **)ptr, bytes) != cudaSuccess) ok = false;
+    if (ok && deft::dev_malloc((void **)ptr, bytes) != cudaSuccess) ok = false;
   };
   const size_t pf = sizeof(float) * off;
   dev(&f->p, pf);
@@ -1885,10 +1886,10 @@ int deft_fno_destroy(deft_fno *f) {
                   (void *)f->mask, (void *)f->target, (void *)f->wt, (void *)f->A, (void *)f->B,
                   (void *)f->S, (void *)f->S2, (void *)f->hb0, (void *)f->hb1, (void *)f->zb,
                   (void *)f->part, (void *)f->loss_d, (void *)f->bulk, (void *)f->part_d})
-    cudaFree(q);
-  for (float *q : f->h) cudaFree(q);
-  for (float *q : f->z) cudaFree(q);
-  for (float2 *q : f->V) cudaFree(q);
+    deft::dev_free(q);
+  for (float *q : f->h) deft::dev_free(q);
+  for (float *q : f->z) deft::dev_free(q);
+  for (float2 *q : f->V) deft::dev_free(q);
   if (f->stream) cudaStreamDestroy(f->stream);
   delete f;
   return DEFT_OK;
@@ -2088,7 +2089,7 @@ int deft_fno_initial_density(deft_fno *f, deft_fmt *fmt, const double *mask_dev,
   if (shape[0] != f->N || shape[1] != f->N || shape[2] != f->N)
     return fno_fail(f, "functional grid does not match the network's N^3", DEFT_ERR_ARG);
   cudaSetDevice(f->device);
-  if (!f->bulk && cudaMalloc((void **)&f->bulk, sizeof(double) * 2 * f->NR) != cudaSuccess) {
+  if (!f->bulk && deft::dev_malloc((void **)&f->bulk, sizeof(double) * 2 * f->NR) != cudaSuccess) {
     f->bulk = nullptr;
     return fno_fail(f, "bulk start buffer", DEFT_ERR_NOMEM);
   }

@@ -1,7 +1,7 @@
 """The host side of a batch (csrc/batch.cu, csrc/dev_mem.h) against a model of
-the CUDA runtime: which error a batch reports, and that the calling thread
-keeps its device.  The sources are compiled with
-g++ against the few calls they make; no GPU."""
+the CUDA runtime: which error a batch reports, that the calling thread
+keeps its device, and that memory its pool holds unused is there for others.
+The sources are compiled with g++ against the few calls they make; no GPU."""
 import os
 import subprocess
 
@@ -39,6 +39,7 @@ cudaError_t cudaGetLastError();
 """
 
 PROGRAM = r"""
+#include <chrono>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -53,6 +54,7 @@ static std::map<void *, Block> blocks;
 static std::map<Pool *, int> pools;
 static size_t used = 0;  // bytes the device has given out (live, being freed, unused in pools)
 static const size_t kCapacity = 100;
+static uint64_t kept = 0;
 static int set_device_calls = 0;
 static bool fail_sync = false;
 static thread_local bool caller = false;
@@ -91,15 +93,22 @@ cudaError_t cudaStreamSynchronize(Stream *s) {
 }
 cudaError_t cudaMemPoolCreate(Pool **p, const cudaMemPoolProps *) { LOCK; *p = new Pool; pools[*p] = 1; return cudaSuccess; }
 cudaError_t cudaMemPoolDestroy(Pool *p) { LOCK; used -= p->unused; p->unused = 0; pools.erase(p); return cudaSuccess; }
-cudaError_t cudaMemPoolSetAttribute(Pool *, cudaMemPoolAttr, void *) { return cudaSuccess; }
+cudaError_t cudaMemPoolSetAttribute(Pool *, cudaMemPoolAttr a, void *v) {
+  if (a == cudaMemPoolAttrReleaseThreshold) kept = *(uint64_t *)v;
+  return cudaSuccess;
+}
 cudaError_t cudaMemPoolTrimTo(Pool *p, size_t) { LOCK; used -= p->unused; p->unused = 0; return cudaSuccess; }
 
 // the C ABI as far as batch.cu uses it; a problem's mu is the status of its
 // solve, its kT the device bytes it needs
 struct deft_ctx { Stream s; };
 struct deft_grid { deft_ctx *c; };
-struct deft_fmt { deft_grid *g; void *mem; int status; };
+struct deft_fmt { deft_grid *g; void *mem; int status; double R; };
 struct deft_cg { deft_fmt *f; };
+static std::atomic<bool> waiting(false), done(false);
+static void until(std::atomic<bool> &b) {
+  for (int i = 0; i < 10000 && !b; i++) std::this_thread::sleep_for(std::chrono::milliseconds(1));
+}
 static thread_local std::string err;
 namespace deft { void set_last_error_message(const std::string &m) { err = m; } }
 extern "C" {
@@ -111,8 +120,10 @@ int deft_grid_create(deft_ctx *c, const double *, int, int, int, deft_grid **g) 
 int deft_grid_destroy(deft_grid *g) { delete g; return 0; }
 int deft_fmt_create(deft_grid *g, const deft_fmt_params *p, deft_fmt **f) {
   void *m = nullptr;
-  if (p->kT > 0 && deft::dev_malloc(&m, (size_t)p->kT) != cudaSuccess) { err = "memory"; return DEFT_ERR_NOMEM; }
-  *f = new deft_fmt{g, m, (int)p->mu};
+  if (p->R == 2) until(waiting);
+  if (p->kT > 0 && deft::dev_malloc(&m, (size_t)p->kT) != cudaSuccess) { err = "memory"; done = true; return DEFT_ERR_NOMEM; }
+  if (p->R == 2) done = true;
+  *f = new deft_fmt{g, m, (int)p->mu, p->R};
   return 0;
 }
 int deft_fmt_destroy(deft_fmt *f) { if (f) deft::dev_free(f->mem); delete f; return 0; }
@@ -122,7 +133,10 @@ int deft_cg_create(deft_fmt *f, const deft_cg_params *, deft_cg **c) { *c = new 
 int deft_cg_destroy(deft_cg *c) { delete c; return 0; }
 int deft_cg_set_x(deft_cg *, const double *, int) { return 0; }
 int deft_cg_get_x(deft_cg *, double *, int) { return 0; }
-int deft_cg_solve(deft_cg *c, deft_cg_status *) { err = "status " + std::to_string(c->f->status); return c->f->status; }
+int deft_cg_solve(deft_cg *c, deft_cg_status *) {
+  if (c->f->R == 1) { waiting = true; until(done); }
+  err = "status " + std::to_string(c->f->status); return c->f->status;
+}
 }
 
 static deft_batch_problem problem(int n, int status, double bytes) {
@@ -130,6 +144,7 @@ static deft_batch_problem problem(int n, int status, double bytes) {
   p.N[0] = p.N[1] = p.N[2] = n;
   p.mu = status;
   p.kT = bytes;
+  p.R = 0;
   return p;
 }
 static int batch(std::vector<deft_batch_problem> pr, int workers, std::vector<deft_cg_status> &st, int device = 0) {
@@ -152,6 +167,36 @@ static int errors() {
   }
   return 0;
 }
+// After a problem of 60 bytes its worker is in another one; 60 bytes are asked
+// for by another worker of the call, by another call, and outside any call.
+static int memory(const char *who) {
+  const std::string w = who;
+  std::vector<deft_cg_status> st, st2;
+  auto big = problem(16, 0, 60), wait = problem(12, 0, 0), next = problem(8, 0, 60);
+  wait.R = 1;  // its solve waits for `done`
+  next.R = 2;  // its functional is made once `wait` is being solved
+  done = waiting = false;
+  int other = -1;
+  if (w == "worker") {
+    WANT(batch({big, wait, next}, 2, st) == DEFT_OK);
+    return 0;
+  }
+  std::thread call([&]() { other = batch({big, wait}, 1, st); });
+  until(waiting);
+  int got;
+  if (w == "call") {
+    got = batch({next}, 1, st2);
+  } else {
+    void *p = nullptr;
+    got = deft::dev_malloc(&p, 60);
+    deft::dev_free(p);
+  }
+  done = true;
+  call.join();
+  WANT(got == 0 && other == 0 && used == 0);
+  WANT(kept > 0 && kept < kCapacity);  // a bound on what a pool may keep
+  return 0;
+}
 static int caller_device() {
   // a batch on another device than the caller's leaves the caller's thread alone
   std::vector<deft_cg_status> st;
@@ -162,7 +207,8 @@ static int caller_device() {
 int main(int argc, char **argv) {
   caller = true;
   const std::string s = argv[1];
-  return s == "errors" ? errors() : s == "caller_device" ? caller_device() : 2;
+  return s == "errors" ? errors() : s == "caller_device" ? caller_device()
+         : s.substr(0, 7) == "memory_" ? memory(argv[1] + 7) : 2;
 }
 """
 
@@ -178,7 +224,8 @@ def program(tmp_path_factory):
     return str(d / "main")
 
 
-@pytest.mark.parametrize("scenario", ["errors", "caller_device"])
+@pytest.mark.parametrize("scenario", ["errors", "caller_device", "memory_worker", "memory_call",
+                                      "memory_alone"])
 def test_batch_host(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
