@@ -59,7 +59,12 @@ inline cudaError_t dev_malloc(void **p, size_t n) {
     if (t.pool) cudaStreamSynchronize(t.stream);
     if (call_pools().trim()) e = get();
   }
-  return e == cudaSuccess && t.pool && n ? cudaStreamSynchronize(t.stream) : e;
+  if (e != cudaSuccess || !t.pool || n == 0) return e;
+  if ((e = cudaStreamSynchronize(t.stream)) != cudaSuccess) {
+    cudaFreeAsync(*p, t.stream);  // callers keep no pointer of a failed allocation
+    *p = nullptr;
+  }
+  return e;
 }
 inline cudaError_t dev_free(void *p) {
   if (!p) return cudaSuccess;

@@ -197,6 +197,21 @@ static int memory(const char *who) {
   WANT(kept > 0 && kept < kCapacity);  // a bound on what a pool may keep
   return 0;
 }
+static int failed_wait() {
+  // an allocation whose stream fails gives its memory back
+  Stream s;
+  cudaMemPool_t pool = deft::make_call_pool(0);
+  deft::thread_pool = {pool, &s};
+  void *p = &s;
+  fail_sync = true;
+  WANT(deft::dev_malloc(&p, 10) == cudaErrorUnknown && p == nullptr);
+  fail_sync = false;
+  cudaStreamSynchronize(&s);
+  WANT(blocks.empty());
+  deft::thread_pool = {};
+  deft::end_call_pool(pool);
+  return 0;
+}
 static int caller_device() {
   // a batch on another device than the caller's leaves the caller's thread alone
   std::vector<deft_cg_status> st;
@@ -208,6 +223,7 @@ int main(int argc, char **argv) {
   caller = true;
   const std::string s = argv[1];
   return s == "errors" ? errors() : s == "caller_device" ? caller_device()
+         : s == "failed_wait" ? failed_wait()
          : s.substr(0, 7) == "memory_" ? memory(argv[1] + 7) : 2;
 }
 """
@@ -225,7 +241,7 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("scenario", ["errors", "caller_device", "memory_worker", "memory_call",
-                                      "memory_alone"])
+                                      "memory_alone", "failed_wait"])
 def test_batch_host(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
