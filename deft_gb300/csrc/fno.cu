@@ -1507,11 +1507,6 @@ void launch_axis(deft_fno *f, const float2 *in, float2 *out, const float2 *E, in
   if (sm <= 96 * 1024) {
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
-    static bool attr[64] = {};  // the shared-memory cap, set once per device
-    if (dev < 0 || dev >= 64 || !attr[dev]) {
-      cudaFuncSetAttribute(k_dft_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-      if (dev >= 0 && dev < 64) attr[dev] = true;
-    }
     // tiles per block pass: fill the 256 threads when a tile has few items
     const int per = (ax_rows(Mout) / kAxMR) * IC;
     int S = per >= 256 ? 1 : 256 / per;
@@ -1539,11 +1534,6 @@ void launch_axis(deft_fno *f, const float2 *in, float2 *out, const float2 *E, in
                                                                               Nin, Mout, inner);
 }
 
-// The shared-memory cap of a kernel, for the current device.
-template <typename K> void allow_smem(K kernel, size_t bytes) {
-  if (bytes > 48 * 1024)
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
 // Calls g(std::integral_constant<int, KB>()) with Kz rounded up to the register tile.
 template <typename F> void with_kb(int Kz, F &&g) {
   switch (kz_block(Kz)) {
@@ -1567,7 +1557,6 @@ void analyse_zy(deft_fno *f, const float *in, const float2 *E) {
   with_kb(f->Kz, [&](auto kb) {
     constexpr int KB = decltype(kb)::value;
     const size_t sm = slab_fwd_smem(N, f->m, KB);
-    allow_smem(k_slab_fwd<KB>, sm);
     k_slab_fwd<KB><<<C * N, 64 * slab_chunks(N), sm, f->stream>>>(in, f->B, E, f->Yc, N, f->Kz,
                                                                   f->m);
   });
@@ -1585,7 +1574,6 @@ void synthesise_yz(deft_fno *f, float *out, const float2 *G, int accumulate) {
   with_kb(f->Kz, [&](auto kb) {
     constexpr int KB = decltype(kb)::value;
     const size_t sm = slab_inv_smem(N, f->m, KB);
-    allow_smem(k_slab_inv<KB>, sm);
     k_slab_inv<KB><<<C * N, 128, sm, f->stream>>>(f->B, out, G, f->Yc, N, f->Kz, f->m, accumulate);
   });
 }
@@ -1614,7 +1602,6 @@ void launch_layer_synth(deft_fno *f, int l) {
   f->launches++;
   if (f->slab) {
     const size_t sm = synth_smem<C>(N, f->m, f->Kz);
-    allow_smem(k_layer_synth<C>, sm);
     // blocks per x: the fewest rounds of two blocks per SM, a round costing
     // its passes and about two more for the block's tables
     const int most = (N + lpb - 1) / lpb;
@@ -1635,7 +1622,6 @@ void launch_layer_synth(deft_fno *f, int l) {
   launch_axis(f, f->B, f->A, f->Eyi, C * N, f->Ky, N, f->Kz);  // [C N N Kz]
   const size_t sm = sizeof(float) * (C * C + ((C + 3) & ~3)) +
                     sizeof(float2) * ((size_t)f->Kz * N + (size_t)lpb * C * f->Kz);
-  allow_smem(k_layer_synth_pw<C>, sm);
   const int lines = N * N;
   int grid = 4 * sms;
   const int need = (lines + lpb - 1) / lpb;
@@ -1643,6 +1629,39 @@ void launch_layer_synth(deft_fno *f, int l) {
   k_layer_synth_pw<C><<<grid, 256, sm, f->stream>>>(f->A, f->Gzi, f->h[l], f->h[l + 1],
                                                     f->pb + f->oWp[l], f->pb + f->ob[l], N, f->Kz,
                                                     act);
+}
+
+// A kernel's shared-memory cap: the device's maximum, whatever this network
+// needs.  The cap belongs to the function, which networks of other sizes launch
+// too, from other threads.
+template <typename K> cudaError_t full_smem(K kernel) {
+  cudaFuncAttributes fa;
+  int dev = 0, most = 0;
+  cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             most - (int)fa.sharedSizeBytes);
+  return e;
+}
+template <int C> cudaError_t synth_caps() {
+  const cudaError_t e = full_smem(k_layer_synth<C>);
+  return e == cudaSuccess ? full_smem(k_layer_synth_pw<C>) : e;
+}
+// The caps of the kernels a network launches, for the current device.
+cudaError_t kernel_caps(const deft_fno *f) {
+  cudaError_t e = full_smem(k_dft_axis);
+  if (e == cudaSuccess) e = full_smem(k_dft_tile);
+  with_kb(f->Kz, [&](auto kb) {
+    constexpr int KB = decltype(kb)::value;
+    if (e == cudaSuccess) e = full_smem(k_dft_z_fwd<KB>);
+    if (e == cudaSuccess) e = full_smem(k_slab_fwd<KB>);
+    if (e == cudaSuccess) e = full_smem(k_slab_inv<KB>);
+  });
+  if (e != cudaSuccess) return e;
+  return f->C == 16 ? synth_caps<16>() : f->C == 8 ? synth_caps<8>() : synth_caps<4>();
 }
 
 // Adjoint of the spectral part for upstream zbar: adds K^T zbar to hin_bar and
@@ -1859,13 +1878,11 @@ int deft_fno_create(int device, int N, int channels, int modes, int layers, unsi
   cudaMemcpy(f->Exf, exf.data(), sizeof(float2) * exf.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(f->Exi, exi.data(), sizeof(float2) * exi.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(f->Yc, yc.data(), sizeof(float2) * yc.size(), cudaMemcpyHostToDevice);
-  const size_t zf = smem_z_fwd(N, f->Kz);
-  cudaFuncSetAttribute(k_dft_z_fwd<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zf);
-  cudaFuncSetAttribute(k_dft_z_fwd<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zf);
-  cudaFuncSetAttribute(k_dft_z_fwd<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zf);
-  cudaFuncSetAttribute(k_dft_z_fwd<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zf);
-  cudaFuncSetAttribute(k_dft_axis, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(sizeof(float2) * 2 * modes * N));
+  if (kernel_caps(f) != cudaSuccess) {
+    check(f, "fno shared memory");
+    deft_fno_destroy(f);
+    return DEFT_ERR_CUDA;
+  }
   k_to_bf16<<<grid_for((long long)off), kT, 0, f->stream>>>(f->p, f->pb, (long long)off);
   if (check(f, "fno create")) {
     deft_fno_destroy(f);
