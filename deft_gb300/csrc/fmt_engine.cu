@@ -4834,16 +4834,14 @@ int noalloc_energy_grad(const GridSpec &s, const FmtSpec &f, const double *n, co
   plan_fill_ns(pz);
 
   const size_t cs = sizeof(double2);
-  const Tiles t = make_tiles(g, cs, kBudget64);
+  Tiles t = make_tiles(g, cs, kBudget64);
   const int pairs = (g.lines + 1) / 2;
   if (t.smem_max() > 227 * 1024) {
     noalloc_fail(err, "grid line too long for one shared-memory tile");
     return 1;
   }
-  const int nblk_phi = (pairs + t.Pphi - 1) / t.Pphi;
-  const int nblk = (f.terms & kTermHS) ? nblk_phi : 4 * 152;
 
-  // scratch layout
+  // scratch layout; the energy partials (a row a Phi tile) come last
   size_t off = 0;
   const size_t o_twx = off; off += align256(cs * g.Nx);
   const size_t o_twy = off; off += align256(cs * g.Ny);
@@ -4853,9 +4851,22 @@ int noalloc_energy_grad(const GridSpec &s, const FmtSpec &f, const double *n, co
   const size_t o_wv = off; off += align256(sizeof(double) * g.NC);
   const size_t o_S0 = off; off += align256(cs * g.NC);
   const size_t o_S5 = off; off += align256(5 * cs * g.NC);
-  const size_t o_part = off; off += align256(sizeof(double) * kNumTerms * nblk);
   const size_t o_res = off; off += align256(sizeof(double) * 8);
   const size_t o_la = off; off += align256(sizeof(LocalArgs));
+  const size_t o_part = off;
+  auto part_bytes = [&](int P) {
+    return align256(sizeof(double) * kNumTerms * ((pairs + P - 1) / P));
+  };
+  if ((f.terms & kTermHS) && off + part_bytes(t.Pphi) > kNoAllocScratchBytes) {
+    // tiles as wide as the shared-memory budget have fewer partials
+    TileChoice widest;
+    const size_t fit = kBudget64 / (10 * (size_t)g.Nz * cs);
+    widest.Pphi = fit >= 15 ? 15 : fit > 1 ? (int)fit : 1;
+    if (widest.Pphi > t.Pphi) t = make_tiles(g, cs, kBudget64, &widest);
+  }
+  const int nblk_phi = (pairs + t.Pphi - 1) / t.Pphi;
+  const int nblk = (f.terms & kTermHS) ? nblk_phi : 4 * 152;
+  off += align256(sizeof(double) * kNumTerms * nblk);
   if (off > kNoAllocScratchBytes) {
     noalloc_fail(err, "no-allocation energy_grad: this grid needs " + std::to_string(off) +
                           " bytes of scratch; the fixed device array holds " +
