@@ -2619,16 +2619,19 @@ __global__ void k_veff_grad(double kT, const double *__restrict__ x, const doubl
 // ---------------------------------------------------------------------------
 // Host side
 
-bool factorize(int n, FftPlan &p) {
+bool factorize(int n, FftPlan &p, bool fp64) {
   int k = 0;
   p.n = n;
   p.reg = 0;
   int e = 0;
   while (n % 2 == 0) { e++; n /= 2; }
   // eights, then fours; a lone radix-2 pass moves every element for one
-  // addition, so 8 x 2 becomes 4 x 4 (x convolutions of an 80^3 grid 60 -> 54
-  // us, Phi at 128^3 297 -> 287)
-  const int eights = e / 3 - (e % 3 == 1 && e > 1 ? 1 : 0);
+  // addition, so double-float takes 8 x 2 as 4 x 4 (x convolutions of an 80^3
+  // grid 60 -> 54 us, Phi at 128^3 297 -> 287) and FP64 8 x 8 x 2 as 8 x 4 x 4
+  // (128^3: 337 -> 334 us) but not 8 x 2, whose first pass is one round of the
+  // block's threads on a tile where 4 x 4's is two (80^3: 102 us as 8 x 2 x 5,
+  // 115 as 4 x 4 x 5; 112^3 283 and 311, 144^3 562 and 621)
+  const int eights = e / 3 - (e % 3 == 1 && e > (fp64 ? 4 : 1) ? 1 : 0);
   for (int i = 0; i < eights; i++, e -= 3) p.radix[k++] = 8;
   for (; e >= 2; e -= 2) p.radix[k++] = 4;
   if (e) p.radix[k++] = 2;
@@ -2717,12 +2720,12 @@ double bulk_density(double R, double kT, double mu, int hs) {
 // Tile widths and shared-memory sizes of every kernel for one precision
 // (cs = bytes of one complex element).
 struct Tiles {
-  int By = 1, Bx = 1, Bxf = 1, Bxc = 1, Pz = 1, Pphi = 1;
-  FastDiv fBy{}, fBx{}, fBxf{}, fBxc{}, f5Bxc{}, fPz{}, fPphi{}, f5Pphi{};
-  size_t smem_y = 0, smem_x2 = 0, smem_xf = 0, smem_xc = 0, smem_z = 0, smem_phi = 0;
+  int By = 1, Bx = 1, Bxf = 1, Bxc = 1, Pz = 1, Pz5 = 1, Pphi = 1;
+  FastDiv fBy{}, fBx{}, fBxf{}, fBxc{}, f5Bxc{}, fPz{}, fPz5{}, fPphi{}, f5Pphi{};
+  size_t smem_y = 0, smem_x2 = 0, smem_xf = 0, smem_xc = 0, smem_z = 0, smem_z5 = 0, smem_phi = 0;
   size_t smem_max() const {
     size_t m = smem_y;
-    for (size_t v : {smem_x2, smem_xf, smem_xc, smem_z, smem_phi}) m = v > m ? v : m;
+    for (size_t v : {smem_x2, smem_xf, smem_xc, smem_z, smem_z5, smem_phi}) m = v > m ? v : m;
     return m;
   }
 };
@@ -2741,6 +2744,7 @@ void finish_tiles(Tiles &t, const Geom &g, size_t cs) {
   t.fBxc = make_fastdiv(t.Bxc);
   t.f5Bxc = make_fastdiv(5 * t.Bxc);
   t.fPz = make_fastdiv(t.Pz);
+  t.fPz5 = make_fastdiv(t.Pz5);
   t.fPphi = make_fastdiv(t.Pphi);
   t.f5Pphi = make_fastdiv(5 * t.Pphi);
   t.smem_y = 2 * (size_t)g.Ny * t.By * cs;
@@ -2748,6 +2752,7 @@ void finish_tiles(Tiles &t, const Geom &g, size_t cs) {
   t.smem_xf = 3 * (size_t)g.Nx * t.Bxf * cs + (cs == 8 ? 3 * (size_t)g.Nx * t.Bxf * 4 : 0);
   t.smem_xc = 10 * (size_t)g.Nx * t.Bxc * cs;
   t.smem_z = 2 * (size_t)g.Nz * t.Pz * cs;
+  t.smem_z5 = 2 * (size_t)g.Nz * t.Pz5 * cs;
   t.smem_phi = 10 * (size_t)g.Nz * t.Pphi * cs;
 }
 
@@ -2782,6 +2787,11 @@ int five_field_tile(const FftPlan &p, int n, int count, size_t budget, int sms) 
   return best;
 }
 
+// FP64 arithmetic: a block per tile and field pays for its extra forward
+// transforms while the blocks of one field leave two fifths of the SMs idle
+// (events, 48^3, 75 tiles: 47 -> 37 us; 64^3, 132 tiles: 53 -> 67).
+bool split_x_fp64(int tiles, int sms) { return 5 * tiles <= 3 * sms; }
+
 // Built-in rule: the widest tiles within `budget` bytes of shared memory (at
 // most 16 columns / pairs), evened out over the lines; overrides from `ov`.
 // The FP64 and double-float kernels (16-byte elements) are issue-bound, so
@@ -2795,7 +2805,18 @@ int five_field_tile(const FftPlan &p, int n, int count, size_t budget, int sms) 
 //   x convolutions: forward 256 / (Nx / smallest radix) columns (96^3: 8, 59 us
 //     against 65 with 16), adjoint four (96^3 63 us against 76 with 6, 77^3 61
 //     against 71 with 7).
-Tiles make_tiles(const Geom &g, size_t cs, size_t budget, const TileChoice *ov = nullptr) {
+// FP64 arithmetic (fp64) is bound by the FP64 pipe: a launch takes its tiles' waves
+// over the SMs, each as long as a tile is wide, and the width B is the one with the
+// least ceil(tiles / SMs) (B + 1).
+//   forward x convolution: 80^3 102 us at 12 columns, 131 at 16; 100^3 234 at 12,
+//     262 at 10; 128^3 343 at 14, 387 at 16.  Where 16 columns leave two fifths of
+//     the SMs idle a block takes one field (split_x_fp64), of 16 columns or of 8
+//     where that is less (its overhead counted as 4: 32^3 16 us at 8, 19 at 16; 48^3
+//     39 and 37)
+//   the z kernel of five fields: 48^3 20 us at 15 pairs, 33 at 3; 64^3 37 at 15, 41
+//     at 7; 80^3 74 at 16, 80 at 15, 84 at 5; 96^3 115 at 13, 122 at 15
+Tiles make_tiles(const Geom &g, size_t cs, size_t budget, const TileChoice *ov = nullptr,
+                 bool fp64 = false) {
   Tiles t;
   const int pairs = (g.lines + 1) / 2;
   auto cap = [](size_t v, int hi) { return (int)(v < (size_t)hi ? v : (size_t)hi); };
@@ -2804,6 +2825,7 @@ Tiles make_tiles(const Geom &g, size_t cs, size_t budget, const TileChoice *ov =
   t.Bxf = even_tiles(g.Ny * g.NzH, cap(budget / (3 * (size_t)g.Nx * cs), 16));
   t.Bxc = even_tiles(g.Ny * g.NzH, cap(budget / (10 * (size_t)g.Nx * cs), 16));
   t.Pz = even_tiles(pairs, cap(budget / (2 * (size_t)g.Nz * cs), 16));
+  t.Pz5 = t.Pz;
   if (t.Pz > 1 && t.Pz % 2 == 0) t.Pz -= 1;  // odd, as Pphi below
   int pm = cap(budget / (10 * (size_t)g.Nz * cs), 15);
   if (pm < 1) pm = 1;
@@ -2816,17 +2838,36 @@ Tiles make_tiles(const Geom &g, size_t cs, size_t budget, const TileChoice *ov =
     pm = most(1, least(most(fit, g.Nz > 192 ? 2 : 1), least((2 * 409 / g.Nz + 1) / 2, most(1, pairs / kSms))));
     if (10 * (size_t)g.Nz * pm * cs > 200 * 1024) pm = 1;
     t.Pz = most(1, least(t.Pz, least(1100 / g.Nz, most(2, pairs / (2 * kSms))) | 1));
-    int rmin = 8;
-    FftPlan px;
-    if (factorize(g.Nx, px))
-      for (int i = 0; i < px.npass; i++) rmin = least(rmin, px.radix[i]);
-    t.Bxf = least(t.Bxf, most(4, 256 * rmin / g.Nx));
+    if (fp64) {
+      // waves of `fields` fields' tiles of B of `count` lines, times B + c
+      auto cost = [&](int count, int B, int fields, int c) {
+        return (fields * ((count + B - 1) / B) + kSms - 1) / kSms * (B + c);
+      };
+      const int J = g.Ny * g.NzH, widest = t.Bxf, half = (widest + 1) / 2;
+      if (split_x_fp64((J + widest - 1) / widest, kSms)) {
+        if (split_x_fp64((J + half - 1) / half, kSms) && cost(J, half, 5, 4) < cost(J, widest, 5, 4))
+          t.Bxf = half;
+      } else {
+        for (int B = widest - 1; B >= 4; B--)
+          if (cost(J, B, 1, 1) < cost(J, t.Bxf, 1, 1)) t.Bxf = B;
+      }
+      for (int P = t.Pz5 - 1; P >= 4; P--)
+        if (cost(pairs, P, 5, 1) < cost(pairs, t.Pz5, 5, 1)) t.Pz5 = P;
+    } else {
+      int rmin = 8;
+      FftPlan px;
+      if (factorize(g.Nx, px, false))
+        for (int i = 0; i < px.npass; i++) rmin = least(rmin, px.radix[i]);
+      t.Bxf = least(t.Bxf, most(4, 256 * rmin / g.Nx));
+      t.Pz5 = t.Pz;
+    }
     t.Bxc = least(t.Bxc, 4);
   } else {
     constexpr int kSms = 152;
     FftPlan px, pz;
     if (factorize_f32(g.Nx, px)) t.Bxc = five_field_tile(px, g.Nx, g.Ny * g.NzH, budget, kSms);
     if (factorize_f32(g.Nz, pz)) pm = five_field_tile(pz, g.Nz, pairs, budget, kSms);
+    t.Pz5 = t.Pz;
   }
   t.Pphi = pm < pairs ? pm : pairs;
   if (ov) {
@@ -2834,7 +2875,7 @@ Tiles make_tiles(const Geom &g, size_t cs, size_t budget, const TileChoice *ov =
     if (ov->Bx > 0) t.Bx = ov->Bx < g.Ny * g.NzH ? ov->Bx : g.Ny * g.NzH;
     if (ov->Bxf > 0) t.Bxf = ov->Bxf < g.Ny * g.NzH ? ov->Bxf : g.Ny * g.NzH;
     if (ov->Bxc > 0) t.Bxc = ov->Bxc < g.Ny * g.NzH ? ov->Bxc : g.Ny * g.NzH;
-    if (ov->Pz > 0) t.Pz = ov->Pz < pairs ? ov->Pz : pairs;
+    if (ov->Pz > 0) t.Pz5 = t.Pz = ov->Pz < pairs ? ov->Pz : pairs;
     if (ov->Pphi > 0) t.Pphi = ov->Pphi < pairs ? ov->Pphi : pairs;
   }
   finish_tiles(t, g, cs);
@@ -2995,8 +3036,11 @@ class EngineImpl {
   double *grad_partials = nullptr;  // k_z_grad's dot-product block sums
   unsigned int *dot_counter = nullptr;
   int dot_blocks = 0;
-  Tiles t64, t32;  // launch shapes of the FP64 and the FP32 kernels
-  template <typename T> const Tiles &tl() const { return sizeof(T) == 4 ? t32 : t64; }
+  // launch shapes of the double-float, FP32 and FP64 kernels
+  Tiles t64, t32, tfp64;
+  template <typename T> const Tiles &tl() const {
+    return sizeof(T) == 4 ? t32 : is_df<T> ? t64 : tfp64;
+  }
   size_t bytes = 0;
   std::string err;
 
@@ -3059,14 +3103,15 @@ class EngineImpl {
 
   int make_plan(int n, FftPlan &p, double2 **tw, FftPlan &pf, float2 **twf, FftPlan &pd,
                 dfc **twd) {
-    if (!factorize(n, p)) {
+    if (!factorize(n, p, true)) {
       err = "grid size " + std::to_string(n) + " has a prime factor above 13";
       return -1;
     }
     plan_fill_ns(p);
     pf = p;
     if (!factorize_f32(n, pf)) pf = p;
-    pd = p;
+    factorize(n, pd, false);
+    plan_fill_ns(pd);
     std::vector<double2> h(n);
     std::vector<float2> hf(n);
     std::vector<dfc> hd(n);
@@ -3165,24 +3210,25 @@ class EngineImpl {
 
     const size_t cs = sizeof(double2);
     t64 = make_tiles(g, sizeof(double2), kBudget64);
+    tfp64 = make_tiles(g, sizeof(double2), kBudget64, nullptr, true);
     t32 = make_tiles(g, sizeof(float2), kBudget32);
     const int pairs = (g.lines + 1) / 2;
     const size_t mx = 227 * 1024;
-    if (t64.smem_max() > mx || t32.smem_max() > mx) {
+    if (t64.smem_max() > mx || tfp64.smem_max() > mx || t32.smem_max() > mx) {
       err = "grid line too long for one shared-memory tile";
       return -1;
     }
-    set_smem(k_z_r2c<double>, t64.smem_z);
-    set_smem(k_z_c2r<double>, t64.smem_z);
-    set_smem(k_y_fft<double, -1>, t64.smem_y);
-    set_smem(k_y_fft<double, +1>, t64.smem_y);
-    set_smem(k_x_fft<double, -1>, t64.smem_x2);
-    set_smem(k_x_fft<double, +1>, t64.smem_x2);
-    set_smem(k_x_conv_fwd<double>, t64.smem_xf);
-    set_smem(k_x_conv_adj<double>, t64.smem_xc);
-    set_smem(k_z_phi<double, false>, t64.smem_phi);
-    set_smem(k_z_phi<double, true>, t64.smem_phi);
-    set_smem(k_z_grad<double>, t64.smem_z);
+    set_smem(k_z_r2c<double>, tfp64.smem_z);
+    set_smem(k_z_c2r<double>, tfp64.smem_z5);
+    set_smem(k_y_fft<double, -1>, tfp64.smem_y);
+    set_smem(k_y_fft<double, +1>, tfp64.smem_y);
+    set_smem(k_x_fft<double, -1>, tfp64.smem_x2);
+    set_smem(k_x_fft<double, +1>, tfp64.smem_x2);
+    set_smem(k_x_conv_fwd<double>, tfp64.smem_xf);
+    set_smem(k_x_conv_adj<double>, tfp64.smem_xc);
+    set_smem(k_z_phi<double, false>, tfp64.smem_phi);
+    set_smem(k_z_phi<double, true>, tfp64.smem_phi);
+    set_smem(k_z_grad<double>, tfp64.smem_z);
     set_smem(k_x_fft<float, -1>, t32.smem_x2);
     set_smem(k_x_fft<float, +1>, t32.smem_x2);
     set_smem(k_z_c2r<float>, t32.smem_z);
@@ -3341,10 +3387,11 @@ class EngineImpl {
       err = "tile choice exceeds shared memory";
       return -1;
     }
-    FftPlan np[3] = {f32 ? pxf : px, f32 ? pyf : py, f32 ? pzf : pz};
+    // FP32's plans, or double-float's and FP64's (one order for both)
+    FftPlan np[3] = {f32 ? pxf : pxd, f32 ? pyf : pyd, f32 ? pzf : pzd}, np64[3] = {px, py, pz};
     for (int a = 0; a < 3; a++) {
       if (!c.radix[a][0] || (f32 && set_reg_order(np[a], c.radix[a]))) continue;
-      if (!set_radix_order(np[a], c.radix[a])) {
+      if (!set_radix_order(np[a], c.radix[a]) || !set_radix_order(np64[a], c.radix[a])) {
         err = "radix order does not factor axis " + std::to_string(a);
         return -1;
       }
@@ -3370,30 +3417,28 @@ class EngineImpl {
       pzf = np[2];
     } else {
       t64 = t;
-      px = np[0];
-      py = np[1];
-      pz = np[2];
-      // the double-float plans share the FP64 radix orders (own twiddles)
-      FftPlan *pd[3] = {&pxd, &pyd, &pzd};
-      for (int a = 0; a < 3; a++) {
-        const void *tw = pd[a]->tw;
-        *pd[a] = np[a];
-        pd[a]->tw = tw;
-      }
+      tfp64 = make_tiles(g, cs, kBudget64, &c, true);
+      pxd = np[0];
+      pyd = np[1];
+      pzd = np[2];
+      px = np64[0];
+      py = np64[1];
+      pz = np64[2];
     }
     return 0;
   }
 
   void get_tiles(int prec, TileChoice *c) const {
     const bool f32 = prec == kPrecisionMixed;
-    const Tiles &t = f32 ? t32 : t64;
+    const Tiles &t = f32 ? t32 : df_on ? t64 : tfp64;
     c->By = t.By;
     c->Bx = t.Bx;
     c->Bxf = t.Bxf;
     c->Bxc = t.Bxc;
     c->Pz = t.Pz;
     c->Pphi = t.Pphi;
-    const FftPlan *pl[3] = {f32 ? &pxf : &px, f32 ? &pyf : &py, f32 ? &pzf : &pz};
+    const FftPlan *pl[3] = {f32 ? &pxf : df_on ? &pxd : &px, f32 ? &pyf : df_on ? &pyd : &py,
+                            f32 ? &pzf : df_on ? &pzd : &pz};
     for (int a = 0; a < 3; a++)
       for (int i = 0; i < 8; i++) {
         if (pl[a]->nord) c->radix[a][i] = i < pl[a]->nord ? pl[a]->order[i] : 0;
@@ -3502,7 +3547,9 @@ class EngineImpl {
   // events: 32^3 (34 tiles) 22.8 -> 13.8 us, 48^3 (75) 27.3 -> 16.5, 56^3 (102)
   // 40.6 -> 33.7; beyond the line 72^3 (267) 38.9 -> 44.5, 96^3 (588) 58.3 -> 83.9.
   // FP32: 24^3 14.5 -> 9.7, 56^3 18.9 -> 13.5; 77^3 (189) 23.8 -> 24.5.
-  bool split_x(int B) const { return x_tiles(B) <= sms; }
+  template <typename T> bool split_x(int B) const {
+    return std::is_same<T, double>::value ? split_x_fp64(x_tiles(B), sms) : x_tiles(B) <= sms;
+  }
 
   // Queues the adjoint x convolution: spec5 -> spec0.
   template <typename T> void x_conv_adj() {
@@ -3652,7 +3699,7 @@ class EngineImpl {
                      &la_dev->R, stream);
     } else {
       with_rn<T>(plan<T>(0), [&](auto rn) {
-        k_x_conv_fwd<T, decltype(rn)::value><<<dim3(x_tiles(t.Bxf), split_x(t.Bxf) ? 5 : 1),
+        k_x_conv_fwd<T, decltype(rn)::value><<<dim3(x_tiles(t.Bxf), split_x<T>(t.Bxf) ? 5 : 1),
                                                kThreads, t.smem_xf, stream>>>(
             spec0<T>(), spec5<T>(), table<T>(0), table<T>(1), table<T>(2), g, plan<T>(0), t.fBxf,
             la_dev);
@@ -4265,13 +4312,13 @@ int Engine::fft(const double *in, double2 *out, Arith a) {
     return e.check("fft");
   }
   e.pre(kK_z_r2c);
-    k_z_r2c<double><<<dim3(e.pairs_tiles(e.t64.Pz), 1), kThreads, e.t64.smem_z, e.stream>>>(
-      in, out, e.g, e.pz, e.t64.fPz, 1.0);
+    k_z_r2c<double><<<dim3(e.pairs_tiles(e.tfp64.Pz), 1), kThreads, e.tfp64.smem_z, e.stream>>>(
+      in, out, e.g, e.pz, e.tfp64.fPz, 1.0);
     e.post(kK_z_r2c);
   e.y_fft<double>(out, 1, -1);
   e.pre(kK_x_fft);
-    k_x_fft<double, -1><<<e.x_tiles(e.t64.Bx), kThreads, e.t64.smem_x2, e.stream>>>(
-      out, e.g, e.px, e.t64.fBx, e.g.dV);
+    k_x_fft<double, -1><<<e.x_tiles(e.tfp64.Bx), kThreads, e.tfp64.smem_x2, e.stream>>>(
+      out, e.g, e.px, e.tfp64.fBx, e.g.dV);
     e.post(kK_x_fft);
   return e.check("fft");
 }
@@ -4313,13 +4360,13 @@ int Engine::ifft(const double2 *in, double *out, Arith a) {
   }
   cudaMemcpyAsync(e.S0, in, sizeof(double2) * e.g.NC, cudaMemcpyDeviceToDevice, e.stream);
   e.pre(kK_x_fft);
-    k_x_fft<double, +1><<<e.x_tiles(e.t64.Bx), kThreads, e.t64.smem_x2, e.stream>>>(
-      e.S0, e.g, e.px, e.t64.fBx, 1.0);
+    k_x_fft<double, +1><<<e.x_tiles(e.tfp64.Bx), kThreads, e.tfp64.smem_x2, e.stream>>>(
+      e.S0, e.g, e.px, e.tfp64.fBx, 1.0);
     e.post(kK_x_fft);
   e.y_fft<double>(e.S0, 1, +1);
   e.pre(kK_z_c2r);
-    k_z_c2r<double><<<dim3(e.pairs_tiles(e.t64.Pz), 1), kThreads, e.t64.smem_z, e.stream>>>(
-      e.S0, out, e.g, e.pz, e.t64.fPz, 1.0 / e.g.vol);
+    k_z_c2r<double><<<dim3(e.pairs_tiles(e.tfp64.Pz), 1), kThreads, e.tfp64.smem_z, e.stream>>>(
+      e.S0, out, e.g, e.pz, e.tfp64.fPz, 1.0 / e.g.vol);
     e.post(kK_z_c2r);
   return e.check("ifft");
 }
@@ -4362,9 +4409,9 @@ int Engine::weighted(const FmtSpec &f, const double *n, double *out5, Arith a) {
   }
   if (e.ensure_table<double>(f.R) || e.forward_weighted<double>(f, n)) return -1;
   e.pre(kK_z_c2r);
-    k_z_c2r<double><<<dim3(e.pairs_tiles(e.t64.Pz), 5), kThreads, e.t64.smem_z, e.stream>>>(
-      e.S5, out5, e.g, e.pz, e.t64.fPz, 1.0);
-    e.post(kK_z_c2r);
+  k_z_c2r<double><<<dim3(e.pairs_tiles(e.tfp64.Pz5), 5), kThreads, e.tfp64.smem_z5, e.stream>>>(
+      e.S5, out5, e.g, e.pz, e.tfp64.fPz5, 1.0);
+  e.post(kK_z_c2r);
   return e.check("weighted");
 }
 
@@ -4791,7 +4838,7 @@ int noalloc_energy_grad(const GridSpec &s, const FmtSpec &f, const double *n, co
       return 1;
     }
   FftPlan px{}, py{}, pz{};
-  if (!factorize(s.Nx, px) || !factorize(s.Ny, py) || !factorize(s.Nz, pz)) {
+  if (!factorize(s.Nx, px, true) || !factorize(s.Ny, py, true) || !factorize(s.Nz, pz, true)) {
     noalloc_fail(err, "no-allocation energy_grad: grid sizes must factor into primes <= 13");
     return 1;
   }
@@ -4834,7 +4881,7 @@ int noalloc_energy_grad(const GridSpec &s, const FmtSpec &f, const double *n, co
   plan_fill_ns(pz);
 
   const size_t cs = sizeof(double2);
-  Tiles t = make_tiles(g, cs, kBudget64);
+  Tiles t = make_tiles(g, cs, kBudget64, nullptr, true);
   const int pairs = (g.lines + 1) / 2;
   if (t.smem_max() > 227 * 1024) {
     noalloc_fail(err, "grid line too long for one shared-memory tile");
@@ -4862,7 +4909,7 @@ int noalloc_energy_grad(const GridSpec &s, const FmtSpec &f, const double *n, co
     TileChoice widest;
     const size_t fit = kBudget64 / (10 * (size_t)g.Nz * cs);
     widest.Pphi = fit >= 15 ? 15 : fit > 1 ? (int)fit : 1;
-    if (widest.Pphi > t.Pphi) t = make_tiles(g, cs, kBudget64, &widest);
+    if (widest.Pphi > t.Pphi) t = make_tiles(g, cs, kBudget64, &widest, true);
   }
   const int nblk_phi = (pairs + t.Pphi - 1) / t.Pphi;
   const int nblk = (f.terms & kTermHS) ? nblk_phi : 4 * 152;

@@ -1,0 +1,62 @@
+"""The launch shapes of the FP64 kernels (the weighted densities' transforms)
+are chosen for FP64 arithmetic: at these sizes neither the five-field z transform
+nor the x convolution is beaten by another tile width.
+
+Times by events, the least of five batches; 15 % allowed for their noise (a
+launch of these takes 10 to 60 us and repeats to 2 or 3 %)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _times(L, g, run):
+    best = {}
+    for _ in range(5):
+        run()
+        L.deft_grid_profile(g.h, 1)
+        for _ in range(10):
+            run()
+        for i in range(L.deft_grid_profile_count(g.h)):
+            name, launches, ms = ctypes.c_char_p(), ctypes.c_longlong(), ctypes.c_double()
+            L.deft_grid_profile_entry(g.h, i, ctypes.byref(name), ctypes.byref(launches),
+                                      ctypes.byref(ms))
+            if launches.value:
+                k, us = name.value.decode(), 1e3 * ms.value / launches.value
+                best[k] = min(us, best.get(k, us))
+    L.deft_grid_profile(g.h, 0)
+    return best
+
+
+@pytest.mark.parametrize("n", [32, 48, 60, 64, 72])
+def test_widths(n):
+    import torch
+    from deft_gb300 import _lib
+    from tests.capi import Ctx, Fmt, Grid
+    L = _lib.load()
+    ctx = Ctx(0)
+    g = Grid(ctx, np.eye(3) * 0.2 * n, (n, n, n))
+    f = Fmt(g, terms=_lib.TERM_HS)
+    dens = torch.full((n, n, n), 0.05, dtype=torch.float64, device="cuda")
+    out = torch.empty((5, n, n, n), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+
+    def run():
+        _lib.check(L.deft_fmt_weighted(f.h, dens.data_ptr(), 1, out.data_ptr()))
+
+    try:
+        own = _times(L, g, run)
+        for what, slot, widths in (("z_c2r", 4, (5, 9, 13, 16)), ("x_conv_fwd", 2, (8, 12, 16))):
+            for w in widths:
+                tiles = np.zeros(6, dtype=np.intc)
+                tiles[slot] = w
+                _lib.check(L.deft_grid_set_tiles(g.h, 0, tiles.ctypes.data, None))
+                t = _times(L, g, run)[what]
+                print(f"{n}^3 {what}: built-in {own[what]:.1f} us, {w} wide {t:.1f}")
+                assert own[what] <= 1.15 * t, (what, w)
+    finally:
+        f.close()
+        g.close()
+        ctx.close()
