@@ -7,6 +7,11 @@ one parameter at a time, the tile width that minimises the time of the
 kernels that parameter shapes, and after that the radix order of each axis.
 Choices change results only by rounding.
 
+Axes whose transforms run in register kernels of a fixed shape (most common
+lengths along x and y, see deft_grid_set_tiles) read neither their tile widths
+nor their radix order: they are found by the evaluation's bits not changing with
+the order, left out of the search, and 0 (the built-in rule) in the entry.
+
 Results are cached in a JSON file keyed by GPU name, grid shape and
 precision; ``load`` registers a file's entries for the current GPU with
 ``deft_tuning_set``, so every grid created afterwards (including the grids
@@ -119,6 +124,28 @@ class _Bench:
         return self.L.deft_grid_set_tiles(self.grid, self.precision, t.ctypes.data,
                                           r.ctypes.data) == 0
 
+    def gradient(self):
+        E = ctypes.c_double()
+        check(self.L.deft_fmt_energy_grad(self.fmt, self.n.data_ptr(), 1, ctypes.addressof(E),
+                                          self.g.data_ptr(), None))
+        return self.g.clone()
+
+    def fixed(self, axis, n):
+        """Whether the axis's transforms (length n) ignore the radix order."""
+        tiles, radix = self.tiles()
+        same, tried = True, 0
+        own = self.gradient()
+        for o in radix_orders(n, 4):
+            cand = radix.copy()
+            cand[8 * axis:8 * axis + 8] = 0
+            cand[8 * axis:8 * axis + len(o)] = o
+            if np.array_equal(cand, radix) or not self.set(tiles, cand):
+                continue
+            tried += 1
+            same = same and bool((self.gradient() == own).all())
+        self.set(tiles, radix)
+        return same and tried > 0
+
     def measure(self, repeats):
         """Per-kernel milliseconds summed over `repeats` workloads."""
         L = self.L
@@ -170,8 +197,10 @@ def tune(shape, precision=_lib.PRECISION_MIXED, device=0, repeats=4, trials=2, l
             return best
 
         before = b.measure(repeats)
+        fixed = [b.fixed(a, shape[a]) for a in range(3)]
+        unread = {p for a in (0, 1) if fixed[a] for p in AXIS_PARAMS[a]}
         for pi, p in enumerate(PARAMS):
-            if p == "Bx":
+            if p == "Bx" or p in unread:
                 continue  # plain x FFTs only serve deft_grid_fft / ifft
             kern = KERNELS[p]
             best_v, best_c = int(tiles[pi]), cost(kern)
@@ -180,8 +209,8 @@ def tune(shape, precision=_lib.PRECISION_MIXED, device=0, repeats=4, trials=2, l
                     continue
                 cand = tiles.copy()
                 cand[pi] = v
-                if not b.set(cand, radix):
-                    continue
+                if not b.set(cand, radix) or b.tiles()[0][pi] != v:
+                    continue  # does not fit, or more than the grid has
                 c = cost(kern)
                 if c < best_c * 0.98:
                     best_v, best_c = v, c
@@ -191,6 +220,8 @@ def tune(shape, precision=_lib.PRECISION_MIXED, device=0, repeats=4, trials=2, l
                 log(f"{shape} prec {precision}: {p} = {best_v} ({best_c / repeats:.4f} ms)")
         N = shape
         for a in range(3):
+            if fixed[a]:
+                continue
             orders = radix_orders(N[a])
             if precision == _lib.PRECISION_MIXED and N[a] in (32, 64, 128, 256):
                 orders = [[16, N[a] // 16]] + orders  # register-resident transform
@@ -220,7 +251,7 @@ def tune(shape, precision=_lib.PRECISION_MIXED, device=0, repeats=4, trials=2, l
             # tiles chosen above need not give: try it jointly with a sweep
             # of that axis's tile widths.
             for a in range(3):
-                if N[a] not in (32, 64, 128, 256):
+                if fixed[a] or N[a] not in (32, 64, 128, 256):
                     continue
                 reg = [16, N[a] // 16]
                 cur = [int(v) for v in radix[8 * a:8 * a + 8] if v]
@@ -251,6 +282,12 @@ def tune(shape, precision=_lib.PRECISION_MIXED, device=0, repeats=4, trials=2, l
                             f"{[int(v) for v in tiles]}")
                 b.set(tiles, radix)
         after = b.measure(repeats)
+        tiles, radix = b.tiles()  # as they took effect
+        for p in unread:
+            tiles[PARAMS.index(p)] = 0
+        for a in range(3):
+            if fixed[a]:
+                radix[8 * a:8 * a + 8] = 0
         return {
             "N": list(shape), "precision": int(precision),
             "tiles": [int(v) for v in tiles], "radix": [int(v) for v in radix],

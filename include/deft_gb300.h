@@ -199,7 +199,13 @@ int deft_grid_profile_entry(deft_grid *grid, int i, const char **name, long long
  * adjoint convolution x tile, z-line pairs per r2c/c2r/gradient tile and per
  * phi/Hessian tile; 0 keeps the built-in rule.  radix[24] (may be NULL) =
  * three 8-entry radix orders for the x, y, z axes, each ending at its first 0
- * (all 0 = built-in).  Results change only by rounding. */
+ * (all 0 = built-in).  Results change only by rounding.
+ * Some transforms along x and y run in register kernels of a fixed shape, which
+ * do not read By, Bxf, Bxc or the axis's radix order (they are still taken and
+ * reported): the mixed form's of length 32, 36, 40, 48, 50, 60, 64, 72, 80, 96,
+ * 100, 120, 128, 144, 160, 192 and 256, and the FP64 form's of length 32, 64, 128
+ * and 256 on grids with enough lines to fill the GPU.  With DEFT_PENCIL=0 in the
+ * environment at grid creation every axis reads them. */
 int deft_grid_set_tiles(deft_grid *grid, int precision, const int tiles[6], const int radix[24]);
 /* The effective choice (built-in values filled in). */
 int deft_grid_get_tiles(deft_grid *grid, int precision, int tiles[6], int radix[24]);
