@@ -5,7 +5,8 @@ table's interval edges, next to 1 and at the limits of their ranges.
 Tolerances.  log_tab adds k ln 2, ln c and log1p r, each rounded to 2^-54 of
 itself, and the sum may be half the size of its terms: 4 x 2^-53.  The
 reciprocal's and square root's last step leaves its own rounding and that of
-its correction: 2^-52.  df_rcp is double-float: 2^-45."""
+its correction: 2^-52.  df_log1m is double-float, some ten operations of 2^-47:
+2^-45."""
 import ctypes
 import os
 import subprocess
@@ -117,6 +118,18 @@ def test_reciprocal_and_root(run):
     assert np.array_equal(run(1, s), [np.inf, -np.inf, 0, -0.0, np.nan], equal_nan=True)
     assert np.array_equal(run(2, np.array([0.0, np.inf, -1.0, np.nan])), [0, np.inf, np.nan, np.nan],
                           equal_nan=True)
+
+
+def test_log1m(run):
+    rng = np.random.default_rng(2)
+    tiny = np.concatenate([s * 2.0 ** -rng.uniform(1, 60, 20000) for s in (-1, 1)])
+    e = np.concatenate([tiny, 1 - _positive(-19, 19), rng.uniform(-0.5, 0.5, 20000)])
+    e = run(4, e)  # double-floats
+    e = e[(1 - e > 2.0 ** -19) & (e != 0)]
+    err = _worst(run(3, e), np.log1p(-e.astype(np.longdouble)))
+    print(f"df_log1m: {err * 2 ** 46:.2f} x 2^-46")
+    assert err <= 2.0 ** -45
+    assert run(3, np.zeros(1))[0] == 0
 
 
 def test_conversions(run):
