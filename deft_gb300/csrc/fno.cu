@@ -1842,7 +1842,7 @@ int deft_fno_create(int device, int N, int channels, int modes, int layers, unsi
   dev(&f->mask, sizeof(float) * f->NR);
   dev(&f->target, sizeof(float) * f->NR);
   dev(&f->wt, sizeof(float) * f->NR);
-  dev(&f->A, sizeof(float2) * C * N * N * f->Kz);
+  if (!f->slab) dev(&f->A, sizeof(float2) * C * N * N * f->Kz);  // between the z and y axes
   dev(&f->B, sizeof(float2) * C * N * f->Ky * f->Kz);
   dev(&f->S, sizeof(float2) * C * f->K);
   dev(&f->S2, sizeof(float2) * C * f->K);
