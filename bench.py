@@ -662,8 +662,8 @@ def run_ours(args, rank, world):
         "roofline": roofline(prof_w1, N, True, peak, peak_kind,
                              vec_bytes=4 if f32_vectors(N, PC == _lib.PC_NONE) else 8),
         "roofline_fp64": dict(roofline(prof_64, N, False, peak, peak_kind),
-                              note="FP64 form: bound by the FP64 pipe (measured 1.0 TFLOP/s "
-                                   "FMA on this GB300), not by HBM"),
+                              note="FP64 form: bound by FP32 issue slots (double-float "
+                                   "arithmetic), not by HBM"),
         "kernels": kernel_table(prof_w1),
         "kernels_fp64": kernel_table(prof_64),
     }

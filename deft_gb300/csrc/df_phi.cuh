@@ -12,8 +12,9 @@
 // points, so that the convolution that follows averages it out; constants
 // that are not exact are three words long (tfl), since their rounding would
 // not be white.  Gradient error against 64-bit arithmetic (relative 2-norm,
-// rms of ten inputs), FP64 Phi / this one: White Bear 64^3 1.56e-14 /
-// 1.32e-14, 77^3 1.94e-14 / 1.77e-14, mark II 128^3 2.93e-14 / 1.84e-14.
+// rms of 40 inputs), with Phi in FP64 and the transforms of that time / now: White
+// Bear 77^3 fcc 2.06e-14 / 1.63e-14, 128^3 2.42e-14 / 2.24e-14, mark II 128^3
+// 2.46e-14 / 1.75e-14.
 //
 // Points the double-float range or the small-density branch of the terms does
 // not cover (1 - n3 outside (2^-20, 2^20), very large weighted densities, a

@@ -2267,11 +2267,12 @@ __global__ void k_precond_dots(const double *__restrict__ n, const double *__res
 }
 
 // FP32-vector forms for the mixed form's FP32 stage: z = g n / (kT dV) on
-// the active points (mask != 0, n > 0) with (z.g, z.h) summed in FP64;
+// the active points (mask != 0, n > 0) with (z.g, z.h);
 // d = alpha g + beta d; y += alpha x; conversions.  Four elements per
 // thread and step (16-byte accesses; the vectors are 256-byte aligned),
-// a scalar tail when the length is not a multiple of 4; per-thread sums in
-// FP32, FP64 across threads and blocks.
+// a scalar tail when the length is not a multiple of 4; sums in FP32 per
+// thread, double-float across a block's threads (block_sum.cuh), FP64 across
+// blocks.
 #define DEFT_V4_LOOP(n)                                                              \
   const int n4_ = (n) >> 2;                                                           \
   const int tid_ = blockIdx.x * blockDim.x + threadIdx.x, nth_ = gridDim.x * blockDim.x; \
@@ -2396,7 +2397,7 @@ __global__ void k_to_f32_scaled(const double *__restrict__ a, double s, float *_
   DEFT_V4_TAIL(n) b[i] = (float)(s * a[i]);
 }
 // The Newton step's linear CG on FP32 vectors: z = M^-1 r with r.z, and
-// the fused update of k_newton_update (per-thread FP32 sums, FP64 across
+// the fused update of k_newton_update (per-thread FP32 sums, double-float and FP64 across
 // threads and blocks in a fixed order).
 __global__ void k_diag_precond_dot32(const float *__restrict__ n, const float *__restrict__ r,
                                      const float *__restrict__ mask, float inv_c,
@@ -2761,11 +2762,11 @@ void finish_tiles(Tiles &t, const Geom &g, size_t cs) {
 // 12 + sum over the passes of rounds x radix (a round: 256 threads, a butterfly
 // each), a launch's as that times ceil(L / R) + L / 10, with L blocks an SM of
 // which R = 3 are resident (registers) or fewer (shared memory).  Measured
-// against the widest tiles of the budget: Phi 128^3 6 pairs 59 us against 66
-// with 9, 96^3 6 pairs 32.7 against 34.8 with 9, 64^3 5 pairs 14.3 against 20.4
-// with 13, 48^3 4 pairs 12.2 against 16.6 with 15; adjoint convolution 96^3 6
-// columns 27.2 against 33.1 with 9, 80^3 8 columns 16.4 against 18.4 with 11,
-// 48^3 4 columns 12.3 against 16.4 with 16.
+// against wider tiles: Phi 128^3 6 pairs 59 us against 66 with 9, 96^3 6 pairs 32.7
+// against 34.8 with 9, 64^3 5 pairs 14.3 against 20.4 with 13, 48^3 4 pairs 12.2
+// against 16.6 with 15; adjoint convolution (lengths without two-pass kernels)
+// 56^3 6 columns 12.3 against 18.0 with 16, 77^3 7 columns 16.3 against 22.5 with
+// 15, 112^3 7 columns 33.6 against 52.7 with 10.
 int five_field_tile(const FftPlan &p, int n, int count, size_t budget, int sms) {
   int best = 1;
   double best_cost = 0;

@@ -31,7 +31,7 @@ struct GridSpec {
 };
 
 enum Precision {
-  kPrecisionFP64 = 0,   // everything FP64
+  kPrecisionFP64 = 0,   // FP64 vectors and sums; transforms, weights and phi in double-float
   kPrecisionMixed = 1,  // FFTs, weights and phi in FP32; reductions FP64
 };
 

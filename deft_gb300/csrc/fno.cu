@@ -325,7 +325,9 @@ size_t slab_inv_smem(int N, int m, int KB) {
   return sizeof(float2) *
          ((size_t)N * KB + (size_t)KB * N + 2 * (size_t)(m + 1) * KB + (size_t)(N / 2 + 1) * (m + 1));
 }
-// Two slab blocks per SM (up to N = 148).
+// Two analysis blocks per SM: up to N = 160 with 4 modes, 152 with 8, 144 with 12,
+// 136 with 16.  The layer kernel needs more (synth_smem): with 16 channels one
+// block fits an SM with 16 modes, and with 12 up to N = 40.
 bool slab_ok(int N, int m) { return slab_fwd_smem(N, m, (m + 3) / 4 * 4) <= 110 * 1024; }
 
 // 16-byte asynchronous copies to shared memory.
@@ -1602,8 +1604,9 @@ void launch_layer_synth(deft_fno *f, int l) {
   f->launches++;
   if (f->slab) {
     const size_t sm = synth_smem<C>(N, f->m, f->Kz);
-    // blocks per x: the fewest rounds of two blocks per SM, a round costing
-    // its passes and about two more for the block's tables
+    // blocks per x: the fewest rounds of two blocks per SM (also assumed where
+    // only one fits), a round costing its passes and about two more for the
+    // block's tables
     const int most = (N + lpb - 1) / lpb;
     int share = 1, best = 0;
     for (int k = 1; k <= most && k <= 16; k++) {
