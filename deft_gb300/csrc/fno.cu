@@ -131,20 +131,20 @@ __global__ void __launch_bounds__(128) k_dft_z_fwd(const float *__restrict__ in,
 // in registers and walks lines of the block's tile, so each 16-byte read of
 // two of a line's coefficients (a broadcast) feeds 16 multiply-adds and the
 // result leaves as one 16-byte store.  The table's strided reads are paid
-// once per tile, so a tile is kZiLines lines where that still leaves every SM
-// two blocks, a quarter of them below.  91 us at
-// 96^3 with 16 channels and 12 modes when a thread held two z (8-byte reads,
-// 4 multiply-adds each), 73 us with four z and 64 lines, 44 us with 256.
+// once per tile of kZiLines lines (grids without slab kernels have two such
+// tiles an SM or more).  91 us at 96^3 with 16 channels and 12 modes when a thread
+// held two z (8-byte reads, 4 multiply-adds each), 73 us with four z and 64
+// lines, 44 us with 256.
 constexpr int kZiLines = 256;
 
 template <int KB>
 __global__ void __launch_bounds__(128) k_dft_z_inv(const float2 *__restrict__ in,
                                                    float *__restrict__ out,
                                                    const float2 *__restrict__ G, int L, int N,
-                                                   int Kz, int accumulate, int lines) {
+                                                   int Kz, int accumulate) {
   __shared__ __align__(16) float2 cs[kZiLines * KB];  // rows of KB, zero beyond Kz
-  const int l0 = blockIdx.x * lines;
-  const int nl = L - l0 < lines ? L - l0 : lines;
+  const int l0 = blockIdx.x * kZiLines;
+  const int nl = L - l0 < kZiLines ? L - l0 : kZiLines;
   for (int i = threadIdx.x; i < nl * KB; i += blockDim.x) {
     const int ll = i / KB, k = i - ll * KB;
     cs[i] = k < Kz ? in[(size_t)(l0 + ll) * Kz + k] : make_float2(0.f, 0.f);
@@ -1492,13 +1492,12 @@ void launch_z_fwd(deft_fno *f, const float *in, float2 *out, const float2 *E) {
 }
 void launch_z_inv(deft_fno *f, const float2 *in, float *out, const float2 *G, int acc) {
   const int L = f->C * f->N * f->N;
-  const int lines = L >= 2 * 152 * kZiLines ? kZiLines : kZiLines / 4;
-  const dim3 grid((L + lines - 1) / lines);
+  const dim3 grid((L + kZiLines - 1) / kZiLines);
   switch (kz_block(f->Kz)) {
-    case 4: k_dft_z_inv<4><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc, lines); break;
-    case 8: k_dft_z_inv<8><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc, lines); break;
-    case 12: k_dft_z_inv<12><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc, lines); break;
-    default: k_dft_z_inv<16><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc, lines); break;
+    case 4: k_dft_z_inv<4><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc); break;
+    case 8: k_dft_z_inv<8><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc); break;
+    case 12: k_dft_z_inv<12><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc); break;
+    default: k_dft_z_inv<16><<<grid, 128, 0, f->stream>>>(in, out, G, L, f->N, f->Kz, acc); break;
   }
 }
 void launch_axis(deft_fno *f, const float2 *in, float2 *out, const float2 *E, int outer, int Nin,
