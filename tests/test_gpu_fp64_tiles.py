@@ -3,7 +3,9 @@ are chosen for FP64 arithmetic: at these sizes neither the five-field z transfor
 nor the x convolution is beaten by another tile width.
 
 Times by events, the least of five batches; 15 % allowed for their noise (a
-launch of these takes 10 to 60 us and repeats to 2 or 3 %)."""
+launch of these takes 10 to 60 us and repeats to 2 or 3 %).  A comparison that
+fails is made again, both sides anew, at most twice: another program's work on
+the host must not decide it."""
 import ctypes
 
 import numpy as np
@@ -46,15 +48,23 @@ def test_widths(n):
     def run():
         _lib.check(L.deft_fmt_weighted(f.h, dens.data_ptr(), 1, out.data_ptr()))
 
+    def times(slot=None, width=0):
+        tiles = np.zeros(6, dtype=np.intc)
+        if slot is not None:
+            tiles[slot] = width
+        _lib.check(L.deft_grid_set_tiles(g.h, 0, tiles.ctypes.data, None))
+        return _times(L, g, run)
+
     try:
-        own = _times(L, g, run)
+        own = times()
         for what, slot, widths in (("z_c2r", 4, (5, 9, 13, 16)), ("x_conv_fwd", 2, (8, 12, 16))):
             for w in widths:
-                tiles = np.zeros(6, dtype=np.intc)
-                tiles[slot] = w
-                _lib.check(L.deft_grid_set_tiles(g.h, 0, tiles.ctypes.data, None))
-                t = _times(L, g, run)[what]
-                print(f"{n}^3 {what}: built-in {own[what]:.1f} us, {w} wide {t:.1f}")
+                for again in (True, True, False):
+                    t = times(slot, w)[what]
+                    print(f"{n}^3 {what}: built-in {own[what]:.1f} us, {w} wide {t:.1f}")
+                    if own[what] <= 1.15 * t or not again:
+                        break
+                    own = times()
                 assert own[what] <= 1.15 * t, (what, w)
     finally:
         f.close()

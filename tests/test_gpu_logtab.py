@@ -101,7 +101,8 @@ def test_log(run):
           f"{_worst(run(0, near), np.log(near.astype(np.longdouble))) * 2 ** 53:.2f}")
     assert err <= 4 * 2.0 ** -53
     s = np.array([0.0, -0.0, np.inf, np.nan, -1.0, -np.inf, 5e-324, 2.0 ** -1030, 1.0])
-    got, want = run(0, s), np.log(np.abs(s))
+    with np.errstate(divide="ignore"):
+        got, want = run(0, s), np.log(np.abs(s))
     assert np.isneginf(got[0]) and np.isneginf(got[1]) and np.isposinf(got[2])
     assert np.all(np.isnan(got[3:6])) and got[8] == 0
     assert np.all(np.abs(got[6:8] / want[6:8] - 1) <= 4 * 2.0 ** -53)
