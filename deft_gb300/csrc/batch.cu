@@ -10,7 +10,8 @@
 // comes from a pool of its own (dev_mem.h), and the largest problems are started
 // first.  12 solves of 32^3 to 96^3 on 8 workers: 64 ms with cudaMalloc and
 // cudaFree in order of the list (49 when nothing was freed), 43 like this; on one
-// worker 82 and 73.
+// worker 82 and 73.  Problems that do not fit beside the others run one by one at
+// the end.
 #include "../../include/deft_gb300.h"
 #include "dev_mem.h"
 
@@ -18,6 +19,7 @@
 #include <atomic>
 #include <climits>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <numeric>
 #include <string>
@@ -127,34 +129,54 @@ extern "C" int deft_batch_solve(int device, int count, const deft_batch_problem 
   // context on another
   std::once_flag pool_made;
   cudaMemPool_t pool = nullptr;
+  // problems that did not fit beside the others: largest first puts the large
+  // ones side by side, whatever their places in the list
+  std::mutex left_mu;
+  std::vector<int> left;
+  // One worker over the problems next_problem() gives, until it gives -1.
+  auto work = [&](const std::function<int()> &next_problem, bool alone) {
+    struct PoolScope {  // outlives w: its clean-up frees to the pool
+      ~PoolScope() { deft::thread_pool = {}; }
+    } scope;
+    Worker w;
+    if (deft_ctx_create(device, &w.ctx) != DEFT_OK) {
+      failed(-1, DEFT_ERR_CUDA, deft_last_error());
+      return;
+    }
+    std::call_once(pool_made, [&]() { pool = deft::make_call_pool(device); });
+    deft::thread_pool = {pool, static_cast<cudaStream_t>(deft_ctx_stream(w.ctx))};
+    for (int i = next_problem(); i >= 0; i = next_problem()) {
+      deft_cg_status &st = status_out[i];
+      memset(&st, 0, sizeof(st));
+      deft::thread_out_of_memory = false;
+      const int s = solve_one(w, probs[i], bp->cg, &st);
+      st.status = s;
+      // what it freed is there for the other workers from here on
+      cudaStreamSynchronize(deft::thread_pool.stream);
+      if (s && deft::thread_out_of_memory && !alone) {
+        std::lock_guard<std::mutex> lock(left_mu);
+        left.push_back(i);
+      } else if (s) {
+        failed(i, s, "problem " + std::to_string(i) + ": " + deft_last_error());
+      }
+    }
+  };
   std::vector<std::thread> threads;
-  for (int t = 0; t < workers; t++) {
+  for (int t = 0; t < workers; t++)
     threads.emplace_back([&]() {
-      struct PoolScope {  // outlives w: its clean-up frees to the pool
-        ~PoolScope() { deft::thread_pool = {}; }
-      } scope;
-      Worker w;
-      if (deft_ctx_create(device, &w.ctx) != DEFT_OK) {
-        failed(-1, DEFT_ERR_CUDA, deft_last_error());
-        return;
-      }
-      std::call_once(pool_made, [&]() { pool = deft::make_call_pool(device); });
-      deft::thread_pool = {pool, static_cast<cudaStream_t>(deft_ctx_stream(w.ctx))};
-      for (;;) {
+      work([&]() {
         const int k = next.fetch_add(1);
-        if (k >= count) break;
-        const int i = order[k];
-        deft_cg_status &st = status_out[i];
-        memset(&st, 0, sizeof(st));
-        const int s = solve_one(w, probs[i], bp->cg, &st);
-        st.status = s;
-        // what it freed is there for the other workers from here on
-        cudaStreamSynchronize(deft::thread_pool.stream);
-        if (s) failed(i, s, "problem " + std::to_string(i) + ": " + deft_last_error());
-      }
+        return k < count ? order[k] : -1;
+      }, false);
     });
-  }
   for (auto &th : threads) th.join();
+  // one after another, with the memory to themselves
+  std::sort(left.begin(), left.end());
+  for (int i : left)
+    std::thread([&]() {
+      bool given = false;
+      work([&]() { return given ? -1 : (given = true, i); }, true);
+    }).join();
   deft::end_call_pool(pool);
   if (first_error != DEFT_OK) deft::set_last_error_message(first_msg);
   return first_error;

@@ -30,6 +30,8 @@ struct ThreadPool {
 // The calling thread's; memory is freed by the thread that allocated it, before
 // that thread's pool is taken away.
 inline thread_local ThreadPool thread_pool;
+// Set when an allocation of the calling thread did not fit.
+inline thread_local bool thread_out_of_memory = false;
 
 // The pools of the calls that are running.
 struct CallPools {
@@ -58,6 +60,7 @@ inline cudaError_t dev_malloc(void **p, size_t n) {
     cudaGetLastError();
     if (t.pool) cudaStreamSynchronize(t.stream);
     if (call_pools().trim()) e = get();
+    if (e == cudaErrorMemoryAllocation) thread_out_of_memory = true;
   }
   if (e != cudaSuccess || !t.pool || n == 0) return e;
   if ((e = cudaStreamSynchronize(t.stream)) != cudaSuccess) {

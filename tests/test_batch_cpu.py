@@ -177,6 +177,19 @@ static int memory(const char *who) {
   next.R = 2;  // its functional is made once `wait` is being solved
   done = waiting = false;
   int other = -1;
+  if (w == "together") {
+    // two problems of 60 bytes that the list keeps apart
+    next.N[0] = next.N[1] = next.N[2] = 16;
+    big.R = 1;
+    WANT(batch({big, problem(8, 0, 0), next}, 2, st) == DEFT_OK);
+    WANT(st[0].status == 0 && st[1].status == 0 && st[2].status == 0 && used == 0);
+    // one that does not fit alone fails, and the others do not
+    waiting = done = true;
+    WANT(batch({problem(8, 0, 0), problem(16, 0, 160), problem(12, 0, 60)}, 2, st) == DEFT_ERR_NOMEM);
+    WANT(!strcmp(deft_last_error(), "problem 1: memory"));
+    WANT(st[0].status == 0 && st[1].status == DEFT_ERR_NOMEM && st[2].status == 0);
+    return 0;
+  }
   if (w == "worker") {
     WANT(batch({big, wait, next}, 2, st) == DEFT_OK);
     return 0;
@@ -240,7 +253,7 @@ def program(tmp_path_factory):
     return str(d / "main")
 
 
-@pytest.mark.parametrize("scenario", ["errors", "caller_device", "memory_worker", "memory_call",
+@pytest.mark.parametrize("scenario", ["errors", "caller_device", "memory_together", "memory_worker", "memory_call",
                                       "memory_alone", "failed_wait"])
 def test_batch_host(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=60)
